@@ -15,9 +15,12 @@
 // This is valid when a group has finished -- and the next lane has consumed
 // its last row -- before the lane's next group starts.  With the band
 // |i(m-1) - j(n-1)| <= W (W = w (min(n,m)-1)) that holds whenever
-// 2W < 31 R (n + m - 2); for a full row (no band) when m <= 31 R + 1; for
-// an LCSS window |i - j| <= delta when delta <= 31 R (32 W lanes: 32 W - 1
-// in place of 31).  Pairs that fail the condition are listed for the next
+// 2W < 31 R (n + m - 2); for a full row (no band) when m <= 31 R + 1 (at
+// R = 1, m <= 31, and not for LCSS: the next lane's first diagonal is the
+// value this lane held one step before its new group starts, which must lie
+// past its old row's end, where LCSS keeps the row's last value -- with more
+// rows that step is inside the new group); for an LCSS window |i - j| <= delta when delta <= 31 R (32 W lanes: 32 W - 1 in
+// place of 31).  Pairs that fail the condition are listed for the next
 // pass, the last one for the round-striped kernel (dp_kernels.cu).
 //
 // A lane's band columns come from integer ramps stepped by additions; its
@@ -55,7 +58,7 @@ constexpr int kNone = 1 << 30;
 __host__ __device__ bool diag_ok(bool lcss, int n, int m, int wd, int R, int lanes) {
   if (n < 2 || m < 2) return false;
   const long long span = (long long)(lanes - 1) * R;  // rows between a lane's groups, less one group
-  if (wd < 0) return m <= span + 1;
+  if (wd < 0) return R > 1 ? m <= span + 1 : !lcss && m <= span;
   if (lcss) return wd <= span;
   const long long W = (long long)wd * ((n < m ? n : m) - 1);
   return 2 * W < span * (n + m - 2);
@@ -488,7 +491,7 @@ int launch_chain(tsim_ctx* ctx, int R0, int warps, const DpArgs& a, int max_m, i
     const long long span = (long long)(lanes - 1) * R;
     const bool lcss = std::is_same<P, PolLcss>::value;
     const int wd = lcss ? a.delta : band_w(a.max_n, max_m, a.band_pct);
-    if (wd < 0) return max_m <= span + 1;
+    if (wd < 0) return R > 1 ? max_m <= span + 1 : !lcss && max_m <= span;
     return wd < span;
   };
   std::vector<int> rs;
@@ -522,7 +525,7 @@ int launch_chain_cta(tsim_ctx* ctx, int R0, const DpArgs& a, int max_m, int* spi
   std::vector<int> rs;
   for (int R = std::max(1, std::min(R0, 8)); R <= 8; R *= 2) {
     rs.push_back(R);
-    if (a.max_n > 0 && max_m <= (kCtaWarps * 32 - 1) * R + 1) break;  // full rows: all fit
+    if (a.max_n > 0 && max_m <= (kCtaWarps * 32 - 1) * R + (R > 1 ? 1 : 0)) break;  // all fit
   }
   const int np = (int)rs.size();
   DpArgs in = a;

@@ -95,3 +95,35 @@ def test_dp_pairs_all_kernels(tsim, cuda_ctx, oracle, measure, kw, lo, hi):
     for kernel in (5, 6):
         assert np.array_equal(fp32[2].view(np.uint32), fp32[kernel].view(np.uint32)), \
             (measure, kernel)
+
+
+@pytest.mark.parametrize("m,kernel", [(31, 2), (32, 2), (33, 2), (63, 4), (64, 4), (65, 4),
+                                      (255, 3), (256, 3), (257, 3)])
+@pytest.mark.parametrize("measure", ["dtw", "frechet", "lcss"])
+def test_dp_full_rows_as_wide_as_the_lanes(tsim, cuda_ctx, oracle, measure, m, kernel):
+    """Full rows of as many columns as a warp, two warps or a CTA has lanes
+    (one row per lane), queries of several rounds of lanes: a group's first
+    diagonal is outside the matrix, not the end of the row above it."""
+    import torch
+    from cudaruntime1_gb300 import api
+    cp, co = G.random_walks(40, m, 900 + m, start_range=2.0)
+    qp, qo = G.random_walks(4, [m + 2, 2 * m + 5, 3 * m, 4 * m + 1], 901 + m, start_range=2.0)
+    pairs = np.stack(np.meshgrid(np.arange(4), np.arange(40), indexing="ij"), -1).reshape(-1, 2)
+    kw, okw = (dict(epsilon=2.0), dict(eps=2.0)) if measure == "lcss" else ({}, {})
+    want = np.array([oracle.pair(measure, qp[qo[a]:qo[a + 1]], cp[co[b]:co[b + 1]], **okw)
+                     for a, b in pairs])
+    want = want ** 2 if measure == "frechet" else want
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+           (qp, np.asarray(qo), cp, np.asarray(co), pairs.astype(np.int32))]
+    for precision in (0,) if measure == "lcss" else (0, 1):
+        out = torch.full((len(pairs),), float("nan"), device="cuda",
+                         dtype=(torch.float32, torch.float64)[precision])
+        api.dp_pairs(cuda_ctx, measure, precision, kernel, dev[0].data_ptr(), dev[1].data_ptr(),
+                     4 * m + 1, dev[2].data_ptr(), dev[3].data_ptr(), m, dev[4].data_ptr(),
+                     len(pairs), out.data_ptr(), out.data_ptr(), **kw)
+        torch.cuda.synchronize()
+        got = out.cpu().numpy().astype(np.float64)
+        # FP32: 4 roundings a cost and one per cell of a path of at most 5 m cells
+        lim = 0.0 if measure == "lcss" else ((5 * m + 8) * 2.0 ** -24 * 1.01 if precision == 0
+                                             else 4.5 * 2.0 ** -24)
+        assert np.all(np.abs(got - want) <= lim * want), (precision, np.abs(got - want).max())
