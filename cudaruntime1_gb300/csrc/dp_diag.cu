@@ -518,41 +518,11 @@ int launch_chain(tsim_ctx* ctx, int R0, int warps, const DpArgs& a, int max_m, i
   return TSIM_OK;
 }
 
-// the chain of launch_chain for a CTA per pair only (R = R0 .. 8)
-template <class P>
-int launch_chain_cta(tsim_ctx* ctx, int R0, const DpArgs& a, int max_m, int* spill, int* nspill,
-                     int* tmp, int* ntmp) {
-  std::vector<int> rs;
-  for (int R = std::max(1, std::min(R0, 8)); R <= 8; R *= 2) {
-    rs.push_back(R);
-    if (a.max_n > 0 && max_m <= (kCtaWarps * 32 - 1) * R + (R > 1 ? 1 : 0)) break;  // all fit
-  }
-  const int np = (int)rs.size();
-  DpArgs in = a;
-  for (int p = 0; p < np; ++p) {
-    const bool to_spill = ((np - 1 - p) & 1) == 0;
-    int* out = to_spill ? spill : tmp;
-    int* nout = to_spill ? nspill : ntmp;
-    TSIM_CUDA(cudaMemsetAsync(nout, 0, 2 * sizeof(int), ctx->stream));  // spills, work counter
-    TSIM_TRY((launch_diag_r<P, kCtaWarps>(ctx, rs[p], in, max_m, out, nout)));
-    in.order = out;
-    in.npairs_dev = nout;
-  }
-  return TSIM_OK;
-}
-
 }  // namespace
 
 int launch_dp_diag(tsim_ctx* ctx, int kind, int R, const DpArgs& a, int max_m, int* spill,
                    int* nspill, int* tmp, int* ntmp, int warps, int rmax) {
   const int W = warps > 2 ? kCtaWarps : warps;
-  if (kind == DP_FRECHET_WIN) {
-    // the exact FP64 Frechet re-score: few, possibly long full-row pairs
-    // (latency), on a CTA per pair only
-    if (W != kCtaWarps)
-      return fail(TSIM_ERR_UNSUPPORTED, "the exact Frechet re-score runs on a CTA per pair");
-    return launch_chain_cta<PolFrechetWin>(ctx, R, a, max_m, spill, nspill, tmp, ntmp);
-  }
   switch (kind) {
     case DP_DTW_SQ: return launch_chain<PolDtwSq>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
     case DP_DTW_EU: return launch_chain<PolDtwEu>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);

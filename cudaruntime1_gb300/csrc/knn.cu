@@ -1707,8 +1707,9 @@ __global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_res
   }
 }
 
-// DP of a pair list: the anti-diagonal kernel for the pairs it can take,
-// the round-striped kernel (G lanes x R rows) for the rest
+// DP of a pair list: the strip kernel for full rows, the anti-diagonal
+// kernels for the banded pairs they can take, the round-striped kernel (G
+// lanes x R rows) for the rest
 // latency: a round of few pairs (seeds, round 1, re-score), whose launch
 // lasts as long as its longest pair.  A step of a warp per pair costs R rows
 // of instructions on one warp; two warps or a CTA of 8 per pair spread the
@@ -1720,6 +1721,19 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
   const bool diag_kind = kind == DP_DTW_SQ || kind == DP_DTW_EU || kind == DP_LCSS ||
                          kind == DP_FRECHET_SQ || kind == DP_DTW_SQC || kind == DP_DTW_EUC ||
                          kind == DP_FRECHET_SQC;
+  if (d.band_pct < 0 && a.wave && strip_kind(kind)) {
+    // full rows: strips of rows, in the latency rounds too (tsim_dp_pairs,
+    // before and after): 8,192 DTW pairs of 128 x 128 points 297 -> 57 us;
+    // 5,120 Frechet pairs of up to 256 x 1,024 points 1,438 us on a CTA of
+    // row groups and 2,317 on a warp (eight passes, R = 1 .. 8) -> 208 us;
+    // the same compensated 4,406 -> 1,004 us
+    TSIM_TRY(launch_dp_strip(ctx, kind, d, d.max_n > 0 ? d.max_n : a.max_qlen, a.max_clen, a.waves,
+                             a.nwaves));
+    DpArgs rest = d;  // pairs with both sides too long to stage
+    rest.order = a.waves;
+    rest.npairs_dev = a.nwaves;
+    return launch_dp(ctx, kind, G, R, rest, a.max_clen);
+  }
   if (!latency && a.lane_gate > 0 && lane_kind(kind)) {
     // many pairs: a lane per pair, with a latency of one pair's cells but a
     // few instructions per cell; the kernel itself passes a round of fewer
@@ -1843,12 +1857,8 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
     r.pairs = a.r64pairs;
     r.out64 = a.r64;
     if (MEAS == M_FRECHET) {  // exact FP64 values from the FP32 ones: no FP64 DP
-      // a CTA of 8 warps per pair, each pair at the fewest rows per lane its
-      // length admits (the pairs are few and up to full rows of 2,041
-      // points: latency); longer ones on the striped kernel
       r.aux = a.rdc;
-      TSIM_TRY(launch_dp_diag(ctx, DP_FRECHET_WIN, 1, r, a.max_clen, a.spill, a.nspill, a.spill2,
-                              a.nspill2, 8));
+      TSIM_TRY(launch_dp_strip(ctx, DP_FRECHET_WIN, r, a.max_qlen, a.max_clen, a.spill, a.nspill));
       DpArgs sp = r;
       sp.order = a.spill;
       sp.npairs_dev = a.nspill;
@@ -2716,7 +2726,7 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
   int G, R;
   dp_shape(kind, max_qlen, max_clen, wd, G, R);
   const bool diag_kind = precision < 2;
-  if (kernel == 1 || (kernel == 0 && (!diag_kind || Rd == 0)) || !diag_kind)
+  if (kernel == 1 || !diag_kind)
     return launch_dp(ctx, kind, G, R, d, max_clen);
   if (Rd == 0) Rd = 16;  // none fits the longest pair: the widest takes the rest
   const int lanes = kernel == 3 ? 256 : 64;  // a CTA of 8 warps, or 2 warps, per pair
@@ -2734,6 +2744,12 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
   int* nrest = arena_take<int>(ctx, 4);
   int* sorted = arena_take<int>(ctx, npairs);
   int* buckets = arena_take<int>(ctx, lane_sort_buckets());
+  if (kernel == 0 && d.band_pct < 0 && strip_kind(kind)) {  // full rows
+    TSIM_TRY(launch_dp_strip(ctx, kind, d, max_qlen, max_clen, spill, nspill));
+    d.order = spill;
+    d.npairs_dev = nspill;
+    return launch_dp(ctx, kind, G, R, d, max_clen);
+  }
   if (kernel == 6 && wave_kind(kind)) {  // band-relative first; wider pairs on the others
     TSIM_TRY(launch_dp_wave(ctx, kind, d, max_qlen, max_clen, npairs <= 4 * ctx->num_sms, rest, nrest));
     d.order = rest;

@@ -11,7 +11,8 @@
 //      memory, evaluates the bound of every candidate (summed in the same
 //      order as the reference CPU code, so values are bit-identical), and
 //      selects the K best by (bound, index) without materialising the matrix;
-//   2. the wavefront DP kernel (dp_kernels.cu) refines the num_t*K pairs;
+//   2. the strip DP kernel (dp_strip.cu; LCSS: dp_kernels.cu) refines the
+//      num_t*K pairs;
 //   3. ref_reduce_kernel keeps the best refined value per query.
 // Outputs equal the reference's CPU functions (dtw.cpp:14-113,
 // lcss.cpp:13-115, frechet.cpp:13-124) bit for bit.
@@ -196,9 +197,14 @@ int ref_batch_core(tsim_ctx* ctx, int measure, const float2* d_t1, const float2*
   a.band_pct = -1;
   a.delta = -1;
   a.eps = eps;
-  int G, R;
-  dp_shape(kind, n, m, -1, G, R);
-  TSIM_TRY(launch_dp(ctx, kind, G, R, a, m));
+  a.max_n = n;
+  if (strip_kind(kind) && std::min(n, m) <= strip_max_cols()) {
+    TSIM_TRY(launch_dp_strip(ctx, kind, a, n, m, nullptr, nullptr));
+  } else {
+    int G, R;
+    dp_shape(kind, n, m, -1, G, R);
+    TSIM_TRY(launch_dp(ctx, kind, G, R, a, m));
+  }
 
   const int tb = 128;
   if (measure == TSIM_LCSS)

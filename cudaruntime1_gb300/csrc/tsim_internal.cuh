@@ -348,6 +348,15 @@ int status_result(tsim_ctx* ctx, unsigned v);
 int set_wait_limit(long long attempts);
 int launch_dp_wave(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, bool latency,
                    int* spill, int* nspill);
+// Strip kernel (dp_strip.cu) for pairs without a band (strip_kind: DTW and
+// Frechet, FP32, compensated, the reference's arithmetic and the exact
+// Frechet re-score): a warp per pair, whose shorter side is at most
+// strip_max_cols() points (else, or past max_n x max_m, in spill[], count in
+// *nspill; both may be null when no pair can be longer).
+bool strip_kind(int kind);
+int strip_max_cols();
+int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
+                    int* nspill);
 // Lane-per-pair kernel (dp_lane.cu) for the FP32 DTW, Frechet and LCSS
 // kinds (lane_kind): a lane runs a whole pair in passes of 8 rows, the row
 // above a pass in a shared-memory ring of `ring` (64 or 128) values per lane

@@ -127,3 +127,64 @@ def test_dp_full_rows_as_wide_as_the_lanes(tsim, cuda_ctx, oracle, measure, m, k
         lim = 0.0 if measure == "lcss" else ((5 * m + 8) * 2.0 ** -24 * 1.01 if precision == 0
                                              else 4.5 * 2.0 ** -24)
         assert np.all(np.abs(got - want) <= lim * want), (precision, np.abs(got - want).max())
+
+
+# the edges of a lane's rows, of a half warp's, a warp's and several strips of
+# rows, and of the staged side; (320, 260): several strips either way round
+STRIP_SHAPES = [(1, 1), (1, 40), (33, 2), (31, 32), (64, 65), (127, 129), (128, 128), (16, 511),
+                (257, 255), (256, 300), (320, 260), (513, 40), (700, 600)]
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("measure,kw", [("dtw", dict(cost=0)), ("dtw", dict(cost=1)),
+                                        ("frechet", {})])
+def test_dp_full_rows_by_strips(tsim, cuda_ctx, measure, kw, many):
+    """Full rows, the kernel chosen by the library, against the round-striped
+    one: the same cells with the same operations, so the same bits; a few
+    pairs (a warp each) and more than eight per SM (two to a warp, where one
+    side is short)."""
+    import torch
+    from cudaruntime1_gb300 import api
+    for shape in STRIP_SHAPES:
+        nc = 1400 if many else 37
+        if many and max(shape) > 520:
+            continue
+        lens = np.full(nc, shape[1])
+        lens[::3] = np.maximum(1, shape[1] - np.arange(len(lens[::3])) % 7)  # ragged
+        qp, qo = G.random_walks(2, [shape[0], max(1, shape[0] - 1)], 77, start_range=10.0)
+        cp, co = G.random_walks(nc, lens, 78, start_range=10.0)
+        pairs = np.stack(np.meshgrid(np.arange(2), np.arange(nc), indexing="ij"), -1)
+        dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+               (qp, np.asarray(qo), cp, np.asarray(co), pairs.reshape(-1, 2).astype(np.int32))]
+        for precision in (0, 1):
+            out = []
+            for kernel in (1, 0):
+                o = torch.full((2 * nc,), float("nan"), device="cuda",
+                               dtype=(torch.float32, torch.float64)[precision])
+                api.dp_pairs(cuda_ctx, measure, precision, kernel, dev[0].data_ptr(),
+                             dev[1].data_ptr(), shape[0], dev[2].data_ptr(), dev[3].data_ptr(),
+                             shape[1], dev[4].data_ptr(), 2 * nc, o.data_ptr(), o.data_ptr(), **kw)
+                torch.cuda.synchronize()
+                out.append(o.cpu().numpy())
+            assert np.array_equal(out[0], out[1]), (shape, precision)
+
+
+def test_frechet_fp64_rescore_of_long_pairs(tsim, cuda_ctx, oracle):
+    """The exact FP64 re-score over one and several strips of rows: bit for
+    bit the oracle's values."""
+    lens = np.concatenate([np.arange(120, 140), np.arange(250, 262), [32, 500, 513]])
+    cp, co = G.random_walks(len(lens), lens, 5, start_range=10.0)
+    qp, qo = G.random_walks(4, [90, 128, 257, 520], 6, start_range=10.0)
+    db = tsim.Database(cuda_ctx, cp, co)
+    want_ids, want = oracle.knn("frechet", qp, qo, cp, co, 20)
+    import torch
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (qp, np.asarray(qo, np.int64))]
+    ids = torch.empty(4 * 20, dtype=torch.int32, device="cuda")
+    d, d64 = torch.empty(80, device="cuda"), torch.empty(80, dtype=torch.float64, device="cuda")
+    for flags in (tsim.api.FLAG_FP64_RESCORE, tsim.api.FLAG_FP64_RESCORE | tsim.api.FLAG_ALWAYS_PRUNE):
+        tsim.knn_device(cuda_ctx, db, dev[0].data_ptr(), dev[1].data_ptr(), 4, 520, ids.data_ptr(),
+                        d.data_ptr(), d64.data_ptr(), "frechet", 20, flags=flags)
+        cuda_ctx.synchronize()
+        assert np.array_equal(ids.cpu().numpy().reshape(4, 20), want_ids)
+        assert np.array_equal(d64.cpu().numpy().reshape(4, 20), want)
+    db.close()
