@@ -154,14 +154,15 @@ struct KArgs {
   int nseg;                 // segments of kSeg entries per query (two-level selection)
   unsigned long long* segkeys;  // [nq*nseg*64] best keys of every segment
   unsigned long long* kthkey;   // [nq] key of the k-th best refined pair
-  int* rraw;                    // [nq] pairs within the re-score bound (before the cap)
+  int* rraw;                    // [nq] pairs within the re-score bound (the first RC are kept)
   int RC;
   int2* rpairs;             // [nq*RC] re-score set
   double* rdc;              // [nq*RC] compensated FP32 (hi+lo) values
   int2* r64pairs;           // [nq*RC] members of ambiguous clusters (else y = -1)
   double* r64;              // [nq*RC] FP64 values of those
-  int* rcnt;                // [nq]
-  int* n64;                 // [1] pairs sent to FP64
+  int* rlist;               // the re-score sets' members, all queries' (entries of rpairs)
+  int* r64list;             // those sent to FP64 (entries of r64pairs)
+  int* n64;                 // [0] pairs sent to FP64, [1] members in rlist
   int force64;              // re-score every pair in FP64 (bit-identical distances)
   // outputs
   int* ids;
@@ -430,7 +431,6 @@ __device__ void seed_threshold(const KArgs& a, int q, int lane) {
     a.cnt0[q] = 0;
     a.cnt1[q] = 0;
     a.cnt2[q] = 0;
-    a.rcnt[q] = 0;
   }
 }
 
@@ -1518,11 +1518,18 @@ __global__ void __launch_bounds__(kSelThreads) final_select_kernel(KArgs a) {
 
 // The re-score set: every refined pair within the FP32 error bound of the
 // k-th value (or, when that is infinite, the k best keys).  Segments of the
-// list in parallel; members are appended in any order (later stages sort).
+// list in parallel; members are appended in any order (later stages sort),
+// to the query's set and to one list of all queries' members: the refine
+// kernels hand out pairs by position, and from sets padded to RC entries
+// some warps drew several pairs and most none (2,560 members in 16,384
+// entries, exact Frechet re-score: RESCORE_BA).
 template <int MEAS>
 __global__ void rescore_collect_kernel(KArgs a) {
   const int q = blockIdx.y;
   const int N = a.S + a.M + a.fcnt[q], base = a.off2[q];
+  // past the list (the grid covers every candidate): before the threshold's
+  // FP64 division, which took most of this kernel's time
+  if (blockIdx.x * kSeg >= N) return;
   const unsigned long long kth = a.kthkey[q];
   const float tk = kth == ~0ull ? TSIM_INF : ord2f((unsigned)(kth >> 32));
   const bool finite = tk < TSIM_INF;
@@ -1539,18 +1546,10 @@ __global__ void rescore_collect_kernel(KArgs a) {
       if (p < a.RC) {
         a.rpairs[(size_t)q * a.RC + p] = make_int2(q, c);
         a.rdc[(size_t)q * a.RC + p] = v;  // pairwise measures re-use their FP32 values
+        a.rlist[atomicAdd(a.n64 + 1, 1)] = q * a.RC + p;
       }
     }
   }
-}
-
-// pad the re-score set to RC entries, count its members (one thread/query)
-__global__ void rescore_pad_kernel(KArgs a) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= a.nq) return;
-  const int rc = min(a.rraw[q], a.RC);
-  for (int p = rc; p < a.RC; ++p) a.rpairs[(size_t)q * a.RC + p] = make_int2(q, -1);
-  a.rcnt[q] = rc;
 }
 
 // Bound on |compensated - FP64| relative to the value, for a path of P
@@ -1596,7 +1595,7 @@ __global__ void __launch_bounds__(32 * kRankWarps) cluster_kernel(KArgs a) {
   RankSlot& S = slots[threadIdx.x >> 5];
   const int q = blockIdx.x * kRankWarps + (threadIdx.x >> 5);
   if (q >= a.nq) return;
-  const int n = min(a.rcnt[q], kMaxRC);
+  const int n = min(a.rraw[q], min(a.RC, kMaxRC));
   const int2* rp = a.rpairs + (size_t)q * a.RC;
   const double* rv = a.rdc + (size_t)q * a.RC;
   int2* r64p = a.r64pairs + (size_t)q * a.RC;
@@ -1612,7 +1611,6 @@ __global__ void __launch_bounds__(32 * kRankWarps) cluster_kernel(KArgs a) {
   __syncwarp();
   for (int i = lane; i < n; i += 32) S.ord[rank_of(S, n, i)] = (unsigned char)i;
   __syncwarp();
-  int sent = 0;
   for (int p = lane; p < n; p += 32) {
     const int i = S.ord[p];
     const double v = S.v[i];
@@ -1628,11 +1626,9 @@ __global__ void __launch_bounds__(32 * kRankWarps) cluster_kernel(KArgs a) {
     }
     if (amb) {
       r64p[i] = rp[i];
-      ++sent;
+      a.r64list[atomicAdd(a.n64, 1)] = q * a.RC + i;
     }
   }
-  for (int o = 16; o; o >>= 1) sent += __shfl_xor_sync(0xffffffffu, sent, o);
-  if (lane == 0 && sent) atomicAdd(a.n64, sent);
 }
 
 // final order: FP64 value for cluster members, compensated value otherwise
@@ -1645,7 +1641,7 @@ __global__ void __launch_bounds__(32 * kRankWarps) final_sort_kernel(KArgs a) {
   RankSlot& S = slots[threadIdx.x >> 5];
   const int q = blockIdx.x * kRankWarps + (threadIdx.x >> 5);
   if (q >= a.nq) return;
-  const int n = min(a.rcnt[q], kMaxRC);
+  const int n = min(a.rraw[q], min(a.RC, kMaxRC));
   const int2* rp = a.rpairs + (size_t)q * a.RC;
   const double* rc = a.rdc + (size_t)q * a.RC;
   const double* r64 = a.r64 + (size_t)q * a.RC;
@@ -1688,7 +1684,7 @@ __global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_res
   for (int q = threadIdx.x; q < a.nq; q += blockDim.x) {
     c1 += a.cnt1[q];
     c2 += a.cnt2[q];
-    rc += with_rescore ? a.rcnt[q] : 0;
+    rc += with_rescore ? min(a.rraw[q], a.RC) : 0;
   }
   for (int o = 16; o; o >>= 1) {
     c1 += __shfl_xor_sync(0xffffffffu, c1, o);
@@ -1832,8 +1828,7 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
   launched(ctx, 2);
   if (MEAS != M_LCSS) {
     rescore_collect_kernel<MEAS><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a);
-    rescore_pad_kernel<<<(nq + 127) / 128, 128, 0, s>>>(a);
-    launched(ctx, 2);
+    launched(ctx);
   }
   TSIM_CUDA(cudaGetLastError());
   stage_end(ctx);
@@ -1846,6 +1841,8 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
     r.coff = a.coff;
     r.pairs = a.rpairs;
     r.npairs = nq * a.RC;
+    r.order = a.rlist;
+    r.npairs_dev = a.n64 + 1;
     r.out64 = a.rdc;
     r.band_pct = d.band_pct;
     r.max_n = a.max_qlen;
@@ -1855,6 +1852,8 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
     if (compensated_rescore(MEAS)) TSIM_TRY(run_dp(ctx, a, dpc, 32, 1, r, true));
     cluster_kernel<MEAS><<<(nq + kRankWarps - 1) / kRankWarps, 32 * kRankWarps, 0, s>>>(a);
     r.pairs = a.r64pairs;
+    r.order = a.r64list;
+    r.npairs_dev = a.n64;
     r.out64 = a.r64;
     if (MEAS == M_FRECHET) {  // exact FP64 values from the FP32 ones: no FP64 DP
       r.aux = a.rdc;
@@ -1866,7 +1865,7 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
     } else if (is_dp(MEAS)) {
       TSIM_TRY(launch_dp(ctx, dp64, 32, 1, r, a.max_clen));
     } else {
-      PwArgs p{a.qpts, a.qoff, a.cpts, a.coff, a.r64pairs, nq * a.RC, nullptr, nullptr, nullptr,
+      PwArgs p{a.qpts, a.qoff, a.cpts, a.coff, a.r64pairs, nq * a.RC, a.n64, a.r64list, nullptr,
                a.r64, nullptr};
       TSIM_TRY(launch_pairwise64(ctx, MEAS == M_HAUSDORFF ? TSIM_HAUSDORFF : TSIM_EUCLIDEAN, p));
     }
@@ -1897,7 +1896,6 @@ __global__ void brute_setup_kernel(KArgs a) {
       a.fcnt[q] = a.C;
       a.cnt1[q] = a.C;
       a.cnt2[q] = a.C;
-      a.rcnt[q] = 0;
       for (int k = 0; k < a.S; ++k) a.seeds[(size_t)q * a.S + k] = make_int2(q, -1);
       for (int k = 0; k < a.M; ++k) a.r1pairs[(size_t)q * a.M + k] = make_int2(q, -1);
     }
@@ -1910,7 +1908,7 @@ int run_brute(tsim_ctx* ctx, KArgs& a, int dp32, int dpc, int dp64) {
   cudaStream_t s = ctx->stream;
   const int nq = a.nq;
   const size_t np = (size_t)nq * a.C;
-  TSIM_CUDA(cudaMemsetAsync(a.n64, 0, sizeof(int), s));
+  TSIM_CUDA(cudaMemsetAsync(a.n64, 0, 2 * sizeof(int), s));
   stage_begin(ctx, TSIM_STAGE_FILTER);
   brute_setup_kernel<<<(unsigned)std::min<size_t>((np + 255) / 256, 4096), 256, 0, s>>>(a);
   TSIM_CUDA(cudaGetLastError());
@@ -1945,7 +1943,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   cudaStream_t s = ctx->stream;
   const int nq = a.nq;
   dim3 g1(a.nch, nq);
-  TSIM_CUDA(cudaMemsetAsync(a.n64, 0, sizeof(int), s));
+  TSIM_CUDA(cudaMemsetAsync(a.n64, 0, 2 * sizeof(int), s));
   stage_begin(ctx, TSIM_STAGE_LB1);
   clear_u32_kernel<<<std::min<size_t>(((size_t)nq * a.Cw + 255) / 256, 4096), 256, 0, s>>>(
       a.seedmap, (size_t)nq * a.Cw);
@@ -2233,7 +2231,8 @@ size_t knn_plan(const tsim_params* p, int nq, int max_qlen, const tsim_db* db, K
                 align256(sizeof(float) * nqC) + align256(sizeof(int) * nq * a.nch * a.T) +
                 align256(sizeof(int2) * nq * a.S) + align256(sizeof(unsigned) * nq * a.Cw) +
                 align256(sizeof(float) * nq * a.S) + align256(sizeof(float) * nq) +
-                5 * align256(sizeof(int) * (nq + 1)) + 2 * align256(sizeof(int) * nqC) +
+                4 * align256(sizeof(int) * (nq + 1)) + 2 * align256(sizeof(int) * nq * (size_t)a.RC) +
+                2 * align256(sizeof(int) * nqC) +
                 align256(sizeof(int) * 4) + align256(sizeof(int2) * nqC) +
                 align256(sizeof(float) * nqC) +
                 align256(sizeof(unsigned long long) * nq * (size_t)a.nseg * 64) +
@@ -2297,7 +2296,6 @@ int knn(tsim_ctx* ctx, const tsim_params* p, const float2* qpts, const int64_t* 
   a.cnt1 = arena_take<int>(ctx, nq + 1);
   a.cnt2 = arena_take<int>(ctx, nq + 1);
   a.off2 = arena_take<int>(ctx, nq + 1);
-  a.rcnt = arena_take<int>(ctx, nq + 1);
   a.list1 = arena_take<int>(ctx, nqC);
   a.list2 = arena_take<int>(ctx, nqC);
   a.npairs = arena_take<int>(ctx, 4);
@@ -2311,6 +2309,8 @@ int knn(tsim_ctx* ctx, const tsim_params* p, const float2* qpts, const int64_t* 
   a.rdc = arena_take<double>(ctx, (size_t)nq * a.RC);
   a.r64pairs = arena_take<int2>(ctx, (size_t)nq * a.RC);
   a.n64 = arena_take<int>(ctx, 4);
+  a.rlist = arena_take<int>(ctx, (size_t)nq * a.RC);
+  a.r64list = arena_take<int>(ctx, (size_t)nq * a.RC);
   a.lb2v = arena_take<float>(ctx, nqC);
   a.r1pairs = arena_take<int2>(ctx, (size_t)nq * a.M);
   a.r1vals = arena_take<float>(ctx, (size_t)nq * a.M);

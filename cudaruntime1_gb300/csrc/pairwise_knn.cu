@@ -184,7 +184,9 @@ __global__ void __launch_bounds__(kPwThreads) pairwise64_kernel(PwArgs a, int eu
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int w = gw; w < a.npairs; w += nw) {
+  const int npairs = a.npairs_dev ? min(*a.npairs_dev, a.npairs) : a.npairs;
+  for (int wk = gw; wk < npairs; wk += nw) {
+    const int w = a.order ? a.order[wk] : wk;
     const int2 pr = a.pairs[w];
     if (pr.y < 0) continue;
     const int64_t qo = a.qoff[pr.x], co = a.coff[pr.y];
