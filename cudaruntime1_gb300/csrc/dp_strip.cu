@@ -420,7 +420,105 @@ int launch_strip_one(tsim_ctx* ctx, const DpArgs& a, int max_n, int max_m, int* 
   return TSIM_OK;
 }
 
+// Exact FP64 Frechet values without a DP where one cell decides.  The FP64
+// optimum is the FP64 cost of some cell whose FP32 cost lies in the window
+// around the pair's FP32 optimum (PolFrechetWin), so when all the window's
+// cells have one FP64 cost, that is the value: a scan of the costs, no
+// dependency between cells, five instructions each.  Of 2,560 pairs of up to
+// 256 x 1,024 points about one in twelve holds two different costs in its
+// window (64 2^-24 wide) and goes on to the DP.  A CTA per pair, a warp every
+// fourth column of 256 rows at a time (a row block's points in registers).
+constexpr int kWinRows = 8;
+__global__ void __launch_bounds__(kStripThreads)
+    frechet_window_kernel(DpArgs a, int* rest, int* nrest) {
+  constexpr int kWarps = kStripThreads / 32;
+  __shared__ double wval[kWarps];
+  __shared__ int wstate[kWarps];  // 0: no window cell, 1: one cost, 2: several
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int npairs = a.npairs_dev ? min(*a.npairs_dev, a.npairs) : a.npairs;
+  for (int wk = blockIdx.x; wk < npairs; wk += gridDim.x) {
+    const int pid = a.order ? a.order[wk] : wk;
+    const int2 pr = a.pairs[pid];
+    if (pr.y < 0) continue;  // uniform over the CTA, as below
+    const int64_t qo = a.qoff[pr.x], co = a.coff[pr.y];
+    const int n = (int)(a.qoff[pr.x + 1] - qo), m = (int)(a.coff[pr.y + 1] - co);
+    const float v32 = (float)a.aux[pid];
+    if (!(v32 >= 1e-20f) || !(v32 < 1e38f)) {  // the relative window does not hold there
+      if (threadIdx.x == 0) rest[atomicAdd(nrest, 1)] = pid;
+      continue;
+    }
+    // costs strictly between lo and hi, as positive floats' bit patterns
+    const unsigned lo = __float_as_uint(__fmul_rd(v32, 1.0f - 32.0f / 16777216.0f));
+    const unsigned span = __float_as_uint(__fmul_ru(v32, 1.0f + 32.0f / 16777216.0f)) - lo - 1;
+    const float2* A = a.qpts + qo;
+    const float2* B = a.cpts + co;
+    double val = 0.0;
+    int state = 0;
+    for (int base = 0; base < n; base += 32 * kWinRows) {
+      float2 p[kWinRows];
+#pragma unroll
+      for (int k = 0; k < kWinRows; ++k) p[k] = __ldg(A + min(base + k * 32 + lane, n - 1));
+#pragma unroll 2
+      for (int j = warp; j < m; j += kWarps) {
+        const float2 c = __ldg(B + j);
+        unsigned first = 0xffffffffu;
+        float d[kWinRows];
+#pragma unroll
+        for (int k = 0; k < kWinRows; ++k) {
+          const float2 t = sub2(p[k], c);
+          d[k] = fmaf(t.y, t.y, t.x * t.x);
+          first = min(first, __float_as_uint(d[k]) - lo - 1u);
+        }
+        if (first < span) {  // some cost of this lane's is inside
+#pragma unroll
+          for (int k = 0; k < kWinRows; ++k)
+            if (__float_as_uint(d[k]) - lo - 1u < span) {
+              const double x = d2_64(p[k].x, p[k].y, c.x, c.y);
+              if (state == 0) {
+                val = x;
+                state = 1;
+              } else if (x != val) {
+                state = 2;
+              }
+            }
+        }
+      }
+    }
+    // the lanes', then the warps' costs together
+    auto meet = [](double& v, int& s, double v2, int s2) {
+      if (s2 == 0) return;
+      if (s == 0) v = v2, s = s2;
+      else if (s2 == 2 || v2 != v) s = 2;
+    };
+    for (int o = 16; o; o >>= 1) {
+      const double v2 = __shfl_xor_sync(0xffffffffu, val, o);
+      const int s2 = __shfl_xor_sync(0xffffffffu, state, o);
+      meet(val, state, v2, s2);
+    }
+    __syncthreads();  // the previous pair's states are read
+    if (lane == 0) wval[warp] = val, wstate[warp] = state;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < kWarps; ++w) meet(val, state, wval[w], wstate[w]);
+      if (state == 1)
+        a.out64[pid] = val;
+      else
+        rest[atomicAdd(nrest, 1)] = pid;
+    }
+  }
+}
+
 }  // namespace
+
+int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest) {
+  TSIM_CUDA(cudaMemsetAsync(nrest, 0, sizeof(int), ctx->stream));
+  if (a.npairs <= 0) return TSIM_OK;
+  const int blocks = std::min(a.npairs, 16 * ctx->num_sms);
+  frechet_window_kernel<<<blocks, kStripThreads, 0, ctx->stream>>>(a, rest, nrest);
+  TSIM_CUDA(cudaGetLastError());
+  launched(ctx);
+  return TSIM_OK;
+}
 
 bool strip_kind(int kind) {
   return kind == DP_DTW_REF || kind == DP_FRECHET_REF || kind == DP_DTW_SQ || kind == DP_DTW_EU ||

@@ -357,6 +357,10 @@ bool strip_kind(int kind);
 int strip_max_cols();
 int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
                     int* nspill);
+// Exact FP64 Frechet values (squared) of the pairs whose window (PolFrechetWin,
+// FP32 values in aux) holds one cost, into out64; the others' entries in rest[]
+// (count in *nrest) for DP_FRECHET_WIN.
+int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest);
 // Lane-per-pair kernel (dp_lane.cu) for the FP32 DTW, Frechet and LCSS
 // kinds (lane_kind): a lane runs a whole pair in passes of 8 rows, the row
 // above a pass in a shared-memory ring of `ring` (64 or 128) values per lane
