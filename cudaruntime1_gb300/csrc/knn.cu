@@ -11,6 +11,8 @@
 //                      pairs the O(1) bound keeps and segfilter_kernel
 //                      bounds them by 8 column segments per candidate and
 //                      32 query row segments (a group of 8 lanes a pair);
+//                      lock-step Euclidean: paa_kernel's segment-mean bound
+//                      of every pair in place of both;
 //   B  seeds           the S best chunk candidates per query are refined
 //                      exactly; the k-th best refined value, widened by the
 //                      FP32 error bound, is the query's pruning threshold;
@@ -19,7 +21,7 @@
 //                      memory for DTW, its candidates fetched by bulk copy
 //                      on databases larger than L2; box distances for
 //                      Frechet and Hausdorff, the windowed eps-box count for
-//                      LCSS; lock-step Euclidean passes the list on);
+//                      LCSS; lock-step Euclidean has none);
 //   D  DP              round 1 (the best survivors by bound) tightens the
 //                      threshold, then the remaining survivors run the
 //                      wavefront DP (or the pairwise distance) with early
@@ -117,7 +119,7 @@ struct KArgs {
   const float4* csegbox;    // [C*kSegs] candidate segment boxes
   const float2* csegsum;    // [C*kSegs] sums of the candidate segments' points
   float2* qpf;              // [nq*(max_qlen+1)] query prefix sums of p_j - p_0, FP32-rounded
-  float* qpe;               // [nq] twice a bound on their FP64 accumulation error
+  float* qpe;               // [nq] bound on the error of a difference of two of them
   int lb2_cap;              // DTW O(length) stage: points per bulk-copy buffer (0: no bulk copies)
   int64_t ctotal;           // points in the database's array (bulk copies stay inside it)
   unsigned* status;         // device status word: bit 0 = a bounded wait ran out
@@ -191,21 +193,20 @@ __device__ __forceinline__ float widen(float t, double g) {
 // ---------------------------------------------------------------------------
 // The query's rows in kQBlocks blocks (block b: rows [b n / kQBlocks,
 // (b+1) n / kQBlocks)), each with its bounding box.  Every query row is
-// coupled to (DTW, Frechet, Euclidean) or has a nearest point in (Hausdorff)
+// coupled to (DTW, Frechet) or has a nearest point in (Hausdorff)
 // the candidate, whose points lie in its box, so a block costs at least its
 // box's distance to the candidate's box per row; LCSS: a row can only match
 // when its block's eps-inflated box meets the candidate's box.
 template <int MEAS>
 __device__ __forceinline__ float block_bound(const KArgs& a, const float4* qblk, int n, float4 cb,
                                              int m) {
-  const int rows_max = MEAS == M_EUCLID ? m : n;  // lock-step: rows 0 .. m-1 only
   float acc = 0.0f;
   int cnt = 0;
   const float e2 = __fmul_ru(a.eps, 1.0f + 1.0f / 1048576.0f);
 #pragma unroll
   for (int b = 0; b < kQBlocks; ++b) {
     const int r0 = (int)((long long)b * n / kQBlocks);
-    const int r1 = min((int)((long long)(b + 1) * n / kQBlocks), rows_max);
+    const int r1 = (int)((long long)(b + 1) * n / kQBlocks);
     if (r1 <= r0) continue;
     const float4 bx = qblk[b];
     if (MEAS == M_LCSS) {
@@ -267,14 +268,6 @@ __device__ __forceinline__ float bound1(const KArgs& a, float4 qb, float4 qe, in
   const float last = pd2_rd(qe.z, qe.w, ce.z, ce.w);
   const float bb = box_box_d2_rd(qb, cb);
   if (MEAS == M_FRECHET) return fmaxf(fmaxf(first, last), bb);
-  if (MEAS == M_EUCLID) {
-    // point i of the candidate is paired with point i of the query; the
-    // query's full box contains its first-m-point prefix
-    if (n < m) return TSIM_INF;
-    if (m == 1) return first;
-    if (n == m) return __fadd_rd(__fadd_rd(first, last), __fmul_rd((float)(m - 2), bb));
-    return __fadd_rd(first, __fmul_rd((float)(m - 1), bb));
-  }
   // DTW: the path has >= max(n,m) cells; (0,0) and (n-1,m-1) are on it
   const int L = max(n, m);
   if (L < 2) return a.cost ? __fsqrt_rd(first) : first;
@@ -322,7 +315,7 @@ __global__ void __launch_bounds__(kChunk) lb1_kernel(KArgs a) {
     const float4 ce = a.cends[c], cb = a.cbox[c];
     const int m = a.clen[c];
     float b = bound1<MEAS>(a, qb, qe, n, cb, ce, m);
-    if (n > 0 && m > 0 && (MEAS != M_EUCLID || n >= m)) {
+    if (n > 0 && m > 0) {
       const float bb = block_bound<MEAS>(a, qblk, n, cb, m);
       b = MEAS == M_LCSS ? fminf(b, fminf(bb, (float)min(n, m))) : fmaxf(b, bb);
     }
@@ -473,31 +466,41 @@ __device__ __forceinline__ void qtable_build(QTable& T, const float2* A, int n, 
   }
 }
 
-// Bytes of the table buffer of a query of up to max_n rows.
-size_t qtable_bytes(int max_n) { return (size_t)qtable_stride(max_n) * sizeof(float4); }
-
 // One CTA per query: its first pruning threshold (warp 0, from the seeds),
-// then its sparse table and, for lock-step Euclidean, its prefix sums in
-// global memory (read by the segment bounds of every pair of the query).
+// then its sparse table in global memory (read by the segment bounds of every
+// pair of the query).
 template <int MEAS>
-__global__ void qtable_global_kernel(KArgs a, int sums) {
-  __shared__ double2 part[256];
+__global__ void qtable_global_kernel(KArgs a) {
   const int q = blockIdx.x;
   if (threadIdx.x < 32) seed_threshold<MEAS>(a, q, threadIdx.x);
+  if (MEAS == M_EUCLID) return;  // its bound needs no table
+  const int n = a.qlen[q];
+  if (n <= 0 || n > a.max_qlen) return;
+  QTable T;
+  qtable_build(T, a.qpts + a.qoff[q], n, a.qtab + (size_t)q * a.tstride);
+}
+
+// columns of candidate segment s: [seg_first(s), seg_first(s + 1))
+__device__ __forceinline__ int seg_first(int s, int m) { return (int)(((long long)s * m) / kSegs); }
+
+// Lock-step Euclidean: the query's prefix sums P[j] = sum of (p_i - p_0) over
+// i = 0 .. j-1, j = 0 .. n, accumulated in FP64 (each difference of two
+// floats exact) and rounded once to float.  One CTA of 256 threads per
+// query, a chunk of points per thread, the chunks joined by shuffle scans.
+// qpe[q] bounds the error of P[b] - P[a] as FP32 computes it: the roundings
+// of P[b], P[a] (2^-24 max|P| each) and of the difference (2^-24 of at most
+// 2 max|P|), with a sixteenth of slack, plus twice the FP64 sums' error
+// (each within n 2^-53 sum |p_i - p_0| of exact in any order).
+__global__ void __launch_bounds__(256) qprefix_kernel(KArgs a) {
+  __shared__ double2 wsum[8], wmag[8];
+  __shared__ float wmax[8];
+  const int q = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n = a.qlen[q];
   if (n <= 0 || n > a.max_qlen) return;
   const float2* A = a.qpts + a.qoff[q];
-  QTable T;
-  qtable_build(T, A, n, a.qtab + (size_t)q * a.tstride);
-  if (!sums) return;  // prefix sums: lock-step Euclidean only
-  // P[j] = sum of (p_i - p_0) over i = 0 .. j-1, j = 0 .. n, in FP64 (each
-  // difference of two floats exact), rounded once to float; a chunk per
-  // thread.  The FP64 sums are within n 2^-53 sum |p_i - p_0| of exact;
-  // qpe[q] keeps twice that, rounded up.
-  __shared__ double2 mag[256];
   float2* P = a.qpf + (size_t)q * (a.max_qlen + 1);
   const double x0 = A[0].x, y0 = A[0].y;
-  const int per = (n + blockDim.x - 1) / blockDim.x;
+  const int per = (n + 255) / 256;
   const int j0 = min(n, (int)threadIdx.x * per), j1 = min(n, j0 + per);
   double sx = 0.0, sy = 0.0, ax = 0.0, ay = 0.0;
   for (int j = j0; j < j1; ++j) {
@@ -507,30 +510,152 @@ __global__ void qtable_global_kernel(KArgs a, int sums) {
     ax += fabs(dx);
     ay += fabs(dy);
   }
-  part[threadIdx.x] = make_double2(sx, sy);
-  mag[threadIdx.x] = make_double2(ax, ay);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double rx = 0.0, ry = 0.0, mx = 0.0, my = 0.0;
-    for (int i = 0; i < (int)blockDim.x; ++i) {
-      const double2 v = part[i];
-      part[i] = make_double2(rx, ry);
-      rx += v.x;
-      ry += v.y;
-      mx += mag[i].x;
-      my += mag[i].y;
-    }
-    P[n] = make_float2((float)rx, (float)ry);
-    // n 2^-53 (1 + 2^-40) max(sum |dx|, sum |dy|), doubled, rounded up
-    a.qpe[q] = __double2float_ru(2.0 * (double)n * 1.1102230246251565e-16 * (1.0 + 1e-12) *
-                                 fmax(mx, my));
+  double ix = sx, iy = sy;  // inclusive sums over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double ux = __shfl_up_sync(0xffffffffu, ix, o), uy = __shfl_up_sync(0xffffffffu, iy, o);
+    if (lane >= o) ix += ux, iy += uy;
   }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    ax += __shfl_xor_sync(0xffffffffu, ax, o);
+    ay += __shfl_xor_sync(0xffffffffu, ay, o);
+  }
+  if (lane == 31) wsum[warp] = make_double2(ix, iy);
+  if (lane == 0) wmag[warp] = make_double2(ax, ay);
   __syncthreads();
-  double rx = part[threadIdx.x].x, ry = part[threadIdx.x].y;
+  double rx = ix - sx, ry = iy - sy, mx = 0.0, my = 0.0;
+  for (int w = 0; w < 8; ++w) {
+    if (w < warp) rx += wsum[w].x, ry += wsum[w].y;
+    mx += wmag[w].x;
+    my += wmag[w].y;
+  }
+  float big = 0.0f;
   for (int j = j0; j < j1; ++j) {
     P[j] = make_float2((float)rx, (float)ry);
+    big = fmaxf(big, fmaxf(fabsf((float)rx), fabsf((float)ry)));
     rx += (double)A[j].x - x0;
     ry += (double)A[j].y - y0;
+  }
+  if (j1 == n && (j0 < n || n == 0)) P[n] = make_float2((float)rx, (float)ry);
+  big = fmaxf(big, fmaxf(fabsf((float)rx), fabsf((float)ry)));
+  for (int o = 16; o; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0) wmax[warp] = big;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) big = fmaxf(big, wmax[w]);
+    // a prefix by difference of sums (rx = ix - sx) takes 16 more additions
+    const double e64 = 2.0 * (n + 16.0) * 1.1102230246251565e-16 * (1.0 + 1e-12) * fmax(mx, my);
+    a.qpe[q] = __double2float_ru(1.0625 * (double)big / 4194304.0 + e64);
+  }
+}
+
+// Lock-step Euclidean, stage A: a lower bound of every pair from the sums of
+// the candidate's kSegs segments and of the query's points at the same
+// indices.  Cauchy-Schwarz: the squared distance over a segment of L points
+// is at least |sum q - sum c|^2 / L; a segment's means lie in its boxes, so
+// this is never below the distance of the segment's boxes.  A thread per
+// candidate, its sums, boundaries and lengths in registers, looped over
+// kPaaQueries queries; 256 candidates a CTA, whose T best by the bound are
+// kept as seed candidates.
+//
+// Against the O(1) bound, compaction and a segment bound on 8 lanes a pair
+// (which evaluated nearly every pair: the O(1) bound hardly prunes random
+// walks): 1,024 x 262,144 pairs 30.5 -> 2.7 ms, and the seeds, picked by
+// this bound, leave 93,000 pairs instead of 38.7 M.  Bound by FP32 issue: 12
+// instructions a segment and pair.
+//
+// Rounding, per coordinate and segment: A = P[b1] - P[b0] within qpe of the
+// query's sum less L p_0; U = fma(-L, p_0, s) within 2^-24 |U| of s - L p_0, s
+// within 2^-24 |s| + 2^-30 L max|c| of the candidate's sum (one rounding of an
+// FP64 sum); |U|, |s| <= L (max|c| + |p_0|) to within those, so both are
+// covered by L 2^-22 (max|c| + |p_0|); D = A - U within 2^-24 |D|, covered by
+// the factor 1 - 2^-22.  What is left of |D| is squared and summed rounding
+// down, and divided by the longest segment's length, rounding down.
+constexpr int kPaaQueries = 8;
+__global__ void __launch_bounds__(kChunk) paa_kernel(KArgs a) {
+  __shared__ unsigned long long keys[kChunk];
+  __shared__ SelScratch red;
+  __shared__ unsigned long long sel[64];
+  __shared__ unsigned wbest[kPaaQueries][kChunk / 32];
+  __shared__ int wcand[kPaaQueries][kChunk / 32];
+  const int chunk = blockIdx.x;
+  const int c = chunk * kChunk + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q0 = blockIdx.y * kPaaQueries, q1 = min(a.nq, q0 + kPaaQueries);
+  const bool in = c < a.C;
+  const int m = in ? a.clen[c] : 0;
+  int b[kSegs + 1];    // segment boundaries
+  float len[kSegs];    // their lengths
+  float2 sum[kSegs];
+  float cmax = 0.0f;
+#pragma unroll
+  for (int s = 0; s <= kSegs; ++s) b[s] = seg_first(s, m);
+#pragma unroll
+  for (int s = 0; s < kSegs; ++s) {
+    len[s] = (float)(b[s + 1] - b[s]);
+    sum[s] = in ? a.csegsum[(size_t)c * kSegs + s] : make_float2(0.0f, 0.0f);
+  }
+  if (in) {
+    const float4 cb = a.cbox[c];
+    cmax = fmaxf(fmaxf(fabsf(cb.x), fabsf(cb.z)), fmaxf(fabsf(cb.y), fabsf(cb.w)));
+  }
+  const float lmax = (float)((m + kSegs - 1) / kSegs);
+  const float rl = __frcp_rd(fmaxf(lmax, 1.0f));
+  const float lc = __fmul_ru(lmax, 1.0f / 4194304.0f);
+  for (int q = q0; q < q1; ++q) {
+    const int n = a.qlen[q];
+    float bound = 0.0f;
+    if (n < 1 || m < 1 || n < m) {
+      bound = TSIM_INF;  // never a neighbour at a finite distance
+    } else if (n <= a.max_qlen && m <= (1 << 26)) {
+      const float4 qe = a.qends[q];
+      const float2* P = a.qpf + (size_t)q * (a.max_qlen + 1);
+      const float e = __fmaf_ru(lc, __fadd_ru(cmax, fmaxf(fabsf(qe.x), fabsf(qe.y))), a.qpe[q]);
+      float2 p0 = make_float2(0.0f, 0.0f);  // P[0]
+      float accx = 0.0f, accy = 0.0f;
+#pragma unroll
+      for (int s = 0; s < kSegs; ++s) {
+        const float2 p1 = __ldg(P + b[s + 1]);
+        const float dx = (p1.x - p0.x) - fmaf(-len[s], qe.x, sum[s].x);
+        const float dy = (p1.y - p0.y) - fmaf(-len[s], qe.y, sum[s].y);
+        const float gx = fmaxf(__fmaf_rd(fabsf(dx), 1.0f - 1.0f / 4194304.0f, -e), 0.0f);
+        const float gy = fmaxf(__fmaf_rd(fabsf(dy), 1.0f - 1.0f / 4194304.0f, -e), 0.0f);
+        accx = __fmaf_rd(gx, gx, accx);
+        accy = __fmaf_rd(gy, gy, accy);
+        p0 = p1;
+      }
+      bound = __fmul_rd(__fadd_rd(accx, accy), rl);
+    }
+    if (in) a.lb1[(size_t)q * a.C + c] = bound;
+    if (a.T == 1) {  // the warp's best; the CTA's after the loop
+      const unsigned o = in ? f2ord(bound) : 0xffffffffu;
+      const unsigned mn = __reduce_min_sync(0xffffffffu, o);
+      const unsigned who = __ballot_sync(0xffffffffu, o == mn);
+      if (lane == 0) {
+        wbest[q - q0][warp] = mn;
+        wcand[q - q0][warp] = mn == 0xffffffffu ? -1 : chunk * kChunk + warp * 32 + __ffs(who) - 1;
+      }
+    } else {
+      keys[threadIdx.x] = in ? pack_key(bound, threadIdx.x) : ~0ull;
+      __syncthreads();
+      block_select_k(keys, kChunk, a.T, sel, red);
+      for (int i = threadIdx.x; i < a.T; i += kChunk) {
+        const int li = key_index(sel[i]);
+        a.chunk_cand[((size_t)q * a.nch + chunk) * a.T + i] = li < 0 ? -1 : chunk * kChunk + li;
+      }
+      __syncthreads();
+    }
+  }
+  if (a.T == 1) {
+    __syncthreads();
+    const int q = q0 + threadIdx.x;
+    if (threadIdx.x < kPaaQueries && q < q1) {
+      int best = 0;
+      for (int w = 1; w < kChunk / 32; ++w)
+        if (wbest[threadIdx.x][w] < wbest[threadIdx.x][best]) best = w;
+      a.chunk_cand[(size_t)q * a.nch + chunk] = wcand[threadIdx.x][best];
+    }
   }
 }
 
@@ -571,9 +696,6 @@ __global__ void lcss_env_kernel(KArgs a) {
 // point is matched, so the maximum over segments; LCSS: a column can only
 // match when the boxes, eps-inflated, meet).  Columns 0 and m-1 are the
 // exact corner cells for DTW.
-// columns of candidate segment s: [seg_first(s), seg_first(s + 1))
-__device__ __forceinline__ int seg_first(int s, int m) { return (int)(((long long)s * m) / kSegs); }
-
 // Row side of the segment bounds: the query's rows in kRowSegs segments;
 // the rows of a segment admit only columns [clo, chi], so each costs at
 // least the distance between the segment's box and the nearest candidate
@@ -634,63 +756,11 @@ __device__ __forceinline__ bool group_any(bool v) {
 // it the row segments are not evaluated.  Called by every lane of a group
 // with the same pair; g is the lane within the group.
 template <int MEAS>
-__device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1, float t, int g,
-                           const QTable& Tq, float4 qbq) {
+__device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1, float t, int g) {
   if (n > a.max_qlen || n < 1 || m < 1) return lb1;
   const float4* sb = a.csegbox + (size_t)c * kSegs;
-  // lock-step Euclidean takes the query's table view and box from the
-  // caller (read once per thread: 765 -> 712 M instructions per 64-query
-  // chunk); the other measures read them per pair, which keeps their kernels
-  // at 48 registers (62 with them held across the loop)
-  QTable T = Tq;
-  float4 qb = qbq;
-  if (MEAS != M_EUCLID) {
-    qb = a.qbox[q];
-    T = qtable_view(a.qtab + (size_t)q * a.tstride, n);
-  }
-  if (MEAS == M_EUCLID) {
-    // lock-step: column j meets row j only, so segment s (L points) costs at
-    // least L times its box's squared distance to the box of the same query
-    // rows, and at least |sum of the query's points - sum of the candidate's|^2
-    // / L per coordinate (Cauchy-Schwarz); the larger of the two per segment
-    if (n < m) return TSIM_INF;
-    const float2* ss = a.csegsum + (size_t)c * kSegs;
-    const float2* P = a.qpf + (size_t)q * (a.max_qlen + 1);
-    const float4 qe = a.qends[q];  // the query's first point: P's origin
-    float part = 0.0f;
-    const int s = g;
-    const int b0 = seg_first(s, m), b1 = seg_first(s + 1, m) - 1;
-    if (b1 >= b0) {
-      const float L = (float)(b1 - b0 + 1);
-      const float4 cb = sb[s];
-      const float d = box_box_d2_rd(qtable_box(T, b0, b1), cb);
-      const float2 sc = ss[s];
-      const float2 f1 = P[b1 + 1], f0 = P[b0];
-      const float e64 = a.qpe[q];
-      // |sum q - sum c| per coordinate, in FP32 from origin-shifted sums:
-      // A = f1 - f0 (the query's, less L p_0), B = sc - L p_0 (the
-      // candidate's), D = |A - B|.  Each rounding -- f1, f0, A, t = L p_0, B,
-      // D, and the candidate sum's (one float rounding of an FP64 sum) -- is
-      // at most 2^-24 of its value, so 2^-22 of the magnitudes below covers
-      // them twice over; e64 covers the query's FP64 prefix sums and 2^-30 L
-      // max|c| the candidate's (at most L^2 2^-53 max|c|, L <= 2^11).
-      auto gap = [&](float a1, float a0, float scv, float p0, float c0, float c1) {
-        const float A = a1 - a0, t = L * p0, B = scv - t, D = fabsf(A - B);
-        float mgn = __fadd_ru(__fadd_ru(fabsf(a1), fabsf(a0)), __fadd_ru(fabsf(t), fabsf(scv)));
-        mgn = __fadd_ru(__fmul_ru(__fadd_ru(mgn, D), 1.0f / 4194304.0f), e64);
-        mgn = __fadd_ru(mgn, __fmul_ru(__fmul_ru(L, fmaxf(fabsf(c0), fabsf(c1))), 1.0f / 1073741824.0f));
-        return fmaxf(0.0f, __fsub_rd(D, mgn));
-      };
-      const float ax = gap(f1.x, f0.x, sc.x, qe.x, cb.x, cb.z);
-      const float ay = gap(f1.y, f0.y, sc.y, qe.y, cb.y, cb.w);
-      // / L as * (1/L within 2 ulp, times 1 - 2^-21 rounded down: below
-      // 1/L), no division sequence
-      const float rl = __fmul_rd(__fdividef(1.0f, L), 0.99999952f);
-      const float cs = __fmul_rd(__fadd_rd(__fmul_rd(ax, ax), __fmul_rd(ay, ay)), rl);
-      part = fmaxf(__fmul_rd(L, d), cs);
-    }
-    return fmaxf(group_sum_rd(part), lb1);
-  }
+  const float4 qb = a.qbox[q];
+  const QTable T = qtable_view(a.qtab + (size_t)q * a.tstride, n);
   if (MEAS == M_FRECHET || MEAS == M_HAUSDORFF) {
     // every point of either set is matched to some point of the other
     float mx = lb1;
@@ -822,8 +892,7 @@ __device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1
 // Append the pair to a per-query list, aggregated over a block of kChunk
 // threads (every thread of the block calls it): warp counts through shared
 // memory, one atomic per block.  A query's list has one counter; with an
-// atomic per warp, a 1M-candidate scan queued on it (compact_kernel: 311 us
-// for 16 queries x 1M candidates at 12 % SM throughput; 86 us per block).
+// atomic per warp, a 1M-candidate scan queued on it.
 __device__ __forceinline__ void block_append(bool take, int* count, int* list, int value) {
   __shared__ int wbase[kChunk / 32];
   __shared__ int bbase;
@@ -846,19 +915,64 @@ __device__ __forceinline__ void block_append(bool take, int* count, int* list, i
 }
 
 // Stage A, first half: the pairs the O(1) bound keeps (seeds excluded) are
-// listed (in list2, free until the O(length) stage) ...
+// listed, in list2 (free until the O(length) stage; lock-step Euclidean,
+// which has no later bound, lists its survivors and their bounds for round 1
+// at once).  kCompact bounds a thread: a block that keeps nothing ends after
+// one vote, one that keeps some makes one atomic for its 2,048 pairs (with
+// 256 pairs a block 16.7 M bounds took 83 to 92 us; now 27).
+constexpr int kCompact = 8;
 template <int MEAS>
 __global__ void __launch_bounds__(kChunk) compact_kernel(KArgs a) {
+  __shared__ int wbase[kChunk / 32];
+  __shared__ int bbase;
   const int q = blockIdx.y;
-  const int c = blockIdx.x * kChunk + threadIdx.x;
+  const int c0 = blockIdx.x * kChunk * kCompact + threadIdx.x;
   const float t = a.thr[q];
-  bool pass = false;
-  if (c < a.C) {
-    const bool seeded = (a.seedmap[(size_t)q * a.Cw + (c >> 5)] >> (c & 31)) & 1u;
-    const float b = a.lb1[(size_t)q * a.C + c];
-    pass = !seeded && (MEAS == M_LCSS ? (b >= t) : (b <= t));
+  const float* lb = a.lb1 + (size_t)q * a.C;
+  float bnd[kCompact];
+  unsigned take = 0;
+#pragma unroll
+  for (int i = 0; i < kCompact; ++i) {
+    const int c = c0 + i * kChunk;
+    bnd[i] = c < a.C ? lb[c] : (MEAS == M_LCSS ? -TSIM_INF : TSIM_INF);
   }
-  block_append(pass, a.cnt0 + q, a.list2 + (size_t)q * a.C, c);
+#pragma unroll
+  for (int i = 0; i < kCompact; ++i) {
+    const int c = c0 + i * kChunk;
+    const bool pass = MEAS == M_LCSS ? bnd[i] >= t : bnd[i] <= t;
+    if (pass && c < a.C && !((a.seedmap[(size_t)q * a.Cw + (c >> 5)] >> (c & 31)) & 1u))
+      take |= 1u << i;
+  }
+  if (!__syncthreads_or((int)take)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int mine = __popc(take);
+  int inc = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) wbase[warp] = inc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kChunk / 32; ++w) {
+      const int n = wbase[w];
+      wbase[w] = total;
+      total += n;
+    }
+    bbase = atomicAdd(MEAS == M_EUCLID ? a.cnt2 + q : a.cnt0 + q, total);
+  }
+  __syncthreads();
+  size_t at = (size_t)q * a.C + bbase + wbase[warp] + inc - mine;
+#pragma unroll
+  for (int i = 0; i < kCompact; ++i)
+    if ((take >> i) & 1u) {
+      a.list2[at] = c0 + i * kChunk;
+      if (MEAS == M_EUCLID) a.lb2v[at] = bnd[i];
+      ++at;
+    }
 }
 
 // ... and their segment bounds are computed with every lane of a warp busy
@@ -873,13 +987,6 @@ __global__ void __launch_bounds__(256) segfilter_kernel(KArgs a) {
   const int n = a.qlen[q];
   const int g = threadIdx.x & (kSegGroup - 1);
   const int per_block = blockDim.x / kSegGroup;  // pairs per block and pass
-  // lock-step Euclidean: the query's table view and box once per thread
-  QTable T{};
-  float4 qb{};
-  if (MEAS == M_EUCLID) {
-    if (n >= 1 && n <= a.max_qlen) T = qtable_view(a.qtab + (size_t)q * a.tstride, n);
-    qb = a.qbox[q];
-  }
   const int start = blockIdx.x * per_block;
   const int stride = gridDim.x * per_block;
   for (int e0 = start; e0 < cnt; e0 += stride) {  // uniform per block: whole blocks iterate
@@ -889,7 +996,7 @@ __global__ void __launch_bounds__(256) segfilter_kernel(KArgs a) {
     if (e < cnt) {  // uniform per group
       c = a.list2[(size_t)q * a.C + e];
       const float b = a.lb1[(size_t)q * a.C + c];
-      const float sbnd = seg_bound<MEAS>(a, q, c, n, a.clen[c], b, t, g, T, qb);
+      const float sbnd = seg_bound<MEAS>(a, q, c, n, a.clen[c], b, t, g);
       pass = g == 0 && (MEAS == M_LCSS ? (sbnd >= t) : (sbnd <= t));
       if (pass) a.lb1[(size_t)q * a.C + c] = sbnd;
     }
@@ -909,23 +1016,6 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int cnt = a.cnt1[q];
   if (cnt == 0) return;  // uniform across the CTA
-  if (MEAS == M_EUCLID) {
-    // no O(length) bound (the exact sum costs the same): the list passes
-    // whole, in order, with the segment bounds -- no append per pair (an
-    // atomic per pair on the query's counter cost 26 ms per 1,024 x 262,144
-    // request)
-    // (an empty trajectory on either side leaves a consumed entry, -1)
-    const int* L1 = a.list1 + (size_t)q * a.C;
-    const bool qok = a.qlen[q] > 0;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
-      const int c = L1[e];
-      const bool ok = qok && a.clen[c] > 0;
-      a.list2[(size_t)q * a.C + e] = ok ? c : -1;
-      a.lb2v[(size_t)q * a.C + e] = ok ? a.lb1[(size_t)q * a.C + c] : TSIM_INF;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.cnt2[q] = cnt;
-    return;
-  }
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
   const float4 qb = a.qbox[q];
@@ -1076,9 +1166,6 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
     float lbv = sbnd;  // the bound (no O(length) bound: stage A's)
     if (n <= 0 || m <= 0) {
       pass = false;
-    } else if (MEAS == M_EUCLID) {
-      // no O(length) bound: the exact sum costs the same
-      pass = true;
     } else if (kTable && !use_table) {
       pass = true;
     } else if (MEAS == M_DTW) {
@@ -1679,10 +1766,10 @@ __global__ void clear_u32_kernel(unsigned* p, size_t n) {
 // Per-request counters, accumulated on the device (no host sync per chunk):
 // counters[2..6] += pairs passing the O(1) bound, the O(length) bound,
 // refined pairs, re-scored pairs, FP64 re-scored pairs.
-__global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_rescore) {
+__global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_rescore, int euclid) {
   unsigned long long c1 = 0, c2 = 0, rc = 0;
   for (int q = threadIdx.x; q < a.nq; q += blockDim.x) {
-    c1 += a.cnt1[q];
+    c1 += euclid ? a.cnt2[q] : a.cnt1[q];  // one bound stage only
     c2 += a.cnt2[q];
     rc += with_rescore ? min(a.rraw[q], a.RC) : 0;
   }
@@ -1878,7 +1965,7 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
     stage_end(ctx);
   }
   if (ctx->count_funnel) {  // a synchronising request that reports its funnel
-    stats_kernel<<<1, 256, 0, s>>>(a, ctx->dcounters, MEAS != M_LCSS ? 1 : 0);
+    stats_kernel<<<1, 256, 0, s>>>(a, ctx->dcounters, MEAS != M_LCSS ? 1 : 0, MEAS == M_EUCLID);
     TSIM_CUDA(cudaGetLastError());
     launched(ctx);
   }
@@ -1950,7 +2037,13 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   stage_begin(ctx, TSIM_STAGE_LB1);
   clear_u32_kernel<<<std::min<size_t>(((size_t)nq * a.Cw + 255) / 256, 4096), 256, 0, s>>>(
       a.seedmap, (size_t)nq * a.Cw);
-  lb1_kernel<MEAS><<<g1, kChunk, 0, s>>>(a);
+  if constexpr (MEAS == M_EUCLID) {
+    qprefix_kernel<<<nq, 256, 0, s>>>(a);
+    paa_kernel<<<dim3(a.nch, (nq + kPaaQueries - 1) / kPaaQueries), kChunk, 0, s>>>(a);
+    launched(ctx);
+  } else {
+    lb1_kernel<MEAS><<<g1, kChunk, 0, s>>>(a);
+  }
   stage_end(ctx);
   launched(ctx, 2);
   stage_begin(ctx, TSIM_STAGE_SEED);
@@ -1998,37 +2091,40 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   stage_end(ctx);
 
   stage_begin(ctx, TSIM_STAGE_FILTER);
-  qtable_global_kernel<MEAS><<<nq, 256, 0, s>>>(a, MEAS == M_EUCLID);  // threshold, segment bounds
+  qtable_global_kernel<MEAS><<<nq, MEAS == M_EUCLID ? 32 : 256, 0, s>>>(a);  // threshold, table
   if (MEAS == M_LCSS && a.qenv) {
     lcss_env_kernel<<<nq, 256, 0, s>>>(a);
     launched(ctx);
   }
-  compact_kernel<MEAS><<<g1, kChunk, 0, s>>>(a);
-  segfilter_kernel<MEAS><<<dim3(std::max(1, std::min(1024, (32 * ctx->num_sms + nq - 1) / nq)), nq),
-                           256, 0, s>>>(a);
-  launched(ctx);
+  compact_kernel<MEAS><<<dim3((a.C + kChunk * kCompact - 1) / (kChunk * kCompact), nq), kChunk, 0,
+                         s>>>(a);
   launched(ctx, 2);
   if (MEAS == M_DTW) d.qtab = a.qtab;  // the survivor round: remaining columns' bound
   // CTAs per query of the grid-stride filter kernels: about 8 per SM over the
   // whole request, so a single query against a large database fills the GPU
   const int ch = std::max(1, std::min(65535, (8 * ctx->num_sms + nq - 1) / nq));
-  // LCSS: the query's grid and window boxes per CTA, and 4x the CTAs per
-  // query (its queries' pair counts vary widely; a CTA's set-up is small)
-  const size_t lb2_smem =
-      MEAS == M_LCSS   ? sizeof(uint32_t) * kGridWords + sizeof(float4) * (size_t)a.env_stride
-      : MEAS == M_DTW ? sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2)
-                       : 0;
-  const int ch2 = MEAS == M_LCSS ? std::max(1, std::min(65535, (32 * ctx->num_sms + nq - 1) / nq))
-                                 : ch;
-  auto lb2 = MEAS == M_DTW ? lb2_dtw_kernel : lb2_kernel<MEAS>;
-  if (lb2_smem > 48 * 1024)
-    TSIM_CUDA(cudaFuncSetAttribute(lb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)lb2_smem));
-  lb2<<<dim3(ch2, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
+  if constexpr (MEAS != M_EUCLID) {
+    segfilter_kernel<MEAS><<<dim3(std::max(1, std::min(1024, (32 * ctx->num_sms + nq - 1) / nq)), nq),
+                             256, 0, s>>>(a);
+    // LCSS: the query's grid and window boxes per CTA, and 4x the CTAs per
+    // query (its queries' pair counts vary widely; a CTA's set-up is small)
+    const size_t lb2_smem =
+        MEAS == M_LCSS   ? sizeof(uint32_t) * kGridWords + sizeof(float4) * (size_t)a.env_stride
+        : MEAS == M_DTW ? sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2)
+                         : 0;
+    const int ch2 = MEAS == M_LCSS ? std::max(1, std::min(65535, (32 * ctx->num_sms + nq - 1) / nq))
+                                   : ch;
+    auto lb2 = MEAS == M_DTW ? lb2_dtw_kernel : lb2_kernel<MEAS>;
+    if (lb2_smem > 48 * 1024)
+      TSIM_CUDA(cudaFuncSetAttribute(lb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)lb2_smem));
+    lb2<<<dim3(ch2, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
+    launched(ctx, 2);
+  }
   seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.M);
   r1_select_kernel<MEAS><<<nq, kSelThreads, 0, s>>>(a);
   TSIM_CUDA(cudaGetLastError());
-  launched(ctx, 5);
+  launched(ctx, 2);
   stage_end(ctx);
 
   // round 1: the best survivors by bound, abandon against the seed threshold
@@ -2353,9 +2449,11 @@ int knn(tsim_ctx* ctx, const tsim_params* p, const float2* qpts, const int64_t* 
 
   stage_begin(ctx, TSIM_STAGE_SUMMARY);
   TSIM_TRY(summarize(ctx, qpts, qoff, nq, qbox, qends, qlen));
-  qblocks_kernel<<<(nq + 3) / 4, 128, 0, ctx->stream>>>(qpts, qoff, nq, a.qblk);
-  TSIM_CUDA(cudaGetLastError());
-  launched(ctx);
+  if (p->measure != TSIM_EUCLIDEAN && !a.brute) {  // read by lb1_kernel only
+    qblocks_kernel<<<(nq + 3) / 4, 128, 0, ctx->stream>>>(qpts, qoff, nq, a.qblk);
+    TSIM_CUDA(cudaGetLastError());
+    launched(ctx);
+  }
   stage_end(ctx);
   switch (p->measure) {
     case TSIM_DTW:

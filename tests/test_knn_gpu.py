@@ -408,3 +408,28 @@ def test_dp_kernel_choices_agree(tsim, cuda_ctx, oracle, measure, kw):
                 assert np.array_equal(got[2].view(np.uint64), base[2].view(np.uint64)), \
                     (measure, extra, choice)
     db.close()
+
+
+@pytest.mark.parametrize("offset", [0.0, 3e5])
+@pytest.mark.parametrize("nc,k", [(300, 40), (5000, 3), (9000, 10)])
+def test_euclidean_segment_means(tsim, cuda_ctx, oracle, nc, k, offset):
+    """The segment-mean bound: ragged candidates down to one point (empty
+    segments), queries of the same, a longer and a too short length, several
+    seed candidates a chunk and one, coordinates far from the origin (whose
+    sums round coarsely): the oracle's ids, and the distances of a request
+    that refines every pair."""
+    lens = np.random.default_rng(nc).integers(1, 70, nc)
+    lens[::5] = 64
+    cp, co = G.random_walks(nc, lens, 31, step="student_t", start_range=20.0)
+    qp, qo = G.random_walks(9, [64, 1, 3, 8, 63, 65, 200, 64, 9], 32, step="student_t",
+                            start_range=20.0)
+    cp, qp = (cp + np.float32(offset)).astype(np.float32), (qp + np.float32(offset)).astype(np.float32)
+    db = tsim.Database(cuda_ctx, cp, co)
+    want_ids, want_d = oracle.knn("euclidean", qp, qo, cp, co, k)
+    ids, d, d64, _ = _device_knn(tsim, cuda_ctx, db, qp, qo, "euclidean", k,
+                                 flags=tsim.api.FLAG_ALWAYS_PRUNE)
+    ids2, d2, d642, _ = _device_knn(tsim, cuda_ctx, db, qp, qo, "euclidean", k,
+                                    flags=tsim.api.FLAG_NO_PRUNE)
+    assert np.array_equal(ids, want_ids)
+    assert np.array_equal(ids, ids2) and np.array_equal(d, d2) and np.array_equal(d64, d642)
+    db.close()
