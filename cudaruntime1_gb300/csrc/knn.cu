@@ -1817,6 +1817,9 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
     rest.npairs_dev = a.nwaves;
     return launch_dp(ctx, kind, G, R, rest, a.max_clen);
   }
+  // bit vectors, in every round: a round's time follows the columns that can
+  // match, not the window's cells, so there is no gate on its size
+  if (a.wave && lcss_window_kind(kind, d.delta)) return launch_lcss_window(ctx, d);
   if (!latency && a.lane_gate > 0 && lane_kind(kind)) {
     // many pairs: a lane per pair, with a latency of one pair's cells but a
     // few instructions per cell; the kernel itself passes a round of fewer
@@ -2100,6 +2103,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
                          s>>>(a);
   launched(ctx, 2);
   if (MEAS == M_DTW) d.qtab = a.qtab;  // the survivor round: remaining columns' bound
+  if (MEAS == M_LCSS) d.qtab = a.qenv;  // columns that cannot match
   // CTAs per query of the grid-stride filter kernels: about 8 per SM over the
   // whole request, so a single query against a large database fills the GPU
   const int ch = std::max(1, std::min(65535, (8 * ctx->num_sms + nq - 1) / nq));
@@ -2135,7 +2139,8 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     r1.npairs = nq * a.M;
     r1.out = a.r1vals;
     r1.thr = a.thr;
-    r1.qtab = nullptr;  // the best pairs by bound rarely abandon: no remaining-columns bound
+    // the best pairs by bound rarely abandon: no remaining-columns bound
+    if (MEAS == M_DTW) r1.qtab = nullptr;
     if (a.plain) {
       for (int i = 0; i < nq * a.M; ++i) {
         DpArgs one = r1;
@@ -2154,13 +2159,20 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   refilter_kernel<MEAS><<<dim3(ch, nq), 256, 0, s>>>(a);
   scan_kernel<<<1, 1024, 0, s>>>(a);
   flatten_kernel<<<dim3(ch, nq), 256, 0, s>>>(a);
-  TSIM_CUDA(cudaMemsetAsync(a.shape_cnt, 0, sizeof(int) * kNumShapes, s));
-  const int sb = ctx->num_sms * 4;
-  shape_hist_kernel<<<sb, 256, 0, s>>>(a);
-  shape_scan_kernel<<<1, 1024, 0, s>>>(a);
-  shape_scatter_kernel<<<sb, 256, 0, s>>>(a);
+  // the shape order serves the kernels whose warps run as long as their
+  // longest pair; the LCSS bit vectors gain more from one query's pairs side
+  // by side
+  const bool sorted = !(MEAS == M_LCSS && a.wave && lcss_window_kind(dp32, a.delta));
+  launched(ctx, 3);
+  if (sorted) {
+    TSIM_CUDA(cudaMemsetAsync(a.shape_cnt, 0, sizeof(int) * kNumShapes, s));
+    const int sb = ctx->num_sms * 4;
+    shape_hist_kernel<<<sb, 256, 0, s>>>(a);
+    shape_scan_kernel<<<1, 1024, 0, s>>>(a);
+    shape_scatter_kernel<<<sb, 256, 0, s>>>(a);
+    launched(ctx, 3);
+  }
   TSIM_CUDA(cudaGetLastError());
-  launched(ctx, 6);
   stage_end(ctx);
 
   stage_begin(ctx, TSIM_STAGE_DP_SURVIVORS);
@@ -2170,7 +2182,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   d.npairs_dev = a.npairs;
   d.out = a.flat_vals;
   d.thr = a.thr2;
-  d.order = a.order;
+  d.order = sorted ? a.order : nullptr;
   if (a.plain) {
     int npairs = 0;
     TSIM_CUDA(cudaMemcpyAsync(&npairs, a.npairs, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2824,6 +2836,7 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
       Rd = R;
       break;
     }
+  if (kernel == 0 && lcss_window_kind(kind, d.delta)) return launch_lcss_window(ctx, d);
   int G, R;
   dp_shape(kind, max_qlen, max_clen, wd, G, R);
   const bool diag_kind = precision < 2;

@@ -253,7 +253,8 @@ struct DpArgs {
   const int* order;   // optional: work item w is pair order[w] (shape-sorted schedule)
   const double* aux;  // optional: a value per pair, passed to the cell policy (else eps)
   const float4* qtab; // optional: queries' sparse tables (qtable_stride(max_n) float4 each):
-                      //   DTW abandoning adds the remaining columns' bound
+                      //   DTW abandoning adds the remaining columns' bound; LCSS: the
+                      //   queries' window boxes (launch_lcss_window)
   int npairs;
   int band_pct;       // DTW/Frechet band, <0 none
   int delta;          // LCSS window, <0 none
@@ -357,6 +358,12 @@ bool strip_kind(int kind);
 int strip_max_cols();
 int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
                     int* nspill);
+// Windowed LCSS by bit vectors (dp_lcss.cu, windows of at most 63 rows): a
+// warp per pair; a.qtab optionally holds the eps-inflated boxes of each
+// query's windows, a.max_n + delta + 1 per query (column j: the box of rows
+// j - delta .. j + delta).  Takes pairs of any length.
+bool lcss_window_kind(int kind, int delta);
+int launch_lcss_window(tsim_ctx* ctx, const DpArgs& a);
 // Exact FP64 Frechet values (squared) of the pairs whose window (PolFrechetWin,
 // FP32 values in aux) holds one cost, into out64; the others' entries in rest[]
 // (count in *nrest) for DP_FRECHET_WIN.

@@ -188,3 +188,39 @@ def test_frechet_fp64_rescore_of_long_pairs(tsim, cuda_ctx, oracle):
         assert np.array_equal(ids.cpu().numpy().reshape(4, 20), want_ids)
         assert np.array_equal(d64.cpu().numpy().reshape(4, 20), want)
     db.close()
+
+
+@pytest.mark.parametrize("delta", [0, 1, 3, 15, 16, 20, 31])
+def test_lcss_window_bit_vectors(tsim, cuda_ctx, oracle, delta):
+    """Windowed LCSS, the kernel chosen by the library, against the oracle:
+    dense and sparse matches, one-point sides, rows and columns past the
+    other side's window, gaps of more than 64 columns between matches; and
+    within kNN, where the queries' window boxes skip columns."""
+    import torch
+    from cudaruntime1_gb300 import api
+    cl = np.array([1, 2, 31, 32, 33, 64, 100, 200, 400] * 4)
+    cp, co = G.random_walks(len(cl), cl, 41, start_range=4.0)
+    qp, qo = G.random_walks(6, [1, 30, 64, 65, 129, 390], 42, start_range=4.0)
+    far = qp[qo[5]:qo[6]].copy()  # a copy of the longest query, far away but for its ends
+    far[8:-8] += 1e4
+    cp = np.concatenate([cp, far])
+    co = np.concatenate([co, [co[-1] + len(far)]])
+    nc = len(co) - 1
+    pairs = np.stack(np.meshgrid(np.arange(6), np.arange(nc), indexing="ij"), -1).reshape(-1, 2)
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+           (qp, np.asarray(qo), cp, np.asarray(co), pairs.astype(np.int32))]
+    for eps in (0.25, 3.0):
+        out = torch.full((len(pairs),), float("nan"), device="cuda")
+        api.dp_pairs(cuda_ctx, "lcss", 0, 0, dev[0].data_ptr(), dev[1].data_ptr(), 390,
+                     dev[2].data_ptr(), dev[3].data_ptr(), 400, dev[4].data_ptr(), len(pairs),
+                     out.data_ptr(), epsilon=eps, delta=delta)
+        torch.cuda.synchronize()
+        want = np.array([oracle.pair("lcss", qp[qo[a]:qo[a + 1]], cp[co[b]:co[b + 1]], eps=eps,
+                                     delta=delta) for a, b in pairs])
+        assert np.array_equal(out.cpu().numpy(), want), eps
+        db = tsim.Database(cuda_ctx, cp, co)
+        ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "lcss", 12, epsilon=eps, delta=delta,
+                             flags=api.FLAG_ALWAYS_PRUNE)
+        wi, wd = oracle.knn("lcss", qp, qo, cp, co, 12, eps=eps, delta=delta)
+        assert np.array_equal(ids, wi) and np.array_equal(d, wd)
+        db.close()
