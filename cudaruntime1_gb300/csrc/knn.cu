@@ -752,11 +752,15 @@ __device__ __forceinline__ bool group_any(bool v) {
   return (__ballot_sync(seg_group_mask(), v) & seg_group_mask()) != 0u;
 }
 
+// hull (LCSS): the first and (<< 8) the last candidate segment that meets its
+// rows' box: columns outside them match nothing.
 // t: the pair's pruning threshold; once the candidate segments' part exceeds
 // it the row segments are not evaluated.  Called by every lane of a group
 // with the same pair; g is the lane within the group.
 template <int MEAS>
-__device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1, float t, int g) {
+__device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1, float t, int g,
+                           int& hull) {
+  hull = (kSegs - 1) << 8;
   if (n > a.max_qlen || n < 1 || m < 1) return lb1;
   const float4* sb = a.csegbox + (size_t)c * kSegs;
   const float4 qb = a.qbox[q];
@@ -793,6 +797,9 @@ __device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1
           b.y <= __fadd_ru(qx.w, e2))
         count = b1 - b0 + 1;
     }
+    const unsigned mk = seg_group_mask();
+    const unsigned meet = (__ballot_sync(mk, count > 0) & mk) >> (__ffs(mk) - 1);
+    hull = meet ? (__ffs(meet) - 1) | ((31 - __clz(meet)) << 8) : (kSegs - 1) << 8;
     count = group_isum(count);
     return fminf(lb1, (float)min(count, min(n, m)));
   }
@@ -889,30 +896,52 @@ __device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1
   return fmaxf(fmaxf(acc, accr), lb1);
 }
 
-// Append the pair to a per-query list, aggregated over a block of kChunk
-// threads (every thread of the block calls it): warp counts through shared
-// memory, one atomic per block.  A query's list has one counter; with an
-// atomic per warp, a 1M-candidate scan queued on it.
-__device__ __forceinline__ void block_append(bool take, int* count, int* list, int value) {
-  __shared__ int wbase[kChunk / 32];
-  __shared__ int bbase;
-  const unsigned ball = __ballot_sync(0xffffffffu, take);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) wbase[warp] = __popc(ball);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int total = 0;
-#pragma unroll
-    for (int w = 0; w < kChunk / 32; ++w) {
-      const int n = wbase[w];
-      wbase[w] = total;
-      total += n;
+// Entries for a per-query list, collected by a warp in shared memory and
+// listed 32 at a time: one atomic on the query's counter and coalesced stores.
+// Lanes with `take` add an entry; the whole warp calls both.
+struct WarpList {
+  int* count;
+  int* list;
+  int* list2;   // a second value per entry, or null
+  int (*buf)[2];  // 64 entries of shared memory, the warp's own
+  int n = 0;
+  __device__ __forceinline__ void add(bool take, int v, int v2) {
+    const int lane = threadIdx.x & 31;
+    const unsigned ball = __ballot_sync(0xffffffffu, take);
+    if (!ball) return;
+    if (take) {
+      const int at = n + __popc(ball & ((1u << lane) - 1));
+      buf[at][0] = v;
+      buf[at][1] = v2;
     }
-    bbase = total ? atomicAdd(count, total) : 0;
+    n += __popc(ball);
+    __syncwarp();
+    if (n < 32) return;
+    store(32);
+    n -= 32;
+    int k = 0, k2 = 0;
+    if (lane < n) k = buf[32 + lane][0], k2 = buf[32 + lane][1];
+    __syncwarp();
+    if (lane < n) buf[lane][0] = k, buf[lane][1] = k2;
+    __syncwarp();
   }
-  __syncthreads();
-  if (take) list[bbase + wbase[warp] + __popc(ball & ((1u << lane) - 1))] = value;
-}
+  __device__ __forceinline__ void flush() {
+    if (n) store(n);
+    n = 0;
+  }
+
+ private:
+  __device__ __forceinline__ void store(int m) {
+    const int lane = threadIdx.x & 31;
+    int pos = 0;
+    if (lane == 0) pos = atomicAdd(count, m);
+    pos = __shfl_sync(0xffffffffu, pos, 0) + lane;
+    if (lane < m) {
+      list[pos] = buf[lane][0];
+      if (list2) list2[pos] = buf[lane][1];
+    }
+  }
+};
 
 // Stage A, first half: the pairs the O(1) bound keeps (seeds excluded) are
 // listed, in list2 (free until the O(length) stage; lock-step Euclidean,
@@ -980,28 +1009,36 @@ __global__ void __launch_bounds__(kChunk) compact_kernel(KArgs a) {
 // the O(1) bound: the O(length) stage and the round-1 order use the tighter
 // of it and their own.
 template <int MEAS>
-__global__ void __launch_bounds__(256) segfilter_kernel(KArgs a) {
+__global__ void __launch_bounds__(256, MEAS == M_DTW ? 5 : 1) segfilter_kernel(KArgs a) {
   const int q = blockIdx.y;
   const int cnt = a.cnt0[q];
   const float t = a.thr[q];
   const int n = a.qlen[q];
   const int g = threadIdx.x & (kSegGroup - 1);
-  const int per_block = blockDim.x / kSegGroup;  // pairs per block and pass
-  const int start = blockIdx.x * per_block;
-  const int stride = gridDim.x * per_block;
-  for (int e0 = start; e0 < cnt; e0 += stride) {  // uniform per block: whole blocks iterate
-    const int e = e0 + (int)threadIdx.x / kSegGroup;
+  __shared__ int buf[256 / 32][64][2];
+  const int warp = threadIdx.x >> 5;
+  constexpr int kPer = 32 / kSegGroup;  // pairs per warp and pass
+  // LCSS: the hull of the columns that can match rides along (in flat_vals,
+  // free until the survivors' round)
+  WarpList out{a.cnt1 + q, a.list1 + (size_t)q * a.C,
+               MEAS == M_LCSS ? reinterpret_cast<int*>(a.flat_vals) + (size_t)q * a.C : nullptr,
+               buf[warp]};
+  const int start = (blockIdx.x * (blockDim.x >> 5) + warp) * kPer;
+  const int stride = gridDim.x * (blockDim.x >> 5) * kPer;
+  for (int e0 = start; e0 < cnt; e0 += stride) {  // uniform per warp
+    const int e = e0 + ((int)threadIdx.x & 31) / kSegGroup;
     bool pass = false;
-    int c = 0;
+    int c = 0, hull = 0;
     if (e < cnt) {  // uniform per group
       c = a.list2[(size_t)q * a.C + e];
       const float b = a.lb1[(size_t)q * a.C + c];
-      const float sbnd = seg_bound<MEAS>(a, q, c, n, a.clen[c], b, t, g);
+      const float sbnd = seg_bound<MEAS>(a, q, c, n, a.clen[c], b, t, g, hull);
       pass = g == 0 && (MEAS == M_LCSS ? (sbnd >= t) : (sbnd <= t));
       if (pass) a.lb1[(size_t)q * a.C + c] = sbnd;
     }
-    block_append(pass, a.cnt1 + q, a.list1 + (size_t)q * a.C, c);
+    out.add(pass, c, hull);
   }
+  out.flush();
 }
 
 // Attempts of a bounded wait on a bulk copy (each may suspend briefly): the
@@ -1009,13 +1046,39 @@ __global__ void __launch_bounds__(256) segfilter_kernel(KArgs a) {
 constexpr uint32_t kWaitLimitDefault = 1u << 22;
 __device__ uint32_t g_wait_limit = kWaitLimitDefault;
 
+// The pairs of query q that pass the O(length) bound, kept a lane each and
+// listed 32 at a time by the whole warp: an atomic and its round trip per pair
+// stop the warp between pairs.
+struct PassList {
+  const KArgs& a;
+  int q;
+  int c = 0, n = 0;
+  float v = 0.0f;
+  __device__ __forceinline__ void add(int cand, float bound) {  // uniform across the warp
+    if ((threadIdx.x & 31) == n) c = cand, v = bound;
+    if (++n == 32) flush();
+  }
+  __device__ __forceinline__ void flush() {
+    if (n == 0) return;
+    const int lane = threadIdx.x & 31;
+    int pos = 0;
+    if (lane == 0) pos = atomicAdd(a.cnt2 + q, n);
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    if (lane < n) {
+      a.list2[(size_t)q * a.C + pos + lane] = c;
+      a.lb2v[(size_t)q * a.C + pos + lane] = v;
+    }
+    n = 0;
+  }
+};
+
 template <int MEAS>
 __device__ __forceinline__ void lb2_body(const KArgs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int q = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int cnt = a.cnt1[q];
-  if (cnt == 0) return;  // uniform across the CTA
+  if (blockIdx.x * kLb2Warps >= cnt) return;  // uniform across the CTA
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
   const float4 qb = a.qbox[q];
@@ -1024,51 +1087,10 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
   // qtable_global_kernel (read through L1: a copy in shared memory per CTA
   // held occupancy to 3 CTAs per SM); a query longer than the table was
   // sized for passes every pair (the bound is skipped, never guessed)
-  constexpr bool kTable = MEAS == M_DTW || MEAS == M_LCSS;
+  constexpr bool kTable = MEAS == M_DTW;
   const bool use_table = n <= a.max_qlen;
   QTable T;
   if (kTable && use_table) T = qtable_view(a.qtab + (size_t)q * a.tstride, n);
-  const float e2 = __fmul_ru(a.eps, 1.0f + 1.0f / 1048576.0f);
-  // LCSS: an occupancy grid of the query in shared memory, cells of side
-  // gs >= 1.01 eps, each query point marking its cell and the 8 around it.
-  // A candidate point within eps (per coordinate) of any query point then
-  // lies in a marked cell: its cell index differs from that query point's
-  // by at most 1 per axis, the index arithmetic's rounding (< 1e-3 cell)
-  // being covered by the 1 % margin.  Points outside the grid match nothing.
-  uint32_t* grid = reinterpret_cast<uint32_t*>(smem_raw);
-  float gx0 = 0.0f, gy0 = 0.0f, ginv = 0.0f;
-  int gnx = 0, gny = 0;
-  if (MEAS == M_LCSS && a.eps > 0.0f) {
-    float gs = __fmul_ru(a.eps, 1.01f);
-    const float W = qb.z - qb.x, H = qb.w - qb.y;
-    while ((W / gs + 3.0f) * (H / gs + 3.0f) > 32.0f * kGridWords) gs *= 1.25f;
-    gnx = (int)(W / gs) + 3;
-    gny = (int)(H / gs) + 3;
-    gx0 = qb.x - gs;
-    gy0 = qb.y - gs;
-    ginv = 1.0f / gs;
-    for (int w = threadIdx.x; w < kGridWords; w += blockDim.x) grid[w] = 0u;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int cx = min(max((int)((A[i].x - gx0) * ginv), 1), gnx - 2);
-      const int cy = min(max((int)((A[i].y - gy0) * ginv), 1), gny - 2);
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int cell = (cy + dy) * gnx + cx + dx;
-          atomicOr(grid + (cell >> 5), 1u << (cell & 31));
-        }
-    }
-    __syncthreads();
-  }
-  // LCSS: the query's window boxes (lcss_env_kernel) in shared memory, next
-  // to the grid: a point's test then reads only its own coordinates from
-  // global memory
-  float4* envs = reinterpret_cast<float4*>(smem_raw + sizeof(uint32_t) * kGridWords);
-  if (MEAS == M_LCSS && a.qenv) {
-    const float4* Eg = a.qenv + (size_t)q * a.env_stride;
-    for (int i = threadIdx.x; i < a.env_stride; i += blockDim.x) envs[i] = Eg[i];
-    __syncthreads();
-  }
   // DTW: a pair's candidate points come by bulk copy into one of the warp's
   // two shared-memory buffers, the next pair's copy in flight while the
   // current one is bounded (the column loop otherwise waits on each point
@@ -1126,6 +1148,7 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
   int m_nx = a.clen[c_nx];
   float s_nx = e + S < cnt ? LB1[c_nx] : 0.0f;
   int slot = 0;
+  PassList pass_list{a, q};
   bool bulk_cur = e < cnt && bulk_ok(o_cur, m_cur);
   if (bulk_cur) issue(0, o_cur, m_cur);
   for (; e < cnt; e += S) {
@@ -1242,7 +1265,7 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
       feasible = __all_sync(0xffffffffu, feasible);
       lbv = feasible ? fmaxf(acc, sbnd) : TSIM_INF;
       pass = lbv <= t;
-    } else if (MEAS == M_FRECHET || MEAS == M_HAUSDORFF) {
+    } else {
       // every point of either trajectory is coupled to (Frechet) or has a
       // nearest point in (Hausdorff) the other, so the squared distance is
       // at least its squared distance to the other's box
@@ -1259,40 +1282,12 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
       for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
       lbv = fmaxf(mx, sbnd);
       pass = lbv <= t;
-    } else {
-      // LCSS: candidate points that can match some query point of their
-      // window (rows [j-delta, j+delta]) inside the eps-inflated box
-      // (the window's inflated box from the query's row boxes; the whole
-      // query's without a window)
-      int count = 0;
-      const float4* E = a.qenv ? envs : nullptr;
-      const float4 qi = make_float4(__fsub_rd(qb.x, e2), __fsub_rd(qb.y, e2), __fadd_ru(qb.z, e2),
-                                    __fadd_ru(qb.w, e2));
-      const int jend = E ? min(m, a.env_stride) : m;  // columns past n-1+delta match nothing
-#pragma unroll 4
-      for (int j = lane; j < jend; j += 32) {
-        const float4 bx = E ? E[j] : qi;
-        const float2 p = B[j];
-        if (p.x >= bx.x && p.x <= bx.z && p.y >= bx.y && p.y <= bx.w) {
-          const float fx = (p.x - gx0) * ginv, fy = (p.y - gy0) * ginv;
-          if (fx >= 0.0f && fy >= 0.0f && fx < (float)gnx && fy < (float)gny) {
-            const int cell = (int)fy * gnx + (int)fx;
-            if ((grid[cell >> 5] >> (cell & 31)) & 1u) ++count;
-          }
-        }
-      }
-      for (int o = 16; o; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
-      lbv = fminf((float)min(count, min(n, m)), sbnd);  // an upper bound on the count
-      pass = lbv >= t;
     }
-    if (pass && lane == 0) {
-      int pos = atomicAdd(a.cnt2 + q, 1);
-      a.list2[(size_t)q * a.C + pos] = c;
-      a.lb2v[(size_t)q * a.C + pos] = lbv;
-    }
+    if (pass) pass_list.add(c, lbv);
     __syncwarp();  // every lane is done with this buffer before it is refilled
     slot ^= 1;
   }
+  pass_list.flush();
   // no copy may be left running into shared memory the next CTA gets
   drain(0);
   drain(1);
@@ -1310,6 +1305,125 @@ __global__ void __launch_bounds__(kLb2Warps * 32) lb2_kernel(KArgs a) {
 // compiler's choice (LCSS spilled in its point loop under the same bound).
 __global__ void __launch_bounds__(kLb2Warps * 32, 5) lb2_dtw_kernel(KArgs a) {
   lb2_body<M_DTW>(a);
+}
+
+// LCSS: an upper bound of a pair's count, the candidate points that can match
+// some query point of their window: inside the eps-inflated box of the
+// window's rows (lcss_env_kernel; the whole query's without a window), and in a
+// marked cell of the query's occupancy grid.  The grid, in shared memory, has
+// cells of side gs >= 1.01 eps, each query point marking its cell and the 8
+// around it.  A candidate point within eps (per coordinate) of any query point
+// then lies in a marked cell: its cell index differs from that query point's
+// by at most 1 per axis, the index arithmetic's rounding (< 1e-3 cell) being
+// covered by the 1 % margin.  Points off the grid count as on its border.
+//
+// What bounds it: the latency of the points, which come from L2 and HBM, and
+// issue; so only the columns of the hull that the segment bound found are read,
+// 64 at a time, the grid is looked up where some lane's point passes its box,
+// and 32 registers leave 64 warps an SM (at 40, 1,197 us; forms that loaded ahead in registers
+// ran 1,606 and 1,790 us, with 1,135 and 848 M instructions).  A CTA takes tiles
+// of kLcssTile pairs, so that a query with few pairs builds few grids: with
+// every query's pairs dealt over 19 CTAs the longest lists set the end.  2.17 M
+// pairs of 256 queries: 1,893 -> 1,053 us, 560 M instructions.
+constexpr int kLcssTile = 512;
+__global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
+  __shared__ uint32_t grid[kGridWords];
+  __shared__ int buf[kLb2Warps][64][2];
+  const int q = blockIdx.y;
+  const int cnt = a.cnt1[q];
+  if ((long long)blockIdx.x * kLcssTile >= cnt) return;  // uniform across the CTA
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float2* A = a.qpts + a.qoff[q];
+  const int n = a.qlen[q];
+  const float4 qb = a.qbox[q];
+  const float t = a.thr[q];
+  const float e2 = __fmul_ru(a.eps, 1.0f + 1.0f / 1048576.0f);
+  const bool skip = n > a.max_qlen;  // longer than its tables were sized for: every pair passes
+  for (int w = threadIdx.x; w < kGridWords; w += blockDim.x) grid[w] = 0u;
+  float gx0 = 0.0f, gy0 = 0.0f, ginv = 0.0f;
+  int gnx = 1, gny = 1;
+  __syncthreads();
+  if (a.eps > 0.0f) {
+    float gs = __fmul_ru(a.eps, 1.01f);
+    const float W = qb.z - qb.x, H = qb.w - qb.y;
+    while ((W / gs + 3.0f) * (H / gs + 3.0f) > 32.0f * kGridWords) gs *= 1.25f;
+    gnx = (int)(W / gs) + 3;
+    gny = (int)(H / gs) + 3;
+    gx0 = qb.x - gs;
+    gy0 = qb.y - gs;
+    ginv = 1.0f / gs;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const int cx = min(max((int)((A[i].x - gx0) * ginv), 1), gnx - 2);
+      const int cy = min(max((int)((A[i].y - gy0) * ginv), 1), gny - 2);
+      for (int dy = -1; dy <= 1; ++dy)
+        for (int dx = -1; dx <= 1; ++dx) {
+          const int cell = (cy + dy) * gnx + cx + dx;
+          atomicOr(grid + (cell >> 5), 1u << (cell & 31));
+        }
+    }
+    __syncthreads();
+  }
+  const float4* E = a.qenv ? a.qenv + (size_t)q * a.env_stride : nullptr;
+  const float4 qi = make_float4(__fsub_rd(qb.x, e2), __fsub_rd(qb.y, e2), __fadd_ru(qb.z, e2),
+                                __fadd_ru(qb.w, e2));
+  const int* L1 = a.list1 + (size_t)q * a.C;
+  const int* H1 = reinterpret_cast<const int*>(a.flat_vals) + (size_t)q * a.C;  // hulls
+  WarpList out{a.cnt2 + q, a.list2 + (size_t)q * a.C,
+               reinterpret_cast<int*>(a.lb2v) + (size_t)q * a.C, buf[warp]};
+  const float gxm = (float)(gnx - 1), gym = (float)(gny - 1);
+  for (long long tile = (long long)blockIdx.x * kLcssTile; tile < cnt;
+       tile += (long long)gridDim.x * kLcssTile) {
+    const int end = (int)min((long long)cnt, tile + kLcssTile);
+    int c_nx = (int)tile + warp < end ? L1[(int)tile + warp] : 0;
+    for (int e = (int)tile + warp; e < end; e += kLb2Warps) {
+      const int c = c_nx;
+      if (e + kLb2Warps < end) c_nx = L1[e + kLb2Warps];
+      const int h = H1[e], m = a.clen[c];
+      const float2* B = a.cpts + a.coff[c];
+      const float sbnd = a.lb1[(size_t)q * a.C + c];
+      // the hull's columns [jb, je); past n-1+delta they match nothing
+      const int jb = seg_first(h & 255, m);
+      int je = seg_first((h >> 8) + 1, m);
+      if (E) je = min(je, a.env_stride);
+      int count = 0;
+#pragma unroll 1
+      for (int j = jb + lane; j - lane < je; j += 64) {
+        float2 p[2];
+        bool in[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          in[u] = j + 32 * u < je;
+          p[u] = in[u] ? __ldg(B + j + 32 * u) : make_float2(0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (in[u]) {
+            const float4 bx = E ? __ldg(E + j + 32 * u) : qi;
+            in[u] = p[u].x >= bx.x && p[u].x <= bx.z && p[u].y >= bx.y && p[u].y <= bx.w;
+          }
+          if (__any_sync(0xffffffffu, in[u])) {
+            // floor by a rounding addition of 2^23 (to a cell below at worst
+            // where the value is whole: within the marks' reach)
+            const float fx = fminf(fmaxf((p[u].x - gx0) * ginv, 0.0f), gxm);
+            const float fy = fminf(fmaxf((p[u].y - gy0) * ginv, 0.0f), gym);
+            const int cx = max(__float_as_int(fx + 8388607.5f) - 0x4b000000, 0);
+            const int cy = max(__float_as_int(fy + 8388607.5f) - 0x4b000000, 0);
+            const int cell = cy * gnx + cx;
+            if (in[u]) count += (grid[cell >> 5] >> (cell & 31)) & 1u;
+          }
+        }
+      }
+      count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
+      bool pass = n > 0 && m > 0;
+      float lbv = sbnd;
+      if (pass && !skip) {
+        lbv = fminf((float)min(count, min(n, m)), sbnd);  // an upper bound on the count
+        pass = lbv >= t;
+      }
+      if (pass) out.add(lane == 0, c, __float_as_int(lbv));
+    }
+  }
+  out.flush();
 }
 
 // Round 1: the M best survivors of each query by their O(length) bound
@@ -2110,19 +2224,18 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   if constexpr (MEAS != M_EUCLID) {
     segfilter_kernel<MEAS><<<dim3(std::max(1, std::min(1024, (32 * ctx->num_sms + nq - 1) / nq)), nq),
                              256, 0, s>>>(a);
-    // LCSS: the query's grid and window boxes per CTA, and 4x the CTAs per
-    // query (its queries' pair counts vary widely; a CTA's set-up is small)
-    const size_t lb2_smem =
-        MEAS == M_LCSS   ? sizeof(uint32_t) * kGridWords + sizeof(float4) * (size_t)a.env_stride
-        : MEAS == M_DTW ? sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2)
-                         : 0;
-    const int ch2 = MEAS == M_LCSS ? std::max(1, std::min(65535, (32 * ctx->num_sms + nq - 1) / nq))
-                                   : ch;
-    auto lb2 = MEAS == M_DTW ? lb2_dtw_kernel : lb2_kernel<MEAS>;
-    if (lb2_smem > 48 * 1024)
-      TSIM_CUDA(cudaFuncSetAttribute(lb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)lb2_smem));
-    lb2<<<dim3(ch2, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
+    if constexpr (MEAS == M_LCSS) {
+      const int tiles = (a.C + kLcssTile - 1) / kLcssTile;
+      lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(a);
+    } else {
+      const size_t lb2_smem =
+          MEAS == M_DTW ? sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2) : 0;
+      auto lb2 = MEAS == M_DTW ? lb2_dtw_kernel : lb2_kernel<MEAS>;
+      if (lb2_smem > 48 * 1024)
+        TSIM_CUDA(cudaFuncSetAttribute(lb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)lb2_smem));
+      lb2<<<dim3(ch, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
+    }
     launched(ctx, 2);
   }
   seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.M);
