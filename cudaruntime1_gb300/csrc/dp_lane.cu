@@ -371,9 +371,15 @@ bool lane_kind(int kind) {
 // database ran its 150 K survivors on lanes in 14.2 ms, on warps in 9.8 ms.
 // DTW and Frechet only: their warp rounds run on the band-relative kernel;
 // LCSS's run on the row-group kernel, whose rate the lanes keep beating.
-int lane_gate_for(int kind, int max_n, int max_m, int band_pct, int delta, int num_sms) {
+// abandon = false: rounds that compute every cell (tsim_dp_pairs): a lane per
+// pair from where the band-relative kernel (500 cells per ns then) needs as
+// long as the lanes' longest pair: 64 queries of 64 to 512 points, band 10 %,
+// against 128 / 256 / 512 / 2,048 candidates: 317 / 547 / 997 / 3,605 us on warps,
+// 527 / 544 / 626 / 1,425 on lanes, and the rule's line at 20,500 pairs (320).
+int lane_gate_for(int kind, int max_n, int max_m, int band_pct, int delta, int num_sms,
+                  bool abandon) {
   constexpr double kLaneStepNs = 70.0, kWarpCellsPerNs = 435.0;  // 435 GCUPS
-  constexpr double kLaneSatCellsPerNs = 1377.0, kWaveCellsPerNs = 700.0;
+  constexpr double kLaneSatCellsPerNs = 1377.0, kWaveCellsPerNs = 700.0, kWaveAllCellsPerNs = 550.0;
   auto cells = [&](int n, int m) {
     const int no = std::max(n, m), ni = std::min(n, m);
     const int wd = kind == DP_LCSS ? delta : (kind == DP_FRECHET_SQ ? -1 : band_w(n, m, band_pct));
@@ -386,6 +392,7 @@ int lane_gate_for(int kind, int max_n, int max_m, int band_pct, int delta, int n
   const double width = cells(max_n, max_m) / no;
   const double latency_ns = std::ceil(no / (double)kLaneR) * (width + kLaneR) * kLaneStepNs;
   const double typical = cells(std::max(2, max_n / 2), std::max(2, max_m / 2));
+  if (!abandon) return (int)std::min(latency_ns * kWaveAllCellsPerNs / typical, 1e9);
   const double gate = 2.0 * latency_ns * kWarpCellsPerNs / typical;
   const double lanes = 3.0 * kLaneThreads * std::max(1, num_sms);  // 3 CTAs per SM
   const double longest_ns = cells(max_n, max_m) / (kLaneSatCellsPerNs / lanes);

@@ -2977,6 +2977,19 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
     d.npairs_dev = nspill;
     return launch_dp(ctx, kind, G, R, d, max_clen);
   }
+  if (kernel == 0 && precision == 0) {
+    // banded FP32 pairs: a lane per pair once they are many, else the
+    // band-relative kernel (64 x 2,048 DTW pairs of 64 to 512 points, band
+    // 10 %: 4.87 ms on row groups, 1.42 on lanes; 64 x 64 of them: 246 us on
+    // row groups, 217 band-relative)
+    const int gate = lane_kind(kind) ? lane_gate_for(kind, max_qlen, max_clen, d.band_pct, d.delta,
+                                                     ctx->num_sms, false)
+                                     : 0;
+    if (gate > 0 && npairs >= gate)
+      kernel = 5;
+    else if (wave_kind(kind))
+      kernel = 6;
+  }
   if (kernel == 6 && wave_kind(kind)) {  // band-relative first; wider pairs on the others
     TSIM_TRY(launch_dp_wave(ctx, kind, d, max_qlen, max_clen, npairs <= 4 * ctx->num_sms, rest, nrest));
     d.order = rest;

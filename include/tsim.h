@@ -325,7 +325,9 @@ TSIM_API int tsim_server_destroy(tsim_server* s);
 /* Values of given (query, candidate) pairs -- d_pairs[2*i] = query index,
  * d_pairs[2*i+1] = candidate index -- for DTW, LCSS or Frechet under p's
  * band / window / cost.  precision: 0 = FP32 (d_out32), 1 = compensated FP32
- * (d_out64), 2 = FP64 (d_out64).  kernel: 0 = automatic, 1 = round-striped
+ * (d_out64), 2 = FP64 (d_out64).  kernel: 0 = automatic (strips for full rows,
+ * bit vectors for LCSS windows of at most 63 rows, lanes or band-relative for
+ * bands by the number of pairs), 1 = round-striped
  * DP, 2 = anti-diagonal DP with a warp per pair, 3 = with a CTA of 8 warps
  * per pair, 4 = with 2 warps per pair (pairs they cannot take fall back to 1),
  * 5 = a lane per pair (FP32 DTW, Frechet and LCSS, the throughput form for
