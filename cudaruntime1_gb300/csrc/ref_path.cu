@@ -7,9 +7,9 @@
 // pair list in again, refines on the GPU and reduces on the host.
 //
 // Here everything after the H2D copy of the trajectories stays on the device:
-//   1. ref_filter_kernel: one CTA per query builds the envelope in shared
-//      memory, evaluates the bound of every candidate (summed in the same
-//      order as the reference CPU code, so values are bit-identical), and
+//   1. ref_filter_kernel: a CTA per one or two queries builds the envelopes
+//      in shared memory, evaluates the bound of every candidate (summed in the
+//      same order as the reference CPU code, so values are bit-identical), and
 //      selects the K best by (bound, index) without materialising the matrix;
 //   2. the strip DP kernel (dp_strip.cu; LCSS: dp_kernels.cu) refines the
 //      num_t*K pairs;
@@ -29,23 +29,63 @@ constexpr size_t kRefSmemCap = 200 * 1024;
 __device__ __forceinline__ float smax(float a, float b) { return (a < b) ? b : a; }
 __device__ __forceinline__ float smin(float a, float b) { return (b < a) ? b : a; }
 
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+union F2 {
+  float2 f;
+  unsigned long long u;
+};
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  F2 x{a}, y{b}, r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(x.u), "l"(y.u));
+  return r.f;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  F2 x{a}, y{b}, r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(x.u), "l"(y.u));
+  return r.f;
+}
+
 // kind: 0 = DTW (sum of envelope distances), 1 = LCSS (eps-box count,
 // descending), 2 = Frechet (max of envelope distances).
-template <int KIND>
+//
+// A CTA takes TQ queries, a thread one candidate at a time for all of them,
+// its points in order (the sums are the reference's, bit for bit).  256
+// candidates' points pass through shared memory kRefCols at a time: read
+// straight from global memory, each lane walks its own row, every load of a
+// warp touches 32 lines and the rows of a CTA do not stay in L1, which set the
+// kernel's time (1,024 x 1,024 x 128 points, DTW: 488 us; now 168, bound by
+// issue: about 17 instructions a point and query, half of them the square
+// root).  Two queries a CTA share the staging where that leaves at least two
+// CTAs per SM.
+//
+// The distances to the envelope, max(0, lo - p, p - hi), take one three-way
+// maximum, equal to the reference's comparisons for every input: a NaN on
+// either side leaves 0 in both.
+constexpr int kRefCols = 8;
+constexpr int kRefStride = kFilterThreads + 2;  // 4 banks from one column to the next
+constexpr size_t kRefTileBytes = sizeof(float2) * kRefCols * kRefStride;
+
+template <int KIND, int TQ>
 __global__ void __launch_bounds__(kFilterThreads)
     ref_filter_kernel(const float2* __restrict__ t1, const float2* __restrict__ t2, int num_t,
                       int n, int m, float eps, int K, unsigned long long* __restrict__ gkeys,
                       int2* __restrict__ pairs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ SelScratch red;
-  const int q = blockIdx.x;
-  // envelope of query point v*n/m for each candidate position v, m entries
-  float4* envv = reinterpret_cast<float4*>(smem_raw);
-  unsigned long long* keys =
-      gkeys ? gkeys + (size_t)q * num_t : reinterpret_cast<unsigned long long*>(envv + m);
-  const float2* A = t1 + (size_t)q * n;
+  const int q0 = blockIdx.x * TQ;
+  // envelope of query point v*n/m for each candidate position v, as (min_x,
+  // min_y, max_x, max_y); LCSS: inflated by eps
+  float4* envv = reinterpret_cast<float4*>(smem_raw);  // [TQ][m]
+  float2* tile = reinterpret_cast<float2*>(envv + (size_t)TQ * m);
+  unsigned long long* skeys = reinterpret_cast<unsigned long long*>(tile + kRefCols * kRefStride);
   const int r = 5;
-  for (int v = threadIdx.x; v < m; v += blockDim.x) {
+  for (int x = threadIdx.x; x < TQ * m; x += blockDim.x) {
+    const int q = min(q0 + x / m, num_t - 1), v = x % m;
+    const float2* A = t1 + (size_t)q * n;
     const int i = (int)(((long long)v * n) / m);
     float min_x = kRefBig, max_x = -kRefBig, min_y = kRefBig, max_y = -kRefBig;
     const int s = max(0, i - r), e = min(n - 1, i + r);
@@ -56,42 +96,86 @@ __global__ void __launch_bounds__(kFilterThreads)
       min_y = smin(min_y, p.y);
       max_y = smax(max_y, p.y);
     }
-    envv[v] = make_float4(min_x, max_x, min_y, max_y);
-  }
-  __syncthreads();
-  const int min_len = min(n, m);
-  for (int j = threadIdx.x; j < num_t; j += blockDim.x) {
-    const float2* C = t2 + (size_t)j * m;
-    float key;
     if (KIND == 1) {
-      int cnt = 0;
-      for (int v = 0; v < m; ++v) {
-        const float4 e = envv[v];
-        const float2 p = __ldg(C + v);
-        if (p.x > __fsub_rn(e.x, eps) && p.x < __fadd_rn(e.y, eps) && p.y > __fsub_rn(e.z, eps) &&
-            p.y < __fadd_rn(e.w, eps))
-          cnt++;
-      }
-      key = -__fdiv_rn((float)cnt, (float)min_len);  // descending ub -> ascending key
-    } else {
-      float acc = 0.0f;
-      for (int v = 0; v < m; ++v) {
-        const float4 e = envv[v];
-        const float2 p = __ldg(C + v);
-        float dx = smax(0.0f, smax(__fsub_rn(e.x, p.x), __fsub_rn(p.x, e.y)));
-        float dy = smax(0.0f, smax(__fsub_rn(e.z, p.y), __fsub_rn(p.y, e.w)));
-        float d = __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
-        acc = (KIND == 0) ? __fadd_rn(acc, d) : smax(acc, d);
-      }
-      key = acc;
+      min_x = __fsub_rn(min_x, eps);
+      min_y = __fsub_rn(min_y, eps);
+      max_x = __fadd_rn(max_x, eps);
+      max_y = __fadd_rn(max_y, eps);
     }
-    keys[j] = pack_key(key, j);
+    envv[x] = make_float4(min_x, min_y, max_x, max_y);
+  }
+  const int min_len = min(n, m);
+  auto point = [&](const float4 e, const float2 p, float& acc) {
+    if (KIND == 1) {
+      if (p.x > e.x && p.x < e.z && p.y > e.y && p.y < e.w) acc += 1.0f;  // exact: below 2^24
+    } else {
+      const float2 lo = sub2(make_float2(e.x, e.y), p), hi = sub2(p, make_float2(e.z, e.w));
+      const float2 d = make_float2(max3f(lo.x, hi.x, 0.0f), max3f(lo.y, hi.y, 0.0f));
+      const float2 dd = mul2(d, d);
+      const float dist = __fsqrt_rn(__fadd_rn(dd.x, dd.y));
+      acc = KIND == 0 ? __fadd_rn(acc, dist) : fmaxf(acc, dist);
+    }
+  };
+  for (int c0 = 0; c0 < num_t; c0 += kFilterThreads) {
+    float2 pre[kRefCols];  // the next columns, in flight while these are used
+    auto fetch = [&](int v0) {
+#pragma unroll
+      for (int i = 0; i < kRefCols; ++i) {
+        const int x = i * kFilterThreads + threadIdx.x;
+        const int j = c0 + x / kRefCols, v = v0 + x % kRefCols;
+        if (j < num_t && v < m) pre[i] = __ldg(t2 + (size_t)j * m + v);
+      }
+    };
+    float acc[TQ];
+#pragma unroll
+    for (int t = 0; t < TQ; ++t) acc[t] = 0.0f;
+    fetch(0);
+    for (int v0 = 0; v0 < m; v0 += kRefCols) {
+      __syncthreads();  // the last columns are used (the first time: the envelopes are written)
+#pragma unroll
+      for (int i = 0; i < kRefCols; ++i) {
+        const int x = i * kFilterThreads + threadIdx.x;
+        tile[(x % kRefCols) * kRefStride + x / kRefCols] = pre[i];
+      }
+      __syncthreads();
+      if (v0 + kRefCols < m) fetch(v0 + kRefCols);
+      if (v0 + kRefCols <= m) {
+#pragma unroll
+        for (int u = 0; u < kRefCols; ++u) {
+          const float2 p = tile[u * kRefStride + threadIdx.x];
+#pragma unroll
+          for (int t = 0; t < TQ; ++t) point(envv[t * m + v0 + u], p, acc[t]);
+        }
+      } else {
+        for (int u = 0; v0 + u < m; ++u) {
+          const float2 p = tile[u * kRefStride + threadIdx.x];
+#pragma unroll
+          for (int t = 0; t < TQ; ++t) point(envv[t * m + v0 + u], p, acc[t]);
+        }
+      }
+    }
+    const int j = c0 + threadIdx.x;
+    if (j < num_t) {
+#pragma unroll
+      for (int t = 0; t < TQ; ++t) {
+        if (q0 + t >= num_t) break;
+        unsigned long long* keys = gkeys ? gkeys + (size_t)(q0 + t) * num_t : skeys + (size_t)t * num_t;
+        // LCSS: descending ub -> ascending key
+        keys[j] = pack_key(KIND == 1 ? -__fdiv_rn(acc[t], (float)min_len) : acc[t], j);
+      }
+    }
   }
   __syncthreads();
   __shared__ unsigned long long sel[64];
-  block_select_k(keys, num_t, K, sel, red);
-  for (int k = threadIdx.x; k < K; k += blockDim.x)
-    pairs[(size_t)q * K + k] = make_int2(q, key_index(sel[k]));
+#pragma unroll 1
+  for (int t = 0; t < TQ && q0 + t < num_t; ++t) {
+    const unsigned long long* keys =
+        gkeys ? gkeys + (size_t)(q0 + t) * num_t : skeys + (size_t)t * num_t;
+    block_select_k(keys, num_t, K, sel, red);
+    for (int k = threadIdx.x; k < K; k += blockDim.x)
+      pairs[(size_t)(q0 + t) * K + k] = make_int2(q0 + t, key_index(sel[k]));
+    __syncthreads();
+  }
 }
 
 // kind 0/2: min of refined distances; 1: max of count / min(n, m).
@@ -118,9 +202,12 @@ __global__ void ref_reduce_kernel(const float* __restrict__ vals, int num_t, int
   }
 }
 
-__global__ void fixed_offsets_kernel(int64_t* off, int count, int len) {
+__global__ void fixed_offsets_kernel(int64_t* off1, int len1, int64_t* off2, int len2, int count) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i <= count) off[i] = (int64_t)i * len;
+  if (i <= count) {
+    off1[i] = (int64_t)i * len1;
+    off2[i] = (int64_t)i * len2;
+  }
 }
 
 }  // namespace
@@ -159,31 +246,33 @@ int ref_batch_core(tsim_ctx* ctx, int measure, const float2* d_t1, const float2*
       keys_in_smem ? nullptr : reinterpret_cast<unsigned long long*>(take(key_bytes * num_t));
 
   stage_begin(ctx, TSIM_STAGE_REF);
-  const size_t smem = env_bytes + (keys_in_smem ? key_bytes : 0);
+  // two queries a CTA where two CTAs per SM are left and their keys fit
+  const size_t one = env_bytes + (keys_in_smem ? key_bytes : 0);
+  const int tq = num_t >= 4 * ctx->num_sms && 2 * one + kRefTileBytes <= 100 * 1024 ? 2 : 1;
+  const size_t smem = tq * one + kRefTileBytes;
   auto launch_filter = [&](auto kern) -> int {
     if (smem > 48 * 1024)
       TSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<num_t, kFilterThreads, smem, ctx->stream>>>(d_t1, d_t2, num_t, n, m, eps, K, gkeys,
-                                                        pairs);
+    kern<<<(num_t + tq - 1) / tq, kFilterThreads, smem, ctx->stream>>>(d_t1, d_t2, num_t, n, m, eps,
+                                                                       K, gkeys, pairs);
     TSIM_CUDA(cudaGetLastError());
     launched(ctx);
     return TSIM_OK;
   };
   int kind;
   if (measure == TSIM_DTW) {
-    TSIM_TRY(launch_filter(ref_filter_kernel<0>));
+    TSIM_TRY(tq == 2 ? launch_filter(ref_filter_kernel<0, 2>) : launch_filter(ref_filter_kernel<0, 1>));
     kind = DP_DTW_REF;
   } else if (measure == TSIM_LCSS) {
-    TSIM_TRY(launch_filter(ref_filter_kernel<1>));
+    TSIM_TRY(tq == 2 ? launch_filter(ref_filter_kernel<1, 2>) : launch_filter(ref_filter_kernel<1, 1>));
     kind = DP_LCSS;
   } else {
-    TSIM_TRY(launch_filter(ref_filter_kernel<2>));
+    TSIM_TRY(tq == 2 ? launch_filter(ref_filter_kernel<2, 2>) : launch_filter(ref_filter_kernel<2, 1>));
     kind = DP_FRECHET_REF;
   }
-  fixed_offsets_kernel<<<(num_t + 256) / 256, 256, 0, ctx->stream>>>(qoff, num_t, n);
-  fixed_offsets_kernel<<<(num_t + 256) / 256, 256, 0, ctx->stream>>>(coff, num_t, m);
+  fixed_offsets_kernel<<<(num_t + 256) / 256, 256, 0, ctx->stream>>>(qoff, n, coff, m, num_t);
   TSIM_CUDA(cudaGetLastError());
-  launched(ctx, 2);
+  launched(ctx);
 
   DpArgs a{};
   a.qpts = d_t1;
