@@ -2,31 +2,11 @@
 // kernels (dp_kernels.cu: round-striped; dp_diag.cu: anti-diagonal).
 #pragma once
 #include "dfloat.cuh"
+#include "f32x2.cuh"
 #include "tsim_internal.cuh"
 
 namespace tsim {
 namespace dp {
-
-// min of three floats in one instruction (the three-operand PTX min.f32 of
-// sm_100+; exact, like two fminf, for the non-NaN values of a DP)
-__device__ __forceinline__ float min3f(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-
-// q - c per coordinate in one packed instruction (sub.rn.f32x2, sm_100 and
-// later): two round-to-nearest subtractions, the bits of two scalar ones
-__device__ __forceinline__ float2 sub2(float2 q, float2 c) {
-  union {
-    float2 f;
-    unsigned long long u;
-  } a, b, r;
-  a.f = q;
-  b.f = c;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(a.u), "l"(b.u));
-  return r.f;
-}
 
 // Minimum of three normalised pairs.  A normalised pair's hi is its value
 // rounded to nearest, so pairs with different hi order as their hi parts;

@@ -16,6 +16,7 @@
 //   3. ref_reduce_kernel keeps the best refined value per query.
 // Outputs equal the reference's CPU functions (dtw.cpp:14-113,
 // lcss.cpp:13-115, frechet.cpp:13-124) bit for bit.
+#include "f32x2.cuh"
 #include "topk.cuh"
 #include "tsim_internal.cuh"
 
@@ -28,26 +29,6 @@ constexpr size_t kRefSmemCap = 200 * 1024;
 
 __device__ __forceinline__ float smax(float a, float b) { return (a < b) ? b : a; }
 __device__ __forceinline__ float smin(float a, float b) { return (b < a) ? b : a; }
-
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-union F2 {
-  float2 f;
-  unsigned long long u;
-};
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-  F2 x{a}, y{b}, r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(x.u), "l"(y.u));
-  return r.f;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  F2 x{a}, y{b}, r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(x.u), "l"(y.u));
-  return r.f;
-}
 
 // kind: 0 = DTW (sum of envelope distances), 1 = LCSS (eps-box count,
 // descending), 2 = Frechet (max of envelope distances).

@@ -433,3 +433,20 @@ def test_euclidean_segment_means(tsim, cuda_ctx, oracle, nc, k, offset):
     assert np.array_equal(ids, want_ids)
     assert np.array_equal(ids, ids2) and np.array_equal(d, d2) and np.array_equal(d64, d642)
     db.close()
+
+
+@pytest.mark.parametrize("pruned", [False, True])
+def test_hausdorff_point_counts(tsim, cuda_ctx, oracle, pruned):
+    """Sides around the kernel's points per lane, its sample's smallest side
+    and the targets staged at a time: the oracle's ids and distances."""
+    sizes = [1, 2, 31, 32, 33, 63, 64, 65, 127, 130, 255, 257, 300, 511, 512, 513, 515, 1030]
+    cp, co = G.random_walks(3 * len(sizes), sizes * 3, 51, start_range=30.0)
+    qp, qo = G.random_walks(6, [1, 33, 64, 161, 513, 1100], 52, start_range=30.0)
+    db = tsim.Database(cuda_ctx, cp, co)
+    flags = tsim.api.FLAG_ALWAYS_PRUNE if pruned else tsim.api.FLAG_NO_PRUNE
+    ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "hausdorff", 7, flags=flags)
+    want_ids, want = oracle.knn("hausdorff", qp, qo, cp, co, 7)
+    assert np.array_equal(ids, want_ids)
+    # one rounded squared distance (8 2^-24), its root and the result's rounding
+    assert np.all(np.abs(d - want) <= 8 * 2.0 ** -24 * want)
+    db.close()
