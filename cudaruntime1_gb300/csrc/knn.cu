@@ -197,22 +197,20 @@ __device__ __forceinline__ float widen(float t, double g) {
 // the candidate, whose points lie in its box, so a block costs at least its
 // box's distance to the candidate's box per row; LCSS: a row can only match
 // when its block's eps-inflated box meets the candidate's box.
+// qblk: the query's block boxes; rows: their row counts (0: a block without
+// rows, whose box is everything).
 template <int MEAS>
-__device__ __forceinline__ float block_bound(const KArgs& a, const float4* qblk, int n, float4 cb,
-                                             int m) {
+__device__ __forceinline__ float block_bound(const KArgs& a, const float4* qblk, const float* rows,
+                                             float4 cb) {
   float acc = 0.0f;
-  int cnt = 0;
   const float e2 = __fmul_ru(a.eps, 1.0f + 1.0f / 1048576.0f);
 #pragma unroll
   for (int b = 0; b < kQBlocks; ++b) {
-    const int r0 = (int)((long long)b * n / kQBlocks);
-    const int r1 = (int)((long long)(b + 1) * n / kQBlocks);
-    if (r1 <= r0) continue;
     const float4 bx = qblk[b];
     if (MEAS == M_LCSS) {
       if (cb.z >= __fsub_rd(bx.x, e2) && cb.x <= __fadd_ru(bx.z, e2) &&
           cb.w >= __fsub_rd(bx.y, e2) && cb.y <= __fadd_ru(bx.w, e2))
-        cnt += r1 - r0;
+        acc += rows[b];
       continue;
     }
     const float d = box_box_d2_rd(bx, cb);
@@ -220,10 +218,10 @@ __device__ __forceinline__ float block_bound(const KArgs& a, const float4* qblk,
       acc = fmaxf(acc, d);
     } else {
       const float c = (MEAS == M_DTW && a.cost) ? __fsqrt_rd(d) : d;
-      acc = __fadd_rd(acc, __fmul_rd((float)(r1 - r0), c));
+      acc = __fmaf_rd(rows[b], c, acc);
     }
   }
-  return MEAS == M_LCSS ? (float)cnt : acc;
+  return acc;
 }
 
 // one warp per query: lane b < kQBlocks reduces block b's box
@@ -260,8 +258,8 @@ __device__ __forceinline__ float bound1(const KArgs& a, float4 qb, float4 qe, in
   if (MEAS == M_HAUSDORFF) {
     // the extreme point of either set along an axis is at least the
     // difference of the two boxes' edges away from every point of the other
-    const float e = fmaxf(fmaxf(absdiff_rd(qb.x, cb.x), absdiff_rd(qb.z, cb.z)),
-                          fmaxf(absdiff_rd(qb.y, cb.y), absdiff_rd(qb.w, cb.w)));
+    const float e = max3f(fmaxf(absdiff_rd(qb.x, cb.x), absdiff_rd(qb.z, cb.z)),
+                          absdiff_rd(qb.y, cb.y), absdiff_rd(qb.w, cb.w));
     return __fmul_rd(e, e);
   }
   const float first = pd2_rd(qe.x, qe.y, ce.x, ce.y);
@@ -298,37 +296,95 @@ __device__ __forceinline__ bool ends_align(int n, int m, int delta) {
   return delta < 0 || abs(n - m) <= delta;
 }
 
+// A chunk's best candidate for each of Q queries (ties: the lowest index)
+template <int Q>
+struct ChunkBest {
+  unsigned ord[Q][kChunk / 32];
+  int cand[Q][kChunk / 32];
+  // the warp's smallest key (~0: none), one lane's candidate each
+  __device__ __forceinline__ void warp_best(int i, unsigned key, int chunk) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned mn = __reduce_min_sync(0xffffffffu, key);
+    const unsigned who = __ballot_sync(0xffffffffu, key == mn);
+    if (lane == 0) {
+      ord[i][warp] = mn;
+      cand[i][warp] = mn == 0xffffffffu ? -1 : chunk * kChunk + warp * 32 + __ffs(who) - 1;
+    }
+  }
+  // after the last query, by the whole block
+  __device__ __forceinline__ void store(const KArgs& a, int q0, int q1, int chunk) {
+    __syncthreads();
+    const int i = threadIdx.x, q = q0 + i;
+    if (i < Q && q < q1) {
+      int w0 = 0;
+      for (int w = 1; w < kChunk / 32; ++w)
+        if (ord[i][w] < ord[i][w0]) w0 = w;
+      a.chunk_cand[(size_t)q * a.nch + chunk] = cand[i][w0];
+    }
+  }
+};
+
+// A thread per candidate, its summary in registers, looped over kLb1Queries
+// queries whose block boxes are in shared memory; 256 candidates a CTA, whose T
+// best are kept as seed candidates: one by a warp reduction per query, more by
+// a block selection.  Bound by issue, 185 to 205 instructions a pair: with a CTA
+// per query and chunk, loads, comparisons, selection and barriers came to 450 to
+// 510 (16.7 M pairs: Hausdorff 247 -> 95 us, Frechet 262 -> 108).
+constexpr int kLb1Queries = 8;
 template <int MEAS>
 __global__ void __launch_bounds__(kChunk) lb1_kernel(KArgs a) {
   __shared__ unsigned long long keys[kChunk];
   __shared__ SelScratch red;
   __shared__ unsigned long long sel[64];
-  const int q = blockIdx.y, chunk = blockIdx.x;
+  __shared__ float4 qblk[kLb1Queries][kQBlocks];
+  __shared__ float rows[kLb1Queries][kQBlocks];
+  __shared__ ChunkBest<kLb1Queries> best;
+  const int chunk = blockIdx.x;
   const int c = chunk * kChunk + threadIdx.x;
-  __shared__ float4 qblk[kQBlocks];
-  const float4 qb = a.qbox[q], qe = a.qends[q];
-  const int n = a.qlen[q];
-  if (threadIdx.x < kQBlocks) qblk[threadIdx.x] = a.qblk[(size_t)q * kQBlocks + threadIdx.x];
+  const int q0 = blockIdx.y * kLb1Queries, q1 = min(a.nq, q0 + kLb1Queries);
+  if (threadIdx.x < kLb1Queries * kQBlocks) {
+    const int i = threadIdx.x / kQBlocks, b = threadIdx.x % kQBlocks;
+    if (q0 + i < q1) {
+      const int n = a.qlen[q0 + i];
+      const int r = (int)((long long)(b + 1) * n / kQBlocks) - (int)((long long)b * n / kQBlocks);
+      rows[i][b] = (float)r;
+      qblk[i][b] = r > 0 ? a.qblk[(size_t)(q0 + i) * kQBlocks + b]
+                         : make_float4(-TSIM_INF, -TSIM_INF, TSIM_INF, TSIM_INF);
+    }
+  }
+  const bool in = c < a.C;
+  float4 ce = make_float4(0.f, 0.f, 0.f, 0.f), cb = ce;
+  int m = 0;
+  if (in) {
+    ce = a.cends[c];
+    cb = a.cbox[c];
+    m = a.clen[c];
+  }
   __syncthreads();
-  unsigned long long key = ~0ull;
-  if (c < a.C) {
-    const float4 ce = a.cends[c], cb = a.cbox[c];
-    const int m = a.clen[c];
+  for (int q = q0; q < q1; ++q) {
+    const float4 qb = a.qbox[q], qe = a.qends[q];
+    const int n = a.qlen[q];
     float b = bound1<MEAS>(a, qb, qe, n, cb, ce, m);
     if (n > 0 && m > 0) {
-      const float bb = block_bound<MEAS>(a, qblk, n, cb, m);
+      const float bb = block_bound<MEAS>(a, qblk[q - q0], rows[q - q0], cb);
       b = MEAS == M_LCSS ? fminf(b, fminf(bb, (float)min(n, m))) : fmaxf(b, bb);
     }
-    a.lb1[(size_t)q * a.C + c] = b;
-    key = pack_key(seed_score<MEAS>(b, qe, ce, ends_align(n, a.clen[c], a.delta)), threadIdx.x);
+    if (in) a.lb1[(size_t)q * a.C + c] = b;
+    const float score = seed_score<MEAS>(b, qe, ce, ends_align(n, m, a.delta));
+    if (a.T == 1) {
+      best.warp_best(q - q0, in ? f2ord(score) : 0xffffffffu, chunk);
+    } else {
+      keys[threadIdx.x] = in ? pack_key(score, threadIdx.x) : ~0ull;
+      __syncthreads();
+      block_select_k(keys, kChunk, a.T, sel, red);
+      for (int i = threadIdx.x; i < a.T; i += kChunk) {
+        const int li = key_index(sel[i]);
+        a.chunk_cand[((size_t)q * a.nch + chunk) * a.T + i] = li < 0 ? -1 : chunk * kChunk + li;
+      }
+      __syncthreads();
+    }
   }
-  keys[threadIdx.x] = key;
-  __syncthreads();
-  block_select_k(keys, kChunk, a.T, sel, red);
-  for (int i = threadIdx.x; i < a.T; i += kChunk) {
-    int li = key_index(sel[i]);
-    a.chunk_cand[((size_t)q * a.nch + chunk) * a.T + i] = li < 0 ? -1 : chunk * kChunk + li;
-  }
+  if (a.T == 1) best.store(a, q0, q1, chunk);
 }
 
 // ---------------------------------------------------------------------------
@@ -577,11 +633,9 @@ __global__ void __launch_bounds__(kChunk) paa_kernel(KArgs a) {
   __shared__ unsigned long long keys[kChunk];
   __shared__ SelScratch red;
   __shared__ unsigned long long sel[64];
-  __shared__ unsigned wbest[kPaaQueries][kChunk / 32];
-  __shared__ int wcand[kPaaQueries][kChunk / 32];
+  __shared__ ChunkBest<kPaaQueries> best;
   const int chunk = blockIdx.x;
   const int c = chunk * kChunk + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q0 = blockIdx.y * kPaaQueries, q1 = min(a.nq, q0 + kPaaQueries);
   const bool in = c < a.C;
   const int m = in ? a.clen[c] : 0;
@@ -628,14 +682,8 @@ __global__ void __launch_bounds__(kChunk) paa_kernel(KArgs a) {
       bound = __fmul_rd(__fadd_rd(accx, accy), rl);
     }
     if (in) a.lb1[(size_t)q * a.C + c] = bound;
-    if (a.T == 1) {  // the warp's best; the CTA's after the loop
-      const unsigned o = in ? f2ord(bound) : 0xffffffffu;
-      const unsigned mn = __reduce_min_sync(0xffffffffu, o);
-      const unsigned who = __ballot_sync(0xffffffffu, o == mn);
-      if (lane == 0) {
-        wbest[q - q0][warp] = mn;
-        wcand[q - q0][warp] = mn == 0xffffffffu ? -1 : chunk * kChunk + warp * 32 + __ffs(who) - 1;
-      }
+    if (a.T == 1) {
+      best.warp_best(q - q0, in ? f2ord(bound) : 0xffffffffu, chunk);
     } else {
       keys[threadIdx.x] = in ? pack_key(bound, threadIdx.x) : ~0ull;
       __syncthreads();
@@ -647,16 +695,7 @@ __global__ void __launch_bounds__(kChunk) paa_kernel(KArgs a) {
       __syncthreads();
     }
   }
-  if (a.T == 1) {
-    __syncthreads();
-    const int q = q0 + threadIdx.x;
-    if (threadIdx.x < kPaaQueries && q < q1) {
-      int best = 0;
-      for (int w = 1; w < kChunk / 32; ++w)
-        if (wbest[threadIdx.x][w] < wbest[threadIdx.x][best]) best = w;
-      a.chunk_cand[(size_t)q * a.nch + chunk] = wcand[threadIdx.x][best];
-    }
-  }
+  if (a.T == 1) best.store(a, q0, q1, chunk);
 }
 
 // LCSS with an index window: column j of any candidate can only match query
@@ -2149,7 +2188,6 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   if (a.brute) return run_brute<MEAS>(ctx, a, dp32, dpc, dp64);
   cudaStream_t s = ctx->stream;
   const int nq = a.nq;
-  dim3 g1(a.nch, nq);
   TSIM_CUDA(cudaMemsetAsync(a.n64, 0, 2 * sizeof(int), s));
   stage_begin(ctx, TSIM_STAGE_LB1);
   clear_u32_kernel<<<std::min<size_t>(((size_t)nq * a.Cw + 255) / 256, 4096), 256, 0, s>>>(
@@ -2159,7 +2197,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     paa_kernel<<<dim3(a.nch, (nq + kPaaQueries - 1) / kPaaQueries), kChunk, 0, s>>>(a);
     launched(ctx);
   } else {
-    lb1_kernel<MEAS><<<g1, kChunk, 0, s>>>(a);
+    lb1_kernel<MEAS><<<dim3(a.nch, (nq + kLb1Queries - 1) / kLb1Queries), kChunk, 0, s>>>(a);
   }
   stage_end(ctx);
   launched(ctx, 2);
