@@ -78,6 +78,15 @@ struct FloorDiv {
       q += 1;
     }
   }
+  // num -= dq * d + dr
+  __device__ __forceinline__ void step_back(int dq, int dr) {
+    q -= dq;
+    r -= dr;
+    if (r < 0) {
+      r += d;
+      q -= 1;
+    }
+  }
 };
 
 // Sparse table of a query for O(1) range boxes: level l holds, for block b,

@@ -187,15 +187,27 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
   if (suffix) {
     const QTable T = qtable_view(a.qtab + (size_t)q * qtable_stride(a.max_n), n);
     float carry = 0.0f;  // bound of the columns after the current block
+    // the band's rows of column j, ceil((j(n-1) - W) / (m-1)) to floor((j(n-1)
+    // + W) / (m-1)), stepped down 32 columns a block
+    const int jl = (((m - 1) >> 5) << 5) + lane, D = m - 1;
+    FloorDiv lo_d{}, hi_d{};
+    int dq = 0, dr = 0;
+    if (W >= 0) {
+      lo_d.init((long long)jl * (n - 1) - W + D - 1, D);
+      hi_d.init((long long)jl * (n - 1) + W, D);
+      divmod_floor(32ll * (n - 1), D, dq, dr);
+    }
     for (int b0 = ((m - 1) >> 5) << 5; b0 >= 0; b0 -= 32) {  // blocks of 32 columns, last first
       const int j = b0 + lane;
       float v = 0.0f;
+      int lo = 0, hi = n - 1;
+      if (W >= 0) {
+        lo = max(0, lo_d.q);
+        hi = min(n - 1, hi_d.q);
+        lo_d.step_back(dq, dr);
+        hi_d.step_back(dq, dr);
+      }
       if (j < m) {
-        int lo = 0, hi = n - 1;
-        if (W >= 0) {
-          lo = max(0, floordiv_i((long long)j * (n - 1) - W + (m - 2), m - 1));  // ceil
-          hi = min(n - 1, floordiv_i((long long)j * (n - 1) + W, m - 1));
-        }
         if (lo <= hi) {
           const float4 bx = qtable_box(T, lo, hi);
           const float2 c = CS(j);
@@ -274,8 +286,10 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
       const V lft = s ? lft1 : v[r];
       const V c = P::combine(cst[r], vmin(mdu, lft));
       const bool in = lane * R + r < L;
+      // a position outside (row past ihi) has its left neighbour outside too
+      // (ihi never falls), so its M is +inf with its V
       nv[r] = in ? c : P::border();
-      nm[r] = in ? vmin(c, lft) : P::border();
+      nm[r] = vmin(nv[r], lft);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
