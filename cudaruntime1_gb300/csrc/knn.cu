@@ -1474,7 +1474,10 @@ __global__ void __launch_bounds__(kSelThreads) r1_select_kernel(KArgs a) {
   __shared__ unsigned long long sel[64];
   const int q = blockIdx.x;
   const int ns = (a.cnt2[q] + kSeg - 1) / kSeg;
-  if (threadIdx.x == 0) a.fcnt[q] = 0;  // round 2's list count (refilter_kernel)
+  if (threadIdx.x == 0) {
+    a.fcnt[q] = 0;  // round 2's list count (refilter_kernel)
+    a.cnt0[q] = 0;  // and what the row side keeps of it (lb_rows_kernel)
+  }
   // the segments' M best (seg_select_kernel) hold the query's M best
   block_select_k(a.segkeys + (size_t)q * a.nseg * 64, ns * a.M, a.M, sel, red);
   for (int i = threadIdx.x; i < a.M; i += kSelThreads) {
@@ -1551,6 +1554,104 @@ __global__ void refilter_kernel(KArgs a) {
       a.list1[(size_t)q * a.C + pos] = c;
     }
   }
+}
+
+// DTW with a band, after the round-1 threshold: the other side of LB_Keogh.
+// Query row i meets the path inside its band columns, so it costs at least the
+// distance from its point to the box of those candidate points.  Where the
+// query is the longer side it has more terms than the column side (a path
+// crosses every row) and narrower windows: DTW queries of up to 2,048 points
+// against 1,000,000 trajectories of 50 to 500: ROWS_PRUNE.  A warp per pair
+// of list1, those that pass to list2: the candidate's boxes over blocks of
+// 8, 16, ... points (at most 64 blocks) and their sparse table in shared
+// memory, then a row a lane.  Rows 0 and n-1 are the exact corner cells.
+// Bound by issue: about 30 instructions a row beside 300 for the table, a
+// fiftieth of the DP it saves.
+constexpr int kRowBlocks = 64, kRowLevels = 7;
+constexpr int kRowWarps = 4;
+__global__ void __launch_bounds__(kRowWarps * 32) lb_rows_kernel(KArgs a) {
+  __shared__ float4 tabs[kRowWarps][kRowLevels][kRowBlocks];
+  __shared__ int buf[kRowWarps][64][2];
+  const int q = blockIdx.y;
+  const int cnt = a.fcnt[q];
+  if (blockIdx.x * kRowWarps >= cnt) return;  // uniform across the CTA
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float t = a.thr2[q];
+  const float2* A = a.qpts + a.qoff[q];
+  const int n = a.qlen[q];
+  float4(*tab)[kRowBlocks] = tabs[warp];
+  WarpList out{a.cnt0 + q, a.list2 + (size_t)q * a.C, nullptr, buf[warp]};
+  for (int e = blockIdx.x * kRowWarps + warp; e < cnt; e += gridDim.x * kRowWarps) {
+    const int c = a.list1[(size_t)q * a.C + e];
+    const int m = a.clen[c];
+    const float2* B = a.cpts + a.coff[c];
+    bool pass = true;
+    if (n >= 2 && m >= 2) {
+      int f = 3;
+      while ((m + (1 << f) - 1) >> f > kRowBlocks) ++f;
+      const int nb = (m + (1 << f) - 1) >> f;
+      const int w = band_w(n, m, a.band_pct);
+      const long long W = (long long)w * (min(n, m) - 1);
+      const int D = n - 1;
+      // the most blocks a row's window touches: its levels are built
+      const int span = (int)min((long long)nb, ((2 * W / D + 2) >> f) + 2);
+      __syncwarp();  // the last pair's table is used
+      for (int b = lane; b < nb; b += 32) {
+        float x0 = TSIM_INF, y0 = TSIM_INF, x1 = -TSIM_INF, y1 = -TSIM_INF;
+        const int j1 = min(m, (b + 1) << f);
+#pragma unroll 4
+        for (int j = b << f; j < j1; ++j) {
+          const float2 p = __ldg(B + j);
+          x0 = fminf(x0, p.x);
+          y0 = fminf(y0, p.y);
+          x1 = fmaxf(x1, p.x);
+          y1 = fmaxf(y1, p.y);
+        }
+        tab[0][b] = make_float4(x0, y0, x1, y1);
+      }
+      __syncwarp();
+      for (int l = 1; (1 << l) <= span; ++l) {
+        for (int b = lane; b + (1 << l) <= nb; b += 32) {
+          const float4 u = tab[l - 1][b], v = tab[l - 1][b + (1 << (l - 1))];
+          tab[l][b] = make_float4(fminf(u.x, v.x), fminf(u.y, v.y), fmaxf(u.z, v.z), fmaxf(u.w, v.w));
+        }
+        __syncwarp();
+      }
+      // columns of row i: ceil((i(m-1) - W) / (n-1)) to floor((i(m-1) + W) / (n-1))
+      FloorDiv lo_d, hi_d;
+      const int i0 = 1 + lane;
+      lo_d.init((long long)i0 * (m - 1) - W + D - 1, D);
+      hi_d.init((long long)i0 * (m - 1) + W, D);
+      int dq, dr;
+      divmod_floor(32ll * (m - 1), D, dq, dr);
+      float acc = 0.0f;
+      if (lane == 0) {
+        const float2 a0 = A[0], a1 = A[n - 1], b0 = B[0], b1 = B[m - 1];
+        const float d0 = pd2_rd(a0.x, a0.y, b0.x, b0.y), d1 = pd2_rd(a1.x, a1.y, b1.x, b1.y);
+        acc = a.cost ? __fadd_rd(__fsqrt_rd(d0), __fsqrt_rd(d1)) : __fadd_rd(d0, d1);
+      }
+      for (int i = i0; i < n - 1; i += 32) {
+        const int lo = max(lo_d.q, 0), hi = min(hi_d.q, m - 1);
+        lo_d.step(dq, dr);
+        hi_d.step(dq, dr);
+        if (lo > hi) {  // a row with no admissible column
+          acc = TSIM_INF;
+          break;
+        }
+        const int k0 = lo >> f, k1 = hi >> f;
+        const int l = 31 - __clz(k1 - k0 + 1);
+        const float4 u = tab[l][k0], v = tab[l][k1 - (1 << l) + 1];
+        const float2 p = __ldg(A + i);
+        const float d = box_pt_d2_rd(fminf(u.x, v.x), fminf(u.y, v.y), fmaxf(u.z, v.z),
+                                     fmaxf(u.w, v.w), p.x, p.y);
+        acc = __fadd_rd(acc, a.cost ? __fsqrt_rd(d) : d);
+      }
+      for (int o = 16; o; o >>= 1) acc = __fadd_rd(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+      pass = acc <= t;
+    }
+    if (pass) out.add(lane == 0, c, 0);
+  }
+  out.flush();
 }
 
 // exclusive scan of fcnt -> off2, total -> npairs (one CTA)
@@ -2308,6 +2409,13 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
 
   stage_begin(ctx, TSIM_STAGE_FILTER);
   refilter_kernel<MEAS><<<dim3(ch, nq), 256, 0, s>>>(a);
+  if (MEAS == M_DTW && a.band_pct >= 0) {
+    lb_rows_kernel<<<dim3(std::max(1, std::min((a.C + kRowWarps - 1) / kRowWarps, 2 * ch)), nq),
+                     kRowWarps * 32, 0, s>>>(a);
+    launched(ctx);
+    a.list1 = a.list2;  // what it kept
+    a.fcnt = a.cnt0;
+  }
   scan_kernel<<<1, 1024, 0, s>>>(a);
   flatten_kernel<<<dim3(ch, nq), 256, 0, s>>>(a);
   // the shape order serves the kernels whose warps run as long as their
