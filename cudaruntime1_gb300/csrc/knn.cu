@@ -1561,15 +1561,16 @@ __global__ void refilter_kernel(KArgs a) {
 // distance from its point to the box of those candidate points.  Where the
 // query is the longer side it has more terms than the column side (a path
 // crosses every row) and narrower windows: DTW queries of up to 2,048 points
-// against 1,000,000 trajectories of 50 to 500: ROWS_PRUNE.  A warp per pair
-// of list1, those that pass to list2: the candidate's boxes over blocks of
-// 8, 16, ... points (at most 64 blocks) and their sparse table in shared
-// memory, then a row a lane.  Rows 0 and n-1 are the exact corner cells.
+// against 1,000,000 trajectories of 50 to 500, 12 queries: 138,000 -> 9,400
+// pairs to the DP (before the column side it cost more than it saved there).  A
+// warp per pair of list1, those that pass to list2: the candidate's boxes over
+// blocks of 8, 16, ... points (at most 64 blocks, a window at most 15) and their
+// sparse table in shared memory, then a row a lane.  Rows 0 and n-1 are the exact corner cells.
 // Bound by issue: about 30 instructions a row beside 300 for the table, a
 // fiftieth of the DP it saves.
-constexpr int kRowBlocks = 64, kRowLevels = 7;
+constexpr int kRowBlocks = 64, kRowLevels = 4;
 constexpr int kRowWarps = 4;
-__global__ void __launch_bounds__(kRowWarps * 32) lb_rows_kernel(KArgs a) {
+__global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
   __shared__ float4 tabs[kRowWarps][kRowLevels][kRowBlocks];
   __shared__ int buf[kRowWarps][64][2];
   const int q = blockIdx.y;
@@ -1587,25 +1588,30 @@ __global__ void __launch_bounds__(kRowWarps * 32) lb_rows_kernel(KArgs a) {
     const float2* B = a.cpts + a.coff[c];
     bool pass = true;
     if (n >= 2 && m >= 2) {
-      int f = 3;
-      while ((m + (1 << f) - 1) >> f > kRowBlocks) ++f;
-      const int nb = (m + (1 << f) - 1) >> f;
       const int w = band_w(n, m, a.band_pct);
       const long long W = (long long)w * (min(n, m) - 1);
       const int D = n - 1;
-      // the most blocks a row's window touches: its levels are built
-      const int span = (int)min((long long)nb, ((2 * W / D + 2) >> f) + 2);
+      // the window's columns, at most; blocks of 2^f points so that a window
+      // touches at most 15 (the table has four levels)
+      const int width = (int)min((long long)m, 2 * W / D + 2);
+      int f = 3;
+      while ((m + (1 << f) - 1) >> f > kRowBlocks || (width >> f) + 2 > 15) ++f;
+      const int nb = (m + (1 << f) - 1) >> f;
+      const int span = min(nb, (width >> f) + 2);
       __syncwarp();  // the last pair's table is used
       for (int b = lane; b < nb; b += 32) {
         float x0 = TSIM_INF, y0 = TSIM_INF, x1 = -TSIM_INF, y1 = -TSIM_INF;
-        const int j1 = min(m, (b + 1) << f);
-#pragma unroll 4
-        for (int j = b << f; j < j1; ++j) {
-          const float2 p = __ldg(B + j);
-          x0 = fminf(x0, p.x);
-          y0 = fminf(y0, p.y);
-          x1 = fmaxf(x1, p.x);
-          y1 = fmaxf(y1, p.y);
+        for (int j = b << f; j < min(m, (b + 1) << f); j += 8) {
+          float2 p[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) p[u] = __ldg(B + min(j + u, m - 1));
+#pragma unroll
+          for (int u = 0; u < 8; u += 2) {
+            x0 = min3f(x0, p[u].x, p[u + 1].x);
+            y0 = min3f(y0, p[u].y, p[u + 1].y);
+            x1 = max3f(x1, p[u].x, p[u + 1].x);
+            y1 = max3f(y1, p[u].y, p[u + 1].y);
+          }
         }
         tab[0][b] = make_float4(x0, y0, x1, y1);
       }
@@ -2410,7 +2416,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   stage_begin(ctx, TSIM_STAGE_FILTER);
   refilter_kernel<MEAS><<<dim3(ch, nq), 256, 0, s>>>(a);
   if (MEAS == M_DTW && a.band_pct >= 0) {
-    lb_rows_kernel<<<dim3(std::max(1, std::min((a.C + kRowWarps - 1) / kRowWarps, 2 * ch)), nq),
+    lb_rows_kernel<<<dim3(std::max(1, std::min((a.C + kRowWarps - 1) / kRowWarps, 8 * ch)), nq),
                      kRowWarps * 32, 0, s>>>(a);
     launched(ctx);
     a.list1 = a.list2;  // what it kept

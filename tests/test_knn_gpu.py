@@ -450,3 +450,24 @@ def test_hausdorff_point_counts(tsim, cuda_ctx, oracle, pruned):
     # one rounded squared distance (8 2^-24), its root and the result's rounding
     assert np.all(np.abs(d - want) <= 8 * 2.0 ** -24 * want)
     db.close()
+
+
+@pytest.mark.parametrize("band,cost", [(0, 0), (1, 0), (10, 0), (10, 1), (45, 0), (100, 0)])
+def test_dtw_row_bounds(tsim, cuda_ctx, oracle, band, cost):
+    """The row side of LB_Keogh: queries shorter, longer and far longer than
+    the candidates, two-point sides, bands from the diagonal to the whole
+    matrix (windows of one block to more than 15): the oracle's ids, and the
+    distances of a request that refines every pair."""
+    lens = np.random.default_rng(7).integers(2, 90, 500)
+    lens[::9] = 300
+    lens[5::50] = 700
+    cp, co = G.random_walks(500, lens, 61, start_range=15.0)
+    qp, qo = G.random_walks(6, [2, 3, 40, 300, 301, 900], 62, start_range=15.0)
+    db = tsim.Database(cuda_ctx, cp, co)
+    kw = dict(band_pct=band, cost=cost)
+    ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 5, flags=tsim.api.FLAG_ALWAYS_PRUNE, **kw)
+    ids2, d2, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 5, flags=tsim.api.FLAG_NO_PRUNE, **kw)
+    want_ids, _ = oracle.knn("dtw", qp, qo, cp, co, 5, **kw)
+    assert np.array_equal(ids, want_ids)
+    assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
+    db.close()
