@@ -1,15 +1,10 @@
 // pairwise_knn.cu -- refine kernels of the exact kNN path for symmetric
 // Hausdorff and lock-step Euclidean: one warp per (query, candidate) pair.
 //
-// Hausdorff (FP32): a lane holds up to 8 points of one side in registers; the
-// other side passes through shared memory, x and y apart, so that a packed
-// instruction takes two points, and each lane keeps its points' minimum
-// squared distances.  The warp maximum is h(Q,C); the reverse direction swaps
-// the roles.  What bounds it is the FP32 pipe: four operations a point pair
-// (two differences, a multiply, an FMA; the minima are a half instruction on
-// another pipe).  A pair whose maximum exceeds the query's threshold is
-// abandoned; most pairs of a pruned round are, so with a threshold a sample of
-// 32 points of either side, spread over it, is tested first.
+// Hausdorff (FP32): the two directions by hausdorff.cuh.  A pair whose maximum
+// exceeds the query's threshold is abandoned; most pairs of a pruned round
+// are, so with a threshold a sample of 32 points of either side, spread over
+// it, is tested first.
 // Reference kernel replaced: hausdorff_tiled_rtree_kernel
 // (CudaRuntime1/hausdorff.cu:84-122), one CTA per query over 256-point tiles.
 //
@@ -21,7 +16,7 @@
 // FP64 kernels compute the oracle's arithmetic (oracle/oracle.c
 // orc_hausdorff64, orc_euclid64) for the pairs the FP32 values cannot order.
 #include "dfloat.cuh"
-#include "f32x2.cuh"
+#include "hausdorff.cuh"
 #include "tsim_internal.cuh"
 
 namespace tsim {
@@ -33,91 +28,10 @@ __device__ __forceinline__ float d2f(float ax, float ay, float bx, float by) {
   return fmaf(dy, dy, dx * dx);
 }
 
-constexpr int kTargets = 512;    // targets staged at a time, per warp
-constexpr int kSampleMin = 64;   // a side is sampled from this many points on
-
-// points T[t0 .. t0 + len) to shared memory (x, then y), padded to a multiple
-// of four with the last one
-__device__ __forceinline__ void stage_targets(const float2* T, int t0, int len, float* sm) {
-  const int lane = threadIdx.x & 31;
-  __syncwarp();  // the last targets are used
-  for (int j = lane; j < ((len + 3) & ~3); j += 32) {
-    const float2 p = __ldg(T + t0 + min(j, len - 1));
-    sm[j] = p.x;
-    sm[kTargets + j] = p.y;
-  }
-  __syncwarp();
-}
-
-// The largest of the minimum squared distances of 32 R points of S to T's;
-// lane's point u is S[row(u)] (a row past the end repeats one of the others).
-template <int R, class Row>
-__device__ __forceinline__ float rows_max_min(const float2* S, const float2* T, int nt, float* sm,
-                                              Row row) {
-  float2 sx[R], sy[R];
-  float mn[R];
-#pragma unroll
-  for (int u = 0; u < R; ++u) {
-    const float2 p = __ldg(S + row(u));
-    sx[u] = make_float2(p.x, p.x);
-    sy[u] = make_float2(p.y, p.y);
-    mn[u] = TSIM_INF;
-  }
-  for (int t0 = 0; t0 < nt; t0 += kTargets) {
-    const int len = min(kTargets, nt - t0);
-    if (nt > kTargets) stage_targets(T, t0, len, sm);  // else staged by the caller
-#pragma unroll 2
-    for (int j = 0; j < len; j += 4) {
-      const float4 X = *reinterpret_cast<const float4*>(sm + j);
-      const float4 Y = *reinterpret_cast<const float4*>(sm + kTargets + j);
-#pragma unroll
-      for (int u = 0; u < R; ++u) {
-        const float2 dx = sub2(make_float2(X.x, X.y), sx[u]), ex = sub2(make_float2(X.z, X.w), sx[u]);
-        const float2 dy = sub2(make_float2(Y.x, Y.y), sy[u]), ey = sub2(make_float2(Y.z, Y.w), sy[u]);
-        const float2 d = fma2(dy, dy, mul2(dx, dx)), e = fma2(ey, ey, mul2(ex, ex));
-        mn[u] = min3f(min3f(mn[u], d.x, d.y), e.x, e.y);
-      }
-    }
-  }
-  float loc = mn[0];
-#pragma unroll
-  for (int u = 1; u < R; ++u) loc = fmaxf(loc, mn[u]);
-  for (int o = 16; o; o >>= 1) loc = fmaxf(loc, __shfl_xor_sync(0xffffffffu, loc, o));
-  return loc;
-}
-
-// max over S of min over T of |s - t|^2 (FP32), at least `run`; stops above
-// `stop`.  *pairs grows by the point pairs compared.  sample: 32 points of S
-// only.
-__device__ float warp_directed(const float2* S, int ns, const float2* T, int nt, float run,
-                               float stop, float* sm, bool sample, long long* pairs) {
-  const int lane = threadIdx.x & 31;
-  if (nt <= kTargets) stage_targets(T, 0, nt, sm);
-  if (sample) {
-    *pairs += 32ll * nt;
-    return fmaxf(run, rows_max_min<1>(S, T, nt, sm, [&](int) {
-                   return (int)((2 * lane + 1) * (long long)ns >> 6);
-                 }));
-  }
-  for (int base = 0; base < ns;) {
-    // as many points a lane as the rest fills
-    const int r = (ns - base + 31) >> 5;
-    const int take = r >= 8 ? 8 : r >= 4 ? 4 : r >= 2 ? 2 : 1;
-    auto row = [&](int u) { return min(base + u * 32 + lane, ns - 1); };
-    const float loc = take == 8   ? rows_max_min<8>(S, T, nt, sm, row)
-                      : take == 4 ? rows_max_min<4>(S, T, nt, sm, row)
-                      : take == 2 ? rows_max_min<2>(S, T, nt, sm, row)
-                                  : rows_max_min<1>(S, T, nt, sm, row);
-    *pairs += (long long)min(32 * take, ns - base) * nt;
-    run = fmaxf(run, loc);
-    if (run > stop) return run;
-    base += 32 * take;
-  }
-  return run;
-}
+constexpr int kSampleMin = 64;  // a side is sampled from this many points on
 
 __global__ void __launch_bounds__(kPwThreads) hausdorff_refine_kernel(PwArgs a) {
-  __shared__ __align__(16) float targets[kPwThreads / 32][2 * kTargets];
+  __shared__ __align__(16) float targets[kPwThreads / 32][haus::kStageFloats];
   const int lane = threadIdx.x & 31;
   float* sm = targets[threadIdx.x >> 5];
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -137,11 +51,11 @@ __global__ void __launch_bounds__(kPwThreads) hausdorff_refine_kernel(PwArgs a) 
       const float stop = a.thr ? a.thr[pr.x] : TSIM_INF;
       v = 0.0f;
       const bool sample = stop < TSIM_INF;
-      if (sample && n >= kSampleMin) v = warp_directed(Q, n, C, m, v, stop, sm, true, &pairs);
+      if (sample && n >= kSampleMin) v = haus::warp_directed<true>(Q, n, C, m, v, stop, sm, true, &pairs);
       if (sample && m >= kSampleMin && v <= stop)
-        v = warp_directed(C, m, Q, n, v, stop, sm, true, &pairs);
-      if (v <= stop) v = warp_directed(Q, n, C, m, v, stop, sm, false, &pairs);
-      if (v <= stop) v = warp_directed(C, m, Q, n, v, stop, sm, false, &pairs);
+        v = haus::warp_directed<true>(C, m, Q, n, v, stop, sm, true, &pairs);
+      if (v <= stop) v = haus::warp_directed<true>(Q, n, C, m, v, stop, sm, false, &pairs);
+      if (v <= stop) v = haus::warp_directed<true>(C, m, Q, n, v, stop, sm, false, &pairs);
       if (v > stop) v = TSIM_INF;  // abandoned: cannot be among the k best
     }
     if (lane == 0) {
