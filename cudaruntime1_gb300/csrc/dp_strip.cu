@@ -508,6 +508,160 @@ __global__ void __launch_bounds__(kStripThreads)
   }
 }
 
+// The value of a pair with several costs in its window, by deciding which of
+// them is the optimum: the smallest cost c for which the cells of cost at most
+// c join the first cell to the last.  Joined or not is one bit a cell, so a
+// column of up to 1,024 rows is a 32-bit word per lane of one warp: a cell is
+// reached from the column before (its row or the row above) or from the row
+// above in its own, and the runs of free cells below the reached ones come
+// from one addition over the column, whose carry ripples through exactly the
+// ones of a run, across the lanes by a second addition on the words' generate
+// and propagate ballots.  The window's costs (at most 64 distinct ones) are
+// found and ordered first; a binary search then takes one pass over the matrix
+// for two costs, six for 64.  The other seven warps turn points into the bits
+// of the next 32 columns meanwhile.
+//
+// What bounds it: the pass's chain of columns, about 80 cycles each, on the one
+// pair in twelve that gets here (a CTA for each).  The DP's chain is as long
+// but takes four cells of 64-bit minima and maxima a step and eight strips for
+// 1,024 rows: the pairs left of 2,560 of up to 256 x 1,024 points 602 -> 52 us.
+// Pairs this cannot take (more rows or costs, a window that does not hold) are
+// left for the DP.
+constexpr int kDecideThreads = 256;
+constexpr int kDecideRows = 1024;
+constexpr int kDecideCosts = 64;
+__global__ void __launch_bounds__(kDecideThreads, 4)
+    frechet_decide_kernel(DpArgs a, int* rest, int* nrest) {
+  __shared__ float2 row[kDecideRows];
+  __shared__ unsigned fw[2][32][33];  // free bits of 32 columns: [column][word of rows]
+  __shared__ double found[kDecideCosts], cost[kDecideCosts];
+  __shared__ int nfound;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int npairs = a.npairs_dev ? min(*a.npairs_dev, a.npairs) : a.npairs;
+  for (int wk = blockIdx.x; wk < npairs; wk += gridDim.x) {
+    const int pid = a.order ? a.order[wk] : wk;
+    const int2 pr = a.pairs[pid];
+    if (pr.y < 0) continue;  // uniform over the CTA, as below
+    const int64_t qo = a.qoff[pr.x], co = a.coff[pr.y];
+    const int n = (int)(a.qoff[pr.x + 1] - qo), m = (int)(a.coff[pr.y + 1] - co);
+    const int rows = min(n, m), cols = max(n, m);
+    const float2* O = n <= m ? a.qpts + qo : a.cpts + co;
+    const float2* I = n <= m ? a.cpts + co : a.qpts + qo;
+    const float v32 = (float)a.aux[pid];
+    if (!(v32 >= 1e-20f) || !(v32 < 1e38f) || rows < 1 || rows > kDecideRows) {
+      if (threadIdx.x == 0) rest[atomicAdd(nrest, 1)] = pid;
+      continue;
+    }
+    // the window of frechet_window_kernel
+    const unsigned lo = __float_as_uint(__fmul_rd(v32, 1.0f - 32.0f / 16777216.0f));
+    const unsigned span = __float_as_uint(__fmul_ru(v32, 1.0f + 32.0f / 16777216.0f)) - lo - 1;
+    const int W = (rows + 31) >> 5;
+    auto d32 = [](float2 p, float2 c) {
+      const float2 t = sub2(p, c);
+      return __float_as_uint(fmaf(t.y, t.y, t.x * t.x));
+    };
+
+    __syncthreads();  // the previous pair's reads are done
+    for (int i = threadIdx.x; i < 32 * W; i += kDecideThreads)
+      row[i] = i < rows ? __ldg(O + i) : make_float2(TSIM_INF, TSIM_INF);  // never free
+    if (threadIdx.x < kDecideCosts) found[threadIdx.x] = -1.0;
+    if (threadIdx.x == 0) nfound = 0;
+    __syncthreads();
+    for (int j = threadIdx.x; j < cols; j += kDecideThreads) {
+      const float2 c = __ldg(I + j);
+      for (int i0 = 0; i0 < 32 * W; i0 += 8) {
+        unsigned first = 0xffffffffu;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) first = min(first, d32(row[i0 + k], c) - lo - 1u);
+        if (first >= span) continue;
+        for (int k = 0; k < 8; ++k) {
+          if (d32(row[i0 + k], c) - lo - 1u >= span) continue;
+          const double x = d2_64(row[i0 + k].x, row[i0 + k].y, c.x, c.y);
+          // (a cost written by another thread meanwhile may be listed twice)
+          bool have = false;
+          const int have_n = min(*(volatile int*)&nfound, kDecideCosts);
+          for (int t = 0; t < have_n; ++t) have = have || *(volatile double*)&found[t] == x;
+          if (have) continue;
+          const int at = atomicAdd(&nfound, 1);
+          if (at < kDecideCosts) *(volatile double*)&found[at] = x;
+        }
+      }
+    }
+    __syncthreads();
+    const int nc = nfound;
+    if (nc < 1 || nc > kDecideCosts) {
+      if (threadIdx.x == 0) rest[atomicAdd(nrest, 1)] = pid;
+      continue;
+    }
+    if (threadIdx.x < nc) {
+      const double x = found[threadIdx.x];
+      int r = 0;
+      for (int t = 0; t < nc; ++t) r += found[t] < x || (found[t] == x && t < (int)threadIdx.x);
+      cost[r] = x;
+    }
+    __syncthreads();
+
+    // free bits of columns 32 ch .. into fw[ch & 1], words w0, w0 + dw, ..
+    auto fill = [&](int ch, double lim, int w0, int dw) {
+      const int j = ch * 32 + lane;
+      const float2 c = j < cols ? __ldg(I + j) : make_float2(TSIM_INF, TSIM_INF);
+      for (int w = w0; w < W; w += dw) {
+        unsigned f = 0, in = 0;
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) {
+          const unsigned d = d32(row[w * 32 + r], c);
+          if (d <= lo) f |= 1u << r;
+          if (d - lo - 1u < span) in |= 1u << r;
+        }
+        while (in) {
+          const int r = __ffs(in) - 1;
+          in &= in - 1;
+          const float2 p = row[w * 32 + r];
+          if (d2_64(p.x, p.y, c.x, c.y) <= lim) f |= 1u << r;
+        }
+        fw[ch & 1][lane][w] = f;
+      }
+    };
+    const int nch = (cols + 31) >> 5;
+    int t0 = 0, t1 = nc - 1;  // the optimum is one of cost[t0 .. t1]
+    while (t0 < t1) {
+      const int mid = (t0 + t1) >> 1;
+      const double lim = cost[mid];
+      unsigned reach = 0;  // warp 0: this lane's 32 rows of the last column done
+      bool joined = false;
+      fill(0, lim, warp, kDecideThreads / 32);
+      __syncthreads();
+      for (int ch = 0; ch < nch; ++ch) {
+        if (warp == 0) {
+          const int w = min(cols - ch * 32, 32);
+#pragma unroll 4
+          for (int c = 0; c < w; ++c) {
+            const unsigned f = lane < W ? fw[ch & 1][c][lane] : 0u;
+            const unsigned tops = __ballot_sync(0xffffffffu, reach >> 31);
+            unsigned from = reach | (reach << 1) | (((tops << 1) >> lane) & 1u);
+            if (ch == 0 && c == 0) from = lane == 0 ? 1u : 0u;
+            const unsigned s = f & from;
+            const unsigned t = f + s;
+            const unsigned gen = __ballot_sync(0xffffffffu, t < f);
+            const unsigned pass = __ballot_sync(0xffffffffu, t == 0xffffffffu);
+            const unsigned carry = (((gen | pass) + gen) ^ pass) >> lane & 1u;
+            reach = (((t + carry) ^ f) | s) & f;
+          }
+          joined = lane == (rows - 1) >> 5 && (reach >> ((rows - 1) & 31) & 1u);
+        } else if (ch + 1 < nch) {
+          fill(ch + 1, lim, warp - 1, kDecideThreads / 32 - 1);
+        }
+        if (!__syncthreads_or(warp == 0 && reach != 0)) break;  // nothing reached in this column
+      }
+      if (__syncthreads_or(joined))  // of the last column done: false after a break
+        t1 = mid;
+      else
+        t0 = mid + 1;
+    }
+    if (threadIdx.x == 0) a.out64[pid] = cost[t0];
+  }
+}
+
 }  // namespace
 
 int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest) {
@@ -515,6 +669,16 @@ int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest)
   if (a.npairs <= 0) return TSIM_OK;
   const int blocks = std::min(a.npairs, 16 * ctx->num_sms);
   frechet_window_kernel<<<blocks, kStripThreads, 0, ctx->stream>>>(a, rest, nrest);
+  TSIM_CUDA(cudaGetLastError());
+  launched(ctx);
+  return TSIM_OK;
+}
+
+int launch_frechet_decide(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest) {
+  TSIM_CUDA(cudaMemsetAsync(nrest, 0, sizeof(int), ctx->stream));
+  if (a.npairs <= 0) return TSIM_OK;
+  const int blocks = std::min(a.npairs, 4 * ctx->num_sms);
+  frechet_decide_kernel<<<blocks, kDecideThreads, 0, ctx->stream>>>(a, rest, nrest);
   TSIM_CUDA(cudaGetLastError());
   launched(ctx);
   return TSIM_OK;

@@ -2210,10 +2210,13 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
       TSIM_TRY(launch_frechet_window(ctx, r, a.spill2, a.nspill2));
       r.order = a.spill2;
       r.npairs_dev = a.nspill2;
-      TSIM_TRY(launch_dp_strip(ctx, DP_FRECHET_WIN, r, a.max_qlen, a.max_clen, a.spill, a.nspill));
+      TSIM_TRY(launch_frechet_decide(ctx, r, a.spill, a.nspill));
+      r.order = a.spill;
+      r.npairs_dev = a.nspill;
+      TSIM_TRY(launch_dp_strip(ctx, DP_FRECHET_WIN, r, a.max_qlen, a.max_clen, a.lanes, a.nlanes));
       DpArgs sp = r;
-      sp.order = a.spill;
-      sp.npairs_dev = a.nspill;
+      sp.order = a.lanes;
+      sp.npairs_dev = a.nlanes;
       TSIM_TRY(launch_dp(ctx, DP_FRECHET_WIN, 32, 1, sp, a.max_clen));
     } else if (is_dp(MEAS)) {
       TSIM_TRY(launch_dp(ctx, dp64, 32, 1, r, a.max_clen));

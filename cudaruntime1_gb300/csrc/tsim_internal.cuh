@@ -368,6 +368,10 @@ int launch_lcss_window(tsim_ctx* ctx, const DpArgs& a);
 // FP32 values in aux) holds one cost, into out64; the others' entries in rest[]
 // (count in *nrest) for DP_FRECHET_WIN.
 int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest);
+// The same of pairs with a few costs in the window, by deciding reachability
+// for them; what is left (many costs, more than 1,024 points on both sides)
+// is for DP_FRECHET_WIN.
+int launch_frechet_decide(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest);
 // Lane-per-pair kernel (dp_lane.cu) for the FP32 DTW, Frechet and LCSS
 // kinds (lane_kind): a lane runs a whole pair in passes of 8 rows, the row
 // above a pass in a shared-memory ring of `ring` (64 or 128) values per lane

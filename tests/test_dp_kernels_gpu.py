@@ -190,6 +190,42 @@ def test_frechet_fp64_rescore_of_long_pairs(tsim, cuda_ctx, oracle):
     db.close()
 
 
+@pytest.mark.parametrize("steps", [1, 16, 100])
+def test_frechet_fp64_among_close_costs(tsim, cuda_ctx, oracle, steps):
+    """Pairs whose optimum is one of several FP64 costs that FP32 cannot tell
+    apart -- a few, up to 64, more -- with cells below and above them, over
+    one to 32 words of rows, more rows than that, and columns around the
+    32-column blocks: bit for bit the oracle's values."""
+    rng = np.random.default_rng(steps)
+
+    def walks(lens, near, far, unit, levels):
+        x = [np.where(rng.random(n) < 0.6, near + rng.integers(0, levels, n) * unit,
+                      rng.choice(far, n)) for n in lens]
+        for w in x:
+            w[0] = w[-1] = near
+        off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+        x = np.concatenate(x)
+        return np.stack([x, np.zeros_like(x)], 1).astype(np.float32), off
+
+    # 0 and 2 are as far from 1; 0.2 is near 0 and far from 2, 1.8 the reverse
+    qp, qo = walks([1, 31, 32, 33, 64, 257, 1024, 1025], 0.0, [2.0], 2.0 ** -26, steps)
+    cp, co = walks([1, 2, 31, 32, 33, 63, 64, 65, 96, 300, 1023, 1024, 1025, 1500], 1.0, [0.2, 1.8],
+                   2.0 ** -23, 3)
+    db = tsim.Database(cuda_ctx, cp, co)
+    want_ids, want = oracle.knn("frechet", qp, qo, cp, co, 14)
+    import torch
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (qp, qo)]
+    ids = torch.empty(8 * 14, dtype=torch.int32, device="cuda")
+    d = torch.empty(8 * 14, device="cuda")
+    d64 = torch.empty(8 * 14, dtype=torch.float64, device="cuda")
+    tsim.knn_device(cuda_ctx, db, dev[0].data_ptr(), dev[1].data_ptr(), 8, 1025, ids.data_ptr(),
+                    d.data_ptr(), d64.data_ptr(), "frechet", 14, flags=tsim.api.FLAG_FP64_RESCORE)
+    cuda_ctx.synchronize()
+    assert np.array_equal(ids.cpu().numpy().reshape(8, 14), want_ids)
+    assert np.array_equal(d64.cpu().numpy().reshape(8, 14), want)
+    db.close()
+
+
 @pytest.mark.parametrize("delta", [0, 1, 3, 15, 16, 20, 31])
 def test_lcss_window_bit_vectors(tsim, cuda_ctx, oracle, delta):
     """Windowed LCSS, the kernel chosen by the library, against the oracle:
