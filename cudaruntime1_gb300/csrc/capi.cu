@@ -94,6 +94,16 @@ int arena_reserve(tsim_ctx* ctx, size_t bytes) {
   return TSIM_OK;
 }
 
+int fresh_counter(tsim_ctx* ctx, int* fallback, int** out) {
+  if (ctx->ctr_used < ctx->ctr_n) {
+    *out = ctx->ctr + kCounterInts * ctx->ctr_used++;
+    return TSIM_OK;
+  }
+  TSIM_CUDA(cudaMemsetAsync(fallback, 0, kCounterInts * sizeof(int), ctx->stream));
+  *out = fallback;
+  return TSIM_OK;
+}
+
 int pinned_reserve(tsim_ctx* ctx, size_t bytes) {
   if (bytes <= ctx->pinned_cap) return TSIM_OK;
   size_t cap = std::max(bytes + bytes / 4, size_t(1) << 20);
@@ -551,11 +561,12 @@ int tsim_db_create(tsim_ctx* ctx, const tsim_point* h_pts, const int64_t* h_off,
   TSIM_CHECK_ARG(ctx && out && h_off && count >= 0, "bad arguments");
   *out = nullptr;
   TSIM_CHECK_ARG(h_off[0] == 0, "offsets must start at 0");
-  int max_len = 0;
+  int max_len = 0, min_len = INT32_MAX;
   for (int t = 0; t < count; ++t) {
     TSIM_CHECK_ARG(h_off[t + 1] > h_off[t], "trajectories must be non-empty (offsets increasing)");
     TSIM_CHECK_ARG(h_off[t + 1] - h_off[t] <= INT32_MAX, "trajectory longer than 2^31 - 1 points");
     max_len = std::max<int64_t>(max_len, h_off[t + 1] - h_off[t]);
+    min_len = std::min<int64_t>(min_len, h_off[t + 1] - h_off[t]);
   }
   TSIM_CHECK_ARG(h_pts != nullptr || count == 0, "h_pts is NULL");
   TSIM_CUDA(cudaSetDevice(ctx->device));
@@ -564,6 +575,7 @@ int tsim_db_create(tsim_ctx* ctx, const tsim_point* h_pts, const int64_t* h_off,
   db->count = count;
   db->total = h_off[count];
   db->max_len = max_len;
+  db->min_len = min_len;
   db->owns = true;
   db->h_off.assign(h_off, h_off + count + 1);
   int s = TSIM_OK;
@@ -614,7 +626,7 @@ int tsim_db_wrap_device(tsim_ctx* ctx, const tsim_point* d_pts, const int64_t* d
     return cuda_fail(e, "tsim_db_wrap_device offsets", __FILE__, __LINE__);
   }
   db->total = db->h_off[count];
-  int ml = 0;
+  int ml = 0, mn = INT32_MAX;
   for (int t = 0; t < count; ++t) {
     if (db->h_off[t + 1] <= db->h_off[t] || db->h_off[0] != 0 ||
         db->h_off[t + 1] - db->h_off[t] > INT32_MAX) {
@@ -622,9 +634,11 @@ int tsim_db_wrap_device(tsim_ctx* ctx, const tsim_point* d_pts, const int64_t* d
       return fail(TSIM_ERR_INVALID_ARG, "tsim_db_wrap_device: offsets must start at 0 and increase by at most 2^31 - 1");
     }
     ml = std::max<int64_t>(ml, db->h_off[t + 1] - db->h_off[t]);
+    mn = std::min<int64_t>(mn, db->h_off[t + 1] - db->h_off[t]);
   }
   (void)max_len;  // the offsets, read here anyway, give the exact value
   db->max_len = ml;
+  db->min_len = mn;
   int s = db_alloc(db);
   if (s == TSIM_OK) s = db_summarize(db);
   if (s == TSIM_OK) {

@@ -197,11 +197,12 @@ extern "C" int tsim_db_load(tsim_ctx* ctx, const char* path, tsim_db** out) {
   const size_t n = (size_t)h.count;
   std::vector<int64_t> off(n + 1);
   TSIM_TRY(read_host(fh.f, s, off.data(), sizeof(int64_t) * (n + 1)));
-  int64_t ml = 0;
+  int64_t ml = 0, mn = INT32_MAX;
   if (off[0] != 0 || off[n] != h.total) return fail(TSIM_ERR_INVALID_ARG, "corrupt offsets");
   for (size_t t = 0; t < n; ++t) {
     if (off[t + 1] <= off[t]) return fail(TSIM_ERR_INVALID_ARG, "corrupt offsets");
     ml = std::max<int64_t>(ml, off[t + 1] - off[t]);
+    mn = std::min<int64_t>(mn, off[t + 1] - off[t]);
   }
   if (ml != h.max_len) return fail(TSIM_ERR_INVALID_ARG, "corrupt header (longest trajectory)");
   TSIM_CUDA(cudaSetDevice(ctx->device));
@@ -210,6 +211,7 @@ extern "C" int tsim_db_load(tsim_ctx* ctx, const char* path, tsim_db** out) {
   db->count = (int)n;
   db->total = h.total;
   db->max_len = (int)ml;
+  db->min_len = (int)mn;
   db->owns = true;
   db->h_off = std::move(off);
   char* pinned = nullptr;

@@ -472,7 +472,7 @@ int launch_diag_r(tsim_ctx* ctx, int R, const DpArgs& a, int max_m, int* spill, 
 
 template <class P>
 int launch_chain(tsim_ctx* ctx, int R0, int warps, const DpArgs& a, int max_m, int* spill,
-                 int* nspill, int* tmp, int* ntmp, int rcap = 0) {
+                 int** nspill, int* tmp, int* ntmp, int rcap, bool* all) {
   // R0, 2 R0, .. Rmax: each pass takes the pairs the previous one spilled, so
   // every pair runs with the fewest rows per lane-group its shape admits
   // (fewer rows in flight, fewer masked cells); the last pass writes `spill`.
@@ -495,17 +495,22 @@ int launch_chain(tsim_ctx* ctx, int R0, int warps, const DpArgs& a, int max_m, i
     return wd < span;
   };
   std::vector<int> rs;
+  if (all) *all = false;
   for (int R = std::max(1, std::min(R0, rmax)); R <= rmax; R *= 2) {
     rs.push_back(R);
-    if (takes_all(R)) break;
+    if (takes_all(R)) {
+      if (all) *all = true;
+      break;
+    }
   }
   const int np = (int)rs.size();
   DpArgs in = a;
   for (int p = 0; p < np; ++p) {
     const bool to_spill = ((np - 1 - p) & 1) == 0;
     int* out = to_spill ? spill : tmp;
-    int* nout = to_spill ? nspill : ntmp;
-    TSIM_CUDA(cudaMemsetAsync(nout, 0, 2 * sizeof(int), ctx->stream));  // spills, work counter
+    int* nout = nullptr;  // spills, work counter
+    TSIM_TRY(fresh_counter(ctx, to_spill ? *nspill : ntmp, &nout));
+    if (to_spill) *nspill = nout;
     if (warps == 1)
       TSIM_TRY((launch_diag_r<P, 1>(ctx, rs[p], in, max_m, out, nout)));
     else if (warps == 2)
@@ -521,18 +526,18 @@ int launch_chain(tsim_ctx* ctx, int R0, int warps, const DpArgs& a, int max_m, i
 }  // namespace
 
 int launch_dp_diag(tsim_ctx* ctx, int kind, int R, const DpArgs& a, int max_m, int* spill,
-                   int* nspill, int* tmp, int* ntmp, int warps, int rmax) {
+                   int** nspill, int* tmp, int* ntmp, int warps, int rmax, bool* all) {
   const int W = warps > 2 ? kCtaWarps : warps;
   switch (kind) {
-    case DP_DTW_SQ: return launch_chain<PolDtwSq>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
-    case DP_DTW_EU: return launch_chain<PolDtwEu>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
-    case DP_LCSS: return launch_chain<PolLcss>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
+    case DP_DTW_SQ: return launch_chain<PolDtwSq>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax, all);
+    case DP_DTW_EU: return launch_chain<PolDtwEu>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax, all);
+    case DP_LCSS: return launch_chain<PolLcss>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax, all);
     case DP_FRECHET_SQ:
-      return launch_chain<PolFrechetSq>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
-    case DP_DTW_SQC: return launch_chain<PolDtwSqC>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
-    case DP_DTW_EUC: return launch_chain<PolDtwEuC>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
+      return launch_chain<PolFrechetSq>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax, all);
+    case DP_DTW_SQC: return launch_chain<PolDtwSqC>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax, all);
+    case DP_DTW_EUC: return launch_chain<PolDtwEuC>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax, all);
     case DP_FRECHET_SQC:
-      return launch_chain<PolFrechetSqC>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax);
+      return launch_chain<PolFrechetSqC>(ctx, R, W, a, max_m, spill, nspill, tmp, ntmp, rmax, all);
   }
   return fail(TSIM_ERR_UNSUPPORTED, "no anti-diagonal kernel for this DP kind");
 }

@@ -412,9 +412,10 @@ int lane_ring_for(int kind, int max_n, int max_m, int band_pct, int delta) {
   return u <= 64 ? 64 : 128;
 }
 
-int launch_dp_lane(tsim_ctx* ctx, int kind, const DpArgs& a, int ring, int* spill, int* nspill,
+int launch_dp_lane(tsim_ctx* ctx, int kind, const DpArgs& a, int ring, int* spill, int** nspill_io,
                    int gate) {
-  TSIM_CUDA(cudaMemsetAsync(nspill, 0, sizeof(int), ctx->stream));
+  TSIM_TRY(fresh_counter(ctx, *nspill_io, nspill_io));
+  int* nspill = *nspill_io;
   if (a.npairs <= 0) return TSIM_OK;
   switch (kind) {
     case DP_DTW_SQ: return launch_lane_ring<PolDtwSq>(ctx, a, ring, spill, nspill, gate);

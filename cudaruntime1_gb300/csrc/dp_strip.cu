@@ -384,8 +384,9 @@ int launch_half(tsim_ctx* ctx, const DpArgs& a, int cap, int* spill, int* nspill
 
 template <class P>
 int launch_strip_one(tsim_ctx* ctx, const DpArgs& a, int max_n, int max_m, int* spill,
-                     int* nspill) {
-  if (nspill) TSIM_CUDA(cudaMemsetAsync(nspill, 0, sizeof(int), ctx->stream));
+                     int** nspill_io) {
+  if (nspill_io) TSIM_TRY(fresh_counter(ctx, *nspill_io, nspill_io));
+  int* nspill = nspill_io ? *nspill_io : nullptr;
   if (a.npairs <= 0) return TSIM_OK;
   // the inner side can always be one of at most the smaller of the longest
   // lengths, so staging is sized for that (with unknown query lengths, for
@@ -664,8 +665,9 @@ __global__ void __launch_bounds__(kDecideThreads, 4)
 
 }  // namespace
 
-int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest) {
-  TSIM_CUDA(cudaMemsetAsync(nrest, 0, sizeof(int), ctx->stream));
+int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int** nrest_io) {
+  TSIM_TRY(fresh_counter(ctx, *nrest_io, nrest_io));
+  int* nrest = *nrest_io;
   if (a.npairs <= 0) return TSIM_OK;
   const int blocks = std::min(a.npairs, 16 * ctx->num_sms);
   frechet_window_kernel<<<blocks, kStripThreads, 0, ctx->stream>>>(a, rest, nrest);
@@ -674,8 +676,9 @@ int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest)
   return TSIM_OK;
 }
 
-int launch_frechet_decide(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest) {
-  TSIM_CUDA(cudaMemsetAsync(nrest, 0, sizeof(int), ctx->stream));
+int launch_frechet_decide(tsim_ctx* ctx, const DpArgs& a, int* rest, int** nrest_io) {
+  TSIM_TRY(fresh_counter(ctx, *nrest_io, nrest_io));
+  int* nrest = *nrest_io;
   if (a.npairs <= 0) return TSIM_OK;
   const int blocks = std::min(a.npairs, 4 * ctx->num_sms);
   frechet_decide_kernel<<<blocks, kDecideThreads, 0, ctx->stream>>>(a, rest, nrest);
@@ -693,7 +696,7 @@ bool strip_kind(int kind) {
 int strip_max_cols() { return kStripMaxCols; }
 
 int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
-                    int* nspill) {
+                    int** nspill) {
   switch (kind) {
     case DP_DTW_REF: return launch_strip_one<PolDtwRef>(ctx, a, max_n, max_m, spill, nspill);
     case DP_FRECHET_REF: return launch_strip_one<PolFrechetRef>(ctx, a, max_n, max_m, spill, nspill);

@@ -419,7 +419,7 @@ int launch_wave_one(tsim_ctx* ctx, const DpArgs& a, int ccap, int qcap, int* spi
 
 template <class P>
 int wave_chain(tsim_ctx* ctx, const DpArgs& a, int max_n, int max_m, bool latency, int* spill,
-               int* nspill) {
+               int** nspill_io) {
   // one launch: R = 1 for the pairs whose widest anti-diagonal fits 32
   // lanes, R = 2 for the others (the longest lengths give the widest band);
   // pairs longer than the staging capacity or wider than 64 cells per
@@ -427,7 +427,8 @@ int wave_chain(tsim_ctx* ctx, const DpArgs& a, int max_n, int max_m, bool latenc
   const int ccap = (std::min(max_m, kWaveMaxLen) + 1) & ~1;
   const int qcap = (std::min(max_n, kWaveMaxLen) + 1) & ~1;
   const int lmax = wave_lmax(max_n, max_m, band_w(max_n, max_m, a.band_pct));
-  TSIM_CUDA(cudaMemsetAsync(nspill, 0, sizeof(int), ctx->stream));
+  TSIM_TRY(fresh_counter(ctx, *nspill_io, nspill_io));
+  int* nspill = *nspill_io;
   if (latency)
     return lmax <= 32 ? launch_wave_one<P, 1, true>(ctx, a, ccap, qcap, spill, nspill)
                       : launch_wave_one<P, 2, true>(ctx, a, ccap, qcap, spill, nspill);
@@ -442,8 +443,17 @@ bool wave_kind(int kind) {
          kind == DP_DTW_EUC || kind == DP_FRECHET_SQC;
 }
 
+bool wave_takes_all(int max_n, int max_m, int band_pct) {
+  if (max_n > kWaveMaxLen || max_m > kWaveMaxLen) return false;
+  // a pair's anti-diagonals hold at most min(n, m) cells and, as
+  // 2 (min(n, m) - 1) <= n + m - 2, at most its band width + 1
+  const int w = band_w(max_n, max_m, band_pct), mn = std::min(max_n, max_m);
+  const int most = w < 0 ? mn : std::min(mn, w + 1);
+  return most <= (wave_lmax(max_n, max_m, w) <= 32 ? 32 : 64);  // cells of the launch's lanes
+}
+
 int launch_dp_wave(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, bool latency,
-                   int* spill, int* nspill) {
+                   int* spill, int** nspill) {
   switch (kind) {
     case DP_DTW_SQ: return wave_chain<PolDtwSq>(ctx, a, max_n, max_m, latency, spill, nspill);
     case DP_DTW_EU: return wave_chain<PolDtwEu>(ctx, a, max_n, max_m, latency, spill, nspill);

@@ -59,6 +59,7 @@ constexpr int kSeg = 2048;       // list entries per CTA of the two-level select
 constexpr int kLb2Warps = 8;
 constexpr int kGridWords = 4096;  // LCSS occupancy grid of a query: 131,072 cells (16 KiB)
 constexpr int kQBlocks = 8;       // row blocks of a query in the O(1) bound
+constexpr int kCallCounters = 48;  // counters a call's launches take (more are cleared one by one)
 
 enum Meas { M_DTW = 0, M_LCSS = 1, M_FRECHET = 2, M_HAUSDORFF = 3, M_EUCLID = 4 };
 
@@ -88,6 +89,10 @@ struct KArgs {
   int C;
   int max_clen;
   int max_qlen;  // shared-memory tables are sized for this query length
+  int min_qlen, min_clen;  // shortest lengths, where known (else 0: not even that no query
+                           // is longer than max_qlen)
+  int* ctr;                // the call's counters (fresh_counter), zeroed by prep_kernel
+  int nctr;
   // parameters
   int k, S, T, nch;
   int plain;    // one DP pair per kernel launch (the unbatched comparison form)
@@ -224,24 +229,76 @@ __device__ __forceinline__ float block_bound(const KArgs& a, const float4* qblk,
   return acc;
 }
 
-// one warp per query: lane b < kQBlocks reduces block b's box
-__global__ void qblocks_kernel(const float2* __restrict__ pts, const int64_t* __restrict__ off,
-                               int nq, float4* __restrict__ qblk) {
+// First kernel of a call.  A warp per query: its row blocks' boxes, and from
+// them its summary (box, first and last point, length).  All threads: what
+// the call starts from zero (seed bits, shape counts, counters), and for a
+// brute-force call the list of all pairs, query by query, with seeds and round
+// 1 left empty.  One launch, because a small call's time is its chain of
+// dependent graph nodes, not their work: with the counters zeroed here (a
+// memset node a DP launch before) and the launches left out for which no pair
+// can be left over (run_dp), one query against 10,000 trajectories went from
+// 382 to 341 us, 4 x 100 all-pairs DTW from 155 to 141.
+__global__ void __launch_bounds__(256) prep_kernel(KArgs a, float4* qbox, float4* qends, int* qlen,
+                                                   int shapes) {
   const int lane = threadIdx.x & 31;
-  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q >= nq || lane >= kQBlocks) return;
-  const int64_t o = off[q];
-  const int n = (int)(off[q + 1] - o);
-  const int r0 = (int)((long long)lane * n / kQBlocks), r1 = (int)((long long)(lane + 1) * n / kQBlocks);
-  float x0 = TSIM_INF, y0 = TSIM_INF, x1 = -TSIM_INF, y1 = -TSIM_INF;
-  for (int r = r0; r < r1; ++r) {
-    const float2 p = pts[o + r];
-    x0 = fminf(x0, p.x);
-    y0 = fminf(y0, p.y);
-    x1 = fmaxf(x1, p.x);
-    y1 = fmaxf(y1, p.y);
+  const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t nthreads = (size_t)gridDim.x * blockDim.x;
+  for (size_t q = tid >> 5; q < (size_t)a.nq; q += nthreads >> 5) {
+    const int64_t o = a.qoff[q];
+    const int n = (int)(a.qoff[q + 1] - o);
+    const float2* A = a.qpts + o;
+    float4 box = make_float4(TSIM_INF, TSIM_INF, -TSIM_INF, -TSIM_INF);
+    for (int b = 0; b < kQBlocks; ++b) {
+      const int r0 = (int)((long long)b * n / kQBlocks), r1 = (int)((long long)(b + 1) * n / kQBlocks);
+      float x0 = TSIM_INF, y0 = TSIM_INF, x1 = -TSIM_INF, y1 = -TSIM_INF;
+      for (int r = r0 + lane; r < r1; r += 32) {
+        const float2 p = A[r];
+        x0 = fminf(x0, p.x);
+        y0 = fminf(y0, p.y);
+        x1 = fmaxf(x1, p.x);
+        y1 = fmaxf(y1, p.y);
+      }
+      for (int s = 16; s; s >>= 1) {
+        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, s));
+        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, s));
+        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, s));
+        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, s));
+      }
+      if (lane == 0) a.qblk[q * kQBlocks + b] = make_float4(x0, y0, x1, y1);
+      box = make_float4(fminf(box.x, x0), fminf(box.y, y0), fmaxf(box.z, x1), fmaxf(box.w, y1));
+    }
+    if (lane == 0) {
+      qbox[q] = box;
+      qlen[q] = n;
+      if (n > 0) {
+        const float2 f = A[0], l = A[n - 1];
+        qends[q] = make_float4(f.x, f.y, l.x, l.y);
+      } else {
+        qends[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
   }
-  qblk[(size_t)q * kQBlocks + lane] = make_float4(x0, y0, x1, y1);
+  for (size_t i = tid; i < (size_t)a.nctr * kCounterInts; i += nthreads) a.ctr[i] = 0;
+  if (tid < 2) a.n64[tid] = 0;
+  if (a.brute) {
+    const size_t np = (size_t)a.nq * a.C;
+    for (size_t i = tid; i < np; i += nthreads) {
+      const int q = (int)(i / a.C), c = (int)(i % a.C);
+      a.flat[i] = make_int2(q, c);
+      if (c == 0) {
+        a.off2[q] = q * a.C;
+        a.fcnt[q] = a.C;
+        a.cnt1[q] = a.C;
+        a.cnt2[q] = a.C;
+        for (int k = 0; k < a.S; ++k) a.seeds[(size_t)q * a.S + k] = make_int2(q, -1);
+        for (int k = 0; k < a.M; ++k) a.r1pairs[(size_t)q * a.M + k] = make_int2(q, -1);
+      }
+      if (i == 0) *a.npairs = (int)np;
+    }
+  } else {
+    for (size_t i = tid; i < (size_t)a.nq * a.Cw; i += nthreads) a.seedmap[i] = 0u;
+    for (size_t i = tid; i < (size_t)shapes; i += nthreads) a.shape_cnt[i] = 0;
+  }
 }
 
 template <int MEAS>
@@ -1686,13 +1743,6 @@ __global__ void __launch_bounds__(1024) scan_kernel(KArgs a) {
   }
 }
 
-__global__ void flatten_kernel(KArgs a) {
-  const int q = blockIdx.y;
-  const int cnt = a.fcnt[q], base = a.off2[q];
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x)
-    a.flat[base + e] = make_int2(q, a.list1[(size_t)q * a.C + e]);
-}
-
 // Shape-sorted schedule of the survivor pairs: counting sort by ((query +
 // candidate length) / 32, longer length / 16), longest first, so that the
 // pairs sharing a warp have similar shapes (a warp runs as long as its
@@ -1708,11 +1758,14 @@ __device__ __forceinline__ int shape_key(int n, int m) {
          min(max(n, m) >> 4, (1 << kShapeBits) - 1);
 }
 
-__global__ void shape_hist_kernel(KArgs a) {
-  const int np = *a.npairs;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const int2 pr = a.flat[i];
-    atomicAdd(a.shape_cnt + (kNumShapes - 1 - shape_key(a.qlen[pr.x], a.clen[pr.y])), 1);
+// the queries' survivor lists side by side, and (sorted) their shape counts
+__global__ void flatten_kernel(KArgs a, int sorted) {
+  const int q = blockIdx.y;
+  const int cnt = a.fcnt[q], base = a.off2[q], n = a.qlen[q];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
+    const int c = a.list1[(size_t)q * a.C + e];
+    a.flat[base + e] = make_int2(q, c);
+    if (sorted) atomicAdd(a.shape_cnt + (kNumShapes - 1 - shape_key(n, a.clen[c])), 1);
   }
 }
 
@@ -2017,12 +2070,6 @@ __global__ void __launch_bounds__(32 * kRankWarps) final_sort_kernel(KArgs a) {
   }
 }
 
-__global__ void clear_u32_kernel(unsigned* p, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    p[i] = 0;
-}
-
 // Per-request counters, accumulated on the device (no host sync per chunk):
 // counters[2..6] += pairs passing the O(1) bound, the O(length) bound,
 // refined pairs, re-scored pairs, FP64 re-scored pairs.
@@ -2070,24 +2117,27 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
     // 5,120 Frechet pairs of up to 256 x 1,024 points 1,438 us on a CTA of
     // row groups and 2,317 on a warp (eight passes, R = 1 .. 8) -> 208 us;
     // the same compensated 4,406 -> 1,004 us
-    TSIM_TRY(launch_dp_strip(ctx, kind, d, d.max_n > 0 ? d.max_n : a.max_qlen, a.max_clen, a.waves,
-                             a.nwaves));
+    int* nw = a.nwaves;
+    const int mq = d.max_n > 0 ? d.max_n : a.max_qlen;
+    TSIM_TRY(launch_dp_strip(ctx, kind, d, mq, a.max_clen, a.waves, &nw));
+    if (a.min_qlen > 0 && std::min(mq, a.max_clen) <= strip_max_cols()) return TSIM_OK;
     DpArgs rest = d;  // pairs with both sides too long to stage
     rest.order = a.waves;
-    rest.npairs_dev = a.nwaves;
+    rest.npairs_dev = nw;
     return launch_dp(ctx, kind, G, R, rest, a.max_clen);
   }
   // bit vectors, in every round: a round's time follows the columns that can
   // match, not the window's cells, so there is no gate on its size
   if (a.wave && lcss_window_kind(kind, d.delta)) return launch_lcss_window(ctx, d);
-  if (!latency && a.lane_gate > 0 && lane_kind(kind)) {
+  if (!latency && a.lane_gate > 0 && d.npairs >= a.lane_gate && lane_kind(kind)) {
     // many pairs: a lane per pair, with a latency of one pair's cells but a
     // few instructions per cell; the kernel itself passes a round of fewer
     // than lane_gate pairs (a count only the device knows) on whole
-    TSIM_TRY(launch_dp_lane(ctx, kind, d, a.lane_ring, a.lanes, a.nlanes, a.lane_gate));
+    int* nl = a.nlanes;
+    TSIM_TRY(launch_dp_lane(ctx, kind, d, a.lane_ring, a.lanes, &nl, a.lane_gate));
     DpArgs rest = d;
     rest.order = a.lanes;
-    rest.npairs_dev = a.nlanes;
+    rest.npairs_dev = nl;
     KArgs b = a;
     b.lane_gate = 0;
     return run_dp(ctx, b, kind, G, R, rest, latency);
@@ -2102,11 +2152,18 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
     // latency rounds and the survivor round (after the lane kernel's gate);
     // pairs with more than 64 cells per anti-diagonal go on to the row-group
     // kernels
-    TSIM_TRY(launch_dp_wave(ctx, kind, d, d.max_n > 0 ? d.max_n : a.max_qlen, a.max_clen, latency,
-                            a.waves, a.nwaves));
+    int* nw = a.nwaves;
+    const int mq = d.max_n > 0 ? d.max_n : a.max_qlen;
+    TSIM_TRY(launch_dp_wave(ctx, kind, d, mq, a.max_clen, latency, a.waves, &nw));
     DpArgs rest = d;
     rest.order = a.waves;
-    rest.npairs_dev = a.nwaves;
+    rest.npairs_dev = nw;
+    if (wave_takes_all(mq, a.max_clen, d.band_pct)) {
+      // only degenerate pairs can be left, which no row-group kernel takes
+      // either; none where every length is known to be at least two
+      if (a.min_qlen >= 2 && a.min_clen >= 2) return TSIM_OK;
+      return launch_dp(ctx, kind, G, R, rest, a.max_clen);
+    }
     KArgs b = a;
     b.wave = 0;
     return run_dp(ctx, b, kind, G, R, rest, latency);
@@ -2121,35 +2178,38 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
   // with abandoning) ran slower on two warps, so they keep one.
   const bool w2 = latency && a.rdiag_w2 > 0 && a.rdiag_w2 <= 2 &&
                   (twofloat || d.npairs <= 4 * ctx->num_sms);
+  int *ns = a.nspill, *ns1 = a.nlanes;
+  bool all = false;  // the row groups take every pair of at least two points a side
   if (!w2 && latency && a.rdiag_cta > 0 && a.rdiag_shape >= (twofloat ? 4 : 8)) {
     // the longest pair needs a CTA, but a round's lengths vary (lognormal
     // Frechet queries): the pairs that fit a warp with up to 8 rows per lane
     // run there, each at its fewest rows, the rest on a CTA per pair from
     // one row per lane up -- instead of every pair at the longest pair's R
-    TSIM_TRY(launch_dp_diag(ctx, kind, 1, d, a.max_clen, a.lanes, a.nlanes, a.spill2, a.nspill2, 1,
+    TSIM_TRY(launch_dp_diag(ctx, kind, 1, d, a.max_clen, a.lanes, &ns1, a.spill2, a.nspill2, 1,
                             twofloat ? 4 : 8));
     DpArgs rest = d;
     rest.order = a.lanes;
-    rest.npairs_dev = a.nlanes;
-    TSIM_TRY(launch_dp_diag(ctx, kind, 1, rest, a.max_clen, a.spill, a.nspill, a.spill2,
-                            a.nspill2, 8));
+    rest.npairs_dev = ns1;
+    TSIM_TRY(launch_dp_diag(ctx, kind, 1, rest, a.max_clen, a.spill, &ns, a.spill2, a.nspill2, 8, 0,
+                            &all));
   } else if (w2 || (latency && twofloat && a.rdiag_shape >= 2 && a.rdiag_w2 > 0)) {
     // two warps per pair: a compensated row per lane and step, for a barrier
     // of two warps
-    TSIM_TRY(launch_dp_diag(ctx, kind, a.rdiag_w2, d, a.max_clen, a.spill, a.nspill, a.spill2,
-                            a.nspill2, 2));
+    TSIM_TRY(launch_dp_diag(ctx, kind, a.rdiag_w2, d, a.max_clen, a.spill, &ns, a.spill2, a.nspill2,
+                            2, 0, &all));
   } else {
     // latency rounds start at the smallest R the longest pair admits; the
     // survivor round at the tuned R (which may be smaller: its first pass
     // then runs the narrow-band pairs with fewer rows per lane and passes the
     // others on)
     const int r0 = latency ? std::max(a.rdiag, a.rdiag_shape) : a.rdiag;
-    TSIM_TRY(launch_dp_diag(ctx, kind, r0, d, a.max_clen, a.spill, a.nspill, a.spill2,
-                            a.nspill2));
+    TSIM_TRY(launch_dp_diag(ctx, kind, r0, d, a.max_clen, a.spill, &ns, a.spill2, a.nspill2, 1, 0,
+                            &all));
   }
+  if (all && a.min_qlen >= 2 && a.min_clen >= 2) return TSIM_OK;
   DpArgs sp = d;
   sp.order = a.spill;
-  sp.npairs_dev = a.nspill;
+  sp.npairs_dev = ns;
   return launch_dp(ctx, kind, G, R, sp, a.max_clen);
 }
 
@@ -2207,17 +2267,20 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
     r.out64 = a.r64;
     if (MEAS == M_FRECHET) {  // exact FP64 values from the FP32 ones: no FP64 DP
       r.aux = a.rdc;
-      TSIM_TRY(launch_frechet_window(ctx, r, a.spill2, a.nspill2));
+      int *ns = a.nspill, *ns2 = a.nspill2, *nl = a.nlanes;
+      TSIM_TRY(launch_frechet_window(ctx, r, a.spill2, &ns2));
       r.order = a.spill2;
-      r.npairs_dev = a.nspill2;
-      TSIM_TRY(launch_frechet_decide(ctx, r, a.spill, a.nspill));
+      r.npairs_dev = ns2;
+      TSIM_TRY(launch_frechet_decide(ctx, r, a.spill, &ns));
       r.order = a.spill;
-      r.npairs_dev = a.nspill;
-      TSIM_TRY(launch_dp_strip(ctx, DP_FRECHET_WIN, r, a.max_qlen, a.max_clen, a.lanes, a.nlanes));
-      DpArgs sp = r;
-      sp.order = a.lanes;
-      sp.npairs_dev = a.nlanes;
-      TSIM_TRY(launch_dp(ctx, DP_FRECHET_WIN, 32, 1, sp, a.max_clen));
+      r.npairs_dev = ns;
+      TSIM_TRY(launch_dp_strip(ctx, DP_FRECHET_WIN, r, a.max_qlen, a.max_clen, a.lanes, &nl));
+      if (a.min_qlen == 0 || std::min(a.max_qlen, a.max_clen) > strip_max_cols()) {
+        DpArgs sp = r;
+        sp.order = a.lanes;
+        sp.npairs_dev = nl;
+        TSIM_TRY(launch_dp(ctx, DP_FRECHET_WIN, 32, 1, sp, a.max_clen));
+      }
     } else if (is_dp(MEAS)) {
       TSIM_TRY(launch_dp(ctx, dp64, 32, 1, r, a.max_clen));
     } else {
@@ -2239,37 +2302,11 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
 }
 
 // Every pair of a small request refined exactly: the bound stages cost more
-// (a chain of dependent launches) than they save.  Seeds and round 1 are
-// left empty; the flat list holds all pairs, query by query.
-__global__ void brute_setup_kernel(KArgs a) {
-  const size_t np = (size_t)a.nq * a.C;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < np;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int q = (int)(i / a.C), c = (int)(i % a.C);
-    a.flat[i] = make_int2(q, c);
-    if (c == 0) {
-      a.off2[q] = q * a.C;
-      a.fcnt[q] = a.C;
-      a.cnt1[q] = a.C;
-      a.cnt2[q] = a.C;
-      for (int k = 0; k < a.S; ++k) a.seeds[(size_t)q * a.S + k] = make_int2(q, -1);
-      for (int k = 0; k < a.M; ++k) a.r1pairs[(size_t)q * a.M + k] = make_int2(q, -1);
-    }
-    if (i == 0) *a.npairs = (int)np;
-  }
-}
-
+// (a chain of dependent launches) than they save.
 template <int MEAS>
 int run_brute(tsim_ctx* ctx, KArgs& a, int dp32, int dpc, int dp64) {
-  cudaStream_t s = ctx->stream;
   const int nq = a.nq;
   const size_t np = (size_t)nq * a.C;
-  TSIM_CUDA(cudaMemsetAsync(a.n64, 0, 2 * sizeof(int), s));
-  stage_begin(ctx, TSIM_STAGE_FILTER);
-  brute_setup_kernel<<<(unsigned)std::min<size_t>((np + 255) / 256, 4096), 256, 0, s>>>(a);
-  TSIM_CUDA(cudaGetLastError());
-  launched(ctx);
-  stage_end(ctx);
   stage_begin(ctx, TSIM_STAGE_DP_SURVIVORS);
   DpArgs d{};
   d.qpts = a.qpts;
@@ -2298,10 +2335,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   if (a.brute) return run_brute<MEAS>(ctx, a, dp32, dpc, dp64);
   cudaStream_t s = ctx->stream;
   const int nq = a.nq;
-  TSIM_CUDA(cudaMemsetAsync(a.n64, 0, 2 * sizeof(int), s));
   stage_begin(ctx, TSIM_STAGE_LB1);
-  clear_u32_kernel<<<std::min<size_t>(((size_t)nq * a.Cw + 255) / 256, 4096), 256, 0, s>>>(
-      a.seedmap, (size_t)nq * a.Cw);
   if constexpr (MEAS == M_EUCLID) {
     qprefix_kernel<<<nq, 256, 0, s>>>(a);
     paa_kernel<<<dim3(a.nch, (nq + kPaaQueries - 1) / kPaaQueries), kChunk, 0, s>>>(a);
@@ -2310,7 +2344,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     lb1_kernel<MEAS><<<dim3(a.nch, (nq + kLb1Queries - 1) / kLb1Queries), kChunk, 0, s>>>(a);
   }
   stage_end(ctx);
-  launched(ctx, 2);
+  launched(ctx);
   stage_begin(ctx, TSIM_STAGE_SEED);
   const size_t seed_smem = sizeof(unsigned long long) * (size_t)a.nch * a.T;
   if (seed_smem > 48 * 1024)
@@ -2426,19 +2460,16 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     a.fcnt = a.cnt0;
   }
   scan_kernel<<<1, 1024, 0, s>>>(a);
-  flatten_kernel<<<dim3(ch, nq), 256, 0, s>>>(a);
   // the shape order serves the kernels whose warps run as long as their
   // longest pair; the LCSS bit vectors gain more from one query's pairs side
   // by side
   const bool sorted = !(MEAS == M_LCSS && a.wave && lcss_window_kind(dp32, a.delta));
+  flatten_kernel<<<dim3(ch, nq), 256, 0, s>>>(a, sorted);
   launched(ctx, 3);
   if (sorted) {
-    TSIM_CUDA(cudaMemsetAsync(a.shape_cnt, 0, sizeof(int) * kNumShapes, s));
-    const int sb = ctx->num_sms * 4;
-    shape_hist_kernel<<<sb, 256, 0, s>>>(a);
     shape_scan_kernel<<<1, 1024, 0, s>>>(a);
-    shape_scatter_kernel<<<sb, 256, 0, s>>>(a);
-    launched(ctx, 3);
+    shape_scatter_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(a);
+    launched(ctx, 2);
   }
   TSIM_CUDA(cudaGetLastError());
   stage_end(ctx);
@@ -2610,21 +2641,21 @@ size_t knn_plan(const tsim_params* p, int nq, int max_qlen, const tsim_db* db, K
                 align256(sizeof(float) * nqC) + align256(sizeof(int) * nq * a.nch * a.T) +
                 align256(sizeof(int2) * nq * a.S) + align256(sizeof(unsigned) * nq * a.Cw) +
                 align256(sizeof(float) * nq * a.S) + align256(sizeof(float) * nq) +
-                4 * align256(sizeof(int) * (nq + 1)) + 2 * align256(sizeof(int) * nq * (size_t)a.RC) +
-                2 * align256(sizeof(int) * nqC) +
+                4 * align256(sizeof(int) * (nq + 1)) + 2 * align256(sizeof(int) * nqC) +
                 align256(sizeof(int) * 4) + align256(sizeof(int2) * nqC) +
                 align256(sizeof(float) * nqC) +
                 align256(sizeof(unsigned long long) * nq * (size_t)a.nseg * 64) +
                 align256(sizeof(unsigned long long) * nq) + align256(sizeof(int) * nq) +
                 2 * align256(sizeof(int2) * nq * a.RC) + 2 * align256(sizeof(double) * nq * a.RC) +
-                align256(sizeof(int) * nqC) + align256(sizeof(int) * kNumShapes) + 256 +
+                align256(sizeof(int) * nqC) + align256(sizeof(int) * kNumShapes) +
+                align256(sizeof(int) * kCounterInts * (5 + kCallCounters)) +
                 align256(sizeof(float) * nqC) + align256(sizeof(int2) * nq * a.M) +
                 align256(sizeof(float) * nq * a.M) + 2 * align256(sizeof(float) * (nq + 1)) +
                 align256(sizeof(float4) * (size_t)nq * a.tstride) +
                 align256(sizeof(float4) * (size_t)nq * a.env_stride) +
                 align256(sizeof(float2) * (size_t)nq * (max_qlen + 1)) + align256(sizeof(float) * nq) +
                 align256(sizeof(float4) * (size_t)nq * kQBlocks) +
-                4 * align256(sizeof(int) * (size_t)nq * std::max(C, a.RC)) + 4 * 256;
+                4 * align256(sizeof(int) * (size_t)nq * std::max(C, a.RC));
   return need;
 }
 
@@ -2687,9 +2718,18 @@ int knn(tsim_ctx* ctx, const tsim_params* p, const float2* qpts, const int64_t* 
   a.r64 = arena_take<double>(ctx, (size_t)nq * a.RC);
   a.rdc = arena_take<double>(ctx, (size_t)nq * a.RC);
   a.r64pairs = arena_take<int2>(ctx, (size_t)nq * a.RC);
-  a.n64 = arena_take<int>(ctx, 4);
-  a.rlist = arena_take<int>(ctx, (size_t)nq * a.RC);
-  a.r64list = arena_take<int>(ctx, (size_t)nq * a.RC);
+  // the re-score sets (distinct candidates, so at most C a query) come when
+  // the bound stages' lists are done with
+  a.rlist = a.list1;
+  a.r64list = a.list2;
+  int* counters_mem = arena_take<int>(ctx, (5 + kCallCounters) * kCounterInts);
+  a.n64 = counters_mem;
+  a.nspill = a.n64 + kCounterInts;
+  a.nspill2 = a.nspill + kCounterInts;
+  a.nlanes = a.nspill2 + kCounterInts;
+  a.nwaves = a.nlanes + kCounterInts;
+  a.ctr = a.nwaves + kCounterInts;
+  a.nctr = kCallCounters;
   a.lb2v = arena_take<float>(ctx, nqC);
   a.r1pairs = arena_take<int2>(ctx, (size_t)nq * a.M);
   a.r1vals = arena_take<float>(ctx, (size_t)nq * a.M);
@@ -2701,13 +2741,9 @@ int knn(tsim_ctx* ctx, const tsim_params* p, const float2* qpts, const int64_t* 
   a.qpe = arena_take<float>(ctx, nq);
   a.qblk = arena_take<float4>(ctx, (size_t)nq * kQBlocks);
   a.spill = arena_take<int>(ctx, (size_t)nq * std::max(C, a.RC));
-  a.nspill = arena_take<int>(ctx, 4);
   a.spill2 = arena_take<int>(ctx, (size_t)nq * std::max(C, a.RC));
-  a.nspill2 = arena_take<int>(ctx, 4);
   a.lanes = arena_take<int>(ctx, (size_t)nq * std::max(C, a.RC));
-  a.nlanes = arena_take<int>(ctx, 4);
   a.waves = arena_take<int>(ctx, (size_t)nq * std::max(C, a.RC));
-  a.nwaves = arena_take<int>(ctx, 4);
   a.csegbox = db->segbox;
   a.csegsum = db->segsum;
   // bulk copies of candidate points (DTW's O(length) stage): buffers of up to
@@ -2727,10 +2763,24 @@ int knn(tsim_ctx* ctx, const tsim_params* p, const float2* qpts, const int64_t* 
   a.shape_cnt = arena_take<int>(ctx, kNumShapes);
   if (!a.shape_cnt) return fail(TSIM_ERR_OUT_OF_MEMORY, "knn scratch carve failed");
 
+  // the call's counters: handed out while this scope lasts
+  struct Counters {
+    tsim_ctx* ctx;
+    Counters(tsim_ctx* c, int* base, int n) : ctx(c) {
+      c->ctr = base;
+      c->ctr_n = n;
+      c->ctr_used = 0;
+    }
+    ~Counters() { ctx->ctr_n = 0; }
+  } counters(ctx, a.ctr, a.nctr);
+  a.min_clen = db->min_len;
+  a.min_qlen = ctx->exact_qlen ? std::max(1, ctx->min_qlen) : 0;
   stage_begin(ctx, TSIM_STAGE_SUMMARY);
-  TSIM_TRY(summarize(ctx, qpts, qoff, nq, qbox, qends, qlen));
-  if (p->measure != TSIM_EUCLIDEAN && !a.brute) {  // read by lb1_kernel only
-    qblocks_kernel<<<(nq + 3) / 4, 128, 0, ctx->stream>>>(qpts, qoff, nq, a.qblk);
+  {
+    const size_t items = a.brute ? nqC : std::max<size_t>((size_t)nq * a.Cw / 4, kNumShapes);
+    const size_t threads = std::max<size_t>((size_t)nq * 32, std::min<size_t>(items, (size_t)1 << 20));
+    prep_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(a, qbox, qends, qlen,
+                                                                            kNumShapes);
     TSIM_CUDA(cudaGetLastError());
     launched(ctx);
   }
@@ -2779,7 +2829,8 @@ std::vector<uint64_t> graph_key(tsim_ctx* ctx, const tsim_params* p, const void*
           eps, (uint64_t)(uint32_t)p->delta, p->flags, (uint64_t)nq, (uint64_t)max_qlen,
           (uint64_t)(uintptr_t)db, (uint64_t)db->count, (uint64_t)(uintptr_t)qpts,
           (uint64_t)(uintptr_t)qoff, (uint64_t)(uintptr_t)ids, (uint64_t)(uintptr_t)dists,
-          (uint64_t)(uintptr_t)d64, (uint64_t)ctx->concurrency, tuned_tag(ctx, p, nq, max_qlen, db)};
+          (uint64_t)(uintptr_t)d64, (uint64_t)ctx->concurrency, tuned_tag(ctx, p, nq, max_qlen, db),
+          (uint64_t)(ctx->exact_qlen ? std::min(ctx->min_qlen, 2) : 0)};
 }
 
 std::vector<uint64_t> arena_gens(tsim_ctx* ctx) {
@@ -2947,7 +2998,11 @@ int knn_request(tsim_ctx* ctx, const tsim_params* p, const tsim_point* d_qpts,
       TSIM_CUDA(cudaStreamWaitEvent(s->stream, ctx->fork_ev, 0));
     }
   }
-  for (tsim_ctx* c : lanes) c->count_funnel = stats != nullptr;
+  for (tsim_ctx* c : lanes) {
+    c->count_funnel = stats != nullptr;
+    c->exact_qlen = ctx->exact_qlen;
+    c->min_qlen = ctx->min_qlen;
+  }
   if (stats)
     for (tsim_ctx* c : lanes)
       TSIM_CUDA(cudaMemsetAsync(c->dcounters + 2, 0, 5 * sizeof(unsigned long long), c->stream));
@@ -2998,10 +3053,11 @@ extern "C" int tsim_knn_host(tsim_ctx* ctx, const tsim_params* p, const tsim_poi
   TSIM_CHECK_ARG(db->ctx == ctx, "database belongs to another (or a destroyed) context");
   TSIM_CHECK_ARG(nq >= 1 && p->k >= 1 && p->k <= 64, "bad nq or k");
   TSIM_CHECK_ARG(h_qoff[0] == 0, "query offsets must start at 0");
-  int max_qlen = 0;
+  int max_qlen = 0, min_qlen = INT32_MAX;
   for (int i = 0; i < nq; ++i) {
     TSIM_CHECK_ARG(h_qoff[i + 1] > h_qoff[i], "queries must be non-empty");
     max_qlen = std::max<int64_t>(max_qlen, h_qoff[i + 1] - h_qoff[i]);
+    min_qlen = std::min<int64_t>(min_qlen, h_qoff[i + 1] - h_qoff[i]);
   }
   TSIM_CUDA(cudaSetDevice(ctx->device));
   const size_t npts = (size_t)h_qoff[nq];
@@ -3027,9 +3083,13 @@ extern "C" int tsim_knn_host(tsim_ctx* ctx, const tsim_params* p, const tsim_poi
   TSIM_CUDA(cudaMemcpyAsync(dp, hp, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
   int* d_ids = (int*)(dp + in_bytes);
   float* d_d = (float*)(dp + in_bytes + tsim::align256(sizeof(int) * nq * p->k));
-  TSIM_TRY(tsim_knn(ctx, p, (const tsim_point*)dp,
-                    (const int64_t*)(dp + tsim::align256(sizeof(tsim_point) * npts)), nq, max_qlen,
-                    db, d_ids, d_d, nullptr, stats));
+  ctx->exact_qlen = true;  // measured above, for this call only
+  ctx->min_qlen = min_qlen;
+  const int st = tsim_knn(ctx, p, (const tsim_point*)dp,
+                          (const int64_t*)(dp + tsim::align256(sizeof(tsim_point) * npts)), nq,
+                          max_qlen, db, d_ids, d_d, nullptr, stats);
+  ctx->exact_qlen = false;
+  TSIM_TRY(st);
   TSIM_CUDA(cudaMemcpyAsync(hp + in_bytes, dp + in_bytes, out_bytes, cudaMemcpyDeviceToHost,
                             ctx->stream));
   // the status word rides with the results (no extra round trip)
@@ -3127,7 +3187,7 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
   int* sorted = arena_take<int>(ctx, npairs);
   int* buckets = arena_take<int>(ctx, lane_sort_buckets());
   if (kernel == 0 && d.band_pct < 0 && strip_kind(kind)) {  // full rows
-    TSIM_TRY(launch_dp_strip(ctx, kind, d, max_qlen, max_clen, spill, nspill));
+    TSIM_TRY(launch_dp_strip(ctx, kind, d, max_qlen, max_clen, spill, &nspill));
     d.order = spill;
     d.npairs_dev = nspill;
     return launch_dp(ctx, kind, G, R, d, max_clen);
@@ -3146,7 +3206,8 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
       kernel = 6;
   }
   if (kernel == 6 && wave_kind(kind)) {  // band-relative first; wider pairs on the others
-    TSIM_TRY(launch_dp_wave(ctx, kind, d, max_qlen, max_clen, npairs <= 4 * ctx->num_sms, rest, nrest));
+    TSIM_TRY(launch_dp_wave(ctx, kind, d, max_qlen, max_clen, npairs <= 4 * ctx->num_sms, rest,
+                            &nrest));
     d.order = rest;
     d.npairs_dev = nrest;
   } else if (kernel == 5 && lane_kind(kind)) {  // a lane per pair first; wider pairs on a warp
@@ -3155,15 +3216,15 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
     d.order = sorted;
     TSIM_TRY(launch_dp_lane(ctx, kind, d,
                             lane_ring_for(kind, max_qlen, max_clen, d.band_pct, d.delta), rest,
-                            nrest));
+                            &nrest));
     d.order = rest;
     d.npairs_dev = nrest;
   }
   if (kernel == 3 || kernel == 4)
-    TSIM_TRY(launch_dp_diag(ctx, kind, Rc, d, max_clen, spill, nspill, tmp, ntmp,
+    TSIM_TRY(launch_dp_diag(ctx, kind, Rc, d, max_clen, spill, &nspill, tmp, ntmp,
                             kernel == 3 ? 8 : 2));
   else
-    TSIM_TRY(launch_dp_diag(ctx, kind, Rd, d, max_clen, spill, nspill, tmp, ntmp));
+    TSIM_TRY(launch_dp_diag(ctx, kind, Rd, d, max_clen, spill, &nspill, tmp, ntmp));
   d.order = spill;
   d.npairs_dev = nspill;
   return launch_dp(ctx, kind, G, R, d, max_clen);

@@ -247,6 +247,8 @@ int launch(tsim_server* s, Slot& sl) {
   int* ids = reinterpret_cast<int*>(base + sl.o_ids);
   float* dists = reinterpret_cast<float*>(base + sl.o_dists);
   const int k = p.k;
+  c->exact_qlen = true;  // the batch's longest query is measured at submit
+  c->min_qlen = 1;
   const float* thr_in = sl.share ? reinterpret_cast<const float*>(base + sl.o_thr_in) : nullptr;
   float* thr_out = sl.share ? reinterpret_cast<float*>(base + sl.o_thr_out) : nullptr;
   for (int q0 = 0; q0 < sl.nq; q0 += sl.qb) {

@@ -81,6 +81,14 @@ struct tsim_ctx {
   double stage_ms[TSIM_STAGE_COUNT] = {};
   int64_t stage_calls[TSIM_STAGE_COUNT] = {};
   unsigned long long* dcounters = nullptr;  // device: [0] DP cells computed, [kStatusSlot] status
+  // device counters of the current kNN call, zeroed by its first kernel and
+  // handed out by fresh_counter (no memset per launch that needs one)
+  int* ctr = nullptr;
+  int ctr_n = 0, ctr_used = 0;
+  // set by the entry points that measured the queries themselves: no query of
+  // the call is shorter than min_qlen or longer than its max_qlen
+  bool exact_qlen = false;
+  int min_qlen = 0;
   bool count_funnel = false;  // requests add their pruning funnel to dcounters[2..6]
   unsigned* status = nullptr;  // device status word (its own dcounters slot; a chunk context: its parent's)
   // concurrency: a request's queries are split into chunks that run on these
@@ -120,6 +128,7 @@ struct tsim_db {
   int count = 0;
   int64_t total = 0;
   int max_len = 0;
+  int min_len = 0;  // shortest trajectory (0: unknown)
   bool owns = false;
   float2* pts = nullptr;      // device [total]
   int64_t* off = nullptr;     // device [count+1]
@@ -145,6 +154,11 @@ T* arena_take(tsim_ctx* ctx, size_t count) {
   return p;
 }
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
+
+// A device counter of four zeroed ints: one of the call's (ctx->ctr), or
+// `fallback`, cleared on the stream.
+constexpr int kCounterInts = 4;
+int fresh_counter(tsim_ctx* ctx, int* fallback, int** out);
 
 int pinned_reserve(tsim_ctx* ctx, size_t bytes);
 // Every device and pinned-host allocation of the library goes through these,
@@ -331,8 +345,12 @@ int launch_dp(tsim_ctx* ctx, int kind, int G, int R, const DpArgs& a, int max_m)
 // per pair (R up to 16), > 1 = a CTA of 8 warps per pair (R up to 4; for few,
 // long, full-row pairs, where the latency of one pair is the launch's).
 // rmax > 0 caps the chain's R (pairs needing more rows go to spill).
+// nspill: in a counter to fall back on, out the one used (here and in the
+// launchers below).  all, if not null: whether only degenerate pairs (a side
+// of one point, or past max_n x max_m) can be left in spill[].
 int launch_dp_diag(tsim_ctx* ctx, int kind, int R, const DpArgs& a, int max_m, int* spill,
-                   int* nspill, int* tmp, int* ntmp, int warps = 1, int rmax = 0);
+                   int** nspill, int* tmp, int* ntmp, int warps = 1, int rmax = 0,
+                   bool* all = nullptr);
 // Band-relative anti-diagonal kernel (dp_wave.cu) for DTW and Frechet, FP32
 // and compensated (wave_kind): a warp per pair, lane p holding the p-th live
 // cells of the anti-diagonal, R = 1 or 2 cells per lane as the pair needs; pairs
@@ -348,7 +366,9 @@ int status_result(tsim_ctx* ctx, unsigned v);
 // Attempts of the bounded waits on bulk copies (< 0: the default); for tests.
 int set_wait_limit(long long attempts);
 int launch_dp_wave(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, bool latency,
-                   int* spill, int* nspill);
+                   int* spill, int** nspill);
+// whether it takes every pair of at least two points a side up to these lengths
+bool wave_takes_all(int max_n, int max_m, int band_pct);
 // Strip kernel (dp_strip.cu) for pairs without a band (strip_kind: DTW and
 // Frechet, FP32, compensated, the reference's arithmetic and the exact
 // Frechet re-score): a warp per pair, whose shorter side is at most
@@ -357,7 +377,7 @@ int launch_dp_wave(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_
 bool strip_kind(int kind);
 int strip_max_cols();
 int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
-                    int* nspill);
+                    int** nspill);
 // Windowed LCSS by bit vectors (dp_lcss.cu, windows of at most 63 rows): a
 // warp per pair; a.qtab optionally holds the eps-inflated boxes of each
 // query's windows, a.max_n + delta + 1 per query (column j: the box of rows
@@ -367,17 +387,17 @@ int launch_lcss_window(tsim_ctx* ctx, const DpArgs& a);
 // Exact FP64 Frechet values (squared) of the pairs whose window (PolFrechetWin,
 // FP32 values in aux) holds one cost, into out64; the others' entries in rest[]
 // (count in *nrest) for DP_FRECHET_WIN.
-int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest);
+int launch_frechet_window(tsim_ctx* ctx, const DpArgs& a, int* rest, int** nrest);
 // The same of pairs with a few costs in the window, by deciding reachability
 // for them; what is left (many costs, more than 1,024 points on both sides)
 // is for DP_FRECHET_WIN.
-int launch_frechet_decide(tsim_ctx* ctx, const DpArgs& a, int* rest, int* nrest);
+int launch_frechet_decide(tsim_ctx* ctx, const DpArgs& a, int* rest, int** nrest);
 // Lane-per-pair kernel (dp_lane.cu) for the FP32 DTW, Frechet and LCSS
 // kinds (lane_kind): a lane runs a whole pair in passes of 8 rows, the row
 // above a pass in a shared-memory ring of `ring` (64 or 128) values per lane
 // (lane_ring_for picks it from the longest pair); pairs wider than the ring,
 // or with fewer than two points on a side, are left in spill[] (count in
-// *nspill, cleared here).  When the list holds fewer than `gate` pairs (read
+// *nspill).  When the list holds fewer than `gate` pairs (read
 // on the device) the kernel computes nothing and copies the whole list, in
 // order, to spill[] for the warp-per-pair kernels.
 bool lane_kind(int kind);
@@ -390,7 +410,7 @@ int lane_sort_buckets();
 int lane_gate_for(int kind, int max_n, int max_m, int band_pct, int delta, int num_sms,
                   bool abandon = true);
 int lane_ring_for(int kind, int max_n, int max_m, int band_pct, int delta);
-int launch_dp_lane(tsim_ctx* ctx, int kind, const DpArgs& a, int ring, int* spill, int* nspill,
+int launch_dp_lane(tsim_ctx* ctx, int kind, const DpArgs& a, int ring, int* spill, int** nspill,
                    int gate = 0);
 // the anti-diagonal kernel's validity condition for a pair shape, R rows
 // per lane-group and `lanes` lanes per pair

@@ -471,3 +471,30 @@ def test_dtw_row_bounds(tsim, cuda_ctx, oracle, band, cost):
     assert np.array_equal(ids, want_ids)
     assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
     db.close()
+
+
+@pytest.mark.parametrize("least", [1, 2])
+@pytest.mark.parametrize("measure,kw,longest", [
+    ("dtw", dict(band_pct=31), (100, 100)), ("dtw", dict(band_pct=32), (100, 100)),
+    ("dtw", dict(band_pct=63), (100, 90)), ("dtw", dict(band_pct=64), (90, 100)),
+    ("dtw", dict(band_pct=100), (33, 400)), ("dtw", dict(band_pct=100), (400, 65)),
+    ("frechet", dict(band_pct=45), (300, 70)), ("dtw", dict(), (64, 2050)),
+    ("frechet", dict(), (2050, 40)), ("lcss", dict(delta=40), (90, 120))])
+def test_known_lengths(tsim, cuda_ctx, oracle, least, measure, kw, longest):
+    """A request whose lengths are known launches no kernel for pairs that
+    cannot be left over: the same results as with a longest query length
+    alone, trajectories of one point among them or not."""
+    rng = np.random.default_rng(9)
+    cl, ql = rng.integers(least, longest[1] + 1, 300), rng.integers(least, longest[0] + 1, 8)
+    cl[:6] = ql[:2] = least
+    cl[6:9], ql[2] = longest[1], longest[0]
+    cp, co = G.random_walks(300, cl, 71, start_range=10.0)
+    qp, qo = G.random_walks(8, ql, 72, start_range=10.0)
+    db = tsim.Database(cuda_ctx, cp, co)
+    want_ids, _ = oracle.knn(measure, qp, qo, cp, co, 5, **kw)
+    for flags in (tsim.api.FLAG_ALWAYS_PRUNE, tsim.api.FLAG_NO_PRUNE):
+        ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, measure, 5, flags=flags, **kw)
+        ids2, d2, _, _ = _device_knn(tsim, cuda_ctx, db, qp, qo, measure, 5, flags=flags, **kw)
+        assert np.array_equal(ids, want_ids)
+        assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
+    db.close()
