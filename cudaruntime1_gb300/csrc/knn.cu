@@ -21,9 +21,11 @@
 //                      memory for DTW, its candidates fetched by bulk copy
 //                      on databases larger than L2; box distances for
 //                      Frechet and Hausdorff, the windowed eps-box count for
-//                      LCSS; lock-step Euclidean has none);
+//                      LCSS, whose pairs pass half of round 1 first; lock-step
+//                      Euclidean has none);
 //   D  DP              round 1 (the best survivors by bound) tightens the
-//                      threshold, then the remaining survivors run the
+//                      threshold, DTW's remaining pairs are bounded from
+//                      their row side too, then the survivors run the
 //                      wavefront DP (or the pairwise distance) with early
 //                      abandon against it;
 //   E  final           the k-th best FP32 value fixes the re-score set (all
@@ -95,6 +97,8 @@ struct KArgs {
   int nctr;
   // parameters
   int k, S, T, nch;
+  int Mr;   // round 1's pairs per query and pass: M, or (LCSS, two passes) half of it
+  int r1n;  // those refined so far
   int plain;    // one DP pair per kernel launch (the unbatched comparison form)
   int brute;    // small request: every pair refined exactly, no bound stages
   int noprune;  // thresholds stay open: every pair is refined
@@ -299,6 +303,12 @@ __global__ void __launch_bounds__(256) prep_kernel(KArgs a, float4* qbox, float4
     for (size_t i = tid; i < (size_t)a.nq * a.Cw; i += nthreads) a.seedmap[i] = 0u;
     for (size_t i = tid; i < (size_t)shapes; i += nthreads) a.shape_cnt[i] = 0;
   }
+}
+
+// entry i of query q among round 1's pairs: the passes' lists one after the other
+__device__ __forceinline__ size_t r1_at(const KArgs& a, int q, int i) {
+  const int pass = i >= a.Mr ? 1 : 0;
+  return ((size_t)pass * a.nq + q) * a.Mr + i - pass * a.Mr;
 }
 
 template <int MEAS>
@@ -995,30 +1005,37 @@ __device__ float seg_bound(const KArgs& a, int q, int c, int n, int m, float lb1
 // Entries for a per-query list, collected by a warp in shared memory and
 // listed 32 at a time: one atomic on the query's counter and coalesced stores.
 // Lanes with `take` add an entry; the whole warp calls both.
+template <int NV>  // values an entry: one to three lists
 struct WarpList {
   int* count;
   int* list;
-  int* list2;   // a second value per entry, or null
-  int (*buf)[2];  // 64 entries of shared memory, the warp's own
+  int* list2;
+  int* list3;
+  int (*buf)[NV];  // 64 entries of shared memory, the warp's own
   int n = 0;
-  __device__ __forceinline__ void add(bool take, int v, int v2) {
+  __device__ __forceinline__ void add(bool take, int v, int v2 = 0, int v3 = 0) {
     const int lane = threadIdx.x & 31;
     const unsigned ball = __ballot_sync(0xffffffffu, take);
     if (!ball) return;
     if (take) {
       const int at = n + __popc(ball & ((1u << lane) - 1));
-      buf[at][0] = v;
-      buf[at][1] = v2;
+      const int x[3] = {v, v2, v3};
+#pragma unroll
+      for (int i = 0; i < NV; ++i) buf[at][i] = x[i];
     }
     n += __popc(ball);
     __syncwarp();
     if (n < 32) return;
     store(32);
     n -= 32;
-    int k = 0, k2 = 0;
-    if (lane < n) k = buf[32 + lane][0], k2 = buf[32 + lane][1];
+    int k[NV] = {};
+    if (lane < n)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) k[i] = buf[32 + lane][i];
     __syncwarp();
-    if (lane < n) buf[lane][0] = k, buf[lane][1] = k2;
+    if (lane < n)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) buf[lane][i] = k[i];
     __syncwarp();
   }
   __device__ __forceinline__ void flush() {
@@ -1034,7 +1051,8 @@ struct WarpList {
     pos = __shfl_sync(0xffffffffu, pos, 0) + lane;
     if (lane < m) {
       list[pos] = buf[lane][0];
-      if (list2) list2[pos] = buf[lane][1];
+      if (NV > 1) list2[pos] = buf[lane][NV > 1 ? 1 : 0];
+      if (NV > 2) list3[pos] = buf[lane][NV > 2 ? 2 : 0];
     }
   }
 };
@@ -1094,7 +1112,7 @@ __global__ void __launch_bounds__(kChunk) compact_kernel(KArgs a) {
 #pragma unroll
   for (int i = 0; i < kCompact; ++i)
     if ((take >> i) & 1u) {
-      a.list2[at] = c0 + i * kChunk;
+      (MEAS == M_LCSS ? a.list1 : a.list2)[at] = c0 + i * kChunk;
       if (MEAS == M_EUCLID) a.lb2v[at] = bnd[i];
       ++at;
     }
@@ -1111,28 +1129,35 @@ __global__ void __launch_bounds__(256, MEAS == M_DTW ? 5 : 1) segfilter_kernel(K
   const float t = a.thr[q];
   const int n = a.qlen[q];
   const int g = threadIdx.x & (kSegGroup - 1);
-  __shared__ int buf[256 / 32][64][2];
+  constexpr bool kLcss = MEAS == M_LCSS;
+  constexpr int kVals = kLcss ? 3 : 1;
+  __shared__ int buf[256 / 32][64][kVals];
   const int warp = threadIdx.x >> 5;
   constexpr int kPer = 32 / kSegGroup;  // pairs per warp and pass
   // LCSS: the hull of the columns that can match rides along (in flat_vals,
-  // free until the survivors' round)
-  WarpList out{a.cnt1 + q, a.list1 + (size_t)q * a.C,
-               MEAS == M_LCSS ? reinterpret_cast<int*>(a.flat_vals) + (size_t)q * a.C : nullptr,
-               buf[warp]};
+  // free until the survivors' round), and the bound (round 1's order)
+  const int* in = (kLcss ? a.list1 : a.list2) + (size_t)q * a.C;
+  WarpList<kVals> out{(kLcss ? a.cnt2 : a.cnt1) + q, (kLcss ? a.list2 : a.list1) + (size_t)q * a.C,
+               kLcss ? reinterpret_cast<int*>(a.flat_vals) + (size_t)q * a.C : nullptr,
+               kLcss ? reinterpret_cast<int*>(a.lb2v) + (size_t)q * a.C : nullptr, buf[warp]};
   const int start = (blockIdx.x * (blockDim.x >> 5) + warp) * kPer;
   const int stride = gridDim.x * (blockDim.x >> 5) * kPer;
   for (int e0 = start; e0 < cnt; e0 += stride) {  // uniform per warp
     const int e = e0 + ((int)threadIdx.x & 31) / kSegGroup;
     bool pass = false;
     int c = 0, hull = 0;
+    float kept = 0.0f;
     if (e < cnt) {  // uniform per group
-      c = a.list2[(size_t)q * a.C + e];
+      c = in[e];
       const float b = a.lb1[(size_t)q * a.C + c];
       const float sbnd = seg_bound<MEAS>(a, q, c, n, a.clen[c], b, t, g, hull);
       pass = g == 0 && (MEAS == M_LCSS ? (sbnd >= t) : (sbnd <= t));
-      if (pass) a.lb1[(size_t)q * a.C + c] = sbnd;
+      if (kLcss)
+        kept = sbnd;
+      else if (pass)
+        a.lb1[(size_t)q * a.C + c] = sbnd;
     }
-    out.add(pass, c, hull);
+    out.add(pass, c, hull, __float_as_int(kept));
   }
   out.flush();
 }
@@ -1421,18 +1446,25 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 5) lb2_dtw_kernel(KArgs a) {
 // of kLcssTile pairs, so that a query with few pairs builds few grids: with
 // every query's pairs dealt over 19 CTAs the longest lists set the end.  2.17 M
 // pairs of 256 queries: 1,893 -> 1,053 us, 560 M instructions.
+//
+// It reads every point where the other measures' bound before round 1 reads
+// boxes, and from the seeds' threshold it kept three pairs in four; so a first
+// pass of round 1, on the pairs best by segment bound, comes before it, and a
+// second on those best by its own: 0.6 M of the 2.17 M pairs left to bound, 339
+// us, for as many pairs in the DP (311 k; 457 k with one pass, before it, and
+// 284 k with one after).  256 queries against 65,536 candidates 1,590 -> 1,390 us.
 constexpr int kLcssTile = 512;
 __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
   __shared__ uint32_t grid[kGridWords];
   __shared__ int buf[kLb2Warps][64][2];
   const int q = blockIdx.y;
-  const int cnt = a.cnt1[q];
+  const int cnt = a.fcnt[q];
   if ((long long)blockIdx.x * kLcssTile >= cnt) return;  // uniform across the CTA
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
   const float4 qb = a.qbox[q];
-  const float t = a.thr[q];
+  const float t = a.thr2[q];
   const float e2 = __fmul_ru(a.eps, 1.0f + 1.0f / 1048576.0f);
   const bool skip = n > a.max_qlen;  // longer than its tables were sized for: every pair passes
   for (int w = threadIdx.x; w < kGridWords; w += blockDim.x) grid[w] = 0u;
@@ -1463,9 +1495,9 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
   const float4 qi = make_float4(__fsub_rd(qb.x, e2), __fsub_rd(qb.y, e2), __fadd_ru(qb.z, e2),
                                 __fadd_ru(qb.w, e2));
   const int* L1 = a.list1 + (size_t)q * a.C;
-  const int* H1 = reinterpret_cast<const int*>(a.flat_vals) + (size_t)q * a.C;  // hulls
-  WarpList out{a.cnt2 + q, a.list2 + (size_t)q * a.C,
-               reinterpret_cast<int*>(a.lb2v) + (size_t)q * a.C, buf[warp]};
+  const int* H1 = a.order + (size_t)q * a.C;  // hulls
+  WarpList<2> out{a.cnt0 + q, a.list2 + (size_t)q * a.C,
+               reinterpret_cast<int*>(a.lb2v) + (size_t)q * a.C, nullptr, buf[warp]};
   const float gxm = (float)(gnx - 1), gym = (float)(gny - 1);
   for (long long tile = (long long)blockIdx.x * kLcssTile; tile < cnt;
        tile += (long long)gridDim.x * kLcssTile) {
@@ -1476,7 +1508,6 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
       if (e + kLb2Warps < end) c_nx = L1[e + kLb2Warps];
       const int h = H1[e], m = a.clen[c];
       const float2* B = a.cpts + a.coff[c];
-      const float sbnd = a.lb1[(size_t)q * a.C + c];
       // the hull's columns [jb, je); past n-1+delta they match nothing
       const int jb = seg_first(h & 255, m);
       int je = seg_first((h >> 8) + 1, m);
@@ -1511,9 +1542,9 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
       }
       count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
       bool pass = n > 0 && m > 0;
-      float lbv = sbnd;
+      float lbv = (float)min(n, m);
       if (pass && !skip) {
-        lbv = fminf((float)min(count, min(n, m)), sbnd);  // an upper bound on the count
+        lbv = fminf((float)count, lbv);  // an upper bound on the count
         pass = lbv >= t;
       }
       if (pass) out.add(lane == 0, c, __float_as_int(lbv));
@@ -1524,27 +1555,28 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
 
 // Round 1: the M best survivors of each query by their O(length) bound
 // (most likely to hold the true neighbours) are refined first; their values
-// tighten the threshold for the rest.  Taken entries are consumed (-1).
-template <int MEAS>
+// tighten the threshold for the rest.  Taken entries are consumed (-1).  LCSS
+// takes them in two passes, half by segment bound and half by O(length) bound.
+template <int MEAS, int PASS>
 __global__ void __launch_bounds__(kSelThreads) r1_select_kernel(KArgs a) {
   __shared__ SelScratch red;
   __shared__ unsigned long long sel[64];
   const int q = blockIdx.x;
-  const int ns = (a.cnt2[q] + kSeg - 1) / kSeg;
-  if (threadIdx.x == 0) {
+  const int ns = ((PASS ? a.cnt0[q] : a.cnt2[q]) + kSeg - 1) / kSeg;
+  if (PASS == 0 && threadIdx.x == 0) {
     a.fcnt[q] = 0;  // round 2's list count (refilter_kernel)
     a.cnt0[q] = 0;  // and what the row side keeps of it (lb_rows_kernel)
   }
   // the segments' M best (seg_select_kernel) hold the query's M best
-  block_select_k(a.segkeys + (size_t)q * a.nseg * 64, ns * a.M, a.M, sel, red);
-  for (int i = threadIdx.x; i < a.M; i += kSelThreads) {
+  block_select_k(a.segkeys + (size_t)q * a.nseg * 64, ns * a.Mr, a.Mr, sel, red);
+  for (int i = threadIdx.x; i < a.Mr; i += kSelThreads) {
     const int pos = key_index(sel[i]);
     int c = -1;
     if (pos >= 0) {
       c = a.list2[(size_t)q * a.C + pos];
       a.list2[(size_t)q * a.C + pos] = -1;
     }
-    a.r1pairs[(size_t)q * a.M + i] = make_int2(q, c);
+    a.r1pairs[r1_at(a, q, PASS * a.Mr + i)] = make_int2(q, c);
   }
 }
 
@@ -1564,9 +1596,9 @@ __device__ float round1_threshold(const KArgs& a, int q, int lane) {
         const float x = a.seed_vals[(size_t)q * a.S + i];
         key[s] = pack_key(MEAS == M_LCSS ? -x : x, i);
       }
-    } else if (i < a.S + a.M) {
-      if (a.r1pairs[(size_t)q * a.M + i - a.S].y >= 0) {
-        const float x = a.r1vals[(size_t)q * a.M + i - a.S];
+    } else if (i < a.S + a.r1n) {
+      if (a.r1pairs[r1_at(a, q, i - a.S)].y >= 0) {
+        const float x = a.r1vals[r1_at(a, q, i - a.S)];
         key[s] = pack_key(MEAS == M_LCSS ? -x : x, i);
       }
     }
@@ -1584,11 +1616,12 @@ __device__ float round1_threshold(const KArgs& a, int q, int lane) {
 }
 
 // Round 2: the remaining survivors whose bound passes the tightened
-// threshold, into list1 (free after stage C).
-template <int MEAS>
+// threshold, into list1 (free after stage C); LCSS's first pass: those that go
+// on to the O(length) bound.
+template <int MEAS, int PASS>
 __global__ void refilter_kernel(KArgs a) {
   const int q = blockIdx.y;
-  const int N = a.cnt2[q];
+  const int N = PASS ? a.cnt0[q] : a.cnt2[q];
   // every CTA of the query derives the tightened threshold (a warp's
   // selection over at most 128 values); the first stores it for the later
   // stages
@@ -1602,15 +1635,25 @@ __global__ void refilter_kernel(KArgs a) {
   }
   __syncthreads();
   const float t = t_sh;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
-    const int c = a.list2[(size_t)q * a.C + e];
-    if (c < 0) continue;
-    const float b = a.lb2v[(size_t)q * a.C + e];
-    if (MEAS == M_LCSS ? (b >= t) : (b <= t)) {
-      const int pos = atomicAdd(a.fcnt + q, 1);
-      a.list1[(size_t)q * a.C + pos] = c;
+  // LCSS, first pass: the hull comes along, for the O(length) bound (in order,
+  // free until the survivors' schedule)
+  constexpr bool kHull = MEAS == M_LCSS && PASS == 0;
+  __shared__ int buf[256 / 32][64][kHull ? 2 : 1];
+  WarpList<kHull ? 2 : 1> out{(PASS ? a.cnt1 : a.fcnt) + q, a.list1 + (size_t)q * a.C,
+               kHull ? a.order + (size_t)q * a.C : nullptr, nullptr, buf[threadIdx.x >> 5]};
+  const int lane = threadIdx.x & 31;
+  for (int e0 = blockIdx.x * blockDim.x + threadIdx.x - lane; e0 < N;  // uniform per warp
+       e0 += gridDim.x * blockDim.x) {
+    const int e = e0 + lane;
+    const int c = e < N ? a.list2[(size_t)q * a.C + e] : -1;
+    bool pass = false;
+    if (c >= 0) {
+      const float b = a.lb2v[(size_t)q * a.C + e];
+      pass = MEAS == M_LCSS ? (b >= t) : (b <= t);
     }
+    out.add(pass, c, kHull && pass ? __float_as_int(a.flat_vals[(size_t)q * a.C + e]) : 0);
   }
+  out.flush();
 }
 
 // DTW with a band, after the round-1 threshold: the other side of LB_Keogh.
@@ -1629,7 +1672,7 @@ constexpr int kRowBlocks = 64, kRowLevels = 4;
 constexpr int kRowWarps = 4;
 __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
   __shared__ float4 tabs[kRowWarps][kRowLevels][kRowBlocks];
-  __shared__ int buf[kRowWarps][64][2];
+  __shared__ int buf[kRowWarps][64][1];
   const int q = blockIdx.y;
   const int cnt = a.fcnt[q];
   if (blockIdx.x * kRowWarps >= cnt) return;  // uniform across the CTA
@@ -1638,7 +1681,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
   float4(*tab)[kRowBlocks] = tabs[warp];
-  WarpList out{a.cnt0 + q, a.list2 + (size_t)q * a.C, nullptr, buf[warp]};
+  WarpList<1> out{a.cnt0 + q, a.list2 + (size_t)q * a.C, nullptr, nullptr, buf[warp]};
   for (int e = blockIdx.x * kRowWarps + warp; e < cnt; e += gridDim.x * kRowWarps) {
     const int c = a.list1[(size_t)q * a.C + e];
     const int m = a.clen[c];
@@ -1836,8 +1879,8 @@ __device__ __forceinline__ void entry(const KArgs& a, int q, int i, int base, in
     c = a.seeds[(size_t)q * a.S + i].y;
     v = a.seed_vals[(size_t)q * a.S + i];
   } else if (i < a.S + a.M) {
-    c = a.r1pairs[(size_t)q * a.M + i - a.S].y;
-    v = a.r1vals[(size_t)q * a.M + i - a.S];
+    c = a.r1pairs[r1_at(a, q, i - a.S)].y;
+    v = a.r1vals[r1_at(a, q, i - a.S)];
   } else {
     c = a.flat[base + i - a.S - a.M].y;
     v = a.flat_vals[base + i - a.S - a.M];
@@ -1854,7 +1897,7 @@ __global__ void __launch_bounds__(kSelThreads) seg_select_kernel(KArgs a, int K)
   __shared__ SelScratch red;
   __shared__ unsigned long long sel[64];
   const int q = blockIdx.y, seg = blockIdx.x;
-  const int N = MODE == 0 ? a.cnt2[q] : a.S + a.M + a.fcnt[q];
+  const int N = MODE == 0 ? a.cnt2[q] : MODE == 2 ? a.cnt0[q] : a.S + a.M + a.fcnt[q];
   const int lo = seg * kSeg;
   if (lo >= N) return;
   const int cnt = min(kSeg, N - lo);
@@ -1862,7 +1905,7 @@ __global__ void __launch_bounds__(kSelThreads) seg_select_kernel(KArgs a, int K)
   for (int t = threadIdx.x; t < cnt; t += kSelThreads) {
     const int i = lo + t;
     unsigned long long key;
-    if (MODE == 0) {
+    if (MODE != 1) {
       const float b = a.lb2v[(size_t)q * a.C + i];
       key = pack_key(MEAS == M_LCSS ? -b : b, i);
     } else {
@@ -2073,11 +2116,14 @@ __global__ void __launch_bounds__(32 * kRankWarps) final_sort_kernel(KArgs a) {
 // Per-request counters, accumulated on the device (no host sync per chunk):
 // counters[2..6] += pairs passing the O(1) bound, the O(length) bound,
 // refined pairs, re-scored pairs, FP64 re-scored pairs.
-__global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_rescore, int euclid) {
+// (LCSS: its O(length) bound follows round 1's first pass, whose pairs count
+// as passing it)
+__global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_rescore, int meas) {
   unsigned long long c1 = 0, c2 = 0, rc = 0;
+  const bool late = meas == M_LCSS && !a.brute;
   for (int q = threadIdx.x; q < a.nq; q += blockDim.x) {
-    c1 += euclid ? a.cnt2[q] : a.cnt1[q];  // one bound stage only
-    c2 += a.cnt2[q];
+    c1 += meas == M_EUCLID || late ? a.cnt2[q] : a.cnt1[q];  // Euclidean: one bound stage only
+    c2 += late ? a.cnt0[q] + min(a.cnt2[q], a.Mr) : a.cnt2[q];
     rc += with_rescore ? min(a.rraw[q], a.RC) : 0;
   }
   for (int o = 16; o; o >>= 1) {
@@ -2294,7 +2340,7 @@ int finish_knn(tsim_ctx* ctx, KArgs& a, int dpc, int dp64) {
     stage_end(ctx);
   }
   if (ctx->count_funnel) {  // a synchronising request that reports its funnel
-    stats_kernel<<<1, 256, 0, s>>>(a, ctx->dcounters, MEAS != M_LCSS ? 1 : 0, MEAS == M_EUCLID);
+    stats_kernel<<<1, 256, 0, s>>>(a, ctx->dcounters, MEAS != M_LCSS ? 1 : 0, MEAS);
     TSIM_CUDA(cudaGetLastError());
     launched(ctx);
   }
@@ -2406,10 +2452,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   if constexpr (MEAS != M_EUCLID) {
     segfilter_kernel<MEAS><<<dim3(std::max(1, std::min(1024, (32 * ctx->num_sms + nq - 1) / nq)), nq),
                              256, 0, s>>>(a);
-    if constexpr (MEAS == M_LCSS) {
-      const int tiles = (a.C + kLcssTile - 1) / kLcssTile;
-      lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(a);
-    } else {
+    if constexpr (MEAS != M_LCSS) {
       const size_t lb2_smem =
           MEAS == M_DTW ? sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2) : 0;
       auto lb2 = MEAS == M_DTW ? lb2_dtw_kernel : lb2_kernel<MEAS>;
@@ -2418,46 +2461,64 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
                                        (int)lb2_smem));
       lb2<<<dim3(ch, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
     }
-    launched(ctx, 2);
+    launched(ctx, MEAS == M_LCSS ? 1 : 2);
   }
-  seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.M);
-  r1_select_kernel<MEAS><<<nq, kSelThreads, 0, s>>>(a);
+  seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
+  r1_select_kernel<MEAS, 0><<<nq, kSelThreads, 0, s>>>(a);
   TSIM_CUDA(cudaGetLastError());
   launched(ctx, 2);
   stage_end(ctx);
 
-  // round 1: the best survivors by bound, abandon against the seed threshold
-  stage_begin(ctx, TSIM_STAGE_DP);
-  {
+  // round 1: the best survivors by bound, abandon against the threshold so far
+  auto round1 = [&](int pass, const float* thr) -> int {
+    stage_begin(ctx, TSIM_STAGE_DP);
     DpArgs r1 = d;
-    r1.pairs = a.r1pairs;
-    r1.npairs = nq * a.M;
-    r1.out = a.r1vals;
-    r1.thr = a.thr;
+    r1.pairs = a.r1pairs + (size_t)pass * nq * a.Mr;
+    r1.npairs = nq * a.Mr;
+    r1.out = a.r1vals + (size_t)pass * nq * a.Mr;
+    r1.thr = thr;
     // the best pairs by bound rarely abandon: no remaining-columns bound
     if (MEAS == M_DTW) r1.qtab = nullptr;
     if (a.plain) {
-      for (int i = 0; i < nq * a.M; ++i) {
+      for (int i = 0; i < nq * a.Mr; ++i) {
         DpArgs one = r1;
-        one.pairs = a.r1pairs + i;
+        one.pairs = r1.pairs + i;
         one.npairs = 1;
-        one.out = a.r1vals + i;
+        one.out = r1.out + i;
         TSIM_TRY(refine32<MEAS>(ctx, a, dp32, Gs, Rs, one));
       }
     } else {
       TSIM_TRY(refine32<MEAS>(ctx, a, dp32, Gs, Rs, r1, true));
     }
-  }
-  stage_end(ctx);
+    a.r1n += a.Mr;
+    stage_end(ctx);
+    return TSIM_OK;
+  };
+  TSIM_TRY(round1(0, a.thr));
 
   stage_begin(ctx, TSIM_STAGE_FILTER);
-  refilter_kernel<MEAS><<<dim3(ch, nq), 256, 0, s>>>(a);
+  // (LCSS: some million pairs whose loads wait on one another: 82 -> 52 us)
+  const int rch = MEAS == M_LCSS ? std::min(4 * ch, 65535) : ch;
+  refilter_kernel<MEAS, 0><<<dim3(rch, nq), 256, 0, s>>>(a);
   if (MEAS == M_DTW && a.band_pct >= 0) {
     lb_rows_kernel<<<dim3(std::max(1, std::min((a.C + kRowWarps - 1) / kRowWarps, 8 * ch)), nq),
                      kRowWarps * 32, 0, s>>>(a);
     launched(ctx);
     a.list1 = a.list2;  // what it kept
     a.fcnt = a.cnt0;
+  }
+  if constexpr (MEAS == M_LCSS) {
+    const int tiles = (a.C + kLcssTile - 1) / kLcssTile;
+    lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(a);
+    seg_select_kernel<MEAS, 2><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
+    r1_select_kernel<MEAS, 1><<<nq, kSelThreads, 0, s>>>(a);
+    launched(ctx, 3);
+    stage_end(ctx);
+    TSIM_TRY(round1(1, a.thr2));
+    stage_begin(ctx, TSIM_STAGE_FILTER);
+    refilter_kernel<MEAS, 1><<<dim3(ch, nq), 256, 0, s>>>(a);
+    launched(ctx);
+    a.fcnt = a.cnt1;
   }
   scan_kernel<<<1, 1024, 0, s>>>(a);
   // the shape order serves the kernels whose warps run as long as their
@@ -2574,6 +2635,8 @@ size_t knn_plan(const tsim_params* p, int nq, int max_qlen, const tsim_db* db, K
   a.k = k;
   a.S = std::min(C, std::min(64, std::max(2 * k, 16)));
   a.M = std::min(64, std::max(2 * k, 32));
+  a.Mr = p->measure == TSIM_LCSS ? a.M / 2 : a.M;
+  a.r1n = 0;
   a.nch = (C + kChunk - 1) / kChunk;
   a.T = std::min(kChunk, std::max(1, (2 * a.S + a.nch - 1) / a.nch));
   a.T = std::min(a.T, 64);
