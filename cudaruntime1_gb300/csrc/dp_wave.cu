@@ -147,18 +147,31 @@ struct WaveGeom {
 #define SFX(j) sfx[TSIM_SIDX(j, ccap + 1)]
 #define QPT(i) (QS ? qs[TSIM_SIDX(i, qcap + kWavePad)] : __ldg(A + min(i, n - 1)))
 
-// One pair on the warp, R cells per lane (its widest anti-diagonal fits 32 R).
-template <class P, int R, bool QS>
+// Half a pair (dp_wave2_kernel): what the warp leaves for the other's half.
+template <class V>
+struct WaveHalf {
+  bool rev = false;  // from the last cell backwards: both point sequences reversed
+  int t_stop = 0;    // its last anti-diagonal
+  V* last = nullptr;  // [32 R] that anti-diagonal's positions, and the one's before
+  V* prev = nullptr;
+  int* geo = nullptr;  // [3] their first rows, and whether the half is alive
+};
+
+// One pair on the warp, R cells per lane (its widest anti-diagonal fits 32 R),
+// or (HALF) its anti-diagonals up to half.t_stop.
+template <class P, int R, bool QS, bool HALF = false>
 __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const int q, const int n,
                                           const int m, const int w, const int64_t qo,
                                           const int64_t co, float2* cs, float* sfx, float2* qs,
-                                          const int ccap, const int qcap) {
+                                          const int ccap, const int qcap,
+                                          const WaveHalf<typename P::V> half = {}) {
+  static_assert(QS || !HALF, "a half stages both sides");
   using V = typename P::V;
   using C = typename P::C;
   const int lane = threadIdx.x & 31;
   const bool check = a.thr != nullptr;
   const int src_dn = (lane + 31) & 31, src_up = (lane + 1) & 31;
-  const int t_end = n + m - 2;
+  const int t_end = HALF ? half.t_stop : n + m - 2;
   const float thr = check ? a.thr[q] : TSIM_INF;
   const int W = w < 0 ? -1 : w * (min(n, m) - 1);
   // the candidate's points are staged; the query's too in the latency
@@ -169,9 +182,11 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
   __syncwarp();
   {
     const float2* B = a.cpts + co;
-    for (int j = lane; j < m; j += 32) CS(j) = __ldg(B + j);
+    const bool rev = HALF && half.rev;
+    for (int j = lane; j < m; j += 32) CS(j) = __ldg(B + (rev ? m - 1 - j : j));
     if (QS)
-      for (int i = lane; i < n; i += 32) qs[TSIM_SIDX(i, qcap + kWavePad)] = __ldg(A + i);
+      for (int i = lane; i < n; i += 32)
+        qs[TSIM_SIDX(i, qcap + kWavePad)] = __ldg(A + (rev ? n - 1 - i : i));
   }
   // Remaining-columns bound (the survivor round): every path crosses every
   // column after the largest one of two consecutive anti-diagonals, and a
@@ -181,7 +196,7 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
   // adds those columns' costs can round below their exact sum by at most
   // (n+m+8) 2^-24 relative, so the check compares with the threshold divided
   // by 1 minus that.
-  const bool suffix = wave_suffix<P>(a) && n <= a.max_n;
+  const bool suffix = !HALF && wave_suffix<P>(a) && n <= a.max_n;
   float thr_chk = thr;
   __syncwarp();
   if (suffix) {
@@ -311,7 +326,7 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
   // blocks of 16 straight-line steps; after each, the abandon test over
   // its last two anti-diagonals (plus the columns after them)
   int t = 1;
-  for (; t + 15 <= t_end; t += 16) {
+  for (; t + 15 <= (HALF ? t_end - 1 : t_end); t += 16) {  // HALF: the last step apart
     float m14 = TSIM_INF;
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
@@ -335,7 +350,21 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
     base += 16;
   }
   if (alive)
-    for (; t <= t_end; ++t) step(t, __shfl_sync(0xffffffffu, win, t + 2 - base));
+    for (; t <= (HALF ? t_end - 1 : t_end); ++t)
+      step(t, __shfl_sync(0xffffffffu, win, t + 2 - base));
+  if (HALF) {
+    if (alive) {
+      // (a lone first anti-diagonal has none before it)
+#pragma unroll
+      for (int r = 0; r < R; ++r) half.prev[lane * R + r] = t_end > 0 ? v[r] : P::border();
+      if (lane == 0) half.geo[1] = ilo;
+      if (t_end > 0) step(t, __shfl_sync(0xffffffffu, win, t + 2 - base)), ++t;
+#pragma unroll
+      for (int r = 0; r < R; ++r) half.last[lane * R + r] = v[r];
+      if (lane == 0) half.geo[0] = ilo;
+    }
+    if (lane == 0) half.geo[2] = alive;
+  }
   if (a.cells) {  // cells of the anti-diagonals computed, inside the band
     const int t_done = alive ? t_end : min(t, t_end);
     long long cells = 0;
@@ -350,7 +379,7 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
     if (lane == 0) atomicAdd(a.cells, (unsigned long long)cells);
   }
   // the result: cell (n-1, m-1), position 0 of the last anti-diagonal
-  if (lane == 0) store_result(a, pid, alive ? v[0] : P::border());
+  if (!HALF && lane == 0) store_result(a, pid, alive ? v[0] : P::border());
 }
 
 // RMAX = 1: pairs whose widest anti-diagonal fits 32 lanes; RMAX = 2: every
@@ -392,6 +421,106 @@ __global__ void __launch_bounds__(kWaveThreads)
   }
 }
 
+__device__ __forceinline__ float path_sum(float a, float b) { return a + b; }
+__device__ __forceinline__ df path_sum(df a, df b) {
+  return a.hi < TSIM_INF && b.hi < TSIM_INF ? df_add(a, b) : df_inf();
+}
+__device__ __forceinline__ void pair_sync(int pair) {  // the two warps of a pair
+  static_assert(kWaveThreads == 128, "two pairs a CTA");
+  if (pair == 0)
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+  else
+    asm volatile("bar.sync 2, 64;" ::: "memory");
+}
+
+// DTW's latency rounds: two warps a pair, one from cell (0, 0) up to the middle
+// anti-diagonal s, one from cell (n-1, m-1) back to s + 1 (the same recurrence
+// on the reversed sequences; the band is symmetric), so the chain of dependent
+// steps is half as long.  A path steps from anti-diagonal s or s - 1 to s + 1,
+// or from s to s + 2: the value is the least sum, over the cells behind and
+// their predecessors before, of the two halves' values.  A sum of two halves
+// rounds no more often than one running sum.
+//
+// What bounds it: the steps' latency (a shuffle, a minimum, an addition, the
+// next cost).  Ten pairs of 333 x 64 to 512 points 47 -> 31 us, compensated 90
+// (two warps of row groups) -> 70.
+template <class P, int RMAX>
+__global__ void __launch_bounds__(kWaveThreads)
+    dp_wave2_kernel(DpArgs a, int ccap, int qcap, int* spill, int* nspill) {
+  using V = typename P::V;
+  extern __shared__ __align__(16) float2 wave_smem[];
+  constexpr int kPairs = kWaveThreads / 64;
+  // forward's last and previous anti-diagonal, backward's
+  __shared__ __align__(8) unsigned char xmem[kPairs][4 * 32 * RMAX * sizeof(V)];
+  __shared__ int geo[kPairs][2][3];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int pair = warp >> 1, side = warp & 1;
+  float2* cs = wave_smem + (size_t)warp * wave_per_warp(ccap, qcap) + kWavePad;
+  float* sfx = reinterpret_cast<float*>(cs + ccap + kWavePad);
+  float2* qs = cs + ccap + kWavePad + (ccap + 2) / 2;
+  V* const x = reinterpret_cast<V*>(xmem[pair]);
+  const int slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 6;
+  const int nslots = (gridDim.x * blockDim.x) >> 6;
+  const int npairs = a.npairs_dev ? min(*a.npairs_dev, a.npairs) : a.npairs;
+
+  for (int wk = slot; wk < npairs; wk += nslots) {  // uniform over the pair's warps
+    const int pid = a.order ? a.order[wk] : wk;
+    const int2 pr = a.pairs[pid];
+    if (pr.y < 0) continue;
+    const int q = pr.x;
+    const int64_t qo = a.qoff[q], co = a.coff[pr.y];
+    const int n = (int)(a.qoff[q + 1] - qo), m = (int)(a.coff[pr.y + 1] - co);
+    const int w = band_w(n, m, a.band_pct);
+    const int lm = wave_lmax(n, m, w);
+    if (n < 2 || m < 2 || n > qcap || m > ccap || lm > 32 * RMAX) {
+      if (threadIdx.x % 64 == 0) spill[atomicAdd(nspill, 1)] = pid;
+      continue;
+    }
+    const int s = (n + m - 3) / 2;  // forward's last anti-diagonal
+    WaveHalf<V> h;
+    h.rev = side;
+    h.t_stop = side ? n + m - 2 - (s + 1) : s;
+    h.last = x + 2 * side * 32 * RMAX;
+    h.prev = h.last + 32 * RMAX;
+    h.geo = geo[pair][side];
+    const bool one = RMAX == 1 || lm <= 32;
+    if (one)
+      wave_pair<P, 1, true, true>(a, pid, q, n, m, w, qo, co, cs, sfx, qs, ccap, qcap, h);
+    else
+      wave_pair<P, RMAX, true, true>(a, pid, q, n, m, w, qo, co, cs, sfx, qs, ccap, qcap, h);
+    pair_sync(pair);
+    if (side == 0) {
+      const int* gf = geo[pair][0];
+      const int* gb = geo[pair][1];
+      const int cells = one ? 32 : 32 * RMAX;
+      const V* f0 = x;
+      const V* f1 = x + 32 * RMAX;
+      const V* b0 = x + 64 * RMAX;
+      const V* b1 = x + 96 * RMAX;
+      V best = P::border();
+      if (gf[2] && gb[2]) {
+        // forward's value of row i on one of its anti-diagonals
+        auto fwd = [&](const V* d, int first, int i) {
+          const int p = i - first;
+          return (unsigned)p < (unsigned)cells ? d[p] : P::border();
+        };
+        for (int p = lane; p < cells; p += 32) {
+          const int i1 = n - 1 - (gb[0] + p);  // row of a cell on s + 1
+          const V before = vmin(vmin(fwd(f0, gf[0], i1 - 1), fwd(f0, gf[0], i1)),
+                                fwd(f1, gf[1], i1 - 1));
+          best = vmin(best, path_sum(before, b0[p]));
+          const int i2 = n - 1 - (gb[1] + p);  // and on s + 2
+          best = vmin(best, path_sum(fwd(f0, gf[0], i2 - 1), b1[p]));
+        }
+      }
+      for (int o = 16; o; o >>= 1) best = vmin(best, wshfl(best, lane ^ o));
+      if (lane == 0) store_result(a, pid, best);
+    }
+    pair_sync(pair);  // before the next pair's halves are written
+  }
+}
+
 #undef CS
 #undef SFX
 #undef QPT
@@ -409,6 +538,26 @@ int launch_wave_one(tsim_ctx* ctx, const DpArgs& a, int ccap, int qcap, int* spi
   if (per_sm < 1) return fail(TSIM_ERR_UNSUPPORTED, "wave kernel does not fit on an SM");
   const long long warps = kWaveThreads / 32;
   const long long blocks = std::min<long long>((a.npairs + warps - 1) / warps,
+                                               (long long)per_sm * ctx->num_sms);
+  kern<<<(unsigned)std::max(blocks, 1ll), kWaveThreads, smem, ctx->stream>>>(a, ccap, qcap, spill,
+                                                                             nspill);
+  TSIM_CUDA(cudaGetLastError());
+  launched(ctx);
+  return TSIM_OK;
+}
+
+template <class P, int R>
+int launch_wave2_one(tsim_ctx* ctx, const DpArgs& a, int ccap, int qcap, int* spill, int* nspill) {
+  if (a.npairs <= 0) return TSIM_OK;
+  auto kern = dp_wave2_kernel<P, R>;
+  const size_t smem = (size_t)(kWaveThreads / 32) * wave_per_warp(ccap, qcap) * sizeof(float2);
+  if (smem > 40 * 1024)
+    TSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  TSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWaveThreads, smem));
+  if (per_sm < 1) return fail(TSIM_ERR_UNSUPPORTED, "wave kernel does not fit on an SM");
+  const long long pairs = kWaveThreads / 64;
+  const long long blocks = std::min<long long>((a.npairs + pairs - 1) / pairs,
                                                (long long)per_sm * ctx->num_sms);
   kern<<<(unsigned)std::max(blocks, 1ll), kWaveThreads, smem, ctx->stream>>>(a, ccap, qcap, spill,
                                                                              nspill);
@@ -450,6 +599,28 @@ bool wave_takes_all(int max_n, int max_m, int band_pct) {
   const int w = band_w(max_n, max_m, band_pct), mn = std::min(max_n, max_m);
   const int most = w < 0 ? mn : std::min(mn, w + 1);
   return most <= (wave_lmax(max_n, max_m, w) <= 32 ? 32 : 64);  // cells of the launch's lanes
+}
+
+// the latency rounds of banded DTW on two warps a pair, from both ends
+template <class P>
+int wave2_chain(tsim_ctx* ctx, const DpArgs& a, int max_n, int max_m, int* spill, int** nspill_io) {
+  const int ccap = (std::min(max_m, kWaveMaxLen) + 1) & ~1;
+  const int qcap = (std::min(max_n, kWaveMaxLen) + 1) & ~1;
+  const int lmax = wave_lmax(max_n, max_m, band_w(max_n, max_m, a.band_pct));
+  TSIM_TRY(fresh_counter(ctx, *nspill_io, nspill_io));
+  return lmax <= 32 ? launch_wave2_one<P, 1>(ctx, a, ccap, qcap, spill, *nspill_io)
+                    : launch_wave2_one<P, 2>(ctx, a, ccap, qcap, spill, *nspill_io);
+}
+
+int launch_dp_wave2(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
+                    int** nspill) {
+  switch (kind) {
+    case DP_DTW_SQ: return wave2_chain<PolDtwSq>(ctx, a, max_n, max_m, spill, nspill);
+    case DP_DTW_EU: return wave2_chain<PolDtwEu>(ctx, a, max_n, max_m, spill, nspill);
+    case DP_DTW_SQC: return wave2_chain<PolDtwSqC>(ctx, a, max_n, max_m, spill, nspill);
+    case DP_DTW_EUC: return wave2_chain<PolDtwEuC>(ctx, a, max_n, max_m, spill, nspill);
+  }
+  return fail(TSIM_ERR_UNSUPPORTED, "no two-ended kernel for this DP kind");
 }
 
 int launch_dp_wave(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, bool latency,

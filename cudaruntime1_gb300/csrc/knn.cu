@@ -240,8 +240,8 @@ __device__ __forceinline__ float block_bound(const KArgs& a, const float4* qblk,
 // 1 left empty.  One launch, because a small call's time is its chain of
 // dependent graph nodes, not their work: with the counters zeroed here (a
 // memset node a DP launch before) and the launches left out for which no pair
-// can be left over (run_dp), one query against 10,000 trajectories went from
-// 382 to 341 us, 4 x 100 all-pairs DTW from 155 to 141.
+// can be left over (run_dp), one query against 16,384 trajectories went from
+// 382 to 334 us, 8 against 1,024 (all pairs refined) from 155 to 141.
 __global__ void __launch_bounds__(256) prep_kernel(KArgs a, float4* qbox, float4* qends, int* qlen,
                                                    int shapes) {
   const int lane = threadIdx.x & 31;
@@ -2190,7 +2190,15 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
   }
   if (!diag_kind || a.rdiag == 0) return launch_dp(ctx, kind, G, R, d, a.max_clen);
   const bool twofloat_kind = kind == DP_DTW_SQC || kind == DP_DTW_EUC || kind == DP_FRECHET_SQC;
-  if (a.wave && wave_kind(kind) && !twofloat_kind) {
+  // Rounds of no more pairs than two an SM -- a query or a few -- run each pair
+  // from both ends on two warps, one a scheduler: a lone query's seeds, round 1
+  // and re-score 47 + 45 + 90 -> 31 + 31 + 70 us.  Larger ones gained nothing
+  // next to other requests (64 queries 402 us either way) and mixed serving
+  // lost 1.8 %: a pair's own latency no longer counts, its staging twice does.
+  const bool two_ended = latency && !a.plain && d.npairs <= 2 * ctx->num_sms &&
+                         (kind == DP_DTW_SQ || kind == DP_DTW_EU || kind == DP_DTW_SQC ||
+                          kind == DP_DTW_EUC);
+  if (a.wave && wave_kind(kind) && (two_ended || !twofloat_kind)) {
     // lanes along the anti-diagonal, straight-line blocks of 16 steps: the
     // shortest FP32 step of the warp-per-pair forms (a lone 512 x 486 pair
     // 83 us against 104 on two warps per pair; compensated pairs are faster
@@ -2200,7 +2208,10 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
     // kernels
     int* nw = a.nwaves;
     const int mq = d.max_n > 0 ? d.max_n : a.max_qlen;
-    TSIM_TRY(launch_dp_wave(ctx, kind, d, mq, a.max_clen, latency, a.waves, &nw));
+    if (two_ended)
+      TSIM_TRY(launch_dp_wave2(ctx, kind, d, mq, a.max_clen, a.waves, &nw));
+    else
+      TSIM_TRY(launch_dp_wave(ctx, kind, d, mq, a.max_clen, latency, a.waves, &nw));
     DpArgs rest = d;
     rest.order = a.waves;
     rest.npairs_dev = nw;

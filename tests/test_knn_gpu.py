@@ -498,3 +498,24 @@ def test_known_lengths(tsim, cuda_ctx, oracle, least, measure, kw, longest):
         assert np.array_equal(ids, want_ids)
         assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
     db.close()
+
+
+@pytest.mark.parametrize("band,cost", [(0, 0), (4, 0), (12, 1), (40, 0), (60, 1)])
+def test_dtw_from_both_ends(tsim, cuda_ctx, oracle, band, cost):
+    """Banded DTW's latency rounds, each pair from both ends to the middle:
+    sums of lengths odd and even, halves around blocks of 16 anti-diagonals,
+    anti-diagonals of up to 32 cells, up to 64 and more, two-point sides."""
+    cp, co = G.random_walks(20, [2, 3, 4, 14, 15, 16, 17, 18, 30, 31, 32, 33, 34, 35, 63, 64, 65, 66,
+                                 120, 200], 81, start_range=10.0)
+    qp, qo = G.random_walks(10, [2, 3, 16, 17, 18, 33, 34, 65, 66, 170], 82, start_range=10.0)
+    db = tsim.Database(cuda_ctx, cp, co)
+    kw = dict(band_pct=band, cost=cost)
+    want_ids, want = oracle.knn("dtw", qp, qo, cp, co, 20, **kw)
+    fin = np.isfinite(want)
+    for flags in (0, tsim.api.FLAG_ALWAYS_PRUNE):
+        ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 20, flags=flags, **kw)
+        assert np.array_equal(ids, want_ids)
+        assert np.array_equal(np.isfinite(d), fin)
+        # costs within 4 2^-24, their compensated sum, the result's rounding
+        assert np.all(np.abs(d[fin] - want[fin]) <= 5 * 2.0 ** -24 * want[fin])
+    db.close()
