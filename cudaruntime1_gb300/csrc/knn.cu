@@ -19,10 +19,10 @@
 //   C  lb2_kernel      the listed pairs get the O(length) bound (banded
 //                      LB_Keogh from the query's sparse table in global
 //                      memory for DTW, its candidates fetched by bulk copy
-//                      on databases larger than L2; box distances for
-//                      Frechet and Hausdorff, the windowed eps-box count for
-//                      LCSS, whose pairs pass half of round 1 first; lock-step
-//                      Euclidean has none);
+//                      on databases larger than L2; after round 1 box
+//                      distances for Frechet and, after half of it, the
+//                      windowed eps-box count for LCSS; Hausdorff and
+//                      lock-step Euclidean have none);
 //   D  DP              round 1 (the best survivors by bound) tightens the
 //                      threshold, DTW's remaining pairs are bounded from
 //                      their row side too, then the survivors run the
@@ -73,6 +73,18 @@ constexpr bool is_dp(int meas) { return meas <= M_FRECHET; }
 constexpr bool compensated_rescore(int meas) { return meas == M_DTW; }
 // values carried in the squared domain (sqrt applied to the reported distance)
 constexpr bool is_squared(int meas) { return meas >= M_FRECHET; }
+
+// Measures whose O(length) bound follows round 1 (LCSS: its first pass), which
+// then goes by the segment bound.  That bound costs as much as a few columns of
+// boxes, the O(length) one reads every point: Hausdorff's kept 1.90 M of 2.00 M
+// pairs for 2.8 of a request's 10.3 ms, and of the 0.47 M that pass round 1's
+// threshold it kept 96 %, so Hausdorff has none (1,024 queries against 262,144
+// candidates 5.43 -> 4.53 ms; 4.80 with it after round 1); Frechet, whose DP
+// costs far more a pair, 523 -> 515 us.  DTW keeps it before round 1: its round
+// lasts longer than the bound.
+constexpr bool late_bound(int meas) {
+  return meas == M_LCSS || meas == M_HAUSDORFF || meas == M_FRECHET;
+}
 
 struct KArgs {
   // queries
@@ -1112,7 +1124,7 @@ __global__ void __launch_bounds__(kChunk) compact_kernel(KArgs a) {
 #pragma unroll
   for (int i = 0; i < kCompact; ++i)
     if ((take >> i) & 1u) {
-      (MEAS == M_LCSS ? a.list1 : a.list2)[at] = c0 + i * kChunk;
+      (late_bound(MEAS) ? a.list1 : a.list2)[at] = c0 + i * kChunk;
       if (MEAS == M_EUCLID) a.lb2v[at] = bnd[i];
       ++at;
     }
@@ -1129,17 +1141,18 @@ __global__ void __launch_bounds__(256, MEAS == M_DTW ? 5 : 1) segfilter_kernel(K
   const float t = a.thr[q];
   const int n = a.qlen[q];
   const int g = threadIdx.x & (kSegGroup - 1);
-  constexpr bool kLcss = MEAS == M_LCSS;
-  constexpr int kVals = kLcss ? 3 : 1;
+  constexpr bool kLcss = MEAS == M_LCSS, kLate = late_bound(MEAS);
+  constexpr int kVals = kLcss ? 3 : kLate ? 2 : 1;
   __shared__ int buf[256 / 32][64][kVals];
   const int warp = threadIdx.x >> 5;
   constexpr int kPer = 32 / kSegGroup;  // pairs per warp and pass
-  // LCSS: the hull of the columns that can match rides along (in flat_vals,
-  // free until the survivors' round), and the bound (round 1's order)
-  const int* in = (kLcss ? a.list1 : a.list2) + (size_t)q * a.C;
-  WarpList<kVals> out{(kLcss ? a.cnt2 : a.cnt1) + q, (kLcss ? a.list2 : a.list1) + (size_t)q * a.C,
-               kLcss ? reinterpret_cast<int*>(a.flat_vals) + (size_t)q * a.C : nullptr,
-               kLcss ? reinterpret_cast<int*>(a.lb2v) + (size_t)q * a.C : nullptr, buf[warp]};
+  // the bound comes along where it orders round 1, and LCSS's hull of the
+  // columns that can match (in flat_vals, free until the survivors' round)
+  const size_t row = (size_t)q * a.C;
+  const int* in = (kLate ? a.list1 : a.list2) + row;
+  int* bounds = reinterpret_cast<int*>(a.lb2v) + row;
+  WarpList<kVals> out{(kLate ? a.cnt2 : a.cnt1) + q, (kLate ? a.list2 : a.list1) + row, bounds,
+                      reinterpret_cast<int*>(a.flat_vals) + row, buf[warp]};
   const int start = (blockIdx.x * (blockDim.x >> 5) + warp) * kPer;
   const int stride = gridDim.x * (blockDim.x >> 5) * kPer;
   for (int e0 = start; e0 < cnt; e0 += stride) {  // uniform per warp
@@ -1152,12 +1165,10 @@ __global__ void __launch_bounds__(256, MEAS == M_DTW ? 5 : 1) segfilter_kernel(K
       const float b = a.lb1[(size_t)q * a.C + c];
       const float sbnd = seg_bound<MEAS>(a, q, c, n, a.clen[c], b, t, g, hull);
       pass = g == 0 && (MEAS == M_LCSS ? (sbnd >= t) : (sbnd <= t));
-      if (kLcss)
-        kept = sbnd;
-      else if (pass)
-        a.lb1[(size_t)q * a.C + c] = sbnd;
+      kept = sbnd;
+      if ((MEAS == M_DTW || MEAS == M_FRECHET) && pass) a.lb1[row + c] = sbnd;
     }
-    out.add(pass, c, hull, __float_as_int(kept));
+    out.add(pass, c, __float_as_int(kept), hull);
   }
   out.flush();
 }
@@ -1173,6 +1184,7 @@ __device__ uint32_t g_wait_limit = kWaitLimitDefault;
 struct PassList {
   const KArgs& a;
   int q;
+  int* count;
   int c = 0, n = 0;
   float v = 0.0f;
   __device__ __forceinline__ void add(int cand, float bound) {  // uniform across the warp
@@ -1183,7 +1195,7 @@ struct PassList {
     if (n == 0) return;
     const int lane = threadIdx.x & 31;
     int pos = 0;
-    if (lane == 0) pos = atomicAdd(a.cnt2 + q, n);
+    if (lane == 0) pos = atomicAdd(count, n);
     pos = __shfl_sync(0xffffffffu, pos, 0);
     if (lane < n) {
       a.list2[(size_t)q * a.C + pos + lane] = c;
@@ -1198,12 +1210,12 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int q = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int cnt = a.cnt1[q];
+  const int cnt = (late_bound(MEAS) ? a.fcnt : a.cnt1)[q];
   if (blockIdx.x * kLb2Warps >= cnt) return;  // uniform across the CTA
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
   const float4 qb = a.qbox[q];
-  const float t = a.thr[q];
+  const float t = (late_bound(MEAS) ? a.thr2 : a.thr)[q];
   // the query's sparse table of row boxes, built in global memory by
   // qtable_global_kernel (read through L1: a copy in shared memory per CTA
   // held occupancy to 3 CTAs per SM); a query longer than the table was
@@ -1269,7 +1281,7 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
   int m_nx = a.clen[c_nx];
   float s_nx = e + S < cnt ? LB1[c_nx] : 0.0f;
   int slot = 0;
-  PassList pass_list{a, q};
+  PassList pass_list{a, q, (late_bound(MEAS) ? a.cnt0 : a.cnt2) + q};
   bool bulk_cur = e < cnt && bulk_ok(o_cur, m_cur);
   if (bulk_cur) issue(0, o_cur, m_cur);
   for (; e < cnt; e += S) {
@@ -1387,9 +1399,8 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
       lbv = feasible ? fmaxf(acc, sbnd) : TSIM_INF;
       pass = lbv <= t;
     } else {
-      // every point of either trajectory is coupled to (Frechet) or has a
-      // nearest point in (Hausdorff) the other, so the squared distance is
-      // at least its squared distance to the other's box
+      // Frechet: every point of either trajectory is coupled to the other, so
+      // the squared distance is at least its squared distance to the other's box
       const float4 cb = a.cbox[c];
       float mx = 0.0f;
       for (int j = lane; j < m; j += 32) {
@@ -1422,8 +1433,7 @@ __global__ void __launch_bounds__(kLb2Warps * 32) lb2_kernel(KArgs a) {
 // DTW's at most 48 registers (5 CTAs of 8 warps per SM where shared memory
 // allows): the bulk-copy pipeline's state took it to 64 (4 CTAs), and the
 // batched workload's step ran 1.4 % slower for it; the few spilled values are
-// per-pair state, outside the column loop.  The other measures keep the
-// compiler's choice (LCSS spilled in its point loop under the same bound).
+// per-pair state, outside the column loop.  Frechet keeps the compiler's choice.
 __global__ void __launch_bounds__(kLb2Warps * 32, 5) lb2_dtw_kernel(KArgs a) {
   lb2_body<M_DTW>(a);
 }
@@ -2116,14 +2126,13 @@ __global__ void __launch_bounds__(32 * kRankWarps) final_sort_kernel(KArgs a) {
 // Per-request counters, accumulated on the device (no host sync per chunk):
 // counters[2..6] += pairs passing the O(1) bound, the O(length) bound,
 // refined pairs, re-scored pairs, FP64 re-scored pairs.
-// (LCSS: its O(length) bound follows round 1's first pass, whose pairs count
-// as passing it)
+// (an O(length) bound after round 1: round 1's pairs count as passing it)
 __global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_rescore, int meas) {
   unsigned long long c1 = 0, c2 = 0, rc = 0;
-  const bool late = meas == M_LCSS && !a.brute;
+  const bool late = late_bound(meas) && !a.brute;
   for (int q = threadIdx.x; q < a.nq; q += blockDim.x) {
-    c1 += meas == M_EUCLID || late ? a.cnt2[q] : a.cnt1[q];  // Euclidean: one bound stage only
-    c2 += late ? a.cnt0[q] + min(a.cnt2[q], a.Mr) : a.cnt2[q];
+    c1 += meas == M_EUCLID || late ? a.cnt2[q] : a.cnt1[q];  // one list of bounded pairs
+    c2 += late && meas != M_HAUSDORFF ? a.cnt0[q] + min(a.cnt2[q], a.Mr) : a.cnt2[q];
     rc += with_rescore ? min(a.rraw[q], a.RC) : 0;
   }
   for (int o = 16; o; o >>= 1) {
@@ -2463,16 +2472,14 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   if constexpr (MEAS != M_EUCLID) {
     segfilter_kernel<MEAS><<<dim3(std::max(1, std::min(1024, (32 * ctx->num_sms + nq - 1) / nq)), nq),
                              256, 0, s>>>(a);
-    if constexpr (MEAS != M_LCSS) {
-      const size_t lb2_smem =
-          MEAS == M_DTW ? sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2) : 0;
-      auto lb2 = MEAS == M_DTW ? lb2_dtw_kernel : lb2_kernel<MEAS>;
+    if constexpr (!late_bound(MEAS)) {
+      const size_t lb2_smem = sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2);
       if (lb2_smem > 48 * 1024)
-        TSIM_CUDA(cudaFuncSetAttribute(lb2, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        TSIM_CUDA(cudaFuncSetAttribute(lb2_dtw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)lb2_smem));
-      lb2<<<dim3(ch, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
+      lb2_dtw_kernel<<<dim3(ch, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
     }
-    launched(ctx, MEAS == M_LCSS ? 1 : 2);
+    launched(ctx, late_bound(MEAS) ? 1 : 2);
   }
   seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
   r1_select_kernel<MEAS, 0><<<nq, kSelThreads, 0, s>>>(a);
@@ -2516,6 +2523,12 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
                      kRowWarps * 32, 0, s>>>(a);
     launched(ctx);
     a.list1 = a.list2;  // what it kept
+    a.fcnt = a.cnt0;
+  }
+  if constexpr (MEAS == M_FRECHET) {
+    lb2_kernel<MEAS><<<dim3(ch, nq), kLb2Warps * 32, 0, s>>>(a);
+    launched(ctx);
+    a.list1 = a.list2;
     a.fcnt = a.cnt0;
   }
   if constexpr (MEAS == M_LCSS) {
