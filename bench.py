@@ -49,7 +49,7 @@ DP_FLOPS_PER_CELL = 8  # 2 sub, mul, fma (2), 2 min, add
 # dram__bytes_read.sum + dram__bytes_write.sum of the survivor-round DP launch
 # of this workload (dp_wave_kernel, single stream), one ncu capture of
 # `python -m cudaruntime1_gb300.profile_pass 1` on a GB300
-SURVIVOR_DP_DRAM_BYTES = 11592448
+SURVIVOR_DP_DRAM_BYTES = 6149120
 L2_FLUSH_BYTES = 512 << 20
 
 
@@ -423,8 +423,9 @@ def refine_roofline(measure, prof, fp32_peak, hbm_peak):
         return None
     fl = FLOPS_PER_UNIT[measure]
     tflops = units * fl / (ms * 1e-3) / 1e12
-    out = {"kernel": {"hausdorff": "hausdorff_refine_kernel", "euclidean": "euclid_refine_kernel"}
-           .get(measure, f"dp_diag_kernel ({measure})") + ", survivor round",
+    out = {"kernel": {"hausdorff": "hausdorff_refine_kernel", "euclidean": "euclid_refine_kernel",
+                      "lcss": "lcss_window_kernel (without a window: a lane or row groups per pair)"}
+           .get(measure, f"dp_strip_kernel or dp_half_kernel ({measure})") + ", survivor round",
            "unit_of_work": "point pair" if measure in ("hausdorff", "euclidean") else "DP cell",
            "units_per_launch": units, "launch_ms": ms, "flops_per_unit": fl,
            "fp32": {"achieved": tflops, "peak": fp32_peak, "unit": "TFLOP/s",

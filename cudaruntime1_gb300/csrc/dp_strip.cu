@@ -246,7 +246,8 @@ __global__ void __launch_bounds__(kStripThreads)
 // all have a side of at most 16 R points: 15 steps of ramp for a strip
 // instead of 31 (128 x 128: 143 steps of 8 rows for two pairs against 159 of
 // 4 rows for one: 8,192 such pairs 61 -> 57 us, and the reference's
-// square-root cost 1,024 x 10 pairs of them 208 -> 138 us).  The halves' pairs differ in length, so a lane outside
+// square-root cost, 1,024 x 10 pairs of them, 131 us, striped 178).  The halves'
+// pairs differ in length, so a lane outside
 // its matrix sits the step out; its last values stay for the result.
 #define HPT(j) pts[TSIM_SIDX(j, cap)]
 template <class P, int R>
