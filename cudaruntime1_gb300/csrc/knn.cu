@@ -80,8 +80,7 @@ constexpr bool is_squared(int meas) { return meas >= M_FRECHET; }
 // pairs for 2.8 of a request's 10.3 ms, and of the 0.47 M that pass round 1's
 // threshold it kept 96 %, so Hausdorff has none (1,024 queries against 262,144
 // candidates 5.43 -> 4.53 ms; 4.80 with it after round 1); Frechet, whose DP
-// costs far more a pair, 523 -> 515 us.  DTW keeps it before round 1: its round
-// lasts longer than the bound.
+// costs far more a pair, 523 -> 515 us.  DTW has both orders (KArgs::late).
 constexpr bool late_bound(int meas) {
   return meas == M_LCSS || meas == M_HAUSDORFF || meas == M_FRECHET;
 }
@@ -111,6 +110,13 @@ struct KArgs {
   int k, S, T, nch;
   int Mr;   // round 1's pairs per query and pass: M, or (LCSS, two passes) half of it
   int r1n;  // those refined so far
+  // DTW: whether the O(length) bound follows round 1, whose pairs then go by
+  // the segment bound, and the row side.  On a database beyond L2, whose points
+  // it reads from HBM: it kept 494 k of 567 k pairs there, and after both is
+  // left 16 k (mixed serving from 1,000,000 trajectories 7.25 -> 6.55 ms).  In
+  // L2 a better round 1 is worth more for few queries (one query 280 us, 284
+  // the other way round).
+  int late;
   int plain;    // one DP pair per kernel launch (the unbatched comparison form)
   int brute;    // small request: every pair refined exactly, no bound stages
   int noprune;  // thresholds stay open: every pair is refined
@@ -315,6 +321,11 @@ __global__ void __launch_bounds__(256) prep_kernel(KArgs a, float4* qbox, float4
     for (size_t i = tid; i < (size_t)a.nq * a.Cw; i += nthreads) a.seedmap[i] = 0u;
     for (size_t i = tid; i < (size_t)shapes; i += nthreads) a.shape_cnt[i] = 0;
   }
+}
+
+template <int MEAS>
+__device__ __forceinline__ bool is_late(const KArgs& a) {
+  return MEAS == M_DTW ? a.late != 0 : late_bound(MEAS);
 }
 
 // entry i of query q among round 1's pairs: the passes' lists one after the other
@@ -1124,7 +1135,7 @@ __global__ void __launch_bounds__(kChunk) compact_kernel(KArgs a) {
 #pragma unroll
   for (int i = 0; i < kCompact; ++i)
     if ((take >> i) & 1u) {
-      (late_bound(MEAS) ? a.list1 : a.list2)[at] = c0 + i * kChunk;
+      (is_late<MEAS>(a) ? a.list1 : a.list2)[at] = c0 + i * kChunk;
       if (MEAS == M_EUCLID) a.lb2v[at] = bnd[i];
       ++at;
     }
@@ -1134,24 +1145,24 @@ __global__ void __launch_bounds__(kChunk) compact_kernel(KArgs a) {
 // (the O(1) bound keeps few pairs of a chunk).  The bound is kept in place of
 // the O(1) bound: the O(length) stage and the round-1 order use the tighter
 // of it and their own.
-template <int MEAS>
+template <int MEAS, bool LATE>
 __global__ void __launch_bounds__(256, MEAS == M_DTW ? 5 : 1) segfilter_kernel(KArgs a) {
   const int q = blockIdx.y;
   const int cnt = a.cnt0[q];
   const float t = a.thr[q];
   const int n = a.qlen[q];
   const int g = threadIdx.x & (kSegGroup - 1);
-  constexpr bool kLcss = MEAS == M_LCSS, kLate = late_bound(MEAS);
-  constexpr int kVals = kLcss ? 3 : kLate ? 2 : 1;
+  constexpr bool kLcss = MEAS == M_LCSS;
+  constexpr int kVals = kLcss ? 3 : LATE ? 2 : 1;
   __shared__ int buf[256 / 32][64][kVals];
   const int warp = threadIdx.x >> 5;
   constexpr int kPer = 32 / kSegGroup;  // pairs per warp and pass
   // the bound comes along where it orders round 1, and LCSS's hull of the
   // columns that can match (in flat_vals, free until the survivors' round)
   const size_t row = (size_t)q * a.C;
-  const int* in = (kLate ? a.list1 : a.list2) + row;
+  const int* in = (LATE ? a.list1 : a.list2) + row;
   int* bounds = reinterpret_cast<int*>(a.lb2v) + row;
-  WarpList<kVals> out{(kLate ? a.cnt2 : a.cnt1) + q, (kLate ? a.list2 : a.list1) + row, bounds,
+  WarpList<kVals> out{(LATE ? a.cnt2 : a.cnt1) + q, (LATE ? a.list2 : a.list1) + row, bounds,
                       reinterpret_cast<int*>(a.flat_vals) + row, buf[warp]};
   const int start = (blockIdx.x * (blockDim.x >> 5) + warp) * kPer;
   const int stride = gridDim.x * (blockDim.x >> 5) * kPer;
@@ -1210,12 +1221,12 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int q = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int cnt = (late_bound(MEAS) ? a.fcnt : a.cnt1)[q];
+  const int cnt = (is_late<MEAS>(a) ? a.fcnt : a.cnt1)[q];
   if (blockIdx.x * kLb2Warps >= cnt) return;  // uniform across the CTA
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
   const float4 qb = a.qbox[q];
-  const float t = (late_bound(MEAS) ? a.thr2 : a.thr)[q];
+  const float t = (is_late<MEAS>(a) ? a.thr2 : a.thr)[q];
   // the query's sparse table of row boxes, built in global memory by
   // qtable_global_kernel (read through L1: a copy in shared memory per CTA
   // held occupancy to 3 CTAs per SM); a query longer than the table was
@@ -1281,7 +1292,7 @@ __device__ __forceinline__ void lb2_body(const KArgs& a) {
   int m_nx = a.clen[c_nx];
   float s_nx = e + S < cnt ? LB1[c_nx] : 0.0f;
   int slot = 0;
-  PassList pass_list{a, q, (late_bound(MEAS) ? a.cnt0 : a.cnt2) + q};
+  PassList pass_list{a, q, (is_late<MEAS>(a) ? a.cnt0 : a.cnt2) + q};
   bool bulk_cur = e < cnt && bulk_ok(o_cur, m_cur);
   if (bulk_cur) issue(0, o_cur, m_cur);
   for (; e < cnt; e += S) {
@@ -2129,7 +2140,7 @@ __global__ void __launch_bounds__(32 * kRankWarps) final_sort_kernel(KArgs a) {
 // (an O(length) bound after round 1: round 1's pairs count as passing it)
 __global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_rescore, int meas) {
   unsigned long long c1 = 0, c2 = 0, rc = 0;
-  const bool late = late_bound(meas) && !a.brute;
+  const bool late = (meas == M_DTW ? a.late != 0 : late_bound(meas)) && !a.brute;
   for (int q = threadIdx.x; q < a.nq; q += blockDim.x) {
     c1 += meas == M_EUCLID || late ? a.cnt2[q] : a.cnt1[q];  // one list of bounded pairs
     c2 += late && meas != M_HAUSDORFF ? a.cnt0[q] + min(a.cnt2[q], a.Mr) : a.cnt2[q];
@@ -2469,17 +2480,24 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   // CTAs per query of the grid-stride filter kernels: about 8 per SM over the
   // whole request, so a single query against a large database fills the GPU
   const int ch = std::max(1, std::min(65535, (8 * ctx->num_sms + nq - 1) / nq));
+  // DTW: banded LB_Keogh from the candidates' columns
+  auto column_side = [&]() -> int {
+    const size_t lb2_smem = sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2);
+    if (lb2_smem > 48 * 1024)
+      TSIM_CUDA(cudaFuncSetAttribute(lb2_dtw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)lb2_smem));
+    lb2_dtw_kernel<<<dim3(ch, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
+    launched(ctx);
+    return TSIM_OK;
+  };
   if constexpr (MEAS != M_EUCLID) {
-    segfilter_kernel<MEAS><<<dim3(std::max(1, std::min(1024, (32 * ctx->num_sms + nq - 1) / nq)), nq),
-                             256, 0, s>>>(a);
-    if constexpr (!late_bound(MEAS)) {
-      const size_t lb2_smem = sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2);
-      if (lb2_smem > 48 * 1024)
-        TSIM_CUDA(cudaFuncSetAttribute(lb2_dtw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)lb2_smem));
-      lb2_dtw_kernel<<<dim3(ch, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
-    }
-    launched(ctx, late_bound(MEAS) ? 1 : 2);
+    constexpr bool kDtw = MEAS == M_DTW;
+    auto segfilter = kDtw && a.late ? segfilter_kernel<MEAS, true>
+                                    : segfilter_kernel<MEAS, kDtw ? false : late_bound(MEAS)>;
+    segfilter<<<dim3(std::max(1, std::min(1024, (32 * ctx->num_sms + nq - 1) / nq)), nq), 256, 0, s>>>(
+        a);
+    launched(ctx);
+    if (MEAS == M_DTW && !a.late) TSIM_TRY(column_side());
   }
   seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
   r1_select_kernel<MEAS, 0><<<nq, kSelThreads, 0, s>>>(a);
@@ -2522,8 +2540,16 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     lb_rows_kernel<<<dim3(std::max(1, std::min((a.C + kRowWarps - 1) / kRowWarps, 8 * ch)), nq),
                      kRowWarps * 32, 0, s>>>(a);
     launched(ctx);
-    a.list1 = a.list2;  // what it kept
+    std::swap(a.list1, a.list2);  // what it kept
     a.fcnt = a.cnt0;
+    a.cnt0 = a.cnt1;
+  }
+  if constexpr (MEAS == M_DTW) {
+    if (a.late) {
+      TSIM_TRY(column_side());
+      a.list1 = a.list2;
+      a.fcnt = a.cnt0;
+    }
   }
   if constexpr (MEAS == M_FRECHET) {
     lb2_kernel<MEAS><<<dim3(ch, nq), kLb2Warps * 32, 0, s>>>(a);
@@ -2845,6 +2871,7 @@ int knn(tsim_ctx* ctx, const tsim_params* p, const float2* qpts, const int64_t* 
                (reinterpret_cast<uintptr_t>(db->pts) & 15) == 0)
                   ? (std::min(db->max_len, 512) + 1) & ~1
                   : 0;
+  a.late = p->measure == TSIM_DTW && db_beyond_l2;
   a.status = ctx->status;
   a.order = arena_take<int>(ctx, nqC);
   a.shape_cnt = arena_take<int>(ctx, kNumShapes);

@@ -519,3 +519,18 @@ def test_dtw_from_both_ends(tsim, cuda_ctx, oracle, band, cost):
         # costs within 4 2^-24, their compensated sum, the result's rounding
         assert np.all(np.abs(d[fin] - want[fin]) <= 5 * 2.0 ** -24 * want[fin])
     db.close()
+
+
+@pytest.mark.parametrize("kw", [dict(band_pct=10), dict(band_pct=10, cost=1), dict(band_pct=-1)])
+def test_dtw_on_a_database_beyond_l2(tsim, cuda_ctx, kw):
+    """Round 1 ahead of LB_Keogh, whose points come from HBM (108 MB of them):
+    the answer of a request that refines every pair, bit for bit."""
+    lens = np.random.default_rng(3).integers(400, 500, 30000)
+    lens[:200] = np.arange(2, 202)
+    cp, co = G.random_walks(30000, lens, 91, start_range=20.0)
+    qp, qo = G.random_walks(3, [2, 100, 700], 92, start_range=20.0)
+    db = tsim.Database(cuda_ctx, cp, co)
+    ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, flags=tsim.api.FLAG_ALWAYS_PRUNE, **kw)
+    ids2, d2, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, flags=tsim.api.FLAG_NO_PRUNE, **kw)
+    assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
+    db.close()
