@@ -86,14 +86,14 @@ __device__ __forceinline__ int strip_cost(int rows, int cols, int rmax, int& R) 
 }
 
 #define PT(j) pts[TSIM_SIDX((j) + kStripPad, cap + 2 * kStripPad)]
-#define ROWBUF(j) buf[TSIM_SIDX((j) + kStripPad, cap + 2 * kStripPad)]
+#define ROWBUF(j) buf[TSIM_SIDX((j) + kStripPad, bufcap)]
 
 // One pair on the warp.  MULTI: rows in several strips.
 template <class P, int R, bool MULTI>
 __device__ __forceinline__ void strip_pair(const DpArgs& a, const int pid, const float2* O,
                                            const int rows, const int cols, const float thr,
                                            const float aux, const float2* pts,
-                                           typename P::V* buf, const int cap) {
+                                           typename P::V* buf, const int cap, const int bufcap) {
   using V = typename P::V;
   const int lane = threadIdx.x & 31;
   const int nstrips = MULTI ? (rows + 32 * R - 1) / (32 * R) : 1;
@@ -195,8 +195,10 @@ __global__ void __launch_bounds__(kStripThreads)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kWarps = kStripThreads / 32;
   float2* pts = strip_smem + (size_t)warp * (cap + 2 * kStripPad);
+  // the row between strips: there only where the launch's longest pair needs it
+  const int bufcap = multi ? cap + 2 * kStripPad : 0;
   V* buf = reinterpret_cast<V*>(strip_smem + (size_t)kWarps * (cap + 2 * kStripPad)) +
-           (multi ? (size_t)warp * (cap + 2 * kStripPad) : 0);
+           (size_t)warp * bufcap;
   const int slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nslots = (gridDim.x * blockDim.x) >> 5;
   const int npairs = a.npairs_dev ? min(*a.npairs_dev, a.npairs) : a.npairs;
@@ -219,9 +221,13 @@ __global__ void __launch_bounds__(kStripThreads)
       continue;
     }
     const bool tr = cc < cq;
+    const int rows = tr ? m : n, cols = tr ? n : m, R = tr ? Rc : Rq;
+    if (rows > 32 * RM && !multi) {  // longer than max_n and max_m: no row to join its strips
+      if (lane == 0) spill[atomicAdd(nspill, 1)] = pid;
+      continue;
+    }
     const float2* O = tr ? a.cpts + co : a.qpts + qo;
     const float2* I = tr ? a.qpts + qo : a.cpts + co;
-    const int rows = tr ? m : n, cols = tr ? n : m, R = tr ? Rc : Rq;
     const float thr = a.thr ? a.thr[pr.x] : TSIM_INF;
     const float aux = a.aux ? (float)a.aux[pid] : a.eps;
     __syncwarp();  // the previous pair's reads are done
@@ -229,13 +235,13 @@ __global__ void __launch_bounds__(kStripThreads)
       PT(j) = (unsigned)j < (unsigned)cols ? __ldg(I + j) : make_float2(TSIM_INF, TSIM_INF);
     __syncwarp();
     if (rows > 32 * RM)
-      strip_pair<P, RM, true>(a, pid, O, rows, cols, thr, aux, pts, buf, cap);
+      strip_pair<P, RM, true>(a, pid, O, rows, cols, thr, aux, pts, buf, cap, bufcap);
     else if (R == 2)
-      strip_pair<P, 2, false>(a, pid, O, rows, cols, thr, aux, pts, buf, cap);
+      strip_pair<P, 2, false>(a, pid, O, rows, cols, thr, aux, pts, buf, cap, bufcap);
     else if (R == 4)
-      strip_pair<P, 4, false>(a, pid, O, rows, cols, thr, aux, pts, buf, cap);
+      strip_pair<P, 4, false>(a, pid, O, rows, cols, thr, aux, pts, buf, cap, bufcap);
     else
-      strip_pair<P, RM, false>(a, pid, O, rows, cols, thr, aux, pts, buf, cap);
+      strip_pair<P, RM, false>(a, pid, O, rows, cols, thr, aux, pts, buf, cap, bufcap);
   }
 }
 

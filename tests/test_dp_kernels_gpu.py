@@ -260,3 +260,47 @@ def test_lcss_window_bit_vectors(tsim, cuda_ctx, oracle, delta):
         wi, wd = oracle.knn("lcss", qp, qo, cp, co, 12, eps=eps, delta=delta)
         assert np.array_equal(ids, wi) and np.array_equal(d, wd)
         db.close()
+
+
+@pytest.mark.parametrize("stated,most", [(100, 200), (128, 128), (250, 60)])
+@pytest.mark.parametrize("measure,kw", [("dtw", {}), ("dtw", dict(cost=1)), ("frechet", {})])
+def test_full_rows_of_queries_longer_than_stated(tsim, cuda_ctx, oracle, measure, kw, stated, most):
+    """Full rows, queries past the stated longest length -- by a point, past
+    one strip of rows, past several -- against candidates that fit the
+    staging: pair values are the bits of the round-striped kernel (given the
+    true length), kNN answers the oracle's."""
+    import torch
+    from cudaruntime1_gb300 import api
+    ql = [stated, stated + 1, 129, 257, 300, 513, 700, 40]
+    cl = np.random.default_rng(3).integers(30, most + 1, 300)
+    cl[0] = most
+    qp, qo = G.random_walks(8, ql, 95, start_range=10.0)
+    cp, co = G.random_walks(300, cl, 96, start_range=10.0)
+    pairs = np.stack(np.meshgrid(np.arange(8), np.arange(300), indexing="ij"), -1).reshape(-1, 2)
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+           (qp, np.asarray(qo), cp, np.asarray(co), pairs.astype(np.int32))]
+    for count in (300, len(pairs)):
+        for precision in (0, 1):
+            out = []
+            for kernel, longest in ((1, max(ql)), (0, stated)):
+                o = torch.full((count,), float("nan"), device="cuda",
+                               dtype=(torch.float32, torch.float64)[precision])
+                api.dp_pairs(cuda_ctx, measure, precision, kernel, dev[0].data_ptr(),
+                             dev[1].data_ptr(), longest, dev[2].data_ptr(), dev[3].data_ptr(), most,
+                             dev[4][len(pairs) - count:].data_ptr(), count, o.data_ptr(),
+                             o.data_ptr(), **kw)
+                torch.cuda.synchronize()
+                out.append(o.cpu().numpy())
+            assert np.array_equal(out[0], out[1]), (count, precision)
+    db = tsim.Database(cuda_ctx, cp, co)
+    want_ids, want = oracle.knn(measure, qp, qo, cp, co, 10, **kw)
+    ids = torch.empty(80, dtype=torch.int32, device="cuda")
+    d, d64 = torch.empty(80, device="cuda"), torch.empty(80, dtype=torch.float64, device="cuda")
+    for flags in (0, tsim.api.FLAG_ALWAYS_PRUNE):
+        tsim.knn_device(cuda_ctx, db, dev[0].data_ptr(), dev[1].data_ptr(), 8, stated,
+                        ids.data_ptr(), d.data_ptr(), d64.data_ptr(), measure, 10,
+                        flags=flags | tsim.api.FLAG_FP64_RESCORE, **kw)
+        cuda_ctx.synchronize()
+        assert np.array_equal(ids.cpu().numpy().reshape(8, 10), want_ids)
+        assert np.array_equal(d64.cpu().numpy().reshape(8, 10), want)
+    db.close()
