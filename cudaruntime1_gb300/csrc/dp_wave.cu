@@ -421,10 +421,6 @@ __global__ void __launch_bounds__(kWaveThreads)
   }
 }
 
-__device__ __forceinline__ float path_sum(float a, float b) { return a + b; }
-__device__ __forceinline__ df path_sum(df a, df b) {
-  return a.hi < TSIM_INF && b.hi < TSIM_INF ? df_add(a, b) : df_inf();
-}
 __device__ __forceinline__ void pair_sync(int pair) {  // the two warps of a pair
   static_assert(kWaveThreads == 128, "two pairs a CTA");
   if (pair == 0)
@@ -439,15 +435,18 @@ __device__ __forceinline__ void pair_sync(int pair) {  // the two warps of a pai
 // steps is half as long.  A path steps from anti-diagonal s or s - 1 to s + 1,
 // or from s to s + 2: the value is the least sum, over the cells behind and
 // their predecessors before, of the two halves' values.  A sum of two halves
-// rounds no more often than one running sum.
+// rounds no more often than one running sum, but not to the same bits, so only
+// rounds that order pairs within an error bound come here, none whose values
+// are returned (the compensated re-score: 70 us instead of 90, but distances
+// then depended on how many queries shared the call).
 //
 // What bounds it: the steps' latency (a shuffle, a minimum, an addition, the
-// next cost).  Ten pairs of 333 x 64 to 512 points 47 -> 31 us, compensated 90
-// (two warps of row groups) -> 70.
+// next cost).  Ten pairs of 333 x 64 to 512 points 47 -> 31 us.
 template <class P, int RMAX>
 __global__ void __launch_bounds__(kWaveThreads)
     dp_wave2_kernel(DpArgs a, int ccap, int qcap, int* spill, int* nspill) {
   using V = typename P::V;
+  static_assert(std::is_same<V, float>::value, "compensated values are one running sum");
   extern __shared__ __align__(16) float2 wave_smem[];
   constexpr int kPairs = kWaveThreads / 64;
   // forward's last and previous anti-diagonal, backward's
@@ -509,9 +508,9 @@ __global__ void __launch_bounds__(kWaveThreads)
           const int i1 = n - 1 - (gb[0] + p);  // row of a cell on s + 1
           const V before = vmin(vmin(fwd(f0, gf[0], i1 - 1), fwd(f0, gf[0], i1)),
                                 fwd(f1, gf[1], i1 - 1));
-          best = vmin(best, path_sum(before, b0[p]));
+          best = vmin(best, before + b0[p]);
           const int i2 = n - 1 - (gb[1] + p);  // and on s + 2
-          best = vmin(best, path_sum(fwd(f0, gf[0], i2 - 1), b1[p]));
+          best = vmin(best, fwd(f0, gf[0], i2 - 1) + b1[p]);
         }
       }
       for (int o = 16; o; o >>= 1) best = vmin(best, wshfl(best, lane ^ o));
@@ -617,8 +616,6 @@ int launch_dp_wave2(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max
   switch (kind) {
     case DP_DTW_SQ: return wave2_chain<PolDtwSq>(ctx, a, max_n, max_m, spill, nspill);
     case DP_DTW_EU: return wave2_chain<PolDtwEu>(ctx, a, max_n, max_m, spill, nspill);
-    case DP_DTW_SQC: return wave2_chain<PolDtwSqC>(ctx, a, max_n, max_m, spill, nspill);
-    case DP_DTW_EUC: return wave2_chain<PolDtwEuC>(ctx, a, max_n, max_m, spill, nspill);
   }
   return fail(TSIM_ERR_UNSUPPORTED, "no two-ended kernel for this DP kind");
 }

@@ -2210,15 +2210,16 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
   }
   if (!diag_kind || a.rdiag == 0) return launch_dp(ctx, kind, G, R, d, a.max_clen);
   const bool twofloat_kind = kind == DP_DTW_SQC || kind == DP_DTW_EUC || kind == DP_FRECHET_SQC;
-  // Rounds of no more pairs than two an SM -- a query or a few -- run each pair
-  // from both ends on two warps, one a scheduler: a lone query's seeds, round 1
-  // and re-score 47 + 45 + 90 -> 31 + 31 + 70 us.  Larger ones gained nothing
-  // next to other requests (64 queries 402 us either way) and mixed serving
-  // lost 1.8 %: a pair's own latency no longer counts, its staging twice does.
+  // FP32 rounds of no more pairs than two an SM -- a query or a few -- run each
+  // pair from both ends on two warps, one a scheduler: a lone query's seeds and
+  // round 1 47 + 45 -> 31 + 31 us.  Larger ones gained nothing next to other
+  // requests (64 queries 402 us either way) and mixed serving lost 1.8 %: a
+  // pair's own latency no longer counts, its staging twice does.  Their values
+  // only order pairs within the FP32 error bound; compensated ones are
+  // returned, and a sum of two halves is not the bits of one running sum.
   const bool two_ended = latency && !a.plain && d.npairs <= 2 * ctx->num_sms &&
-                         (kind == DP_DTW_SQ || kind == DP_DTW_EU || kind == DP_DTW_SQC ||
-                          kind == DP_DTW_EUC);
-  if (a.wave && wave_kind(kind) && (two_ended || !twofloat_kind)) {
+                         (kind == DP_DTW_SQ || kind == DP_DTW_EU);
+  if (a.wave && wave_kind(kind) && !twofloat_kind) {
     // lanes along the anti-diagonal, straight-line blocks of 16 steps: the
     // shortest FP32 step of the warp-per-pair forms (a lone 512 x 486 pair
     // 83 us against 104 on two warps per pair; compensated pairs are faster

@@ -367,9 +367,9 @@ int status_result(tsim_ctx* ctx, unsigned v);
 int set_wait_limit(long long attempts);
 int launch_dp_wave(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, bool latency,
                    int* spill, int** nspill);
-// The same of DTW on two warps a pair, from both ends to the middle: latency
-// rounds whose values only order pairs within an error bound, or are
-// compensated (a sum of halves is not the bits of one running sum).
+// The same of FP32 DTW on two warps a pair, from both ends to the middle:
+// latency rounds whose values only order pairs within an error bound (a sum of
+// halves is not the bits of one running sum).
 int launch_dp_wave2(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
                     int** nspill);
 // whether it takes every pair of at least two points a side up to these lengths

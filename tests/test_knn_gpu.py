@@ -534,3 +534,32 @@ def test_dtw_on_a_database_beyond_l2(tsim, cuda_ctx, kw):
     ids2, d2, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, flags=tsim.api.FLAG_NO_PRUNE, **kw)
     assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
     db.close()
+
+
+@pytest.mark.parametrize("cost", [0, 1])
+def test_distances_alone_and_in_a_batch(tsim, cuda_ctx, cost):
+    """Banded DTW's distances do not depend on how many queries share the
+    call, nor on the kernels chosen: the bits of each query alone, of a few
+    together, and of all of them with the row-group kernels."""
+    rng = np.random.default_rng(97)
+    cp, co = _db(3000, 16, 300, 97)
+    qp, qo = G.random_walks(24, G.uniform_lengths(24, 16, 300, 98), 99)
+    for c in range(480):  # near copies, whose costs span more bits than a pair of floats holds
+        src = np.linspace(qo[c % 24], qo[c % 24 + 1] - 1, co[c + 1] - co[c]).round().astype(int)
+        scale = 2.0 ** rng.uniform(-16, 3, (len(src), 1))
+        cp[co[c]:co[c + 1]] = qp[src] + scale * rng.standard_normal((len(src), 2))
+    db = tsim.Database(cuda_ctx, cp, co)
+    kw = dict(band_pct=10, cost=cost)
+    for flags in (0, tsim.api.FLAG_ALWAYS_PRUNE):
+        want = _device_knn(tsim, cuda_ctx, db, qp, qo, "dtw", 10, flags=flags, **kw)
+        off = _device_knn(tsim, cuda_ctx, db, qp, qo, "dtw", 10,
+                          flags=flags | tsim.api.FLAG_NO_WAVE_DP, **kw)
+        assert np.array_equal(off[0], want[0])
+        assert np.array_equal(off[2].view(np.uint64), want[2].view(np.uint64))
+        for q0, q1 in [(q, q + 1) for q in range(0, 24, 3)] + [(1, 4), (5, 9)]:
+            got = _device_knn(tsim, cuda_ctx, db, qp[qo[q0]:qo[q1]], qo[q0:q1 + 1] - qo[q0], "dtw",
+                              10, flags=flags, **kw)
+            assert np.array_equal(got[0], want[0][q0:q1])
+            assert np.array_equal(got[1].view(np.uint32), want[1][q0:q1].view(np.uint32))
+            assert np.array_equal(got[2].view(np.uint64), want[2][q0:q1].view(np.uint64))
+    db.close()
