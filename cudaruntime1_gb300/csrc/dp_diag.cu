@@ -442,8 +442,7 @@ int launch_diag_one(tsim_ctx* ctx, const DpArgs& a, int max_m, int* spill, int* 
   if (diag_suffix<P, W>(a))
     smem += (size_t)pairs_per_cta * (col_cap + 1 + diag_checks(a.max_n, col_cap)) * sizeof(float);
   auto kern = dp_diag_kernel<P, R, W>;
-  if (smem > 48 * 1024)
-    TSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSIM_CUDA(allow_dynamic_smem(kern, smem));
   int per_sm = 0;
   TSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
   long long blocks = std::min<long long>((a.npairs + pairs_per_cta - 1) / pairs_per_cta,

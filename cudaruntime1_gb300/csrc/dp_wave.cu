@@ -550,8 +550,7 @@ int launch_wave2_one(tsim_ctx* ctx, const DpArgs& a, int ccap, int qcap, int* sp
   if (a.npairs <= 0) return TSIM_OK;
   auto kern = dp_wave2_kernel<P, R>;
   const size_t smem = (size_t)(kWaveThreads / 32) * wave_per_warp(ccap, qcap) * sizeof(float2);
-  if (smem > 40 * 1024)
-    TSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSIM_CUDA(allow_dynamic_smem(kern, smem));
   int per_sm = 0;
   TSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWaveThreads, smem));
   if (per_sm < 1) return fail(TSIM_ERR_UNSUPPORTED, "wave kernel does not fit on an SM");

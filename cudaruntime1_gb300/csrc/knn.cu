@@ -2425,9 +2425,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   launched(ctx);
   stage_begin(ctx, TSIM_STAGE_SEED);
   const size_t seed_smem = sizeof(unsigned long long) * (size_t)a.nch * a.T;
-  if (seed_smem > 48 * 1024)
-    TSIM_CUDA(cudaFuncSetAttribute(seed_kernel<MEAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)seed_smem));
+  TSIM_CUDA(allow_dynamic_smem(seed_kernel<MEAS>, seed_smem));
   seed_kernel<MEAS><<<nq, kSelThreads, seed_smem, s>>>(a);
   TSIM_CUDA(cudaGetLastError());
   launched(ctx);
@@ -2484,9 +2482,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   // DTW: banded LB_Keogh from the candidates' columns
   auto column_side = [&]() -> int {
     const size_t lb2_smem = sizeof(float2) * (size_t)kLb2Warps * 2 * (a.lb2_cap + 2);
-    if (lb2_smem > 48 * 1024)
-      TSIM_CUDA(cudaFuncSetAttribute(lb2_dtw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)lb2_smem));
+    TSIM_CUDA(allow_dynamic_smem(lb2_dtw_kernel, lb2_smem));
     lb2_dtw_kernel<<<dim3(ch, nq), kLb2Warps * 32, lb2_smem, s>>>(a);
     launched(ctx);
     return TSIM_OK;

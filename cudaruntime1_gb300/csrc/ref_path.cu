@@ -232,8 +232,7 @@ int ref_batch_core(tsim_ctx* ctx, int measure, const float2* d_t1, const float2*
   const int tq = num_t >= 4 * ctx->num_sms && 2 * one + kRefTileBytes <= 100 * 1024 ? 2 : 1;
   const size_t smem = tq * one + kRefTileBytes;
   auto launch_filter = [&](auto kern) -> int {
-    if (smem > 48 * 1024)
-      TSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TSIM_CUDA(allow_dynamic_smem(kern, smem));
     kern<<<(num_t + tq - 1) / tq, kFilterThreads, smem, ctx->stream>>>(d_t1, d_t2, num_t, n, m, eps,
                                                                        K, gkeys, pairs);
     TSIM_CUDA(cudaGetLastError());

@@ -160,6 +160,15 @@ inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr int kCounterInts = 4;
 int fresh_counter(tsim_ctx* ctx, int* fallback, int** out);
 
+// Lets launches of a kernel that also has static shared memory (at most
+// 16 KiB) take `dynamic` bytes: past 48 KiB of the two together they are
+// refused otherwise.
+template <class K>
+cudaError_t allow_dynamic_smem(K kern, size_t dynamic) {
+  if (dynamic <= 32 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic);
+}
+
 int pinned_reserve(tsim_ctx* ctx, size_t bytes);
 // Every device and pinned-host allocation of the library goes through these,
 // so tsim_debug_fail_allocations can make any of them fail as out of memory.

@@ -563,3 +563,18 @@ def test_distances_alone_and_in_a_batch(tsim, cuda_ctx, cost):
             assert np.array_equal(got[1].view(np.uint32), want[1][q0:q1].view(np.uint32))
             assert np.array_equal(got[2].view(np.uint64), want[2][q0:q1].view(np.uint64))
     db.close()
+
+
+@pytest.mark.parametrize("count,length", [(6010 * 256, 2), (33000, 381), (33000, 382), (33000, 383)])
+def test_shared_memory_around_48_kib(tsim, cuda_ctx, count, length):
+    """Databases whose seed keys, or whose longest candidate's copies, take
+    about 48 KiB of a block's shared memory: the answer of a request that
+    refines every pair."""
+    cp, co = G.random_walks(count, length, 17)
+    qp, qo = G.random_walks(2, 30, 18)
+    db = tsim.Database(cuda_ctx, cp, co)
+    ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, band_pct=20)
+    ids2, d2, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, band_pct=20,
+                           flags=tsim.api.FLAG_NO_PRUNE)
+    assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
+    db.close()

@@ -104,3 +104,22 @@ def test_euclidean_csr_and_pipeline(tsim, cuda_ctx, oracle):
     c2 = oracle.mbr_knn(t1, n, t2, n, k)
     want2 = oracle.ref_euclid_cands(t1, t2, n, c2, np.arange(0, num_t * k + 1, k, dtype=np.int32))
     assert np.array_equal(_bits(got2), _bits(want2))
+
+
+@pytest.mark.parametrize("num_t,m", [(16, 1860), (16, 1908), (16, 1950), (16, 2020), (16, 2040),
+                                     (608, 655), (608, 700), (608, 716), (608, 717), (1, 12790)])
+def test_candidate_lengths_around_48_kib(tsim, cuda_ctx, oracle, num_t, m):
+    """Envelopes, keys and staged columns of about 48 KiB, with one query a
+    block and with two, and of the most the filter takes."""
+    import torch
+    from cudaruntime1_gb300 import api
+    t1 = G.ref_base_trajectories(num_t, 24, 7, r=300.0)
+    t2 = G.ref_similar_trajectories(t1, num_t, 24, m, 2.0, 9, r=300.0)
+    d1, d2 = (torch.from_numpy(np.ascontiguousarray(t, np.float32)).cuda() for t in (t1, t2))
+    out = torch.empty(num_t, device="cuda")
+    for measure in ("dtw", "lcss", "frechet"):
+        api.ref_batch_device(cuda_ctx, measure, d1.data_ptr(), d2.data_ptr(), num_t, 24, m,
+                             out.data_ptr())
+        cuda_ctx.synchronize()
+        assert np.array_equal(_bits(out.cpu().numpy()),
+                              _bits(oracle.ref_batch(measure, t1, t2, 24, m, eps=0.5))), measure
