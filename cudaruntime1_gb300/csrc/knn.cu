@@ -1456,8 +1456,8 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 5) lb2_dtw_kernel(KArgs a) {
 // cells of side gs >= 1.01 eps, each query point marking its cell and the 8
 // around it.  A candidate point within eps (per coordinate) of any query point
 // then lies in a marked cell: its cell index differs from that query point's
-// by at most 1 per axis, the index arithmetic's rounding (< 1e-3 cell) being
-// covered by the 1 % margin.  Points off the grid count as on its border.
+// by at most 1 per axis, the index arithmetic's rounding (two a point, of an
+// index below 43,691: 0.0046 cell) being covered by the 1 % margin.  Points off the grid count as on its border.
 //
 // What bounds it: the latency of the points, which come from L2 and HBM, and
 // issue; so only the columns of the hull that the segment bound found are read,
@@ -1493,8 +1493,12 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
   int gnx = 1, gny = 1;
   __syncthreads();
   if (a.eps > 0.0f) {
-    float gs = __fmul_ru(a.eps, 1.01f);
-    const float W = qb.z - qb.x, H = qb.w - qb.y;
+    // an extent that is not finite (points at infinity, NaNs alone on an axis)
+    // still gives cells inside the grid: points that match nothing may share
+    // one; and a cell side that growing by a quarter does not round back to
+    float gs = fmaxf(__fmul_ru(a.eps, 1.01f), FLT_MIN);
+    const float W = fminf(fmaxf(qb.z - qb.x, 0.0f), FLT_MAX);
+    const float H = fminf(fmaxf(qb.w - qb.y, 0.0f), FLT_MAX);
     while ((W / gs + 3.0f) * (H / gs + 3.0f) > 32.0f * kGridWords) gs *= 1.25f;
     gnx = (int)(W / gs) + 3;
     gny = (int)(H / gs) + 3;

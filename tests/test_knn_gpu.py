@@ -578,3 +578,27 @@ def test_shared_memory_around_48_kib(tsim, cuda_ctx, count, length):
                            flags=tsim.api.FLAG_NO_PRUNE)
     assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
     db.close()
+
+
+@pytest.mark.parametrize("delta", [-1, 6])
+@pytest.mark.parametrize("eps", [1e-45, 0.5, 3e38])
+def test_lcss_without_a_finite_extent(tsim, cuda_ctx, oracle, eps, delta):
+    """LCSS queries with NaNs or infinities among their points, alone on an
+    axis, or everywhere, and the smallest and largest epsilon: the oracle's
+    counts."""
+    cp, co = G.random_walks(400, G.uniform_lengths(400, 3, 60, 5), 6, start_range=4.0)
+    cp[co[7]:co[8]], cp[co[9]:co[10], 0] = np.nan, np.inf
+    ql = [40] * 9
+    qp, qo = G.random_walks(9, ql, 7, start_range=4.0)
+    bad = [(0, np.nan), (0, np.inf), (1, -np.inf), (slice(None), np.nan), (slice(None), np.inf)]
+    for q, (axis, v) in enumerate(bad):
+        qp[qo[q]:qo[q + 1], axis] = v
+    qp[qo[5] + 3, 0], qp[qo[6] + 5, 1], qp[qo[7], 0], qp[qo[7] + 1, 0] = np.inf, np.nan, -np.inf, np.inf
+    cp[co[20]:co[21]] = qp[qo[8]:qo[9]][:co[21] - co[20]][:1]  # equal points: they match at any epsilon
+    db = tsim.Database(cuda_ctx, cp, co)
+    want_ids, want = oracle.knn("lcss", qp, qo, cp, co, 10, eps=eps, delta=delta)
+    for flags in (0, tsim.api.FLAG_ALWAYS_PRUNE, tsim.api.FLAG_NO_PRUNE):
+        ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "lcss", 10, epsilon=eps, delta=delta, flags=flags)
+        assert np.array_equal(d, want), flags
+        assert np.array_equal(ids, want_ids), flags
+    db.close()
