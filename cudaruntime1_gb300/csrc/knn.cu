@@ -2044,6 +2044,13 @@ struct RankSlot {
   int c[kMaxRC];
   unsigned char ord[kMaxRC];  // entry index by rank
 };
+// a NaN (points that are not finite) orders as no distance at all: with it as
+// it is the ranks would not be a permutation, and the entries read by rank
+// not all written
+__device__ __forceinline__ double ordered(double v) {
+  const double inf = __longlong_as_double(0x7ff0000000000000ll);
+  return v < inf ? v : inf;
+}
 __device__ __forceinline__ bool before(double dv, int dc, int di, double v, int c, int i) {
   return dv < v || (dv == v && (dc < c || (dc == c && di < i)));
 }
@@ -2072,7 +2079,7 @@ __global__ void __launch_bounds__(32 * kRankWarps) cluster_kernel(KArgs a) {
                                              : 2.0 * gamma_dp(MEAS, a.qlen[q], a.max_clen);
   const double inf = __longlong_as_double(0x7ff0000000000000ll);
   for (int i = lane; i < n; i += 32) {
-    S.v[i] = rv[i];
+    S.v[i] = ordered(rv[i]);
     S.c[i] = rp[i].y;
   }
   for (int i = lane; i < a.RC; i += 32) r64p[i] = make_int2(q, -1);
@@ -2117,7 +2124,7 @@ __global__ void __launch_bounds__(32 * kRankWarps) final_sort_kernel(KArgs a) {
   for (int i = lane; i < n; i += 32) {
     double d = r64p[i].y >= 0 ? r64[i] : rc[i];
     if (is_squared(MEAS)) d = __dsqrt_rn(d);
-    S.v[i] = d;
+    S.v[i] = ordered(d);
     S.c[i] = rp[i].y;
   }
   __syncwarp();

@@ -602,3 +602,32 @@ def test_lcss_without_a_finite_extent(tsim, cuda_ctx, oracle, eps, delta):
         assert np.array_equal(d, want), flags
         assert np.array_equal(ids, want_ids), flags
     db.close()
+
+
+@pytest.mark.parametrize("measure,kw", [("dtw", dict(band_pct=10)), ("dtw", dict(cost=1)),
+                                        ("frechet", {}), ("hausdorff", {}), ("euclidean", {})])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_candidates_without_a_finite_distance(tsim, cuda_ctx, oracle, measure, kw, bad):
+    """Fewer candidates at a finite distance than neighbours asked for, the
+    others with a point at infinity or a NaN, and queries of which one has no
+    finite distance at all: the oracle's answer among the finite ones, then
+    distinct candidates at infinity."""
+    if measure == "frechet" and np.isnan(bad):
+        pytest.skip("a maximum passes over a NaN cost: such a pair's distance is finite")
+    cp, co = G.random_walks(300, 40, 15, start_range=10.0)
+    qp, qo = G.random_walks(9, 40, 16, start_range=10.0)
+    good = np.array([5, 100, 101, 200, 255, 299])
+    rng = np.random.default_rng(17)
+    for c in np.setdiff1d(np.arange(300), good):
+        cp[co[c] + rng.choice([0, 20, 39]), 1] = bad
+    qp[qo[8] + 20, 0] = bad
+    gp = np.concatenate([cp[co[c]:co[c + 1]] for c in good])
+    want_ids, want = oracle.knn(measure, qp[:qo[8]], qo[:9], gp, np.arange(7) * 40, 6, **kw)
+    db = tsim.Database(cuda_ctx, cp, co)
+    for flags in (0, tsim.api.FLAG_ALWAYS_PRUNE, tsim.api.FLAG_FP64_RESCORE):
+        ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, measure, 10, flags=flags, **kw)
+        assert np.array_equal(ids[:8, :6], good[want_ids]), flags
+        assert np.all(np.abs(d[:8, :6] - want) <= 1e-5 * want), flags
+        assert np.all(np.isposinf(d[:8, 6:])) and np.all(np.isposinf(d[8])), flags
+        assert all(len(set(row)) == 10 and min(row) >= 0 for row in ids.tolist()), flags
+    db.close()
