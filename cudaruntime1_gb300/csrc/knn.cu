@@ -1778,7 +1778,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
         acc = __fadd_rd(acc, a.cost ? __fsqrt_rd(d) : d);
       }
       for (int o = 16; o; o >>= 1) acc = __fadd_rd(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-      pass = acc <= t;
+      pass = !(acc > t);  // a corner that is no number bounds nothing
     }
     if (pass) out.add(lane == 0, c, 0);
   }

@@ -631,3 +631,20 @@ def test_candidates_without_a_finite_distance(tsim, cuda_ctx, oracle, measure, k
         assert np.all(np.isposinf(d[:8, 6:])) and np.all(np.isposinf(d[8])), flags
         assert all(len(set(row)) == 10 and min(row) >= 0 for row in ids.tolist()), flags
     db.close()
+
+
+@pytest.mark.parametrize("cost", [0, 1])
+def test_dtw_row_bounds_of_corners_that_are_no_number(tsim, cuda_ctx, cost):
+    """Banded DTW where most corner cells are NaN and no threshold exists: the
+    row side of LB_Keogh keeps what the column side keeps, the candidates of a
+    request that refines every pair."""
+    cp, co = G.random_walks(300, 40, 19, start_range=10.0)
+    qp, qo = G.random_walks(3, 40, 20, start_range=10.0)
+    cp[co[:-1][np.arange(300) % 60 != 7]] = np.nan
+    db = tsim.Database(cuda_ctx, cp, co)
+    ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, band_pct=10, cost=cost,
+                         flags=tsim.api.FLAG_ALWAYS_PRUNE)
+    ids2, d2, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, band_pct=10, cost=cost,
+                           flags=tsim.api.FLAG_NO_PRUNE)
+    assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
+    db.close()
