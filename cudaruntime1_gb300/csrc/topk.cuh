@@ -10,10 +10,9 @@
 
 namespace tsim {
 
-// (a NaN, whose bits have no place in f2ord's order, comes after +inf)
+// (a NaN, whose bits have no place in f2ord's order, counts as +inf)
 __device__ __forceinline__ unsigned long long pack_key(float key, int idx) {
-  const unsigned o = key <= TSIM_INF ? f2ord(key) : 0xffffffffu;
-  return ((unsigned long long)o << 32) | (unsigned)idx;
+  return ((unsigned long long)f2ord(key <= TSIM_INF ? key : TSIM_INF) << 32) | (unsigned)idx;
 }
 
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
