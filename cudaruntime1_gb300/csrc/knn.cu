@@ -1464,8 +1464,8 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 5) lb2_dtw_kernel(KArgs a) {
 // 64 at a time, the grid is looked up where some lane's point passes its box,
 // and 32 registers leave 64 warps an SM (at 40, 1,197 us; forms that loaded ahead in registers
 // ran 1,606 and 1,790 us, with 1,135 and 848 M instructions).  A CTA takes tiles
-// of kLcssTile pairs, so that a query with few pairs builds few grids: with
-// every query's pairs dealt over 19 CTAs the longest lists set the end.  2.17 M
+// of up to kLcssTile pairs, so that a query with few pairs builds few grids:
+// with every query's pairs dealt over 19 CTAs the longest lists set the end.  2.17 M
 // pairs of 256 queries: 1,893 -> 1,053 us, 560 M instructions.
 //
 // It reads every point where the other measures' bound before round 1 reads
@@ -1474,13 +1474,13 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 5) lb2_dtw_kernel(KArgs a) {
 // second on those best by its own: 0.6 M of the 2.17 M pairs left to bound, 339
 // us, for as many pairs in the DP (311 k; 457 k with one pass, before it, and
 // 284 k with one after).  256 queries against 65,536 candidates 1,590 -> 1,390 us.
-constexpr int kLcssTile = 512;
-__global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
+constexpr int kLcssTile = 512;  // at most
+__global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a, int tile_len) {
   __shared__ uint32_t grid[kGridWords];
   __shared__ int buf[kLb2Warps][64][2];
   const int q = blockIdx.y;
   const int cnt = a.fcnt[q];
-  if ((long long)blockIdx.x * kLcssTile >= cnt) return;  // uniform across the CTA
+  if ((long long)blockIdx.x * tile_len >= cnt) return;  // uniform across the CTA
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
@@ -1524,9 +1524,9 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a) {
   WarpList<2> out{a.cnt0 + q, a.list2 + (size_t)q * a.C,
                reinterpret_cast<int*>(a.lb2v) + (size_t)q * a.C, nullptr, buf[warp]};
   const float gxm = (float)(gnx - 1), gym = (float)(gny - 1);
-  for (long long tile = (long long)blockIdx.x * kLcssTile; tile < cnt;
-       tile += (long long)gridDim.x * kLcssTile) {
-    const int end = (int)min((long long)cnt, tile + kLcssTile);
+  for (long long tile = (long long)blockIdx.x * tile_len; tile < cnt;
+       tile += (long long)gridDim.x * tile_len) {
+    const int end = (int)min((long long)cnt, tile + tile_len);
     int c_nx = (int)tile + warp < end ? L1[(int)tile + warp] : 0;
     for (int e = (int)tile + warp; e < end; e += kLb2Warps) {
       const int c = c_nx;
@@ -2566,8 +2566,14 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     a.fcnt = a.cnt0;
   }
   if constexpr (MEAS == M_LCSS) {
-    const int tiles = (a.C + kLcssTile - 1) / kLcssTile;
-    lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(a);
+    // fewer pairs a tile for few queries, whose lists are all the work there
+    // is: 2,813 pairs of one query were six CTAs (16,384 candidates, epsilon 0.25,
+    // windows of 11 and 41 rows: 189 and 213 us a call, now 129 and 147; 16
+    // queries 296 and 318, now 231 and 246)
+    const int tile_len = std::max(32, std::min(kLcssTile, kLcssTile / 64 * nq));
+    const int tiles = (a.C + tile_len - 1) / tile_len;
+    lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(
+        a, tile_len);
     seg_select_kernel<MEAS, 2><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
     r1_select_kernel<MEAS, 1><<<nq, kSelThreads, 0, s>>>(a);
     launched(ctx, 3);
