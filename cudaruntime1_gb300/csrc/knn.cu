@@ -1785,29 +1785,41 @@ __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
   out.flush();
 }
 
-// exclusive scan of fcnt -> off2, total -> npairs (one CTA)
-__global__ void __launch_bounds__(1024) scan_kernel(KArgs a) {
-  __shared__ int part[1024];
+// exclusive scan of fcnt -> off2, total -> npairs[0] (one CTA).  LCSS: the
+// pairs of queries whose threshold is at least `dense` of their length come
+// last, when there are at least `gate` of them: npairs[1] pairs, then npairs[2].
+__global__ void __launch_bounds__(1024) scan_kernel(KArgs a, float dense, int gate) {
+  __shared__ unsigned long long part[1024];  // dense queries' pairs << 32 | the others'
   const int per = (a.nq + 1023) / 1024;
   const int b = threadIdx.x * per, e = min(a.nq, b + per);
-  int s = 0;
-  for (int i = b; i < e; ++i) s += a.fcnt[i];
+  auto pairs = [&](int i) {
+    const bool d = dense > 0.0f && a.thr2[i] >= dense * (float)a.qlen[i];
+    return (unsigned long long)a.fcnt[i] << (d ? 32 : 0);
+  };
+  unsigned long long s = 0;
+  for (int i = b; i < e; ++i) s += pairs(i);
   part[threadIdx.x] = s;
   __syncthreads();
   for (int o = 1; o < 1024; o <<= 1) {
-    int v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
+    const unsigned long long v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
     __syncthreads();
     part[threadIdx.x] += v;
     __syncthreads();
   }
-  int run = part[threadIdx.x] - s;
+  const int nd = (int)(part[1023] >> 32), ns = (int)part[1023];
+  const bool last = nd > 0 && nd >= gate;
+  unsigned long long run = part[threadIdx.x] - s;
   for (int i = b; i < e; ++i) {
-    a.off2[i] = run;
-    run += a.fcnt[i];
+    const unsigned long long p = pairs(i);
+    const int before_d = (int)(run >> 32), before_s = (int)run;
+    a.off2[i] = !last ? before_d + before_s : p >> 32 ? ns + before_d : before_s;
+    run += p;
   }
   if (threadIdx.x == 1023) {
-    a.off2[a.nq] = part[1023];
-    *a.npairs = part[1023];
+    a.off2[a.nq] = ns + nd;
+    a.npairs[0] = ns + nd;
+    a.npairs[1] = last ? ns : ns + nd;
+    a.npairs[2] = last ? nd : 0;
   }
 }
 
@@ -1826,14 +1838,19 @@ __device__ __forceinline__ int shape_key(int n, int m) {
          min(max(n, m) >> 4, (1 << kShapeBits) - 1);
 }
 
-// the queries' survivor lists side by side, and (sorted) their shape counts
+// the queries' survivor lists side by side, and (sorted) their shape counts;
+// else the list of those that scan_kernel put last
 __global__ void flatten_kernel(KArgs a, int sorted) {
   const int q = blockIdx.y;
   const int cnt = a.fcnt[q], base = a.off2[q], n = a.qlen[q];
+  const int first = sorted ? 0 : a.npairs[1];
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
     const int c = a.list1[(size_t)q * a.C + e];
     a.flat[base + e] = make_int2(q, c);
-    if (sorted) atomicAdd(a.shape_cnt + (kNumShapes - 1 - shape_key(n, a.clen[c])), 1);
+    if (sorted)
+      atomicAdd(a.shape_cnt + (kNumShapes - 1 - shape_key(n, a.clen[c])), 1);
+    else if (base >= first)
+      a.order[base - first + e] = base + e;
   }
 }
 
@@ -2204,7 +2221,8 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
     return launch_dp(ctx, kind, G, R, rest, a.max_clen);
   }
   // bit vectors, in every round: a round's time follows the columns that can
-  // match, not the window's cells, so there is no gate on its size
+  // match, not the window's cells, so there is no gate on its size (the
+  // survivor round leaves out the pairs that match densely, where many)
   if (a.wave && lcss_window_kind(kind, d.delta)) return launch_lcss_window(ctx, d);
   if (!latency && a.lane_gate > 0 && d.npairs >= a.lane_gate && lane_kind(kind)) {
     // many pairs: a lane per pair, with a latency of one pair's cells but a
@@ -2584,11 +2602,16 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     launched(ctx);
     a.fcnt = a.cnt1;
   }
-  scan_kernel<<<1, 1024, 0, s>>>(a);
+  // LCSS pairs that match densely run a lane each where they are many
+  // (lcss_dense_from); the lanes' kernel costs a request without any an empty
+  // launch, so small requests, which cannot fill it, go without
+  const bool lcss_bits = MEAS == M_LCSS && a.wave && lcss_window_kind(dp32, a.delta);
+  const bool lanes_too = lcss_bits && a.lane_gate > 0 && (size_t)nq * a.C >= (size_t)a.lane_gate;
+  scan_kernel<<<1, 1024, 0, s>>>(a, lanes_too ? lcss_dense_from(a.delta) : 0.0f, a.lane_gate);
   // the shape order serves the kernels whose warps run as long as their
   // longest pair; the LCSS bit vectors gain more from one query's pairs side
   // by side
-  const bool sorted = !(MEAS == M_LCSS && a.wave && lcss_window_kind(dp32, a.delta));
+  const bool sorted = !lcss_bits;
   flatten_kernel<<<dim3(ch, nq), 256, 0, s>>>(a, sorted);
   launched(ctx, 3);
   if (sorted) {
@@ -2621,6 +2644,20 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
       TSIM_TRY(refine32<MEAS>(ctx, a, dp32, Gs, Rs, one));
     }
   } else {
+    if (lanes_too) {
+      int* nl = a.nlanes;
+      DpArgs l = d;
+      l.order = a.order;
+      l.npairs_dev = a.npairs + 2;
+      TSIM_TRY(launch_dp_lane(ctx, dp32, l, lane_ring_for(dp32, INT32_MAX, INT32_MAX, -1, a.delta),
+                              a.lanes, &nl));
+      if (a.min_qlen < 2 || a.min_clen < 2) {  // pairs with a side of one point
+        l.order = a.lanes;
+        l.npairs_dev = nl;
+        TSIM_TRY(launch_lcss_window(ctx, l));
+      }
+      d.npairs_dev = a.npairs + 1;
+    }
     TSIM_TRY(refine32<MEAS>(ctx, a, dp32, G, R, d));
   }
   stage_end(ctx);

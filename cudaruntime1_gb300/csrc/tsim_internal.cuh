@@ -398,6 +398,8 @@ int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max
 // j - delta .. j + delta).  Takes pairs of any length.
 bool lcss_window_kind(int kind, int delta);
 int launch_lcss_window(tsim_ctx* ctx, const DpArgs& a);
+// the part of a pair's columns that match from which a lane per pair is faster
+float lcss_dense_from(int delta);
 // Exact FP64 Frechet values (squared) of the pairs whose window (PolFrechetWin,
 // FP32 values in aux) holds one cost, into out64; the others' entries in rest[]
 // (count in *nrest) for DP_FRECHET_WIN.
