@@ -653,25 +653,28 @@ def test_dtw_row_bounds_of_corners_that_are_no_number(tsim, cuda_ctx, cost):
 
 @pytest.mark.parametrize("nq", [1, 4, 5, 40])
 @pytest.mark.parametrize("delta", [-1, 3, 20, 31])
-def test_lcss_dense_and_sparse_queries(tsim, cuda_ctx, oracle, nq, delta):
+def test_lcss_dense_and_sparse_queries(tsim, oracle, nq, delta):
     """LCSS of one query, a few and many, alternately matching nearly every
     point and few: lists shorter and longer than a block's tile, and enough
-    densely matching pairs for a lane each, one-point sides among them: the
-    oracle's counts, with and without the lanes."""
-    cl = G.uniform_lengths(2500, 20, 60, 21)
+    densely matching pairs for a lane each (74,000 of 40 queries, one stream),
+    one-point sides among them: the oracle's counts, with and without the lanes."""
+    ctx = tsim.Context(0)
+    ctx.set_concurrency(1)
+    cl = G.uniform_lengths(6000, 20, 60, 21)
     cl[:40] = 1
-    cp, co = G.random_walks(2500, cl, 22, start_range=10.0)
+    cp, co = G.random_walks(6000, cl, 22, start_range=10.0)
     ql = np.resize([60, 50, 30, 55, 1, 45], nq)
     qp, qo = G.random_walks(nq, ql, 23, start_range=10.0)
     for q in range(1, nq, 2):  # every other query far away but for its ends
         qp[qo[q] + 3:max(qo[q] + 3, qo[q + 1] - 3)] += 1e4
-    db = tsim.Database(cuda_ctx, cp, co)
+    db = tsim.Database(ctx, cp, co)
     for eps in (0.5, 20.0):
         want_ids, want = oracle.knn("lcss", qp, qo, cp, co, 5, eps=eps, delta=delta)
         for flags in (0, tsim.api.FLAG_ALWAYS_PRUNE,
                       tsim.api.FLAG_ALWAYS_PRUNE | tsim.api.FLAG_NO_LANE_DP):
-            ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "lcss", 5, epsilon=eps, delta=delta,
+            ids, d, _ = tsim.knn(ctx, db, qp, qo, "lcss", 5, epsilon=eps, delta=delta,
                                  flags=flags)
             assert np.array_equal(d, want), (eps, flags)
             assert np.array_equal(ids, want_ids), (eps, flags)
     db.close()
+    ctx.close()
