@@ -2592,15 +2592,21 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     const int tiles = (a.C + tile_len - 1) / tile_len;
     lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(
         a, tile_len);
-    seg_select_kernel<MEAS, 2><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
-    r1_select_kernel<MEAS, 1><<<nq, kSelThreads, 0, s>>>(a);
-    launched(ctx, 3);
-    stage_end(ctx);
-    TSIM_TRY(round1(1, a.thr2));
-    stage_begin(ctx, TSIM_STAGE_FILTER);
-    refilter_kernel<MEAS, 1><<<dim3(ch, nq), 256, 0, s>>>(a);
     launched(ctx);
-    a.fcnt = a.cnt1;
+    if (a.Mr == a.M) {  // round 1 was one pass
+      a.list1 = a.list2;
+      a.fcnt = a.cnt0;
+    } else {
+      seg_select_kernel<MEAS, 2><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
+      r1_select_kernel<MEAS, 1><<<nq, kSelThreads, 0, s>>>(a);
+      launched(ctx, 2);
+      stage_end(ctx);
+      TSIM_TRY(round1(1, a.thr2));
+      stage_begin(ctx, TSIM_STAGE_FILTER);
+      refilter_kernel<MEAS, 1><<<dim3(ch, nq), 256, 0, s>>>(a);
+      launched(ctx);
+      a.fcnt = a.cnt1;
+    }
   }
   // LCSS pairs that match densely run a lane each where they are many
   // (lcss_dense_from); the lanes' kernel costs a request without any an empty
@@ -2736,7 +2742,11 @@ size_t knn_plan(const tsim_params* p, int nq, int max_qlen, const tsim_db* db, K
   a.k = k;
   a.S = std::min(C, std::min(64, std::max(2 * k, 16)));
   a.M = std::min(64, std::max(2 * k, 32));
-  a.Mr = p->measure == TSIM_LCSS ? a.M / 2 : a.M;
+  // LCSS: two passes, but for a few queries against up to 2 M candidates in
+  // all, whose O(length) bound costs less than a pass: one query against 16,384
+  // trajectories 129 -> 115 us, 147 -> 119 with 41 rows, against 262,144 182 ->
+  // 150; four densely matching queries 459 -> 429, but sixteen 552 -> 647
+  a.Mr = p->measure == TSIM_LCSS && (nq > 4 || (int64_t)nq * C > 2000000) ? a.M / 2 : a.M;
   a.r1n = 0;
   a.nch = (C + kChunk - 1) / kChunk;
   a.T = std::min(kChunk, std::max(1, (2 * a.S + a.nch - 1) / a.nch));
