@@ -2191,6 +2191,21 @@ __global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_res
   }
 }
 
+// Whether a compensated full-row pair of the longest lengths takes longer on a
+// warp's strips of 128 rows than on a CTA of row groups.  A strip's step (four
+// rows) is about 0.21 us on a lone warp, a CTA's 0.125 a row of each lane; ten
+// pairs of 130 / 260 / 500 / 1,000 / 2,040 points a side take 50 / 143 / 462 / 1,714
+// / 6,781 us on strips and 49 / 107 / 192 / 634 / 2,331 on CTAs, but 64 x 1,000 points
+// 195 and 361: a lane's rows are the query's.  (FP32 strips hold eight rows a
+// lane and cost less a step.)
+bool strip_slower(const KArgs& a, int kind, int n) {
+  if ((kind != DP_DTW_SQC && kind != DP_DTW_EUC) || a.rdiag_cta <= 0) return false;
+  const double m = a.max_clen, r = a.rdiag_cta;
+  const double strips = 0.21 * std::min(std::ceil(n / 128.0) * (m + 31), std::ceil(m / 128) * (n + 31));
+  const double cta = 0.125 * r * std::ceil(n / (256 * r)) * (m + std::min(256.0, std::ceil(n / r)));
+  return cta + 20.0 < strips;
+}
+
 // DP of a pair list: the strip kernel for full rows, the anti-diagonal
 // kernels for the banded pairs they can take, the round-striped kernel (G
 // lanes x R rows) for the rest
@@ -2211,8 +2226,20 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
     // 5,120 Frechet pairs of up to 256 x 1,024 points 1,438 us on a CTA of
     // row groups and 2,317 on a warp (eight passes, R = 1 .. 8) -> 208 us;
     // the same compensated 4,406 -> 1,004 us
-    int* nw = a.nwaves;
     const int mq = d.max_n > 0 ? d.max_n : a.max_qlen;
+    if (latency && d.npairs <= ctx->num_sms && strip_slower(a, kind, mq)) {
+      // a compensated round of at most a pair an SM: eight warps a pair
+      int* ns = a.nspill;
+      bool all = false;
+      TSIM_TRY(launch_dp_diag(ctx, kind, a.rdiag_cta, d, a.max_clen, a.spill, &ns, a.spill2,
+                              a.nspill2, 8, 0, &all));
+      if (all && a.min_qlen >= 2 && a.min_clen >= 2) return TSIM_OK;
+      DpArgs rest = d;
+      rest.order = a.spill;
+      rest.npairs_dev = ns;
+      return launch_dp(ctx, kind, G, R, rest, a.max_clen);
+    }
+    int* nw = a.nwaves;
     TSIM_TRY(launch_dp_strip(ctx, kind, d, mq, a.max_clen, a.waves, &nw));
     if (a.min_qlen > 0 && std::min(mq, a.max_clen) <= strip_max_cols()) return TSIM_OK;
     DpArgs rest = d;  // pairs with both sides too long to stage

@@ -536,9 +536,10 @@ def test_dtw_on_a_database_beyond_l2(tsim, cuda_ctx, kw):
     db.close()
 
 
+@pytest.mark.parametrize("band", [10, -1])
 @pytest.mark.parametrize("cost", [0, 1])
-def test_distances_alone_and_in_a_batch(tsim, cuda_ctx, cost):
-    """Banded DTW's distances do not depend on how many queries share the
+def test_distances_alone_and_in_a_batch(tsim, cuda_ctx, cost, band):
+    """DTW's distances do not depend on how many queries share the
     call, nor on the kernels chosen: the bits of each query alone, of a few
     together, and of all of them with the row-group kernels."""
     rng = np.random.default_rng(97)
@@ -549,7 +550,7 @@ def test_distances_alone_and_in_a_batch(tsim, cuda_ctx, cost):
         scale = 2.0 ** rng.uniform(-16, 3, (len(src), 1))
         cp[co[c]:co[c + 1]] = qp[src] + scale * rng.standard_normal((len(src), 2))
     db = tsim.Database(cuda_ctx, cp, co)
-    kw = dict(band_pct=10, cost=cost)
+    kw = dict(band_pct=band, cost=cost)
     for flags in (0, tsim.api.FLAG_ALWAYS_PRUNE):
         want = _device_knn(tsim, cuda_ctx, db, qp, qo, "dtw", 10, flags=flags, **kw)
         off = _device_knn(tsim, cuda_ctx, db, qp, qo, "dtw", 10,
