@@ -3388,6 +3388,12 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
   int* nrest = arena_take<int>(ctx, 4);
   int* sorted = arena_take<int>(ctx, npairs);
   int* buckets = arena_take<int>(ctx, lane_sort_buckets());
+  // Past 1,710 points a side the compensated strips' rows leave one CTA of four
+  // pairs an SM: more pairs than that take turns, 1,216 pairs of 2,040 points
+  // 14.0 ms and 4,096 48.8, round-striped 9.1 and 27.6 (608: 7.1 and 8.0)
+  if (kernel == 0 && precision == 1 && d.band_pct < 0 && std::min(max_qlen, max_clen) > 1710 &&
+      npairs > 4 * ctx->num_sms)
+    return launch_dp(ctx, kind, 32, 8, d, max_clen);
   if (kernel == 0 && d.band_pct < 0 && strip_kind(kind)) {  // full rows
     TSIM_TRY(launch_dp_strip(ctx, kind, d, max_qlen, max_clen, spill, &nspill));
     d.order = spill;

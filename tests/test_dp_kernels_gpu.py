@@ -304,3 +304,30 @@ def test_full_rows_of_queries_longer_than_stated(tsim, cuda_ctx, oracle, measure
         assert np.array_equal(ids.cpu().numpy().reshape(8, 10), want_ids)
         assert np.array_equal(d64.cpu().numpy().reshape(8, 10), want)
     db.close()
+
+
+@pytest.mark.parametrize("measure", ["dtw", "frechet"])
+@pytest.mark.parametrize("longest", [1710, 1712])
+def test_compensated_full_rows_past_one_cta_an_sm(tsim, cuda_ctx, measure, longest):
+    """Compensated full rows of more pairs than one block an SM holds, on both
+    sides of the length from which they are round-striped: the same bits, for
+    pairs of every length, as from fewer pairs."""
+    import torch
+    from cudaruntime1_gb300 import api
+    qp, qo = G.random_walks(2, [longest, 33], 99, start_range=10.0)
+    cp, co = G.random_walks(12, [longest, 1, 2, 31, 32, 33, 64, 100, 255, 256, 257, 300], 100,
+                            start_range=10.0)
+    pairs = np.stack(np.meshgrid(np.arange(2), np.arange(12), indexing="ij"), -1).reshape(-1, 2)
+    pairs = np.concatenate([pairs] + [pairs[13:]] * 60).astype(np.int32)  # short ones again and again
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+           (qp, np.asarray(qo), cp, np.asarray(co), pairs)]
+    out = []
+    for count in (len(pairs), 24):
+        o = torch.full((len(pairs),), float("nan"), dtype=torch.float64, device="cuda")
+        api.dp_pairs(cuda_ctx, measure, 1, 0, dev[0].data_ptr(), dev[1].data_ptr(), longest,
+                     dev[2].data_ptr(), dev[3].data_ptr(), longest, dev[4].data_ptr(), count, 0,
+                     o.data_ptr())
+        torch.cuda.synchronize()
+        out.append(o.cpu().numpy())
+    assert len(pairs) > 608 and np.array_equal(out[0][:24], out[1][:24])
+    assert np.array_equal(out[0][24:], np.tile(out[1][13:24], 60))
