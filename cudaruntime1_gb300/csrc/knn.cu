@@ -108,7 +108,7 @@ struct KArgs {
   int nctr;
   // parameters
   int k, S, T, nch;
-  int Mr;   // round 1's pairs per query and pass: M, or (LCSS, two passes) half of it
+  int M0;   // round 1's pairs per query of its first pass: M, or (LCSS, knn_plan) half or none
   int r1n;  // those refined so far
   // DTW: whether the O(length) bound follows round 1, whose pairs then go by
   // the segment bound, and the row side.  On a database beyond L2, whose points
@@ -328,10 +328,11 @@ __device__ __forceinline__ bool is_late(const KArgs& a) {
   return MEAS == M_DTW ? a.late != 0 : late_bound(MEAS);
 }
 
-// entry i of query q among round 1's pairs: the passes' lists one after the other
+// entry i of query q among round 1's pairs: the passes' lists (M0 pairs a query,
+// then M - M0) one after the other
 __device__ __forceinline__ size_t r1_at(const KArgs& a, int q, int i) {
-  const int pass = i >= a.Mr ? 1 : 0;
-  return ((size_t)pass * a.nq + q) * a.Mr + i - pass * a.Mr;
+  return i < a.M0 ? (size_t)q * a.M0 + i
+                  : (size_t)a.nq * a.M0 + (size_t)q * (a.M - a.M0) + i - a.M0;
 }
 
 template <int MEAS>
@@ -1581,7 +1582,7 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a, in
 // Round 1: the M best survivors of each query by their O(length) bound
 // (most likely to hold the true neighbours) are refined first; their values
 // tighten the threshold for the rest.  Taken entries are consumed (-1).  LCSS
-// takes them in two passes, half by segment bound and half by O(length) bound.
+// takes them in up to two passes, by segment bound and by O(length) bound (knn_plan).
 template <int MEAS, int PASS>
 __global__ void __launch_bounds__(kSelThreads) r1_select_kernel(KArgs a) {
   __shared__ SelScratch red;
@@ -1593,15 +1594,16 @@ __global__ void __launch_bounds__(kSelThreads) r1_select_kernel(KArgs a) {
     a.cnt0[q] = 0;  // and what the row side keeps of it (lb_rows_kernel)
   }
   // the segments' M best (seg_select_kernel) hold the query's M best
-  block_select_k(a.segkeys + (size_t)q * a.nseg * 64, ns * a.Mr, a.Mr, sel, red);
-  for (int i = threadIdx.x; i < a.Mr; i += kSelThreads) {
+  const int K = PASS ? a.M - a.M0 : a.M0;
+  block_select_k(a.segkeys + (size_t)q * a.nseg * 64, ns * K, K, sel, red);
+  for (int i = threadIdx.x; i < K; i += kSelThreads) {
     const int pos = key_index(sel[i]);
     int c = -1;
     if (pos >= 0) {
       c = a.list2[(size_t)q * a.C + pos];
       a.list2[(size_t)q * a.C + pos] = -1;
     }
-    a.r1pairs[r1_at(a, q, PASS * a.Mr + i)] = make_int2(q, c);
+    a.r1pairs[r1_at(a, q, PASS * a.M0 + i)] = make_int2(q, c);
   }
 }
 
@@ -2171,7 +2173,7 @@ __global__ void stats_kernel(KArgs a, unsigned long long* counters, int with_res
   const bool late = (meas == M_DTW ? a.late != 0 : late_bound(meas)) && !a.brute;
   for (int q = threadIdx.x; q < a.nq; q += blockDim.x) {
     c1 += meas == M_EUCLID || late ? a.cnt2[q] : a.cnt1[q];  // one list of bounded pairs
-    c2 += late && meas != M_HAUSDORFF ? a.cnt0[q] + min(a.cnt2[q], a.Mr) : a.cnt2[q];
+    c2 += late && meas != M_HAUSDORFF ? a.cnt0[q] + min(a.cnt2[q], a.M0) : a.cnt2[q];
     rc += with_rescore ? min(a.rraw[q], a.RC) : 0;
   }
   for (int o = 16; o; o >>= 1) {
@@ -2552,24 +2554,28 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     launched(ctx);
     if (MEAS == M_DTW && !a.late) TSIM_TRY(column_side());
   }
-  seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
+  if (a.M0 > 0) {
+    seg_select_kernel<MEAS, 0><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.M0);
+    launched(ctx);
+  }
   r1_select_kernel<MEAS, 0><<<nq, kSelThreads, 0, s>>>(a);
   TSIM_CUDA(cudaGetLastError());
-  launched(ctx, 2);
+  launched(ctx);
   stage_end(ctx);
 
   // round 1: the best survivors by bound, abandon against the threshold so far
   auto round1 = [&](int pass, const float* thr) -> int {
     stage_begin(ctx, TSIM_STAGE_DP);
+    const int per = pass ? a.M - a.M0 : a.M0;
     DpArgs r1 = d;
-    r1.pairs = a.r1pairs + (size_t)pass * nq * a.Mr;
-    r1.npairs = nq * a.Mr;
-    r1.out = a.r1vals + (size_t)pass * nq * a.Mr;
+    r1.pairs = a.r1pairs + (size_t)pass * nq * a.M0;
+    r1.npairs = nq * per;
+    r1.out = a.r1vals + (size_t)pass * nq * a.M0;
     r1.thr = thr;
     // the best pairs by bound rarely abandon: no remaining-columns bound
     if (MEAS == M_DTW) r1.qtab = nullptr;
     if (a.plain) {
-      for (int i = 0; i < nq * a.Mr; ++i) {
+      for (int i = 0; i < nq * per; ++i) {
         DpArgs one = r1;
         one.pairs = r1.pairs + i;
         one.npairs = 1;
@@ -2579,11 +2585,11 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     } else {
       TSIM_TRY(refine32<MEAS>(ctx, a, dp32, Gs, Rs, r1, true));
     }
-    a.r1n += a.Mr;
+    a.r1n += per;
     stage_end(ctx);
     return TSIM_OK;
   };
-  TSIM_TRY(round1(0, a.thr));
+  if (a.M0 > 0) TSIM_TRY(round1(0, a.thr));
 
   stage_begin(ctx, TSIM_STAGE_FILTER);
   // (LCSS: some million pairs whose loads wait on one another: 82 -> 52 us)
@@ -2620,11 +2626,11 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(
         a, tile_len);
     launched(ctx);
-    if (a.Mr == a.M) {  // round 1 was one pass
+    if (a.M0 == a.M) {  // round 1 was one pass
       a.list1 = a.list2;
       a.fcnt = a.cnt0;
     } else {
-      seg_select_kernel<MEAS, 2><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.Mr);
+      seg_select_kernel<MEAS, 2><<<dim3(a.nseg, nq), kSelThreads, 0, s>>>(a, a.M - a.M0);
       r1_select_kernel<MEAS, 1><<<nq, kSelThreads, 0, s>>>(a);
       launched(ctx, 2);
       stage_end(ctx);
@@ -2769,11 +2775,23 @@ size_t knn_plan(const tsim_params* p, int nq, int max_qlen, const tsim_db* db, K
   a.k = k;
   a.S = std::min(C, std::min(64, std::max(2 * k, 16)));
   a.M = std::min(64, std::max(2 * k, 32));
-  // LCSS: two passes, but for a few queries against up to 2 M candidates in
-  // all, whose O(length) bound costs less than a pass: one query against 16,384
-  // trajectories 129 -> 115 us, 147 -> 119 with 41 rows, against 262,144 182 ->
-  // 150; four densely matching queries 459 -> 429, but sixteen 552 -> 647
-  a.Mr = p->measure == TSIM_LCSS && (nq > 4 || (int64_t)nq * C > 2000000) ? a.M / 2 : a.M;
+  a.M0 = a.M;
+  if (p->measure == TSIM_LCSS) {
+    // Where round 1 comes.  Without the bit vectors (no window, or one of more
+    // than 63 rows) the DP costs most and goes by the O(length) bound alone: 60
+    // queries against 10,000 trajectories, 81 rows, 478 us (532 in two passes, 753
+    // in one before that bound), 6 against 200,000 without a window 444 (724,
+    // 1,564).  With them that bound costs more than a round, which goes by the
+    // segment bound ahead of it where pairs are few (one query against 16,384
+    // 129 us in two passes, 115 in one; six against 60,000 135 and 117) and is
+    // divided where they are many: the batched workload's 17 M, and 64 densely
+    // matching queries against 16,384 1,023 us (1,583 in one pass).
+    const int64_t pairs = (int64_t)nq * C;
+    if (!lcss_window_kind(DP_LCSS, p->delta))
+      a.M0 = 0;
+    else if (pairs > (nq > 4 ? 100000 : 2000000))
+      a.M0 = a.M / 2;
+  }
   a.r1n = 0;
   a.nch = (C + kChunk - 1) / kChunk;
   a.T = std::min(kChunk, std::max(1, (2 * a.S + a.nch - 1) / a.nch));
