@@ -98,9 +98,9 @@ __global__ void __launch_bounds__(kLcssThreads) lcss_window_kernel(DpArgs a) {
       }
       const int r0 = j - delta;
       const bool inner = lane >= k || (r0 >= 0 && r0 + 8 * chunks <= n);
-      auto bits = [&](auto row) {
-        if (lane >= k) return;
-        for (int ch = 0; ch < chunks; ++ch) {
+      // rows ch0 .. of 8, to ch1
+      auto bits = [&](int ch0, int ch1, auto row) {
+        for (int ch = ch0; ch < ch1; ++ch) {
           unsigned w = 0;
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
@@ -112,11 +112,13 @@ __global__ void __launch_bounds__(kLcssThreads) lcss_window_kernel(DpArgs a) {
         M &= wmask;  // rows past the window (its chunks of 8)
       };
       if (__all_sync(0xffffffffu, inner)) {
-        bits([&](int r) { return __ldg(A + r); });
-      } else {  // some window reaches over an end of the query
-        bits([&](int r) { return __ldg(A + min(max(r, 0), n - 1)); });
+        if (lane < k) bits(0, chunks, [&](int r) { return __ldg(A + r); });
+      } else {  // some window reaches over an end of the query: the rows that exist
+        const int e0 = max(0, -r0), e1 = min(2 * delta, n - 1 - r0);
+        if (lane < k)
+          bits(e0 >> 3, (e1 >> 3) + 1, [&](int r) { return __ldg(A + min(max(r, 0), n - 1)); });
         // rows -r0 .. n-1-r0 of the window exist (a column with none: mc)
-        M &= (~0ull << max(0, -r0)) & ((2ull << min(2 * delta, n - 1 - r0)) - 1);
+        M &= (~0ull << e0) & ((2ull << e1) - 1);
         if (lane >= k) M = 0;
       }
       unsigned todo = __ballot_sync(0xffffffffu, M != 0);
