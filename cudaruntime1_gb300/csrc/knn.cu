@@ -2249,10 +2249,16 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
     rest.npairs_dev = nw;
     return launch_dp(ctx, kind, G, R, rest, a.max_clen);
   }
-  // bit vectors, in every round: a round's time follows the columns that can
-  // match, not the window's cells, so there is no gate on its size (the
-  // survivor round leaves out the pairs that match densely, where many)
-  if (a.wave && lcss_window_kind(kind, d.delta)) return launch_lcss_window(ctx, d);
+  // bit vectors, in every round of a pruned request: a round's time follows the
+  // columns that can match, not the window's cells, so there is no gate on its
+  // size (the survivor round leaves out the pairs that match densely, where
+  // many).  A brute-force round has no boxes that skip columns and short pairs:
+  // on lanes where many, 60,000 pairs of 16 / 32 / 64 points 50 / 71 / 99 us with
+  // windows of 17 rows, on bit vectors 86 / 85 / 103 with few matches and 114 /
+  // 153 / 253 with matches everywhere
+  if (a.wave && lcss_window_kind(kind, d.delta) &&
+      !(a.brute && a.lane_gate > 0 && d.npairs >= a.lane_gate))
+    return launch_lcss_window(ctx, d);
   if (!latency && a.lane_gate > 0 && d.npairs >= a.lane_gate && lane_kind(kind)) {
     // many pairs: a lane per pair, with a latency of one pair's cells but a
     // few instructions per cell; the kernel itself passes a round of fewer
