@@ -415,15 +415,15 @@ struct ChunkBest {
   }
 };
 
-// A thread per candidate, its summary in registers, looped over kLb1Queries
+// A thread per candidate, its summary in registers, looped over up to kLb1Queries
 // queries whose block boxes are in shared memory; 256 candidates a CTA, whose T
 // best are kept as seed candidates: one by a warp reduction per query, more by
 // a block selection.  Bound by issue, 185 to 205 instructions a pair: with a CTA
 // per query and chunk, loads, comparisons, selection and barriers came to 450 to
 // 510 (16.7 M pairs: Hausdorff 247 -> 95 us, Frechet 262 -> 108).
-constexpr int kLb1Queries = 8;
+constexpr int kLb1Queries = 8;  // at most
 template <int MEAS>
-__global__ void __launch_bounds__(kChunk) lb1_kernel(KArgs a) {
+__global__ void __launch_bounds__(kChunk) lb1_kernel(KArgs a, int per) {
   __shared__ unsigned long long keys[kChunk];
   __shared__ SelScratch red;
   __shared__ unsigned long long sel[64];
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kChunk) lb1_kernel(KArgs a) {
   __shared__ ChunkBest<kLb1Queries> best;
   const int chunk = blockIdx.x;
   const int c = chunk * kChunk + threadIdx.x;
-  const int q0 = blockIdx.y * kLb1Queries, q1 = min(a.nq, q0 + kLb1Queries);
+  const int q0 = blockIdx.y * per, q1 = min(a.nq, q0 + per);
   if (threadIdx.x < kLb1Queries * kQBlocks) {
     const int i = threadIdx.x / kQBlocks, b = threadIdx.x % kQBlocks;
     if (q0 + i < q1) {
@@ -719,15 +719,15 @@ __global__ void __launch_bounds__(256) qprefix_kernel(KArgs a) {
 // covered by L 2^-22 (max|c| + |p_0|); D = A - U within 2^-24 |D|, covered by
 // the factor 1 - 2^-22.  What is left of |D| is squared and summed rounding
 // down, and divided by the longest segment's length, rounding down.
-constexpr int kPaaQueries = 8;
-__global__ void __launch_bounds__(kChunk) paa_kernel(KArgs a) {
+constexpr int kPaaQueries = 8;  // at most
+__global__ void __launch_bounds__(kChunk) paa_kernel(KArgs a, int per) {
   __shared__ unsigned long long keys[kChunk];
   __shared__ SelScratch red;
   __shared__ unsigned long long sel[64];
   __shared__ ChunkBest<kPaaQueries> best;
   const int chunk = blockIdx.x;
   const int c = chunk * kChunk + threadIdx.x;
-  const int q0 = blockIdx.y * kPaaQueries, q1 = min(a.nq, q0 + kPaaQueries);
+  const int q0 = blockIdx.y * per, q1 = min(a.nq, q0 + per);
   const bool in = c < a.C;
   const int m = in ? a.clen[c] : 0;
   int b[kSegs + 1];    // segment boundaries
@@ -2471,6 +2471,18 @@ int run_brute(tsim_ctx* ctx, KArgs& a, int dp32, int dpc, int dp64) {
   return finish_knn<MEAS>(ctx, a, dpc, dp64);
 }
 
+// Queries a CTA of the O(1) bounds takes, one after the other (each with a block
+// selection where chunks are few): fewer than eight while that leaves less
+// than four CTAs an SM.  200 queries against 2,000 trajectories in eight chunks,
+// ten neighbours, in us: Hausdorff 14, 20 with two CTAs an SM (19 with a CTA per
+// query and chunk); 20 queries with 64 neighbours 64 with eight queries a CTA, now
+// 14.
+int bound_queries(int nq, int nch, int num_sms) {
+  static_assert(kLb1Queries == kPaaQueries, "one rule");
+  const int64_t per = (int64_t)nq * nch / (4 * (int64_t)num_sms);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(kLb1Queries, per));
+}
+
 template <int MEAS>
 int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, tsim_stats* st) {
   (void)st;
@@ -2478,12 +2490,13 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   cudaStream_t s = ctx->stream;
   const int nq = a.nq;
   stage_begin(ctx, TSIM_STAGE_LB1);
+  const int per = bound_queries(nq, a.nch, ctx->num_sms);
   if constexpr (MEAS == M_EUCLID) {
     qprefix_kernel<<<nq, 256, 0, s>>>(a);
-    paa_kernel<<<dim3(a.nch, (nq + kPaaQueries - 1) / kPaaQueries), kChunk, 0, s>>>(a);
+    paa_kernel<<<dim3(a.nch, (nq + per - 1) / per), kChunk, 0, s>>>(a, per);
     launched(ctx);
   } else {
-    lb1_kernel<MEAS><<<dim3(a.nch, (nq + kLb1Queries - 1) / kLb1Queries), kChunk, 0, s>>>(a);
+    lb1_kernel<MEAS><<<dim3(a.nch, (nq + per - 1) / per), kChunk, 0, s>>>(a, per);
   }
   stage_end(ctx);
   launched(ctx);

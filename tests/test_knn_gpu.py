@@ -679,3 +679,21 @@ def test_lcss_dense_and_sparse_queries(tsim, oracle, nq, delta):
             assert np.array_equal(ids, want_ids), (eps, flags)
     db.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("nq", [5, 20, 43])
+@pytest.mark.parametrize("measure,kw", [("dtw", dict(band_pct=20)), ("lcss", dict(epsilon=0.5, delta=3)),
+                                        ("frechet", {}), ("hausdorff", {}), ("euclidean", {})])
+def test_first_bound_queries_a_block(tsim, measure, kw, nq):
+    """Requests whose first bound takes one query a block, a few and eight, the
+    last block with fewer: the answer of a request that refines every pair."""
+    ctx = tsim.Context(0)
+    ctx.set_concurrency(1)
+    cp, co = G.random_walks(33000, G.uniform_lengths(33000, 8, 24, 31), 32, start_range=60.0)
+    qp, qo = G.random_walks(nq, 24, 33, start_range=60.0)
+    db = tsim.Database(ctx, cp, co)
+    ids, d, _ = tsim.knn(ctx, db, qp, qo, measure, 10, **kw)
+    ids2, d2, _ = tsim.knn(ctx, db, qp, qo, measure, 10, flags=tsim.api.FLAG_NO_PRUNE, **kw)
+    assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
+    db.close()
+    ctx.close()
