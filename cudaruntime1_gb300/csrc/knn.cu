@@ -2639,8 +2639,10 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
     // fewer pairs a tile for few queries, whose lists are all the work there
     // is: 2,813 pairs of one query were six CTAs (16,384 candidates, epsilon 0.25,
     // windows of 11 and 41 rows: 189 and 213 us a call, now 129 and 147; 16
-    // queries 296 and 318, now 231 and 246)
-    const int tile_len = std::max(32, std::min(kLcssTile, kLcssTile / 64 * nq));
+    // queries 296 and 318, now 231 and 246); nor more than spread over the GPU
+    const int64_t even = (int64_t)nq * a.C / (8 * ctx->num_sms);  // eight CTAs an SM
+    const int tile_len = (int)std::max<int64_t>(
+        32, std::min<int64_t>(std::min(kLcssTile, kLcssTile / 64 * nq), even));
     const int tiles = (a.C + tile_len - 1) / tile_len;
     lb2_lcss_kernel<<<dim3(std::max(1, std::min(tiles, 8 * ch)), nq), kLb2Warps * 32, 0, s>>>(
         a, tile_len);
