@@ -27,7 +27,8 @@
 //    j mod RING, laid out [slot][thread] so that every lane reads and writes
 //    its own bank.  A pair fits when the union of a pass's bands is at most
 //    RING columns wide; pairs that do not fit (or that have fewer than two
-//    points on a side) are listed in spill[] for the other kernels.
+//    points on a side, or a band so narrow that rows may have no cell in it)
+//    are listed in spill[] for the other kernels.
 //  - Passes end on the last row: the first pass starts at row (no mod R) - R
 //    when R does not divide the row count, its rows above row 0 being empty;
 //    the empty row just above row 0 carries the origin D(-1,-1) to cell
@@ -121,7 +122,9 @@ __global__ void __launch_bounds__(kLaneThreads, 3)
       rp = make_ramps(no, ni, wd, kLcss);
       dq = (int)(rp.a / rp.d);
       dr = (int)(rp.a % rp.d);
-      if (lane_union_bound(rp, dq, dr) > RING) {
+      // (a band less than a column wide can leave rows without a cell, which the
+      // other kernels know)
+      if (lane_union_bound(rp, dq, dr) > RING || (P::kMin && rp.Wl + rp.Wh < rp.d - 1)) {
         spill[atomicAdd(nspill, 1)] = id;
         continue;
       }

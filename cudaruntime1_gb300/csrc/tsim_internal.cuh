@@ -411,9 +411,9 @@ int launch_frechet_decide(tsim_ctx* ctx, const DpArgs& a, int* rest, int** nrest
 // Lane-per-pair kernel (dp_lane.cu) for the FP32 DTW, Frechet and LCSS
 // kinds (lane_kind): a lane runs a whole pair in passes of 8 rows, the row
 // above a pass in a shared-memory ring of `ring` (64 or 128) values per lane
-// (lane_ring_for picks it from the longest pair); pairs wider than the ring,
-// or with fewer than two points on a side, are left in spill[] (count in
-// *nspill).  When the list holds fewer than `gate` pairs (read
+// (lane_ring_for picks it from the longest pair); pairs wider than the ring, or
+// with fewer than two points on a side, or whose band can leave rows without a
+// cell, are left in spill[] (count in *nspill).  When the list holds fewer than `gate` pairs (read
 // on the device) the kernel computes nothing and copies the whole list, in
 // order, to spill[] for the warp-per-pair kernels.
 bool lane_kind(int kind);

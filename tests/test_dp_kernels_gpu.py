@@ -331,3 +331,47 @@ def test_compensated_full_rows_past_one_cta_an_sm(tsim, cuda_ctx, measure, longe
         out.append(o.cpu().numpy())
     assert len(pairs) > 608 and np.array_equal(out[0][:24], out[1][:24])
     assert np.array_equal(out[0][24:], np.tile(out[1][13:24], 60))
+
+
+@pytest.mark.parametrize("band", [0, 1, 2])
+@pytest.mark.parametrize("cost", [0, 1])
+def test_dp_pairs_with_rows_the_band_leaves_empty(tsim, cuda_ctx, oracle, band, cost):
+    """Narrow bands of sides of very different lengths, where some rows (or
+    columns) admit no cell and the pair has no path: the oracle's infinities on
+    every kernel, few pairs and enough for a lane each, and its answer in kNN."""
+    import torch
+    from cudaruntime1_gb300 import api
+    ql = [2, 9, 20, 31, 40, 60, 200]
+    cl = np.concatenate([np.arange(2, 22), [40, 60, 100, 200, 399]] * 30)
+    qp, qo = G.random_walks(7, ql, 103, start_range=10.0)
+    cp, co = G.random_walks(len(cl), cl, 104, start_range=10.0)
+    pairs = np.stack(np.meshgrid(np.arange(7), np.arange(len(cl)), indexing="ij"), -1).reshape(-1, 2)
+    want = np.array([oracle.pair("dtw", qp[qo[a]:qo[a + 1]], cp[co[b]:co[b + 1]], band_pct=band,
+                                 cost=cost) for a, b in pairs])
+    assert np.isinf(want).any() and np.isfinite(want).any()
+    lens = np.diff(qo)[pairs[:, 0]] + np.diff(co)[pairs[:, 1]]
+    many = np.tile(pairs, (12, 1))
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+           (qp, np.asarray(qo), cp, np.asarray(co), many.astype(np.int32))]
+    for count in (len(pairs), len(many)):
+        for kernel in range(7):
+            o = torch.full((count,), float("nan"), device="cuda")
+            api.dp_pairs(cuda_ctx, "dtw", 0, kernel, dev[0].data_ptr(), dev[1].data_ptr(), 200,
+                         dev[2].data_ptr(), dev[3].data_ptr(), 399, dev[4].data_ptr(), count,
+                         o.data_ptr(), band_pct=band, cost=cost)
+            torch.cuda.synchronize()
+            got = o.cpu().numpy().astype(np.float64).reshape(-1, len(pairs))
+            fin = np.isfinite(want)
+            assert np.array_equal(np.isfinite(got), np.broadcast_to(fin, got.shape)), (count, kernel)
+            # 4 roundings a cost and one per cell of the path
+            lim = (lens[fin] + 8) * 2.0 ** -24 * 1.01 * want[fin]
+            assert np.all(np.abs(got[:, fin] - want[fin]) <= lim), (count, kernel)
+    cp, co = G.random_walks(6000, G.uniform_lengths(6000, 4, 20, 105), 106, start_range=10.0)
+    qp, qo = G.random_walks(20, [13, 20, 40, 70] * 5, 107, start_range=10.0)
+    db = tsim.Database(cuda_ctx, cp, co)
+    want_ids, want = oracle.knn("dtw", qp, qo, cp, co, 10, band_pct=band, cost=cost)
+    for flags in (0, api.FLAG_NO_PRUNE):
+        ids, d, _ = tsim.knn(cuda_ctx, db, qp, qo, "dtw", 10, band_pct=band, cost=cost, flags=flags)
+        assert np.array_equal(ids, want_ids), flags
+        assert np.array_equal(np.isfinite(d), np.isfinite(want)), flags
+    db.close()
