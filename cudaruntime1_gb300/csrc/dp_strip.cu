@@ -52,10 +52,14 @@ constexpr int strip_rmax() {
 // Policies whose cost takes a square root test whether the lane's column is
 // inside the matrix instead: the square root of an infinite cost leaves the
 // fast path, for the whole warp, on every step that has a lane outside.
+// Compensated Frechet too: a pair's cost at infinity is no number, and among
+// three cells that are none (a point at infinity on the matrix's edge) the
+// maximum passes over them.
 template <class P>
 constexpr bool strip_guard() {
   return std::is_same<P, PolDtwRef>::value || std::is_same<P, PolFrechetRef>::value ||
-         std::is_same<P, PolDtwEu>::value || std::is_same<P, PolDtwEuC>::value;
+         std::is_same<P, PolDtwEu>::value || std::is_same<P, PolDtwEuC>::value ||
+         std::is_same<P, PolFrechetSqC>::value;
 }
 
 // a cell from packed points where the policy has that form

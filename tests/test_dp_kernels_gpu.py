@@ -375,3 +375,40 @@ def test_dp_pairs_with_rows_the_band_leaves_empty(tsim, cuda_ctx, oracle, band, 
         assert np.array_equal(ids, want_ids), flags
         assert np.array_equal(np.isfinite(d), np.isfinite(want)), flags
     db.close()
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("measure,kw", [("dtw", dict(cost=0)), ("dtw", dict(cost=1)), ("frechet", {})])
+def test_full_rows_with_points_that_are_not_finite(tsim, cuda_ctx, measure, kw, bad):
+    """The strips' own points at infinity beside a trajectory's: the same pairs
+    have a finite value as on the round-striped kernel, and the same bits;
+    strips of a pair and of two pairs a warp."""
+    import torch
+    from cudaruntime1_gb300 import api
+    for longest, nc in ((40, 30), (120, 700), (300, 30)):
+        ql, cl = G.uniform_lengths(4, 2, longest, 61), G.uniform_lengths(nc, 2, longest, 62)
+        qp, qo = G.random_walks(4, ql, 63, start_range=10.0)
+        cp, co = G.random_walks(nc, cl, 64, start_range=10.0)
+        rng = np.random.default_rng(65)
+        for q in (0, 1):  # one in the middle; the last one
+            qp[qo[q] + (ql[q] // 2 if q else ql[q] - 1), q] = bad
+        for c in range(0, nc, 3):
+            cp[co[c] + rng.integers(0, cl[c]), rng.integers(0, 2)] = bad if c % 2 else np.inf
+        pairs = np.stack(np.meshgrid(np.arange(4), np.arange(nc), indexing="ij"), -1)
+        dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+               (qp, qo, cp, co, pairs.reshape(-1, 2).astype(np.int32))]
+        for precision in (0, 1):
+            out = []
+            for kernel in (1, 0):
+                o = torch.zeros(4 * nc, device="cuda",
+                                dtype=(torch.float32, torch.float64)[precision])
+                api.dp_pairs(cuda_ctx, measure, precision, kernel, dev[0].data_ptr(),
+                             dev[1].data_ptr(), int(ql.max()), dev[2].data_ptr(),
+                             dev[3].data_ptr(), int(cl.max()), dev[4].data_ptr(), 4 * nc,
+                             o.data_ptr(), o.data_ptr(), **kw)
+                torch.cuda.synchronize()
+                out.append(o.cpu().numpy())
+            fin = np.isfinite(out[0])
+            assert fin.any() and not fin.all()
+            assert np.array_equal(fin, np.isfinite(out[1])), (longest, precision)
+            assert np.array_equal(out[0][fin], out[1][fin]), (longest, precision)
