@@ -152,8 +152,9 @@ template <class V>
 struct WaveHalf {
   bool rev = false;  // from the last cell backwards: both point sequences reversed
   int t_stop = 0;    // its last anti-diagonal
-  V* last = nullptr;  // [32 R] that anti-diagonal's positions, and the one's before
+  V* last = nullptr;  // [cap] that anti-diagonal's positions, and the one's before
   V* prev = nullptr;
+  int cap = 0;  // of each: 32 RMAX
   int* geo = nullptr;  // [3] their first rows, and whether the half is alive
 };
 
@@ -356,11 +357,11 @@ __device__ __forceinline__ void wave_pair(const DpArgs& a, const int pid, const 
     if (alive) {
       // (a lone first anti-diagonal has none before it)
 #pragma unroll
-      for (int r = 0; r < R; ++r) half.prev[lane * R + r] = t_end > 0 ? v[r] : P::border();
+      for (int r = 0; r < R; ++r) half.prev[TSIM_SIDX(lane * R + r, half.cap)] = t_end > 0 ? v[r] : P::border();
       if (lane == 0) half.geo[1] = ilo;
       if (t_end > 0) step(t, __shfl_sync(0xffffffffu, win, t + 2 - base)), ++t;
 #pragma unroll
-      for (int r = 0; r < R; ++r) half.last[lane * R + r] = v[r];
+      for (int r = 0; r < R; ++r) half.last[TSIM_SIDX(lane * R + r, half.cap)] = v[r];
       if (lane == 0) half.geo[0] = ilo;
     }
     if (lane == 0) half.geo[2] = alive;
@@ -482,6 +483,7 @@ __global__ void __launch_bounds__(kWaveThreads)
     h.t_stop = side ? n + m - 2 - (s + 1) : s;
     h.last = x + 2 * side * 32 * RMAX;
     h.prev = h.last + 32 * RMAX;
+    h.cap = 32 * RMAX;
     h.geo = geo[pair][side];
     const bool one = RMAX == 1 || lm <= 32;
     if (one)
@@ -502,15 +504,15 @@ __global__ void __launch_bounds__(kWaveThreads)
         // forward's value of row i on one of its anti-diagonals
         auto fwd = [&](const V* d, int first, int i) {
           const int p = i - first;
-          return (unsigned)p < (unsigned)cells ? d[p] : P::border();
+          return (unsigned)p < (unsigned)cells ? d[TSIM_SIDX(p, 32 * RMAX)] : P::border();
         };
         for (int p = lane; p < cells; p += 32) {
           const int i1 = n - 1 - (gb[0] + p);  // row of a cell on s + 1
           const V before = vmin(vmin(fwd(f0, gf[0], i1 - 1), fwd(f0, gf[0], i1)),
                                 fwd(f1, gf[1], i1 - 1));
-          best = vmin(best, before + b0[p]);
+          best = vmin(best, before + b0[TSIM_SIDX(p, 32 * RMAX)]);
           const int i2 = n - 1 - (gb[1] + p);  // and on s + 2
-          best = vmin(best, fwd(f0, gf[0], i2 - 1) + b1[p]);
+          best = vmin(best, fwd(f0, gf[0], i2 - 1) + b1[TSIM_SIDX(p, 32 * RMAX)]);
         }
       }
       for (int o = 16; o; o >>= 1) best = vmin(best, wshfl(best, lane ^ o));

@@ -45,6 +45,7 @@
 
 #include "bounds.cuh"
 #include "bulk_copy.cuh"
+#include "debug_bounds.cuh"
 #include "topk.cuh"
 #include "tsim_internal.cuh"
 
@@ -1512,7 +1513,7 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a, in
       for (int dy = -1; dy <= 1; ++dy)
         for (int dx = -1; dx <= 1; ++dx) {
           const int cell = (cy + dy) * gnx + cx + dx;
-          atomicOr(grid + (cell >> 5), 1u << (cell & 31));
+          atomicOr(grid + TSIM_SIDX(cell >> 5, kGridWords), 1u << (cell & 31));
         }
     }
     __syncthreads();
@@ -1562,7 +1563,7 @@ __global__ void __launch_bounds__(kLb2Warps * 32, 8) lb2_lcss_kernel(KArgs a, in
             const int cx = max(__float_as_int(fx + 8388607.5f) - 0x4b000000, 0);
             const int cy = max(__float_as_int(fy + 8388607.5f) - 0x4b000000, 0);
             const int cell = cy * gnx + cx;
-            if (in[u]) count += (grid[cell >> 5] >> (cell & 31)) & 1u;
+            if (in[u]) count += (grid[TSIM_SIDX(cell >> 5, kGridWords)] >> (cell & 31)) & 1u;
           }
         }
       }
@@ -1708,6 +1709,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
   const float2* A = a.qpts + a.qoff[q];
   const int n = a.qlen[q];
   float4(*tab)[kRowBlocks] = tabs[warp];
+#define TAB(l, b) tab[TSIM_SIDX(l, kRowLevels)][TSIM_SIDX(b, kRowBlocks)]
   WarpList<1> out{a.cnt0 + q, a.list2 + (size_t)q * a.C, nullptr, nullptr, buf[warp]};
   for (int e = blockIdx.x * kRowWarps + warp; e < cnt; e += gridDim.x * kRowWarps) {
     const int c = a.list1[(size_t)q * a.C + e];
@@ -1740,13 +1742,13 @@ __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
             y1 = max3f(y1, p[u].y, p[u + 1].y);
           }
         }
-        tab[0][b] = make_float4(x0, y0, x1, y1);
+        TAB(0, b) = make_float4(x0, y0, x1, y1);
       }
       __syncwarp();
       for (int l = 1; (1 << l) <= span; ++l) {
         for (int b = lane; b + (1 << l) <= nb; b += 32) {
-          const float4 u = tab[l - 1][b], v = tab[l - 1][b + (1 << (l - 1))];
-          tab[l][b] = make_float4(fminf(u.x, v.x), fminf(u.y, v.y), fmaxf(u.z, v.z), fmaxf(u.w, v.w));
+          const float4 u = TAB(l - 1, b), v = TAB(l - 1, b + (1 << (l - 1)));
+          TAB(l, b) = make_float4(fminf(u.x, v.x), fminf(u.y, v.y), fmaxf(u.z, v.z), fmaxf(u.w, v.w));
         }
         __syncwarp();
       }
@@ -1773,7 +1775,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
         }
         const int k0 = lo >> f, k1 = hi >> f;
         const int l = 31 - __clz(k1 - k0 + 1);
-        const float4 u = tab[l][k0], v = tab[l][k1 - (1 << l) + 1];
+        const float4 u = TAB(l, k0), v = TAB(l, k1 - (1 << l) + 1);
         const float2 p = __ldg(A + i);
         const float d = box_pt_d2_rd(fminf(u.x, v.x), fminf(u.y, v.y), fmaxf(u.z, v.z),
                                      fmaxf(u.w, v.w), p.x, p.y);
@@ -1785,6 +1787,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 12) lb_rows_kernel(KArgs a) {
     if (pass) out.add(lane == 0, c, 0);
   }
   out.flush();
+#undef TAB
 }
 
 // exclusive scan of fcnt -> off2, total -> npairs[0] (one CTA).  LCSS: the

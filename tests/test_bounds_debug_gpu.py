@@ -71,3 +71,40 @@ def test_no_shared_memory_index_out_of_bounds(tsim):
     assert r.returncode == 0, r.stderr[-3000:]
     out = json.loads(r.stdout.strip().splitlines()[-1])
     assert out["violations"] == 0, out
+
+
+CHILD_FEW_QUERIES = r"""
+import ctypes as C, json, sys
+import numpy as np, torch
+sys.path.insert(0, ROOT)
+import cudaruntime1_gb300 as T
+from cudaruntime1_gb300 import _lib, api, datagen as G
+L = _lib.load()
+ctx = T.Context(0)
+cp, co = G.random_walks(1500, G.uniform_lengths(1500, 2, 300, 21), 22)
+db = T.Database(ctx, cp, co)
+for nq, lo, hi in ((1, 40, 40), (3, 2, 300), (2, 1800, 2048)):
+    qp, qo = G.random_walks(nq, G.uniform_lengths(nq, lo, hi, 23 + nq), 24 + nq)
+    for measure, kw in (("dtw", dict(band_pct=2)), ("dtw", dict(band_pct=10, cost=1)),
+                        ("dtw", dict(band_pct=60)), ("lcss", dict(epsilon=1e-4, delta=9)),
+                        ("lcss", dict(epsilon=20.0, delta=-1))):
+        for flags in (api.FLAG_ALWAYS_PRUNE, 0):
+            T.knn(ctx, db, qp, qo, measure, 10, stats=False, flags=flags, **kw)
+db.close()
+torch.cuda.synchronize()
+n, f = C.c_int64(), C.c_int64()
+assert L.tsim_debug_bounds_violations(C.byref(n), C.byref(f)) == 0
+print(json.dumps({"violations": n.value, "first": f.value}))
+"""
+
+
+def test_few_queries_index_no_shared_memory_out_of_bounds(tsim):
+    """The two-ended kernel's exchange arrays, the row side's table and LCSS's
+    occupancy grid: few queries, and queries far longer than candidates."""
+    from cudaruntime1_gb300 import buildlib as B
+    env = dict(os.environ, TSIM_LIB=B.build(debug_bounds=True))
+    r = subprocess.run([sys.executable, "-c", "ROOT = %r\n" % ROOT + CHILD_FEW_QUERIES], env=env,
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stderr[-3000:]
+    out = json.loads(r.stdout.strip().splitlines()[-1])
+    assert out["violations"] == 0, out
