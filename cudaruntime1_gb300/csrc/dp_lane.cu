@@ -373,12 +373,14 @@ bool lane_kind(int kind) {
 // it a 16-query DTW request of up to 2,048 points against the 1M serving
 // database ran its 150 K survivors on lanes in 14.2 ms, on warps in 9.8 ms.
 // DTW and Frechet only: their warp rounds run on the band-relative kernel;
-// LCSS's run on the row-group kernel, whose rate the lanes keep beating.
+// LCSS's (no window, or one of more than 63 rows; others mostly go to the bit
+// vectors) run on the row-group kernel, whose rate the lanes keep beating.
 // abandon = false: rounds that compute every cell (tsim_dp_pairs): a lane per
-// pair from where the band-relative kernel (500 cells per ns then) needs as
+// pair from where the band-relative kernel (550 cells per ns then) needs as
 // long as the lanes' longest pair: 64 queries of 64 to 512 points, band 10 %,
 // against 128 / 256 / 512 / 2,048 candidates: 317 / 547 / 997 / 3,605 us on warps,
-// 527 / 544 / 626 / 1,425 on lanes, and the rule's line at 20,500 pairs (320).
+// 527 / 544 / 626 / 1,425 on lanes: they meet near 16,400 pairs (256), the rule's
+// line is at 20,500 (320).
 int lane_gate_for(int kind, int max_n, int max_m, int band_pct, int delta, int num_sms,
                   bool abandon) {
   constexpr double kLaneStepNs = 70.0, kWarpCellsPerNs = 435.0;  // 435 GCUPS

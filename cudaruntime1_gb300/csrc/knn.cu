@@ -164,9 +164,10 @@ struct KArgs {
   const float* thr_in;      // optional [nq]: a pruning threshold known beforehand (an earlier
                             //   identical query's), combined with the seeds' (else null)
   float* thr_out;           // optional [nq]: the final pruning threshold, for later requests
-  int* waves;               // what the band-relative kernel leaves to the row-group ones
+  int* waves;               // what the strips or the band-relative kernel leave to the others
   int* nwaves;
-  int wave;                 // DTW / Frechet rounds start on the band-relative kernel
+  int wave;                 // full rows go to the strips, banded FP32 DTW to the band-relative
+                            // kernel, LCSS windows of at most 63 rows to the bit vectors
   int rdiag;                // rows per lane-group of the anti-diagonal kernel (0: off)
   int rdiag_shape;          // the smallest R a warp per pair admits for the longest pair
   int rdiag_cta;            // the same for a CTA per pair (0: no R fits the longest pair)
@@ -2326,8 +2327,8 @@ int run_dp(tsim_ctx* ctx, const KArgs& a, int kind, int G, int R, const DpArgs& 
   int *ns = a.nspill, *ns1 = a.nlanes;
   bool all = false;  // the row groups take every pair of at least two points a side
   if (!w2 && latency && a.rdiag_cta > 0 && a.rdiag_shape >= (twofloat ? 4 : 8)) {
-    // the longest pair needs a CTA, but a round's lengths vary (lognormal
-    // Frechet queries): the pairs that fit a warp with up to 8 rows per lane
+    // the longest pair needs a CTA, but a round's lengths vary (wide bands,
+    // LCSS without a window): the pairs that fit a warp with up to 8 rows per lane
     // run there, each at its fewest rows, the rest on a CTA per pair from
     // one row per lane up -- instead of every pair at the longest pair's R
     TSIM_TRY(launch_dp_diag(ctx, kind, 1, d, a.max_clen, a.lanes, &ns1, a.spill2, a.nspill2, 1,

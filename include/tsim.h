@@ -79,9 +79,10 @@ typedef enum tsim_cost {
 #define TSIM_FLAG_NO_LANE_DP 0x20u  /* survivor rounds stay on the warp-per-pair DP
                                        kernels even when they hold many pairs (the
                                        lane-per-pair kernel is off); same values */
-#define TSIM_FLAG_NO_WAVE_DP 0x40u  /* DTW / Frechet rounds skip the band-relative DP
-                                       kernel (lanes along the anti-diagonal) and start
-                                       on the row-group ones; same values */
+#define TSIM_FLAG_NO_WAVE_DP 0x40u  /* rounds skip the strips (DTW without a band,
+                                       Frechet), the band-relative DP kernel (banded
+                                       DTW) and the LCSS bit vectors and start on the
+                                       lane-per-pair or row-group ones; same values */
 #define TSIM_FLAG_SHARE_THRESHOLDS 0x80u /* server requests: a query's pruning threshold
                                              starts from the final one of an earlier
                                              identical query (same parameters, points and
