@@ -697,3 +697,27 @@ def test_first_bound_queries_a_block(tsim, measure, kw, nq):
     assert np.array_equal(ids, ids2) and np.array_equal(d, d2)
     db.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("measure,kw", [("lcss", dict(epsilon=0.5, delta=40)),
+                                        ("lcss", dict(epsilon=0.5, delta=-1)),
+                                        ("lcss", dict(epsilon=2.0, delta=12)),
+                                        ("dtw", dict(band_pct=-1, cost=0))])
+def test_dp_kernel_choices_agree_past_strips_and_bit_vectors(tsim, cuda_ctx, oracle, measure, kw):
+    """LCSS without bit vectors (a lane or a warp a pair), with them, and DTW's
+    full rows: what the kernel choices still differ in where strips and bit
+    vectors come first."""
+    cp, co = _db(3000, 8, 150, 94)
+    qp, qo = G.random_walks(14, G.uniform_lengths(14, 8, 150, 95), 96)
+    db = tsim.Database(cuda_ctx, cp, co)
+    okw = {("eps" if k == "epsilon" else k): v for k, v in kw.items()}
+    want_ids, _ = oracle.knn(measure, qp, qo, cp, co, 10, **okw)
+    for extra in (0, tsim.api.FLAG_ALWAYS_PRUNE, tsim.api.FLAG_NO_PRUNE):
+        base = None
+        for choice in (0, tsim.api.FLAG_NO_LANE_DP, tsim.api.FLAG_NO_WAVE_DP,
+                       tsim.api.FLAG_NO_LANE_DP | tsim.api.FLAG_NO_WAVE_DP):
+            got = _device_knn(tsim, cuda_ctx, db, qp, qo, measure, 10, flags=extra | choice, **kw)
+            assert np.array_equal(got[0], want_ids), (extra, choice)
+            base = base or got
+            assert np.array_equal(got[1].view(np.uint32), base[1].view(np.uint32)), (extra, choice)
+    db.close()
