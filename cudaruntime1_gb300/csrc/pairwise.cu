@@ -10,33 +10,57 @@ namespace tsim {
 
 namespace {
 
-constexpr int kHdThreads = 128;
-
 // One CTA per query, its top_k candidates in two passes (the reference's
 // hausdorff_tiled_rtree_kernel takes them in turn, CudaRuntime1/hausdorff.cu:
 // 84-122).  First a warp per candidate bounds the symmetric Hausdorff^2 from
 // below by 32 points of either side; then the candidate with the smallest
-// bound is computed, a warp per direction, and the others only where their
-// bound is still below the best.  Minima and maxima are exact in any order,
-// so the value is the sequential loop's.  Bound by the FP32 pipe (hausdorff.cuh);
-// 1,024 queries of 128 points, ten candidates: 69 us computing every candidate
-// on 256 threads a query, 38 now.
+// bound is computed, each direction's points dealt over half of the warps, and
+// the others only where their bound is still below the best: a warp per
+// candidate, or, where they are fewer than the warps, the whole CTA for each (a
+// candidate's long sides on a warp or two left the others idle: 4 queries of
+// 8,192 points, two candidates, 24.8 ms, 13.7 on 256 threads a candidate, 6.7
+// now).  A lone candidate needs no bound.
+// Minima and maxima are exact in any order, so the value is the sequential
+// loop's.  Bound by the FP32 pipe (hausdorff.cuh); 1,024 queries of 128
+// points, ten candidates: 69 us computing every candidate on 256 threads a
+// query, 36 now.
 constexpr int kMaxCandSlots = 1024;  // bounds kept in shared memory at a time
-__global__ void __launch_bounds__(kHdThreads)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
     hausdorff_cands_kernel(const float2* __restrict__ t1, int n, const float2* __restrict__ t2,
                            int num_t2, int m, const int* __restrict__ cand, int top_k,
                            float* __restrict__ out) {
-  constexpr int kWarps = kHdThreads / 32;
+  constexpr int kWarps = THREADS / 32, kHalf = kWarps / 2;
   __shared__ __align__(16) float targets[kWarps][haus::kStageFloats];
   __shared__ float bound[kMaxCandSlots];
   __shared__ unsigned best_bits;  // of a non-negative float: ordered as unsigned
-  __shared__ float dir[2];
+  __shared__ float part[kWarps];
   __shared__ int first;
   const int q = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float* sm = targets[warp];
   const float2* A = t1 + (size_t)q * n;
   long long pairs = 0;
+  // the candidate in slot k by the whole CTA: this warp's points of its direction
+  auto together = [&](int k, float stop) {
+    const float2* B = t2 + (size_t)cand[(size_t)q * top_k + k] * m;
+    const bool back = warp >= kHalf;
+    const float2 *S = back ? B : A, *D = back ? A : B;
+    const int ns = back ? m : n, w = back ? warp - kHalf : warp;
+    const int r0 = (int)((long long)w * ns / kHalf), r1 = (int)((long long)(w + 1) * ns / kHalf);
+    const float v = r1 > r0 ? haus::warp_directed<false>(S + r0, r1 - r0, D, back ? n : m, 0.0f,
+                                                         stop, sm, false, &pairs)
+                            : 0.0f;
+    if (lane == 0) part[warp] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float h = part[0];
+#pragma unroll
+      for (int i = 1; i < kWarps; ++i) h = fmaxf(h, part[i]);
+      best_bits = min(best_bits, __float_as_uint(h));
+    }
+    __syncthreads();
+  };
   if (threadIdx.x == 0) best_bits = __float_as_uint(TSIM_INF);
   for (int k0 = 0; k0 < top_k; k0 += kMaxCandSlots) {
     const int kn = min(kMaxCandSlots, top_k - k0);
@@ -46,8 +70,11 @@ __global__ void __launch_bounds__(kHdThreads)
       float v = TSIM_INF;  // out-of-range candidate slots are ignored
       if (c >= 0 && c < num_t2) {
         const float2* B = t2 + (size_t)c * m;
-        v = haus::warp_directed<false>(A, n, B, m, 0.0f, TSIM_INF, sm, true, &pairs);
-        v = haus::warp_directed<false>(B, m, A, n, v, TSIM_INF, sm, true, &pairs);
+        v = 0.0f;
+        if (kn > 1) {
+          v = haus::warp_directed<false>(A, n, B, m, 0.0f, TSIM_INF, sm, true, &pairs);
+          v = haus::warp_directed<false>(B, m, A, n, v, TSIM_INF, sm, true, &pairs);
+        }
       }
       if (lane == 0) bound[k] = v;
     }
@@ -66,17 +93,15 @@ __global__ void __launch_bounds__(kHdThreads)
     }
     __syncthreads();
     const int f = first;
-    if (f >= 0 && bound[f] < __uint_as_float(best_bits)) {  // uniform over the CTA
-      const float2* B = t2 + (size_t)cand[(size_t)q * top_k + k0 + f] * m;
-      if (warp < 2) {
-        const float v = haus::warp_directed<false>(warp ? B : A, warp ? m : n, warp ? A : B,
-                                                   warp ? n : m, 0.0f, TSIM_INF, sm, false, &pairs);
-        if (lane == 0) dir[warp] = v;
+    if (f >= 0 && bound[f] < __uint_as_float(best_bits))  // uniform over the CTA, as below
+      together(k0 + f, TSIM_INF);
+    if (kn <= kWarps) {
+      for (int k = 0; k < kn; ++k) {
+        const float best = __uint_as_float(best_bits);
+        if (k != f && bound[k] < best) together(k0 + k, best);
       }
-      __syncthreads();
-      if (threadIdx.x == 0) atomicMin(&best_bits, __float_as_uint(fmaxf(dir[0], dir[1])));
+      continue;
     }
-    __syncthreads();
     for (int k = warp; k < kn; k += kWarps) {
       const float best = __uint_as_float(*(volatile unsigned*)&best_bits);
       if (k == f || !(bound[k] < best)) continue;
@@ -240,7 +265,13 @@ int hausdorff_cands(tsim_ctx* ctx, const float2* t1, int num_t1, int n, const fl
                     int m, const int* cand, int top_k, float* out) {
   TSIM_CHECK_ARG(sizeof(float2) * ((size_t)n + m) <= 200 * 1024,
                  "trajectories too long for the Hausdorff kernel");
-  hausdorff_cands_kernel<<<num_t1, kHdThreads, 0, ctx->stream>>>(t1, n, t2, num_t2, m, cand, top_k,
+  // eight warps a query where four leave the GPU half empty (200 queries of 2,048
+  // points, four candidates: 2.3 ms on four, 1.0)
+  if (num_t1 <= 2 * ctx->num_sms)
+    hausdorff_cands_kernel<256><<<num_t1, 256, 0, ctx->stream>>>(t1, n, t2, num_t2, m, cand, top_k,
+                                                                 out);
+  else
+    hausdorff_cands_kernel<128><<<num_t1, 128, 0, ctx->stream>>>(t1, n, t2, num_t2, m, cand, top_k,
                                                                  out);
   TSIM_CUDA(cudaGetLastError());
   return TSIM_OK;

@@ -123,3 +123,39 @@ def test_candidate_lengths_around_48_kib(tsim, cuda_ctx, oracle, num_t, m):
         cuda_ctx.synchronize()
         assert np.array_equal(_bits(out.cpu().numpy()),
                               _bits(oracle.ref_batch(measure, t1, t2, 24, m, eps=0.5))), measure
+
+
+@pytest.mark.parametrize("top_k", [1023, 1025, 2500])
+def test_hausdorff_many_given_candidates(tsim, cuda_ctx, oracle, top_k):
+    """More candidates a query than are bounded at a time, some slots empty,
+    the nearest one first, in the middle and last."""
+    num_t1, num_t2, n, m = 3, 3000, 20, 35
+    t1 = G.ref_base_trajectories(num_t1, n, 41, r=200.0)
+    t2 = G.ref_base_trajectories(num_t2, m, 42, r=200.0)
+    cand = np.random.default_rng(43).integers(0, num_t2, (num_t1, top_k)).astype(np.int32)
+    for q, at in enumerate((0, top_k // 2, top_k - 1)):
+        c = 100 * q
+        src = np.linspace(0, n - 1, m).round().astype(int)
+        t2[c * m:(c + 1) * m] = t1[q * n + src] + np.float32(0.25)
+        cand[q, at] = c
+    cand[:, 5] = -1
+    got, _ = tsim.launch_hausdorff_rtree_gpu(t1, num_t1, n, t2, num_t2, m, cand, top_k)
+    valid = np.where(cand < 0, cand[:, :1], cand)  # an empty slot: one there is already
+    want = oracle.ref_hausdorff_cands(t1, n, t2, m, valid.ravel())
+    assert np.array_equal(_bits(got), _bits(want))
+
+
+@pytest.mark.parametrize("num_t1,n,m,top_k", [(2, 3, 5, 1), (2, 1, 300, 3), (5, 300, 2, 4),
+                                              (3, 1300, 900, 4), (3, 600, 1100, 8),
+                                              (3, 600, 1100, 9), (320, 70, 90, 4),
+                                              (320, 70, 90, 5), (320, 520, 40, 1)])
+def test_hausdorff_candidates_by_the_whole_block(tsim, cuda_ctx, oracle, num_t1, n, m, top_k):
+    """Fewer candidates than warps, sides shorter than the warps and longer
+    than a warp's registers and staged targets."""
+    num_t2 = max(num_t1, 20)
+    t1 = G.ref_base_trajectories(num_t1, n, 51, r=200.0)
+    t2 = G.ref_base_trajectories(num_t2, m, 52, r=200.0)
+    cand = np.random.default_rng(53).integers(0, num_t2, (num_t1, top_k)).astype(np.int32)
+    got, _ = tsim.launch_hausdorff_rtree_gpu(t1, num_t1, n, t2, num_t2, m, cand, top_k)
+    want = oracle.ref_hausdorff_cands(t1, n, t2, m, cand.ravel())
+    assert np.array_equal(_bits(got), _bits(want))
