@@ -706,6 +706,13 @@ bool strip_kind(int kind) {
 
 int strip_max_cols() { return kStripMaxCols; }
 
+int strip_pairs_per_sm(int max_n, int max_m) {
+  const int cap = std::min((std::min(max_n, max_m) + 1) & ~1, kStripMaxCols);
+  constexpr int kWarps = kStripThreads / 32;
+  const int cta = kWarps * (cap + 2 * kStripPad) * (int)(sizeof(float2) + sizeof(float)) + 1024;
+  return kWarps * (228 * 1024 / cta);
+}
+
 int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
                     int** nspill) {
   switch (kind) {

@@ -267,7 +267,19 @@ int ref_batch_core(tsim_ctx* ctx, int measure, const float2* d_t1, const float2*
   a.delta = -1;
   a.eps = eps;
   a.max_n = n;
-  if (strip_kind(kind) && std::min(n, m) <= strip_max_cols()) {
+  // The reference's square roots make a lone warp's step long, and a strip's
+  // time hardly depends on the warps beside it: one pair more than the SMs hold
+  // doubles the launch.  Round-striped, whose pairs stage no points, from there
+  // on: where an SM holds eight pairs for any number (2,440 pairs of 2,040 points
+  // 10.9 ms, 17.8 on strips, 3,700 of them 18.6 and 24.2; 1,000 7.8 and 6.3), else
+  // as long as it does not take turns itself (of 1,000 points 2,440 2.8 ms and 3.3,
+  // 3,300 4.4 and 3.6).
+  const int held = strip_pairs_per_sm(n, m);
+  const bool turns = a.npairs > held * ctx->num_sms && std::max(n, m) <= strip_max_cols() &&
+                     (held <= 8 || a.npairs <= 20 * ctx->num_sms);
+  if (strip_kind(kind) && turns) {
+    TSIM_TRY(launch_dp(ctx, kind, 32, 8, a, m));
+  } else if (strip_kind(kind) && std::min(n, m) <= strip_max_cols()) {
     TSIM_TRY(launch_dp_strip(ctx, kind, a, n, m, nullptr, nullptr));
   } else {
     int G, R;

@@ -390,6 +390,8 @@ bool wave_takes_all(int max_n, int max_m, int band_pct);
 // *nspill; both may be null when no pair can be longer).
 bool strip_kind(int kind);
 int strip_max_cols();
+// pairs of long 4-byte strips that an SM's shared memory holds
+int strip_pairs_per_sm(int max_n, int max_m);
 int launch_dp_strip(tsim_ctx* ctx, int kind, const DpArgs& a, int max_n, int max_m, int* spill,
                     int** nspill);
 // Windowed LCSS by bit vectors (dp_lcss.cu, windows of at most 63 rows): a

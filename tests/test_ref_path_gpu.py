@@ -159,3 +159,16 @@ def test_hausdorff_candidates_by_the_whole_block(tsim, cuda_ctx, oracle, num_t1,
     got, _ = tsim.launch_hausdorff_rtree_gpu(t1, num_t1, n, t2, num_t2, m, cand, top_k)
     want = oracle.ref_hausdorff_cands(t1, n, t2, m, cand.ravel())
     assert np.array_equal(_bits(got), _bits(want))
+
+
+@pytest.mark.parametrize("measure", ["dtw", "frechet"])
+@pytest.mark.parametrize("num_t", [121, 122])
+def test_long_sides_past_what_the_strips_hold(tsim, cuda_ctx, oracle, measure, num_t):
+    """One pair of long sides fewer than the strips' shared memory holds on
+    152 SMs, and more."""
+    n, m = 1990, 2040
+    t1 = G.ref_base_trajectories(num_t, n, 61, r=200.0)
+    t2 = G.ref_base_trajectories(num_t, m, 62, r=200.0)
+    got, _ = FN[measure](tsim, t1, t2, n, m, num_t, 0.5)
+    want = oracle.ref_batch(measure, t1, t2, n, m, eps=0.5)
+    assert np.array_equal(_bits(got), _bits(want))
