@@ -405,7 +405,8 @@ int lane_gate_for(int kind, int max_n, int max_m, int band_pct, int delta, int n
   return (int)std::min(std::max(gate, gate_tail), 1e9);
 }
 
-int lane_ring_for(int kind, int max_n, int max_m, int band_pct, int delta) {
+// a bound on the columns of a pass's bands, for pairs up to max_n x max_m
+static long long lane_union_for(int kind, int max_n, int max_m, int band_pct, int delta) {
   const int mn = std::min(max_n, max_m), mx = std::max(max_n, max_m);
   long long u;
   if (kind == DP_LCSS)
@@ -414,7 +415,15 @@ int lane_ring_for(int kind, int max_n, int max_m, int band_pct, int delta) {
     u = mn;
   else  // the widest band of pairs up to these lengths: 2w + 1 columns, plus a pass's slope
     u = std::min<long long>(mn, 2ll * band_w(mx, mx, band_pct) + 2 + (kLaneR - 1));
-  return u <= 64 ? 64 : 128;
+  return u;
+}
+
+int lane_ring_for(int kind, int max_n, int max_m, int band_pct, int delta) {
+  return lane_union_for(kind, max_n, max_m, band_pct, delta) <= 64 ? 64 : 128;
+}
+
+bool lane_takes_all(int kind, int max_n, int max_m, int band_pct, int delta) {
+  return lane_union_for(kind, max_n, max_m, band_pct, delta) <= 128;
 }
 
 int launch_dp_lane(tsim_ctx* ctx, int kind, const DpArgs& a, int ring, int* spill, int** nspill_io,

@@ -3415,7 +3415,25 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
   const bool diag_kind = precision < 2;
   if (kernel == 1 || !diag_kind)
     return launch_dp(ctx, kind, G, R, d, max_clen);
-  if (Rd == 0) Rd = 16;  // none fits the longest pair: the widest takes the rest
+  // Automatic, and the longest pair's band too wide for the row groups:
+  // round-striped.  Row groups first, which take the shorter pairs, pay only in
+  // FP32 and for few pairs hardly any of which they leave, or many whose band is
+  // not so wide that the striped rows waste little (in us, striped / both: 300
+  // pairs of 64 to 512 points, band 100 %, 766 / 267, of 300 to 600 2,690 /
+  // 3,173; 3,000 of 500 to 1,000, 60 %, 6,285 / 8,416, 12,000 of them 17,672 /
+  // 11,767, but 12,000 of 64 to 512, 100 %, 1,379 / 2,969).
+  const bool wide = Rd == 0;
+  const bool lanes_fit =
+      !wide || (lane_kind(kind) && lane_takes_all(kind, max_qlen, max_clen, d.band_pct, d.delta));
+  if (kernel == 0 && !lanes_fit && !(d.band_pct < 0 && strip_kind(kind))) {
+    const int n9 = max_qlen * 0.9, m9 = max_clen * 0.9;
+    const bool few = kind != DP_LCSS && npairs <= 4 * ctx->num_sms &&
+                     diag_ok(false, n9, m9, band_w(n9, m9, d.band_pct), 16);
+    const bool many = kind != DP_LCSS && d.band_pct <= 60 &&
+                      npairs > 0.6 * d.band_pct * ctx->num_sms;
+    if (precision == 1 || !(few || many)) return launch_dp(ctx, kind, G, R, d, max_clen);
+  }
+  if (wide) Rd = 16;  // none fits the longest pair: the widest takes the rest
   const int lanes = kernel == 3 ? 256 : 64;  // a CTA of 8 warps, or 2 warps, per pair
   int Rc = 4;  // the smallest R that fits the longest pair
   for (int R2 : {8, 4, 2, 1})  // R = 8 for a CTA only
@@ -3447,14 +3465,25 @@ extern "C" int tsim_dp_pairs(tsim_ctx* ctx, const tsim_params* p, int precision,
     // banded FP32 pairs: a lane per pair once they are many, else the
     // band-relative kernel (64 x 2,048 DTW pairs of 64 to 512 points, band
     // 10 %: 4.87 ms on row groups, 1.42 on lanes; 64 x 64 of them: 246 us on
-    // row groups, 217 band-relative)
+    // row groups, 217 band-relative) where it takes every pair: in two launches
+    // one after the other, each as long as its longest pair, it lost more than
+    // it saved (10 pairs of 500 to 1,000 points, band 10 %, 232 us on row groups,
+    // 301 with both).  Nor where pairs are so long that their staging leaves
+    // two CTAs an SM and many take turns (3,000 of 1,000 to 2,000 points, band 3 %,
+    // 753 us on row groups, 940).
     const int gate = lane_kind(kind) ? lane_gate_for(kind, max_qlen, max_clen, d.band_pct, d.delta,
                                                      ctx->num_sms, false)
                                      : 0;
-    if (gate > 0 && npairs >= gate)
+    if (gate > 0 && npairs >= gate && lanes_fit) {
       kernel = 5;
-    else if (wave_kind(kind))
-      kernel = 6;
+    } else if (wave_kind(kind) && wave_takes_all(max_qlen, max_clen, d.band_pct) &&
+               (max_clen <= 1500 || npairs <= 8 * ctx->num_sms)) {
+      TSIM_TRY(launch_dp_wave(ctx, kind, d, max_qlen, max_clen, npairs <= 4 * ctx->num_sms, rest,
+                              &nrest));
+      d.order = rest;  // pairs with a side of one point, which no row group takes either
+      d.npairs_dev = nrest;
+      return launch_dp(ctx, kind, G, R, d, max_clen);
+    }
   }
   if (kernel == 6 && wave_kind(kind)) {  // band-relative first; wider pairs on the others
     TSIM_TRY(launch_dp_wave(ctx, kind, d, max_qlen, max_clen, npairs <= 4 * ctx->num_sms, rest,

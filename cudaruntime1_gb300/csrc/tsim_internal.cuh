@@ -428,6 +428,8 @@ int lane_sort_buckets();
 int lane_gate_for(int kind, int max_n, int max_m, int band_pct, int delta, int num_sms,
                   bool abandon = true);
 int lane_ring_for(int kind, int max_n, int max_m, int band_pct, int delta);
+// whether that holds every pair of these lengths
+bool lane_takes_all(int kind, int max_n, int max_m, int band_pct, int delta);
 int launch_dp_lane(tsim_ctx* ctx, int kind, const DpArgs& a, int ring, int* spill, int** nspill,
                    int gate = 0);
 // the anti-diagonal kernel's validity condition for a pair shape, R rows

@@ -412,3 +412,33 @@ def test_full_rows_with_points_that_are_not_finite(tsim, cuda_ctx, measure, kw, 
             assert fin.any() and not fin.all()
             assert np.array_equal(fin, np.isfinite(out[1])), (longest, precision)
             assert np.array_equal(out[0][fin], out[1][fin]), (longest, precision)
+
+
+@pytest.mark.parametrize("lo,hi,band,npairs", [
+    (480, 520, 100, 20), (480, 520, 100, 900), (300, 620, 100, 20), (500, 900, 60, 50),
+    (900, 1100, 30, 3000), (2, 90, 60, 40), (2, 140, 60, 2000), (600, 1510, 3, 1500),
+    (1500, 1502, 3, 1000), (1, 60, 5, 300)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_dp_pairs_picks_a_kernel_for_any_band(tsim, cuda_ctx, lo, hi, band, npairs, precision):
+    """The kernel chosen by the library for banded pairs against the
+    round-striped one: the same bits, wide bands and narrow ones, few pairs
+    and many."""
+    import torch
+    from cudaruntime1_gb300 import api
+    ql, cl = G.uniform_lengths(9, lo, hi, 71), G.uniform_lengths(40, lo, hi, 72)
+    ql[0], cl[0] = hi, hi
+    qp, qo = G.random_walks(9, ql, 73)
+    cp, co = G.random_walks(40, cl, 74)
+    rng = np.random.default_rng(75)
+    pairs = np.stack([rng.integers(0, 9, npairs), rng.integers(0, 40, npairs)], 1).astype(np.int32)
+    pairs[0] = 0
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (qp, qo, cp, co, pairs)]
+    out = []
+    for kernel in (1, 0):
+        o = torch.zeros(npairs, device="cuda", dtype=(torch.float32, torch.float64)[precision])
+        api.dp_pairs(cuda_ctx, "dtw", precision, kernel, dev[0].data_ptr(), dev[1].data_ptr(), hi,
+                     dev[2].data_ptr(), dev[3].data_ptr(), hi, dev[4].data_ptr(), npairs,
+                     o.data_ptr(), o.data_ptr(), band_pct=band)
+        torch.cuda.synchronize()
+        out.append(o.cpu().numpy())
+    assert np.array_equal(out[0], out[1])
