@@ -1656,7 +1656,9 @@ __global__ void refilter_kernel(KArgs a) {
   // stages
   __shared__ float t_sh;
   if (threadIdx.x < 32) {
-    const float tq = round1_threshold<MEAS>(a, q, threadIdx.x);
+    // (with none of round 1 refined yet: the seeds', a selection of 64 from which
+    // takes 30 us)
+    const float tq = a.r1n ? round1_threshold<MEAS>(a, q, threadIdx.x) : a.thr[q];
     if (threadIdx.x == 0) {
       t_sh = tq;
       if (blockIdx.x == 0) a.thr2[q] = tq;
