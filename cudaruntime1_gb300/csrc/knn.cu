@@ -2810,10 +2810,11 @@ size_t knn_plan(const tsim_params* p, int nq, int max_qlen, const tsim_db* db, K
     // in one before that bound), 6 against 200,000 without a window 444 (724,
     // 1,564).  With them that bound costs more than a round, which goes by the
     // segment bound ahead of it where pairs are few (one query against 16,384
-    // 129 us in two passes, 115 in one; two against 30,000 162 and 135) and is
+    // 129 us in two passes, 115 in one) and is
     // divided where they are many: the batched workload's 17 M, and 64 densely
     // matching queries against 16,384 1,023 us (1,583 in one pass).  One pass is
-    // some 30 us shorter for any few queries, but where fewer candidates match
+    // some 30 us shorter for any few queries (four against 30,000, epsilon 2, windows
+    // of 11 rows, 152 and 185), but where fewer candidates match
     // than neighbours are asked for and the segment bound does not find them,
     // every pair is refined, 1 us a thousand: two queries against 900,000, epsilon
     // 0.1, 32 neighbours, 2,671 us, 1,028 in two; so the line is where that is 100 us.
