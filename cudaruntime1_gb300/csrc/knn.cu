@@ -2479,13 +2479,14 @@ int run_brute(tsim_ctx* ctx, KArgs& a, int dp32, int dpc, int dp64) {
 
 // Queries a CTA of the O(1) bounds takes, one after the other (each with a block
 // selection where chunks are few): fewer than eight while that leaves less
-// than four CTAs an SM.  200 queries against 2,000 trajectories in eight chunks,
+// than four CTAs an SM, or, without those selections, two (64 queries against
+// 16,384 trajectories next to other requests 407 us, 411 with four).  200 queries against 2,000 trajectories in eight chunks,
 // ten neighbours, in us: Hausdorff 14, 20 with two CTAs an SM (19 with a CTA per
 // query and chunk); 20 queries with 64 neighbours 64 with eight queries a CTA, now
 // 14.
-int bound_queries(int nq, int nch, int num_sms) {
+int bound_queries(int nq, int nch, int T, int num_sms) {
   static_assert(kLb1Queries == kPaaQueries, "one rule");
-  const int64_t per = (int64_t)nq * nch / (4 * (int64_t)num_sms);
+  const int64_t per = (int64_t)nq * nch / ((T > 1 ? 4 : 2) * (int64_t)num_sms);
   return (int)std::max<int64_t>(1, std::min<int64_t>(kLb1Queries, per));
 }
 
@@ -2496,7 +2497,7 @@ int run_knn(tsim_ctx* ctx, KArgs& a, int max_qlen, int dp32, int dpc, int dp64, 
   cudaStream_t s = ctx->stream;
   const int nq = a.nq;
   stage_begin(ctx, TSIM_STAGE_LB1);
-  const int per = bound_queries(nq, a.nch, ctx->num_sms);
+  const int per = bound_queries(nq, a.nch, a.T, ctx->num_sms);
   if constexpr (MEAS == M_EUCLID) {
     qprefix_kernel<<<nq, 256, 0, s>>>(a);
     paa_kernel<<<dim3(a.nch, (nq + per - 1) / per), kChunk, 0, s>>>(a, per);
